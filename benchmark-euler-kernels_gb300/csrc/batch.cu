@@ -66,8 +66,11 @@ struct GridState {
     void* cons[2][5] = {};
     void* lo[2][5] = {};
     void* cs[2] = {};
+    void* h[2] = {}; // FP64: e + p
     bool loaded = false;
     int items = 0;          // work items of this grid in the current item list
+    TileSplit sx{}, sy{};   // its tiles (FP64) and chunk length: the batch's, evened out over the grid
+    int kchunk = 0;
     bool ghost_fix = false; // FP64: copy 0 still holds the loaded ghost prim; fixed after the next step
 };
 
@@ -167,8 +170,10 @@ int upload_params(eulr_batch* b)
             if (is_f64(b)) {
                 p.prim = cbundle_of<T>(G.prim[in]);
                 p.cs = static_cast<const T*>(G.cs[in]);
+                p.h = static_cast<const T*>(G.h[in]);
                 p.prim_out = bundle_of<T>(G.prim[out]);
                 p.cs_out = static_cast<T*>(G.cs[out]);
+                p.h_out = static_cast<T*>(G.h[out]);
             }
             p.cons_in = cbundle_of<T>(G.cons[in]);
             p.cons_out = bundle_of<T>(G.cons[out]);
@@ -191,7 +196,9 @@ int upload_params(eulr_batch* b)
             p.invdx2 = ix2;
             p.wmax = &b->sc[g].wmax;
             p.status = &b->sc[g].status;
-            p.kchunk = b->kchunk;
+            p.sx = G.sx;
+            p.sy = G.sy;
+            p.kchunk = G.kchunk;
             p.fin = &b->sc[g];
             p.grid_items = G.items;
             fp[g] = p;
@@ -227,7 +234,16 @@ int build_items(eulr_batch* b, int shape, int kchunk)
         int const ix = G.n0 - 2, iy = G.n1 - 2, iz = G.n2 - 2;
         size_t const before = items.size();
         if (ix > 0 && iy > 0 && iz > 0) {
-            int const ntx = (ix + tx - 1) / tx, nty = (iy + ty - 1) / ty, nkc = (iz + kchunk - 1) / kchunk;
+            // FP64: the same number of tiles and chunks, of even size instead of
+            // full ones and a remainder.  FP32 tiles are whole, so only the
+            // chunks are evened out.
+            int const ntx = (ix + tx - 1) / tx, nty = (iy + ty - 1) / ty;
+            int nkc = (iz + kchunk - 1) / kchunk;
+            GridState& S = b->grids[g];
+            S.sx = split_tiles(ix, ntx, 1);
+            S.sy = split_tiles(iy, nty, 1);
+            S.kchunk = (iz + nkc - 1) / nkc;
+            nkc = (iz + S.kchunk - 1) / S.kchunk;
             for (int kc = 0; kc < nkc; ++kc) {
                 for (int y = 0; y < nty; ++y) {
                     for (int x = 0; x < ntx; ++x) {
@@ -315,6 +331,7 @@ int ghost_copy(eulr_batch* b, int g, int in, int out)
     q.cons_out = bundle_of<double>(G.cons[out]);
     q.prim_out = bundle_of<double>(G.prim[out]);
     q.cs_out = static_cast<double*>(G.cs[out]);
+    q.h_out = static_cast<double*>(G.h[out]);
     q.comp = kCompNone;
     q.gamma = G.gamma;
     q.gm1 = G.gamma - 1.0;
@@ -369,7 +386,8 @@ int prepare_grid(eulr_batch* b, int g)
         // sound speed and first wavespeed as a loaded simulation computes them
         B_CUDA(launch_load_prim<double>(cbundle_of<double>(G.prim[0]), Bundle<double>{}, static_cast<double*>(G.cs[0]),
                                         n, G.gamma, 1.0 / G.dx[0], 1.0 / G.dx[1], 1.0 / G.dx[2], &b->sc[g].wmax,
-                                        b->sms, b->stream),
+                                        b->sms, b->stream, static_cast<double*>(G.h[0]),
+                                        static_cast<const double*>(G.cons[0][1])),
                "load");
         B_CUDA(launch_finalize_dt<double>(&b->sc[g], b->cfl, 0, b->stream), "finalize");
         // copy 1's ghost layer once (after the first dt, which the loaded
@@ -530,7 +548,7 @@ int eulr_batch_create(int precision, int ngrids, const eulr_grid_desc* grids, do
         b->own_stream = true;
     }
     b->grids.resize(ngrids);
-    int const per_copy = is_f64(b) ? 11 : (b->comp == kCompHiLo ? 10 : 5);
+    int const per_copy = is_f64(b) ? 12 : (b->comp == kCompHiLo ? 10 : 5);
     size_t bytes = 0;
     size_t max_items = 0;
     for (int g = 0; g < ngrids; ++g) {
@@ -567,6 +585,8 @@ int eulr_batch_create(int precision, int ngrids, const eulr_grid_desc* grids, do
                     p += field;
                 }
                 G.cs[c] = p;
+                p += field;
+                G.h[c] = p;
                 p += field;
             }
             for (int f = 0; f < 5; ++f) {

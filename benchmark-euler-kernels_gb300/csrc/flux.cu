@@ -2,19 +2,22 @@
 // simulation step share one z-marching tile engine.
 //
 // Work decomposition: the interior [1,n0-1) x [1,n1-1) x [1,n2-1) is cut into
-// TX x TY columns and each column into chunks of kchunk planes; a persistent
-// grid of CTAs walks the (tile, chunk) items round-robin.  A CTA marches up
-// its chunk one plane at a time through a ring of plane slots in shared
+// tiles of at most TX x TY columns.  FP64, single grid: tiles of even size,
+// their extent chosen for the grid (choose_tiles), and one run of planes per
+// CTA, all tiles' planes divided evenly among a resident grid of CTAs.  FP64
+// batch: even tiles and chunks of planes popped from a queue.  FP32: whole
+// tiles and chunks of kchunk planes, walked round-robin.  A CTA marches up
+// its run one plane at a time through a ring of plane slots in shared
 // memory, each slot holding the 7 face inputs (d, p, u0, u1, u2, c, e) of a
 // (TX+2) x (TY+2) plane with its one-cell halo.  Per plane:
 //   1. face phase -- every x face and y face of plane k and every z face
 //      between planes k and k+1 is solved ONCE (the reference solves each
 //      interior face twice, once from each side, godunov.hpp:48-82).  FP64
-//      (bound by the FP64 pipe): the x, y and z faces share one index space,
-//      and each face's family, cells and axis permutation are chosen by
-//      selects, so a warp whose lanes straddle two families still runs the
-//      HLLC once -- the 800 faces of a 16x16 tile take exactly 25
-//      warp-passes.  FP32 (bound by instruction issue): each family in its
+//      (bound by the FP64 pipe): the x, y and z faces share one index space
+//      of exactly the tile's faces, and each face's family, cells and axis
+//      permutation are chosen by selects, so a warp whose lanes straddle two
+//      families still runs the HLLC once -- the 800 faces of a 16x16 tile
+//      take exactly 25 warp-passes.  FP32 (bound by instruction issue): each family in its
 //      own warp-aligned range with compile-time axes, on a 32x8 tile.
 //      Fluxes go to shared memory in global axes;
 //   2. cell phase -- each thread owns one column cell and applies
@@ -25,14 +28,17 @@
 // and the next step's CFL max-wavespeed, reduced warp -> block -> one
 // atomicMax per CTA, so dt never leaves the device.
 //
-// Staging: in the fused step the seven input fields of a plane slot are
-// fetched by TMA (cp.async.bulk.tensor, one 18x18x1 FP64 box per field) into a
-// ring of three slots, two planes ahead of the plane being solved, each slot
-// completing on its own mbarrier.  Grids whose row pitch is not a multiple of
-// 16 bytes (odd n0) and the per-operator godunov (arbitrary caller pointers)
-// stage with plain cooperative loads instead.  Every mbarrier wait is bounded:
-// a wait that runs out sets bit 1 of the status word, waits (bounded) for the
-// copies still in flight and ends the CTA.
+// Staging: in the fused FP64 step the seven input fields of a plane slot are
+// fetched into a ring of three slots, two planes ahead of the plane being
+// solved: by TMA (cp.async.bulk.tensor, one 18x18x1 box per field, each slot
+// completing on its own mbarrier) where the row pitch is a multiple of 16
+// bytes, else and in the batch by 8-byte cp.async (20 steps of a
+// 99 x 128 x 75 grid, odd pitch: 7.0 -> 5.9 ms against synchronous loads and
+// whole tiles).  The per-operator godunov (arbitrary caller pointers, values
+// computed while staged) and the FP32 states stage with plain cooperative
+// loads instead.  Every mbarrier wait is bounded: a wait that runs out sets
+// bit 1 of the status word, waits (bounded) for the copies still in flight
+// and ends the CTA.
 #include "euler_device.cuh"
 #include "kernels.h"
 #include "step_common.cuh"
@@ -44,6 +50,15 @@ namespace eulr {
 namespace {
 
 constexpr int kWaitTries = 1 << 20; // mbarrier.try_wait attempts before giving up
+
+// How a plane slot is filled.
+enum Staging {
+    kStageTma,   // fused FP64 step, row pitch a multiple of 16 bytes: TMA boxes, ring of three slots
+    kStageAsync, // fused FP64 step, any pitch, and the batch: 8-byte cp.async, the same ring
+    kStageLoad,  // values are computed while staged (per-operator godunov, FP32 states): plain loads, two slots
+};
+template <int STAGE>
+constexpr int kStageSlots = STAGE == kStageLoad ? 2 : 3;
 
 template <class T, int TX, int TY, int NSLOT>
 struct TileLayout {
@@ -136,18 +151,88 @@ __device__ __forceinline__ void issue_plane(T* smem, unsigned long long* bars, i
     }
 }
 
-// Stage plane k with plain loads.  Godunov mode derives c and e from prim;
-// step mode reads the stored sound speed and the conservative energy.  Cells
-// outside the array get a benign uniform state; no face touching them is
-// ever used.
-template <class T, int TX, int TY, int NSLOT, int MODE, int COMP>
-__device__ __forceinline__ void load_plane(T* smem, int slot, FluxParams<T> const& p, int i0, int j0, int k)
+// The tile of one work item: its cells and the magic divisors of its face
+// and cell indexes (div_runtime).
+struct TileDims {
+    int w, h;            // interior cells along x and y
+    unsigned mw, mw1, mw2; // magics of w, w + 1 and w + 2
+};
+
+__device__ __forceinline__ TileDims tile_dims(int w, int h)
+{
+    return TileDims{w, h, div_magic20(w), div_magic20(w + 1), div_magic20(w + 2)};
+}
+
+// The halo cells a thread stages of every plane (a tile and its halo hold at
+// most two cells per thread): their offset within a plane of the grid and
+// their place in a slot's field (-1: none).  Found once per work item.
+template <int N>
+struct StageCells {
+    long long src[N];
+    int dst[N];
+};
+
+template <int TX, int TY>
+constexpr int kStagePerThread = ((TX + 2) * (TY + 2) + TX * TY - 1) / (TX * TY);
+
+template <class T, int TX, int TY>
+__device__ __forceinline__ StageCells<kStagePerThread<TX, TY>> stage_cells(FluxParams<T> const& p, TileDims const& t,
+                                                                         int i0, int j0)
+{
+    StageCells<kStagePerThread<TX, TY>> s;
+#pragma unroll
+    for (int r = 0; r < kStagePerThread<TX, TY>; ++r) {
+        int const c = threadIdx.x + r * TX * TY;
+        int const hy = div_runtime(c, t.mw2);
+        int const hx = c - hy * (t.w + 2);
+        s.dst[r] = hy < t.h + 2 ? hy * (TX + 2) + hx : -1;
+        s.src[r] = p.g.at(i0 - 1 + hx, j0 - 1 + hy, 0);
+    }
+    return s;
+}
+
+// Start copying plane k of the tile and its halo into `slot` (fused FP64
+// step: every staged value is stored, none is computed).
+template <class T, int TX, int TY, int NSLOT>
+__device__ __forceinline__ void issue_plane_async(T* smem, int slot, FluxParams<T> const& p,
+                                                  StageCells<kStagePerThread<TX, TY>> const& s, int k)
 {
     using L = TileLayout<T, TX, TY, NSLOT>;
+    static_assert(sizeof(T) == 8, "8-byte copies");
+    unsigned const base = smem_u32(slot_field<T, TX, TY, NSLOT>(smem, slot, 0));
+    long long const plane = p.g.s2 * k;
+#pragma unroll
+    for (int r = 0; r < kStagePerThread<TX, TY>; ++r) {
+        if (s.dst[r] >= 0) {
+            long long const o = s.src[r] + plane;
+#pragma unroll
+            for (int f = 0; f < kFields; ++f) {
+                const T* const src = (f < 5 ? p.prim.f[f] : (f == 5 ? p.cs : p.h)) + o;
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(
+                                     base + static_cast<unsigned>((f * L::PLANE_PAD + s.dst[r]) * sizeof(T))),
+                             "l"(src)
+                             : "memory");
+            }
+        }
+    }
+}
+
+// Stage plane k of the tile and its halo with plain loads.  Godunov mode
+// derives c and e + p from prim, the FP32 states rebuild prim from cons.
+// FP32 tiles are whole (TX x TY): their cells outside the array get a benign
+// uniform state, and no face touching them is ever used.
+template <class T, int TX, int TY, int NSLOT, int MODE, int COMP>
+__device__ __forceinline__ void load_plane(T* smem, int slot, FluxParams<T> const& p, TileDims const& t, int i0, int j0,
+                                           int k)
+{
+    using L = TileLayout<T, TX, TY, NSLOT>;
+    constexpr bool kWhole = sizeof(T) == 4;
     T* q = slot_field<T, TX, TY, NSLOT>(smem, slot, 0);
-    for (int c = threadIdx.x; c < L::PLANE; c += L::NT) {
-        int const hx = c % L::HX;
-        int const hy = c / L::HX;
+    int const n = kWhole ? L::PLANE : (t.w + 2) * (t.h + 2);
+    for (int cc = threadIdx.x; cc < n; cc += L::NT) {
+        int const hy = kWhole ? cc / L::HX : div_runtime(cc, t.mw2);
+        int const hx = cc - hy * (kWhole ? L::HX : t.w + 2);
+        int const c = hy * L::HX + hx;
         int const i = i0 - 1 + hx;
         int const j = j0 - 1 + hy;
         T d = T(1), pr = T(1), u0 = T(0), u1 = T(0), u2 = T(0), cs = T(1), e = T(2.5);
@@ -160,10 +245,7 @@ __device__ __forceinline__ void load_plane(T* smem, int slot, FluxParams<T> cons
                 u1 = __ldg(p.prim.f[3] + o);
                 u2 = __ldg(p.prim.f[4] + o);
             }
-            if (MODE == kModeStep) {
-                cs = __ldg(p.cs + o);
-                e = __ldg(p.cons_in.f[1] + o);
-            } else if (MODE == kModeStepCons) {
+            if (MODE == kModeStepCons) {
                 // cons-only FP32 state: cons_to_prim on chip
                 T const m0 = __ldg(p.cons_in.f[2] + o);
                 T const m1 = __ldg(p.cons_in.f[3] + o);
@@ -258,34 +340,42 @@ __device__ __forceinline__ bool wait_slot(TileCtx<T>& c, int s)
     return ok;
 }
 
-// One work item: interior planes [kb, ke) of the TX x TY column whose first
-// cell is (1 + tx*TX, 1 + ty*TY), with update coefficients k0..k2 (dt/dv
-// times the face areas).  Returns false when a staged plane never arrived.
-template <class T, int TX, int TY, int NSLOT, int MODE, bool TMA, int COMP>
+// One work item: interior planes [kb, ke) of tile (tx, ty), with update
+// coefficients k0..k2 (dt/dv times the face areas).  FP64 tiles are at most
+// TX x TY cells, cut evenly out of the grid (p.sx, p.sy), so a warp solves no
+// face and updates no cell that is not the grid's; FP32 tiles are whole.
+// Returns false when a staged plane never arrived.
+template <class T, int TX, int TY, int MODE, int STAGE, int COMP>
 __device__ __forceinline__ bool tile_item(TileCtx<T>& c, FluxParams<T> const& p, TmaMaps const& maps, T k0, T k1,
-                                          T k2, int tx, int ty, int kc)
+                                          T k2, int tx, int ty, int kb, int ke)
 {
+    constexpr int NSLOT = kStageSlots<STAGE>;
+    constexpr bool kWhole = sizeof(T) == 4;
     using L = TileLayout<T, TX, TY, NSLOT>;
     int const tid = threadIdx.x;
-    int const ti = tid % TX;
-    int const tj = tid / TX;
-    int const center = (tj + 1) * L::HX + ti + 1;
     bool const cubic = p.invdx0 == p.invdx1 && p.invdx1 == p.invdx2;
     T* const smem = c.smem;
     T* const fx = c.fx;
     T* const fy = c.fy;
     T* const fz = c.fz;
 
-    int const i0 = 1 + tx * TX;
-    int const j0 = 1 + ty * TY;
-    int const kb = 1 + kc * p.kchunk;
-    int const ke = min(kb + p.kchunk, p.g.n2 - 1);
+    int const i0 = 1 + (kWhole ? tx * TX : p.sx.start(tx));
+    int const j0 = 1 + (kWhole ? ty * TY : p.sy.start(ty));
+    TileDims const t = tile_dims(kWhole ? TX : 1 + p.sx.start(tx + 1) - i0, kWhole ? TY : 1 + p.sy.start(ty + 1) - j0);
+    int const tj = kWhole ? tid / TX : div_runtime(tid, t.mw);
+    int const ti = tid - tj * (kWhole ? TX : t.w);
+    int const center = (tj + 1) * L::HX + ti + 1;
     int const i = i0 + ti;
     int const j = j0 + tj;
-    bool const own = (i < p.g.n0 - 1) && (j < p.g.n1 - 1);
+    bool const own = kWhole ? (i < p.g.n0 - 1) && (j < p.g.n1 - 1) : tj < t.h;
+
+    StageCells<kStagePerThread<TX, TY>> cells;
+    if (STAGE == kStageAsync) {
+        cells = stage_cells<T, TX, TY>(p, t, i0, j0);
+    }
 
     __syncthreads(); // the previous item's readers of slots and fluxes are done
-    if (TMA) {
+    if (STAGE == kStageTma) {
         // planes kb-1, kb, kb+1 -> slots 0, 1, 2 (kb+1 <= ke always)
         if (tid == 0) {
             issue_plane<T, TX, TY, NSLOT>(smem, c.bars, 0, maps, i0, j0, kb - 1);
@@ -295,15 +385,21 @@ __device__ __forceinline__ bool tile_item(TileCtx<T>& c, FluxParams<T> const& p,
         c.inflight |= 7u;
         c.timed_out |= !wait_slot<T, NSLOT>(c, 0);
         c.timed_out |= !wait_slot<T, NSLOT>(c, 1);
+    } else if constexpr (STAGE == kStageAsync) {
+        for (int s = 0; s < NSLOT; ++s) {
+            issue_plane_async<T, TX, TY, NSLOT>(smem, s, p, cells, kb - 1 + s);
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncthreads();
     } else {
-        load_plane<T, TX, TY, NSLOT, MODE, COMP>(smem, 0, p, i0, j0, kb - 1);
-        load_plane<T, TX, TY, NSLOT, MODE, COMP>(smem, 1, p, i0, j0, kb);
+        load_plane<T, TX, TY, NSLOT, MODE, COMP>(smem, 0, p, t, i0, j0, kb - 1);
+        load_plane<T, TX, TY, NSLOT, MODE, COMP>(smem, 1, p, t, i0, j0, kb);
         __syncthreads();
     }
     // z face below the chunk's first plane, kept in registers in global
     // axes (the z face frame has n = mx2, t1 = mx0, t2 = mx1)
-    T zlo[5];
-    {
+    T zlo[5] = {T(0), T(0), T(0), T(0), T(0)};
+    if (kWhole || own) {
         Flux<T> const f0 = hllc_flux(load_side<T, L::PLANE_PAD>(slot_field<T, TX, TY, NSLOT>(smem, 0, 0), center, 2),
                                      load_side<T, L::PLANE_PAD>(slot_field<T, TX, TY, NSLOT>(smem, 1, 0), center, 2));
         zlo[0] = f0.d;
@@ -315,14 +411,22 @@ __device__ __forceinline__ bool tile_item(TileCtx<T>& c, FluxParams<T> const& p,
     if (__syncthreads_or(c.timed_out)) { // slot 0 is refilled next
         return false;
     }
-    if (TMA) {
+    if (STAGE == kStageTma) {
         if (kb + 2 <= ke) {
             if (tid == 0) {
                 issue_plane<T, TX, TY, NSLOT>(smem, c.bars, 0, maps, i0, j0, kb + 2);
             }
             c.inflight |= 1u;
         }
+    } else if constexpr (STAGE == kStageAsync) {
+        if (kb + 2 <= ke) {
+            issue_plane_async<T, TX, TY, NSLOT>(smem, 0, p, cells, kb + 2);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
     }
+    int const nfx = (t.w + 1) * t.h; // FP64: the faces of each family
+    int const nfy = t.w * (t.h + 1);
+    int const nface = nfx + nfy + t.w * t.h;
 
     // FP64 step: the next step's CFL wavespeed is screened (WaveScreen); the
     // running max carries over from the CTA's previous item of the same grid
@@ -346,10 +450,10 @@ __device__ __forceinline__ bool tile_item(TileCtx<T>& c, FluxParams<T> const& p,
                 }
             }
         }
-        if (TMA) {
+        if (STAGE == kStageTma) {
             c.timed_out |= !wait_slot<T, NSLOT>(c, nxt);
-        } else {
-            load_plane<T, TX, TY, NSLOT, MODE, COMP>(smem, nxt, p, i0, j0, k + 1);
+        } else if (STAGE == kStageLoad) {
+            load_plane<T, TX, TY, NSLOT, MODE, COMP>(smem, nxt, p, t, i0, j0, k + 1);
             __syncthreads();
         }
 
@@ -361,12 +465,12 @@ __device__ __forceinline__ bool tile_item(TileCtx<T>& c, FluxParams<T> const& p,
             // families; each face's family, left cell and right cell are
             // chosen by selects, so a warp that straddles two families still
             // runs the HLLC once
-            for (int f = tid; f < L::NFACE; f += L::NT) {
-                bool const is_x = f < L::NFX;
-                bool const is_y = !is_x && f < L::NFX + L::NFY;
-                int const g = is_x ? f : (is_y ? f - L::NFX : f - L::NFX - L::NFY);
-                int const gj = is_x ? div_small<TX + 1>(g) : div_small<TX>(g);
-                int const gi = g - gj * (is_x ? TX + 1 : TX);
+            for (int f = tid; f < nface; f += L::NT) {
+                bool const is_x = f < nfx;
+                bool const is_y = !is_x && f < nfx + nfy;
+                int const g = is_x ? f : (is_y ? f - nfx : f - nfx - nfy);
+                int const gj = div_runtime(g, is_x ? t.mw1 : t.mw);
+                int const gi = g - gj * (is_x ? t.w + 1 : t.w);
                 int const a = (is_y ? gj : gj + 1) * L::HX + (is_x ? gi : gi + 1);
                 int const dir = is_x ? 0 : (is_y ? 1 : 2);
                 T const* const qr = is_x || is_y ? qc : qn;
@@ -411,14 +515,19 @@ __device__ __forceinline__ bool tile_item(TileCtx<T>& c, FluxParams<T> const& p,
         if (__syncthreads_or(c.timed_out)) {
             return false;
         }
-        if (TMA) {
-            // plane k is no longer read: refill its slot with plane k+3
+        // plane k is no longer read: refill its slot with plane k+3
+        if (STAGE == kStageTma) {
             if (k + 3 <= ke) {
                 if (tid == 0) {
                     issue_plane<T, TX, TY, NSLOT>(smem, c.bars, cur, maps, i0, j0, k + 3);
                 }
                 c.inflight |= 1u << cur;
             }
+        } else if constexpr (STAGE == kStageAsync) {
+            if (k + 3 <= ke) {
+                issue_plane_async<T, TX, TY, NSLOT>(smem, cur, p, cells, k + 3);
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
         }
 
         // ---- cell phase
@@ -429,13 +538,14 @@ __device__ __forceinline__ bool tile_item(TileCtx<T>& c, FluxParams<T> const& p,
         }
         T wv[4] = {T(0), T(0), T(0), T(0)}; // FP64 step: the new cs, v0, v1, v2, for the screened wavespeed
         if (own) {
-            int const xl = tj * (TX + 1) + ti;
-            int const yb = tj * TX + ti;
+            int const tw = kWhole ? TX : t.w;
+            int const xl = tj * (tw + 1) + ti;
+            int const yb = tj * tw + ti;
 #pragma unroll
             for (int f = 0; f < 5; ++f) {
                 if (COMP == kCompNone) {
                     T const ax = fx[f * L::NFX + xl + 1] - fx[f * L::NFX + xl];
-                    T const ay = fy[f * L::NFY + yb + TX] - fy[f * L::NFY + yb];
+                    T const ay = fy[f * L::NFY + yb + tw] - fy[f * L::NFY + yb];
                     T const az = fza[f] - zlo[f];
                     u[f] = u[f] - k0 * ax - k1 * ay - k2 * az;
                 } else {
@@ -537,6 +647,9 @@ __device__ __forceinline__ bool tile_item(TileCtx<T>& c, FluxParams<T> const& p,
         for (int f = 0; f < 5; ++f) {
             zlo[f] = fza[f];
         }
+        if (STAGE == kStageAsync) {
+            asm volatile("cp.async.wait_group 1;" ::: "memory"); // plane k+2 landed (k+3 may be in flight)
+        }
         __syncthreads(); // fluxes are rewritten by the next face phase
     }
     c.wrun = screen.run;
@@ -612,19 +725,19 @@ __device__ __forceinline__ TileCtx<T> make_ctx(unsigned char* smem_dyn)
     return c;
 }
 
-template <class T, int TX, int TY, int NSLOT, int MODE, bool TMA, int COMP>
+template <class T, int TX, int TY, int MODE, int STAGE, int COMP>
 __global__ void __launch_bounds__(TX* TY) flux_tile_kernel(const __grid_constant__ FluxParams<T> p,
                                                            const __grid_constant__ TmaMaps maps)
 {
     static_assert(COMP == kCompNone || (sizeof(T) == 4 && MODE == kModeStepCons), "compensation is for the FP32 step");
-    static_assert(!TMA || NSLOT == 3, "the TMA ring has three slots");
+    constexpr int NSLOT = kStageSlots<STAGE>;
     extern __shared__ __align__(128) unsigned char smem_dyn[];
     TileCtx<T> c = make_ctx<T, TX, TY, NSLOT>(smem_dyn);
     T const dtodv = dt_over_dv(p);
     // cons -= dt/dv * sum_d ds_d (F_R - F_L), coefficients folded
     T const k0 = dtodv * p.ds0, k1 = dtodv * p.ds1, k2 = dtodv * p.ds2;
 
-    if (TMA) {
+    if (STAGE == kStageTma) {
         if (threadIdx.x == 0) {
             for (int s = 0; s < NSLOT; ++s) {
                 mbar_init(&c.bars[s], 1);
@@ -634,17 +747,32 @@ __global__ void __launch_bounds__(TX* TY) flux_tile_kernel(const __grid_constant
         __syncthreads();
     }
 
-    int const tiles_xy = p.tiles_x * p.tiles_y;
-    for (int w = blockIdx.x; w < p.nwork; w += gridDim.x) {
-        int const tx = w % p.tiles_x;
-        int const ty = (w / p.tiles_x) % p.tiles_y;
-        int const kc = w / tiles_xy;
-        if (!tile_item<T, TX, TY, NSLOT, MODE, TMA, COMP>(c, p, maps, k0, k1, k2, tx, ty, kc)) {
-            break;
+    if constexpr (sizeof(T) == 8) {
+        // CTA b's share of all tiles' planes, counted tile by tile: a run of
+        // planes up one tile, and on into the next
+        int const iz = p.g.n2 - 2;
+        long long w = static_cast<long long>(p.nwork) * blockIdx.x / gridDim.x;
+        long long const end = static_cast<long long>(p.nwork) * (blockIdx.x + 1) / gridDim.x;
+        while (w < end) {
+            int const tile = static_cast<int>(w) / iz;
+            int const k = static_cast<int>(w) - tile * iz;
+            int const run = static_cast<int>(min(end - w, static_cast<long long>(iz - k)));
+            if (!tile_item<T, TX, TY, MODE, STAGE, COMP>(c, p, maps, k0, k1, k2, tile % p.tiles_x, tile / p.tiles_x,
+                                                         1 + k, 1 + k + run)) {
+                break;
+            }
+            w += run;
+        }
+    } else {
+        int const tiles_xy = p.tiles_x * p.tiles_y;
+        for (int w = blockIdx.x; w < p.nwork; w += gridDim.x) {
+            int const kb = 1 + w / tiles_xy * p.kchunk;
+            tile_item<T, TX, TY, MODE, STAGE, COMP>(c, p, maps, k0, k1, k2, w % p.tiles_x, (w / p.tiles_x) % p.tiles_y,
+                                                    kb, min(kb + p.kchunk, p.g.n2 - 1));
         }
     }
 
-    if (TMA && __syncthreads_or(c.timed_out)) {
+    if (STAGE == kStageTma && __syncthreads_or(c.timed_out)) {
         // a staged plane never arrived: report, wait (bounded) for the copies
         // still in flight so none lands after the CTA is gone, and stop
         if (threadIdx.x == 0) {
@@ -668,11 +796,13 @@ __global__ void __launch_bounds__(TX* TY) flux_tile_kernel(const __grid_constant
 // (grid, tile, chunk) items from a global queue (largest grids first),
 // copies the item's grid parameters to shared memory and runs the same tile
 // engine; each item's wavespeed goes to its own grid's accumulator, so every
-// grid keeps its own dt.  Plain-load staging (grids of any shape).
+// grid keeps its own dt.  No TMA (grids of any shape): the FP64 state stages
+// by cp.async, the FP32 states by plain loads.
 template <class T, int TX, int TY, int MODE, int COMP>
 __global__ void __launch_bounds__(TX* TY) flux_batch_kernel(const __grid_constant__ BatchParams<T> b)
 {
-    constexpr int NSLOT = 2;
+    constexpr int STAGE = sizeof(T) == 8 ? kStageAsync : kStageLoad;
+    constexpr int NSLOT = kStageSlots<STAGE>;
     constexpr int NT = TX * TY;
     static_assert(sizeof(FluxParams<T>) % 4 == 0, "parameter copy in 4-byte words");
     extern __shared__ __align__(128) unsigned char smem_dyn[];
@@ -697,7 +827,9 @@ __global__ void __launch_bounds__(TX* TY) flux_batch_kernel(const __grid_constan
         __syncthreads();
         T const dtodv = dt_over_dv(gp);
         T const k0 = dtodv * gp.ds0, k1 = dtodv * gp.ds1, k2 = dtodv * gp.ds2;
-        tile_item<T, TX, TY, NSLOT, MODE, false, COMP>(c, gp, TmaMaps{}, k0, k1, k2, it.y, it.z, it.w);
+        int const kb = 1 + it.w * gp.kchunk;
+        tile_item<T, TX, TY, MODE, STAGE, COMP>(c, gp, TmaMaps{}, k0, k1, k2, it.y, it.z, kb,
+                                                min(kb + gp.kchunk, gp.g.n2 - 1));
         flush_wavespeed<T, NT>(c, gp.wmax, gp.status);
         item_done(gp);
     }
@@ -828,9 +960,11 @@ __global__ void finalize_dt_kernel(SimScalars* s, T cfl, int add_time, const dou
     }
 }
 
-// The single-grid tile.  FP64: 16x16 columns, whose 800 faces per plane
-// fill exactly 25 warp-passes (a 32x8 tile's 808 need 26) with the same 256
-// threads, 18x18 TMA boxes and two resident CTAs per SM.  FP32 (the state
+// The single-grid tile, at most.  FP64: 16x16 columns, whose 800 faces per
+// plane fill exactly 25 warp-passes (a 32x8 tile's 808 need 26) with the same
+// 256 threads, 18x18 TMA boxes and two resident CTAs per SM.  (A 16x8 kernel
+// with four CTAs of 128 threads per SM measured 33.2 ms a 512^3 step against
+// 32.9, and no better on small grids.)  FP32 (the state
 // with stored low words; the other FP32 states run the column engine):
 // 32x8, measured faster there (26.9 against 21.9 Gcell/s at 512^3).
 template <class T>
@@ -842,21 +976,79 @@ struct StepTile<float> {
     static constexpr int X = 32, Y = 8;
 };
 
-template <class T, int MODE, bool TMA, int COMP>
+// Tiles per axis of a single-grid FP64 launch.
+struct TilePlan {
+    int nx, ny;
+};
+
+// Picks them by the time of the busiest SM.  The kernel divides all tiles'
+// planes evenly among its CTAs, so with U planes in all on G CTAs, r of them
+// on an SM, each solves m = ceil(U/G) planes of cost c and the z faces below
+// its first plane, z: the SM's FP64 pipe is busy r (m c + z), and every plane
+// adds a wait that its neighbour does not cover (its barriers and its last,
+// partly filled pass of faces).  c and z count FP64 warp instructions, 27 a
+// face and 49 a cell of the step (30 of the operator's update, and 15 a cell
+// that it stages), each holding its SM for 9.0 ns; the wait measured
+// 1.1 us a plane with two CTAs on the SM and 1.6 us with one.  Whole
+// 16 x 16 tiles are the best for large grids (256^3: 4.14 ms a step, 4.42 in
+// 16 x 8), smaller ones where their number leaves SMs idle.  Against whole
+// 16 x 16 tiles in chunks of at least 8 planes: 16^3 97 -> 12.5 us a step,
+// 48^3 97 -> 46, 64^3 97 -> 86, 99 x 128 x 75 311 -> 270.
+TilePlan choose_tiles(int ix, int iy, int iz, int sms, int per_sm, bool step, int q)
+{
+    constexpr int kTX = StepTile<double>::X, kTY = StepTile<double>::Y;
+    constexpr double kInstr = 9.0e-3, kWait2 = 1.1, kWait1 = 1.6; // us
+    int const units = (ix + q - 1) / q;
+    TilePlan best{};
+    double best_us = 1e300;
+    int last_nx = 0;
+    for (int w = kTX / q; w >= 1; --w) {
+        int const nx = (units + w - 1) / w;
+        int const tw = (units + nx - 1) / nx * q;
+        if (nx == last_nx) {
+            continue; // the same tiles as the previous extent's
+        }
+        last_nx = nx;
+        int last_ny = 0;
+        for (int h = kTY; h >= 1; --h) {
+            int const ny = (iy + h - 1) / h;
+            int const th = (iy + ny - 1) / ny;
+            if (ny == last_ny) {
+                continue;
+            }
+            last_ny = ny;
+            int const faces = (tw + 1) * th + tw * (th + 1) + tw * th;
+            int const rows = (tw * th + 31) / 32;
+            int const c = 27 * ((faces + 31) / 32) +
+                          (step ? 49 * rows : 30 * rows + 15 * (((tw + 2) * (th + 2) + 31) / 32));
+            long long const u = static_cast<long long>(nx) * ny * iz;
+            long long const ctas = u < static_cast<long long>(sms) * per_sm ? u : static_cast<long long>(sms) * per_sm;
+            long long const r = (ctas + sms - 1) / sms;
+            long long const m = (u + ctas - 1) / ctas;
+            double const us = m * (r * c * kInstr + (r > 1 ? kWait2 : kWait1)) + r * 27 * rows * kInstr;
+            if (us < best_us * (1.0 - 1e-9)) {
+                best_us = us;
+                best = TilePlan{nx, ny};
+            }
+        }
+    }
+    return best;
+}
+
+template <class T, int MODE, int STAGE, int COMP>
 struct FluxKernel {
-    static constexpr int NSLOT = TMA ? 3 : 2;
     static constexpr int TX = StepTile<T>::X, TY = StepTile<T>::Y;
-    using L = TileLayout<T, TX, TY, NSLOT>;
-    static auto fn() { return flux_tile_kernel<T, TX, TY, NSLOT, MODE, TMA, COMP>; }
+    using L = TileLayout<T, TX, TY, kStageSlots<STAGE>>;
+    static auto fn() { return flux_tile_kernel<T, TX, TY, MODE, STAGE, COMP>; }
 };
 
 // Opts the kernel into its dynamic shared memory size and returns its
 // resident CTAs per SM.  Called outside any stream capture (by the entry
 // points before they enqueue work), and cheap to repeat.
-template <class T, int MODE, bool TMA, int COMP>
+template <class T, int MODE, int STAGE, int COMP>
 cudaError_t configure_flux_impl(int* per_sm)
 {
-    using K = FluxKernel<T, MODE, TMA, COMP>;
+    using K = FluxKernel<T, MODE, STAGE, COMP>;
     auto kern = K::fn();
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          static_cast<int>(K::L::BYTES));
@@ -872,10 +1064,10 @@ cudaError_t configure_flux_impl(int* per_sm)
     return cudaSuccess;
 }
 
-template <class T, int MODE, bool TMA, int COMP>
+template <class T, int MODE, int STAGE, int COMP>
 cudaError_t launch_flux_impl(FluxParams<T> p, TmaMaps const& maps, int sms, cudaStream_t s)
 {
-    using K = FluxKernel<T, MODE, TMA, COMP>;
+    using K = FluxKernel<T, MODE, STAGE, COMP>;
     int const per_sm = p.per_sm > 0 ? p.per_sm : 1;
     int const ix = p.g.n0 - 2;
     int const iy = p.g.n1 - 2;
@@ -883,10 +1075,18 @@ cudaError_t launch_flux_impl(FluxParams<T> p, TmaMaps const& maps, int sms, cuda
     if (ix <= 0 || iy <= 0 || iz <= 0) {
         return cudaSuccess; // no interior cell
     }
-    p.tiles_x = (ix + K::TX - 1) / K::TX;
-    p.tiles_y = (iy + K::TY - 1) / K::TY;
     long long const slots = static_cast<long long>(sms) * per_sm;
-    if (p.kchunk <= 0) {
+    if constexpr (sizeof(T) == 8) {
+        int const q = STAGE == kStageTma ? 2 : 1;
+        TilePlan const plan = choose_tiles(ix, iy, iz, sms, per_sm, MODE == kModeStep, q);
+        p.sx = split_tiles(ix, plan.nx, q);
+        p.sy = split_tiles(iy, plan.ny, 1);
+        p.tiles_x = plan.nx;
+        p.tiles_y = plan.ny;
+        p.kchunk = 1; // the kernel divides the planes themselves among its CTAs
+    } else {
+        p.tiles_x = (ix + K::TX - 1) / K::TX;
+        p.tiles_y = (iy + K::TY - 1) / K::TY;
         p.kchunk = choose_kchunk(p.tiles_x * p.tiles_y, iz, slots);
     }
     int const kchunks = (iz + p.kchunk - 1) / p.kchunk;
@@ -907,7 +1107,7 @@ constexpr int kNumBatchShapes = 3;
 
 template <class T, int TX, int TY, int MODE, int COMP>
 struct BatchKernel {
-    using L = TileLayout<T, TX, TY, 2>;
+    using L = TileLayout<T, TX, TY, kStageSlots<(sizeof(T) == 8 ? kStageAsync : kStageLoad)>>;
     static auto fn() { return flux_batch_kernel<T, TX, TY, MODE, COMP>; }
     static cudaError_t configure(int* per_sm)
     {
@@ -980,21 +1180,21 @@ struct FluxDispatch<double> {
     static cudaError_t configure(int mode, bool tma, int /*comp*/, int* per_sm)
     {
         if (mode == kModeStep) {
-            return tma ? configure_flux_impl<double, kModeStep, true, kCompNone>(per_sm)
-                       : configure_flux_impl<double, kModeStep, false, kCompNone>(per_sm);
+            return tma ? configure_flux_impl<double, kModeStep, kStageTma, kCompNone>(per_sm)
+                       : configure_flux_impl<double, kModeStep, kStageAsync, kCompNone>(per_sm);
         }
-        return configure_flux_impl<double, kModeGodunov, false, kCompNone>(per_sm);
+        return configure_flux_impl<double, kModeGodunov, kStageLoad, kCompNone>(per_sm);
     }
     static cudaError_t launch(FluxParams<double> const& p, TmaMaps const* maps, int mode, int /*comp*/, int sms,
                               cudaStream_t s)
     {
         if (mode == kModeStep) {
             if (maps != nullptr) {
-                return launch_flux_impl<double, kModeStep, true, kCompNone>(p, *maps, sms, s);
+                return launch_flux_impl<double, kModeStep, kStageTma, kCompNone>(p, *maps, sms, s);
             }
-            return launch_flux_impl<double, kModeStep, false, kCompNone>(p, TmaMaps{}, sms, s);
+            return launch_flux_impl<double, kModeStep, kStageAsync, kCompNone>(p, TmaMaps{}, sms, s);
         }
-        return launch_flux_impl<double, kModeGodunov, false, kCompNone>(p, TmaMaps{}, sms, s);
+        return launch_flux_impl<double, kModeGodunov, kStageLoad, kCompNone>(p, TmaMaps{}, sms, s);
     }
 };
 
@@ -1007,11 +1207,11 @@ struct FluxDispatch<float> {
             // double-float state keeps the shared-memory tile engine
             switch (comp) {
             case kCompSum: return configure_step_f32col(kCompSum, per_sm);
-            case kCompHiLo: return configure_flux_impl<float, kModeStepCons, false, kCompHiLo>(per_sm);
+            case kCompHiLo: return configure_flux_impl<float, kModeStepCons, kStageLoad, kCompHiLo>(per_sm);
             default: return configure_step_f32col(kCompNone, per_sm);
             }
         }
-        return configure_flux_impl<float, kModeGodunov, false, kCompNone>(per_sm);
+        return configure_flux_impl<float, kModeGodunov, kStageLoad, kCompNone>(per_sm);
     }
     static cudaError_t launch(FluxParams<float> const& p, TmaMaps const* /*maps*/, int mode, int comp, int sms,
                               cudaStream_t s)
@@ -1019,11 +1219,11 @@ struct FluxDispatch<float> {
         if (mode == kModeStep) {
             switch (comp) {
             case kCompSum: return launch_step_f32col(p, kCompSum, sms, s);
-            case kCompHiLo: return launch_flux_impl<float, kModeStepCons, false, kCompHiLo>(p, TmaMaps{}, sms, s);
+            case kCompHiLo: return launch_flux_impl<float, kModeStepCons, kStageLoad, kCompHiLo>(p, TmaMaps{}, sms, s);
             default: return launch_step_f32col(p, kCompNone, sms, s);
             }
         }
-        return launch_flux_impl<float, kModeGodunov, false, kCompNone>(p, TmaMaps{}, sms, s);
+        return launch_flux_impl<float, kModeGodunov, kStageLoad, kCompNone>(p, TmaMaps{}, sms, s);
     }
 };
 

@@ -32,6 +32,25 @@ struct SimScalars {
     unsigned long long ghost_wmax; // FP32 states: max invdt of the ghost layer, which never changes (set at load)
 };
 
+// n interior cells cut into `parts` tiles of even size: `base` or base + 1
+// units of q cells each, the longer ones first.  q = 2 keeps every tile's
+// first cell at an odd index, whose halo (one cell lower) starts on the
+// 16-byte boundary a TMA box needs.
+struct TileSplit {
+    int n, parts, base, longer, q;
+    __host__ __device__ int start(int t) const
+    {
+        int const s = q * (t * base + (t < longer ? t : longer));
+        return s < n ? s : n;
+    }
+};
+
+inline TileSplit split_tiles(int n, int parts, int q)
+{
+    int const units = (n + q - 1) / q;
+    return TileSplit{n, parts, units / parts, units % parts, q};
+}
+
 // TMA descriptors of the seven staged fields (d, p, u0, u1, u2, c, e) of the
 // step's input copy: 3D tensors (n0, n1, n2), boxes of (TX+2) x (TY+2) x 1.
 struct TmaMaps {
@@ -61,7 +80,9 @@ struct FluxParams {
     T invdx0, invdx1, invdx2;
     unsigned long long* wmax; // step mode: atomicMax of the next max invdt
     int* status;              // step mode: set to 1 on a non-physical cell
-    int tiles_x, tiles_y, kchunk, nwork; // work decomposition (kchunk <= 0: default)
+    const T* h;          // FP64 step mode: stored e + p of prim
+    TileSplit sx, sy;                    // FP64: the tiles along x and y
+    int tiles_x, tiles_y, kchunk, nwork; // work decomposition (FP64 single grid: nwork planes of tiles, no chunks)
     int per_sm;                          // resident CTAs per SM (from configure_flux)
     SimScalars* fin;  // step mode, when set: the kernel finalizes the step itself (next dt, clock)
     T* h_out;         // FP64 step mode, when set: e + p of the new state (interior), the HLLC's

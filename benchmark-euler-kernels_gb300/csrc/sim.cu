@@ -278,6 +278,7 @@ int enqueue_step_t(eulr_sim* s, int in, cudaEvent_t* ev)
     if (is_f64(s)) {
         p.prim = cbundle_of<T>(s->prim[in]);
         p.cs = static_cast<const T*>(s->cs[in]);
+        p.h = static_cast<const T*>(s->h[in]);
         p.prim_out = bundle_of<T>(s->prim[out]);
         p.cs_out = static_cast<T*>(s->cs[out]);
         p.h_out = static_cast<T*>(s->h[out]);

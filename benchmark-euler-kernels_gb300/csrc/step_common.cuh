@@ -15,15 +15,21 @@ constexpr long long kInfBits = 0x7ff0000000000000LL;
 
 // g / D for 0 <= g < 2^12 and a compile-time 0 < D < 256, as one product and
 // a shift: floor(g (floor(2^20/D) + 1) / 2^20) exceeds g/D by less than
-// g/2^20 < 2^-8, which stays below the gap 1/D to the next integer.  The
-// tile engine's face index takes one of two constant divisors by a select,
-// which the compiler otherwise turned into a runtime integer division.
+// g/2^20 < 2^-8, which stays below the gap 1/D to the next integer.
 template <int D>
 __device__ __forceinline__ int div_small(int g)
 {
     static_assert(D > 0 && D < 256, "divisor range");
     constexpr unsigned kM = (1u << 20) / D + 1u;
     return static_cast<int>((static_cast<unsigned>(g) * kM) >> 20);
+}
+
+// The same with a divisor known at run time (an FP64 tile's extents are its
+// grid's): the magic once per work item, a product and a shift per use.
+__device__ __forceinline__ unsigned div_magic20(int d) { return (1u << 20) / static_cast<unsigned>(d) + 1u; }
+__device__ __forceinline__ int div_runtime(int g, unsigned magic)
+{
+    return static_cast<int>((static_cast<unsigned>(g) * magic) >> 20);
 }
 
 __device__ __forceinline__ unsigned smem_u32(const void* p)
