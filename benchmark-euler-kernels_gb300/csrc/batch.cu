@@ -712,6 +712,9 @@ int eulr_batch_autotune(eulr_batch* b, int trial_steps, int* shape_out, int* kch
     int best_shape = 0, best_kc = 32;
     int st = EULR_SUCCESS;
     for (int shape = 0; shape < batch_shape_count() && st == EULR_SUCCESS; ++shape) {
+        if (!batch_shape_built(shape, is_f64(b))) {
+            continue;
+        }
         for (int kc : kKchunks) {
             st = build_items(b, shape, kc);
             if (st != EULR_SUCCESS) {

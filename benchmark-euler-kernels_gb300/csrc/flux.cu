@@ -1,25 +1,22 @@
-// Godunov/HLLC flux kernels (sm_103a): the per-operator godunov and the fused
-// simulation step share one z-marching tile engine.
+// FP64 Godunov/HLLC flux kernels (sm_103a): the per-operator godunov and the
+// fused simulation step share one z-marching tile engine.  (The FP32 ones run
+// on the column engine of flux_f32.cu.)
 //
 // Work decomposition: the interior [1,n0-1) x [1,n1-1) x [1,n2-1) is cut into
-// tiles of at most TX x TY columns.  FP64, single grid: tiles of even size,
-// their extent chosen for the grid (choose_tiles), and one run of planes per
-// CTA, all tiles' planes divided evenly among a resident grid of CTAs.  FP64
-// batch: even tiles and chunks of planes popped from a queue.  FP32: whole
-// tiles and chunks of kchunk planes, walked round-robin.  A CTA marches up
-// its run one plane at a time through a ring of plane slots in shared
-// memory, each slot holding the 7 face inputs (d, p, u0, u1, u2, c, e) of a
+// tiles of at most TX x TY columns, of even size.  Single grid: their extent
+// is chosen for the grid (choose_tiles), and all tiles' planes are divided
+// evenly among a resident grid of CTAs, a run of planes each.  Batch: chunks
+// of planes popped from a queue.  A CTA marches up its run one plane at a
+// time through a ring of plane slots in shared memory, each slot holding the 7 face inputs (d, p, u0, u1, u2, c, e) of a
 // (TX+2) x (TY+2) plane with its one-cell halo.  Per plane:
 //   1. face phase -- every x face and y face of plane k and every z face
 //      between planes k and k+1 is solved ONCE (the reference solves each
-//      interior face twice, once from each side, godunov.hpp:48-82).  FP64
-//      (bound by the FP64 pipe): the x, y and z faces share one index space
+//      interior face twice, once from each side, godunov.hpp:48-82).  The
+//      FP64 pipe is the bound: the x, y and z faces share one index space
 //      of exactly the tile's faces, and each face's family, cells and axis
 //      permutation are chosen by selects, so a warp whose lanes straddle two
 //      families still runs the HLLC once -- the 800 faces of a 16x16 tile
-//      take exactly 25 warp-passes.  FP32 (bound by instruction issue): each family in its
-//      own warp-aligned range with compile-time axes, on a 32x8 tile.
-//      Fluxes go to shared memory in global axes;
+//      take exactly 25 warp-passes.  Fluxes go to shared memory in global axes;
 //   2. cell phase -- each thread owns one column cell and applies
 //      cons -= dt/dv * sum_d ds_d (F_R - F_L) (godunov.hpp:84-90) with the
 //      face-area and dt/dv factors folded into three coefficients.  The z
@@ -35,8 +32,7 @@
 // bytes, else and in the batch by 8-byte cp.async (20 steps of a
 // 99 x 128 x 75 grid, odd pitch: 7.0 -> 5.9 ms against synchronous loads and
 // whole tiles).  The per-operator godunov (arbitrary caller pointers, values
-// computed while staged) and the FP32 states stage with plain cooperative
-// loads instead.  Every mbarrier wait is bounded: a wait that runs out sets
+// computed while staged) stages with plain cooperative loads instead.  Every mbarrier wait is bounded: a wait that runs out sets
 // bit 1 of the status word, waits (bounded) for the copies still in flight
 // and ends the CTA.
 #include "euler_device.cuh"
@@ -55,12 +51,12 @@ constexpr int kWaitTries = 1 << 20; // mbarrier.try_wait attempts before giving 
 enum Staging {
     kStageTma,   // fused FP64 step, row pitch a multiple of 16 bytes: TMA boxes, ring of three slots
     kStageAsync, // fused FP64 step, any pitch, and the batch: 8-byte cp.async, the same ring
-    kStageLoad,  // values are computed while staged (per-operator godunov, FP32 states): plain loads, two slots
+    kStageLoad,  // values are computed while staged (per-operator godunov): plain loads, two slots
 };
 template <int STAGE>
 constexpr int kStageSlots = STAGE == kStageLoad ? 2 : 3;
 
-template <class T, int TX, int TY, int NSLOT>
+template <int TX, int TY, int NSLOT>
 struct TileLayout {
     static constexpr int HX = TX + 2;
     static constexpr int HY = TY + 2;
@@ -69,15 +65,9 @@ struct TileLayout {
     static constexpr int NFX = (TX + 1) * TY;
     static constexpr int NFY = TX * (TY + 1);
     static constexpr int NFZ = TX * TY;
-    static constexpr int NFACE = NFX + NFY + NFZ;
-    // FP32's index space: each face family starts on a warp boundary
-    static constexpr int NFX_W = (NFX + 31) / 32 * 32;
-    static constexpr int NFY_W = (NFY + 31) / 32 * 32;
-    static constexpr int NFACE_W = NFX_W + NFY_W + NFZ;
-    static_assert(NFACE_W >= NFACE && NFACE_W - NFACE < 64, "padding of at most one warp per family");
-    static_assert(NFX < 4096 && NFY < 4096 && NFZ < 4096, "face index range of div_small");
+    static_assert(NFX < 4096 && NFY < 4096 && NFZ < 4096, "face index range of div_runtime");
     static constexpr int NT = TX * TY;
-    // shared memory, in T elements after a 128-byte mbarrier block
+    // shared memory, in double elements after a 128-byte mbarrier block
     static constexpr int Q_ELEMS = NSLOT * kFields * PLANE_PAD;
     static constexpr int FX_OFF = Q_ELEMS;
     static constexpr int FY_OFF = FX_OFF + 5 * NFX;
@@ -85,8 +75,8 @@ struct TileLayout {
     static constexpr int ELEMS = FZ_OFF + 5 * NFZ;
     static constexpr int MBAR_BYTES = 128;
     // + 128 bytes of slack to align the dynamic region to 128 bytes at run time
-    static constexpr size_t BYTES = 128 + MBAR_BYTES + sizeof(T) * static_cast<size_t>(ELEMS);
-    static constexpr unsigned TX_BYTES = kFields * PLANE * sizeof(T); // bytes one slot's TMA delivers
+    static constexpr size_t BYTES = 128 + MBAR_BYTES + sizeof(double) * static_cast<size_t>(ELEMS);
+    static constexpr unsigned TX_BYTES = kFields * PLANE * sizeof(double); // bytes one slot's TMA delivers
 };
 
 __device__ __forceinline__ void mbar_init(unsigned long long* bar, unsigned count)
@@ -130,24 +120,24 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, i
             : "memory");
 }
 
-template <class T, int TX, int TY, int NSLOT>
-__device__ __forceinline__ T* slot_field(T* smem, int slot, int field)
+template <int TX, int TY, int NSLOT>
+__device__ __forceinline__ double* slot_field(double* smem, int slot, int field)
 {
-    using L = TileLayout<T, TX, TY, NSLOT>;
+    using L = TileLayout<TX, TY, NSLOT>;
     return smem + (slot * kFields + field) * L::PLANE_PAD;
 }
 
 // Issue the TMA loads of plane k (x origin i0-1, y origin j0-1) into `slot`.
-template <class T, int TX, int TY, int NSLOT>
-__device__ __forceinline__ void issue_plane(T* smem, unsigned long long* bars, int slot, TmaMaps const& maps, int i0,
+template <int TX, int TY, int NSLOT>
+__device__ __forceinline__ void issue_plane(double* smem, unsigned long long* bars, int slot, TmaMaps const& maps, int i0,
                                             int j0, int k)
 {
-    using L = TileLayout<T, TX, TY, NSLOT>;
+    using L = TileLayout<TX, TY, NSLOT>;
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     mbar_expect_tx(&bars[slot], L::TX_BYTES);
 #pragma unroll
     for (int f = 0; f < kFields; ++f) {
-        tma_load_3d(slot_field<T, TX, TY, NSLOT>(smem, slot, f), &maps.m[f], i0 - 1, j0 - 1, k, &bars[slot]);
+        tma_load_3d(slot_field<TX, TY, NSLOT>(smem, slot, f), &maps.m[f], i0 - 1, j0 - 1, k, &bars[slot]);
     }
 }
 
@@ -175,8 +165,8 @@ struct StageCells {
 template <int TX, int TY>
 constexpr int kStagePerThread = ((TX + 2) * (TY + 2) + TX * TY - 1) / (TX * TY);
 
-template <class T, int TX, int TY>
-__device__ __forceinline__ StageCells<kStagePerThread<TX, TY>> stage_cells(FluxParams<T> const& p, TileDims const& t,
+template <int TX, int TY>
+__device__ __forceinline__ StageCells<kStagePerThread<TX, TY>> stage_cells(FluxParams<double> const& p, TileDims const& t,
                                                                          int i0, int j0)
 {
     StageCells<kStagePerThread<TX, TY>> s;
@@ -193,13 +183,12 @@ __device__ __forceinline__ StageCells<kStagePerThread<TX, TY>> stage_cells(FluxP
 
 // Start copying plane k of the tile and its halo into `slot` (fused FP64
 // step: every staged value is stored, none is computed).
-template <class T, int TX, int TY, int NSLOT>
-__device__ __forceinline__ void issue_plane_async(T* smem, int slot, FluxParams<T> const& p,
+template <int TX, int TY, int NSLOT>
+__device__ __forceinline__ void issue_plane_async(double* smem, int slot, FluxParams<double> const& p,
                                                   StageCells<kStagePerThread<TX, TY>> const& s, int k)
 {
-    using L = TileLayout<T, TX, TY, NSLOT>;
-    static_assert(sizeof(T) == 8, "8-byte copies");
-    unsigned const base = smem_u32(slot_field<T, TX, TY, NSLOT>(smem, slot, 0));
+    using L = TileLayout<TX, TY, NSLOT>;
+    unsigned const base = smem_u32(slot_field<TX, TY, NSLOT>(smem, slot, 0));
     long long const plane = p.g.s2 * k;
 #pragma unroll
     for (int r = 0; r < kStagePerThread<TX, TY>; ++r) {
@@ -207,9 +196,9 @@ __device__ __forceinline__ void issue_plane_async(T* smem, int slot, FluxParams<
             long long const o = s.src[r] + plane;
 #pragma unroll
             for (int f = 0; f < kFields; ++f) {
-                const T* const src = (f < 5 ? p.prim.f[f] : (f == 5 ? p.cs : p.h)) + o;
+                const double* const src = (f < 5 ? p.prim.f[f] : (f == 5 ? p.cs : p.h)) + o;
                 asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(
-                                     base + static_cast<unsigned>((f * L::PLANE_PAD + s.dst[r]) * sizeof(T))),
+                                     base + static_cast<unsigned>((f * L::PLANE_PAD + s.dst[r]) * sizeof(double))),
                              "l"(src)
                              : "memory");
             }
@@ -217,81 +206,45 @@ __device__ __forceinline__ void issue_plane_async(T* smem, int slot, FluxParams<
     }
 }
 
-// Stage plane k of the tile and its halo with plain loads.  Godunov mode
-// derives c and e + p from prim, the FP32 states rebuild prim from cons.
-// FP32 tiles are whole (TX x TY): their cells outside the array get a benign
-// uniform state, and no face touching them is ever used.
-template <class T, int TX, int TY, int NSLOT, int MODE, int COMP>
-__device__ __forceinline__ void load_plane(T* smem, int slot, FluxParams<T> const& p, TileDims const& t, int i0, int j0,
+// Stage plane k of the tile and its halo for the per-operator godunov with
+// plain loads: prim as it is, the sound speed and e + p derived from it.
+template <int TX, int TY, int NSLOT>
+__device__ __forceinline__ void load_plane(double* smem, int slot, FluxParams<double> const& p, TileDims const& t, int i0, int j0,
                                            int k)
 {
-    using L = TileLayout<T, TX, TY, NSLOT>;
-    constexpr bool kWhole = sizeof(T) == 4;
-    T* q = slot_field<T, TX, TY, NSLOT>(smem, slot, 0);
-    int const n = kWhole ? L::PLANE : (t.w + 2) * (t.h + 2);
+    using L = TileLayout<TX, TY, NSLOT>;
+    double* q = slot_field<TX, TY, NSLOT>(smem, slot, 0);
+    int const n = (t.w + 2) * (t.h + 2);
     for (int cc = threadIdx.x; cc < n; cc += L::NT) {
-        int const hy = kWhole ? cc / L::HX : div_runtime(cc, t.mw2);
-        int const hx = cc - hy * (kWhole ? L::HX : t.w + 2);
+        int const hy = div_runtime(cc, t.mw2);
+        int const hx = cc - hy * (t.w + 2);
         int const c = hy * L::HX + hx;
-        int const i = i0 - 1 + hx;
-        int const j = j0 - 1 + hy;
-        T d = T(1), pr = T(1), u0 = T(0), u1 = T(0), u2 = T(0), cs = T(1), e = T(2.5);
-        if (i < p.g.n0 && j < p.g.n1) {
-            long long const o = p.g.at(i, j, k);
-            if (MODE != kModeStepCons) {
-                d = __ldg(p.prim.f[0] + o);
-                pr = __ldg(p.prim.f[1] + o);
-                u0 = __ldg(p.prim.f[2] + o);
-                u1 = __ldg(p.prim.f[3] + o);
-                u2 = __ldg(p.prim.f[4] + o);
-            }
-            if (MODE == kModeStepCons) {
-                // cons-only FP32 state: cons_to_prim on chip
-                T const m0 = __ldg(p.cons_in.f[2] + o);
-                T const m1 = __ldg(p.cons_in.f[3] + o);
-                T const m2 = __ldg(p.cons_in.f[4] + o);
-                d = __ldg(p.cons_in.f[0] + o);
-                e = __ldg(p.cons_in.f[1] + o);
-                T const r = rcp_rn(d); // = 1/d correctly rounded, without the division routine
-                u0 = m0 * r;
-                u1 = m1 * r;
-                u2 = m2 * r;
-                pr = cons_pressure<COMP>(d, e, m0, m1, m2, r, p.gm1, nullptr);
-                cs = fast_sound_speed(p.gamma * pr * r);
-            } else {
-                if constexpr (sizeof(T) == 8) {
-                    // sqrt(gamma p / rho) from one reciprocal square root, and
-                    // e + p = p gamma/(gamma-1) + (rho/2) |u|^2 with the
-                    // halving on the integer pipe: 4 FP64 instructions and a
-                    // seed fewer per staged cell than 1/rho, a square root
-                    // and e formed before p is added
-                    cs = sqrt_quotient_faithful(p.gamma * pr, d);
-                    e = pr * (p.inv_gm1 + T(1)) + half_exact(d) * (u0 * u0 + u1 * u1 + u2 * u2);
-                } else {
-                    cs = sqrt(p.gamma * pr * (T(1) / d));
-                    e = pr * p.inv_gm1 + T(0.5) * d * (u0 * u0 + u1 * u1 + u2 * u2);
-                }
-            }
-            if (MODE != kModeGodunov || sizeof(T) == 4) {
-                e += pr; // the HLLC takes e + p (formed once per staged cell, not per face)
-            }
-        }
+        long long const o = p.g.at(i0 - 1 + hx, j0 - 1 + hy, k);
+        double const d = __ldg(p.prim.f[0] + o);
+        double const pr = __ldg(p.prim.f[1] + o);
+        double const u0 = __ldg(p.prim.f[2] + o);
+        double const u1 = __ldg(p.prim.f[3] + o);
+        double const u2 = __ldg(p.prim.f[4] + o);
         q[0 * L::PLANE_PAD + c] = d;
         q[1 * L::PLANE_PAD + c] = pr;
         q[2 * L::PLANE_PAD + c] = u0;
         q[3 * L::PLANE_PAD + c] = u1;
         q[4 * L::PLANE_PAD + c] = u2;
-        q[5 * L::PLANE_PAD + c] = cs;
-        q[6 * L::PLANE_PAD + c] = e;
+        // sqrt(gamma p / rho) from one reciprocal square root, and
+        // e + p = p gamma/(gamma-1) + (rho/2) |u|^2 with the halving on the
+        // integer pipe: 4 FP64 instructions and a seed fewer per staged cell
+        // than 1/rho, a square root and e formed before p is added
+        q[5 * L::PLANE_PAD + c] = sqrt_quotient_faithful(p.gamma * pr, d);
+        q[6 * L::PLANE_PAD + c] = pr * (p.inv_gm1 + 1.0) + half_exact(d) * (u0 * u0 + u1 * u1 + u2 * u2);
     }
 }
 
-template <class T, int PLANE_PAD>
-__device__ __forceinline__ Side<T> load_side(T const* q, int c, int dir)
+template <int PLANE_PAD>
+__device__ __forceinline__ Side<double> load_side(double const* q, int c, int dir)
 {
     int const d1 = dir == 2 ? 0 : dir + 1; // the axes after the normal, cyclically
     int const d2 = dir == 0 ? 2 : dir - 1;
-    Side<T> s;
+    Side<double> s;
     s.d = q[0 * PLANE_PAD + c];
     s.p = q[1 * PLANE_PAD + c];
     s.un = q[(2 + dir) * PLANE_PAD + c];
@@ -302,8 +255,7 @@ __device__ __forceinline__ Side<T> load_side(T const* q, int c, int dir)
     return s;
 }
 
-template <class T>
-__device__ __forceinline__ void store_flux(T* out, int stride, int idx, int dir, Flux<T> const& f)
+__device__ __forceinline__ void store_flux(double* out, int stride, int idx, int dir, Flux<double> const& f)
 {
     int const d1 = dir == 2 ? 0 : dir + 1;
     int const d2 = dir == 0 ? 2 : dir - 1;
@@ -315,24 +267,22 @@ __device__ __forceinline__ void store_flux(T* out, int stride, int idx, int dir,
 }
 
 // Per-CTA state of the tile engine that lives across work items.
-template <class T>
 struct TileCtx {
     unsigned long long* bars; // one mbarrier per slot (TMA ring)
-    T* smem;                  // plane slots
-    T* fx;                    // x-face fluxes (5 fields)
-    T* fy;                    // y-face fluxes
-    T* fz;                    // z-face fluxes
+    double* smem;                  // plane slots
+    double* fx;                    // x-face fluxes (5 fields)
+    double* fy;                    // y-face fluxes
+    double* fz;                    // z-face fluxes
     unsigned phase;           // bit s: parity of slot s's next completion (TMA ring)
     unsigned inflight;        // bit s: a TMA into slot s has not been waited for
     bool timed_out;           // a bounded mbarrier wait ran out
-    long long wkey;           // ordered bits of this thread's max wavespeed (FP64)
-    unsigned wrun;            // FP64 step: the warp's running max of wavespeed estimates (WaveScreen)
-    float wmaxf;              // this thread's max wavespeed (FP32 states: keyed once, at the flush)
+    long long wkey;           // ordered bits of this thread's max wavespeed
+    unsigned wrun;            // fused step: the warp's running max of wavespeed estimates (WaveScreen)
     bool bad;                 // this thread saw a non-physical cell
 };
 
-template <class T, int NSLOT>
-__device__ __forceinline__ bool wait_slot(TileCtx<T>& c, int s)
+template <int NSLOT>
+__device__ __forceinline__ bool wait_slot(TileCtx& c, int s)
 {
     bool const ok = mbar_wait(&c.bars[s], (c.phase >> s) & 1u);
     c.phase ^= 1u << s;
@@ -341,67 +291,65 @@ __device__ __forceinline__ bool wait_slot(TileCtx<T>& c, int s)
 }
 
 // One work item: interior planes [kb, ke) of tile (tx, ty), with update
-// coefficients k0..k2 (dt/dv times the face areas).  FP64 tiles are at most
+// coefficients k0..k2 (dt/dv times the face areas).  Tiles are at most
 // TX x TY cells, cut evenly out of the grid (p.sx, p.sy), so a warp solves no
-// face and updates no cell that is not the grid's; FP32 tiles are whole.
-// Returns false when a staged plane never arrived.
-template <class T, int TX, int TY, int MODE, int STAGE, int COMP>
-__device__ __forceinline__ bool tile_item(TileCtx<T>& c, FluxParams<T> const& p, TmaMaps const& maps, T k0, T k1,
-                                          T k2, int tx, int ty, int kb, int ke)
+// face and updates no cell that is not the grid's.  Returns false when a staged plane never arrived.
+template <int TX, int TY, int MODE, int STAGE>
+__device__ __forceinline__ bool tile_item(TileCtx& c, FluxParams<double> const& p, TmaMaps const& maps, double k0, double k1,
+                                          double k2, int tx, int ty, int kb, int ke)
 {
     constexpr int NSLOT = kStageSlots<STAGE>;
-    constexpr bool kWhole = sizeof(T) == 4;
-    using L = TileLayout<T, TX, TY, NSLOT>;
+    using L = TileLayout<TX, TY, NSLOT>;
     int const tid = threadIdx.x;
     bool const cubic = p.invdx0 == p.invdx1 && p.invdx1 == p.invdx2;
-    T* const smem = c.smem;
-    T* const fx = c.fx;
-    T* const fy = c.fy;
-    T* const fz = c.fz;
+    double* const smem = c.smem;
+    double* const fx = c.fx;
+    double* const fy = c.fy;
+    double* const fz = c.fz;
 
-    int const i0 = 1 + (kWhole ? tx * TX : p.sx.start(tx));
-    int const j0 = 1 + (kWhole ? ty * TY : p.sy.start(ty));
-    TileDims const t = tile_dims(kWhole ? TX : 1 + p.sx.start(tx + 1) - i0, kWhole ? TY : 1 + p.sy.start(ty + 1) - j0);
-    int const tj = kWhole ? tid / TX : div_runtime(tid, t.mw);
-    int const ti = tid - tj * (kWhole ? TX : t.w);
+    int const i0 = 1 + p.sx.start(tx);
+    int const j0 = 1 + p.sy.start(ty);
+    TileDims const t = tile_dims(1 + p.sx.start(tx + 1) - i0, 1 + p.sy.start(ty + 1) - j0);
+    int const tj = div_runtime(tid, t.mw);
+    int const ti = tid - tj * t.w;
     int const center = (tj + 1) * L::HX + ti + 1;
     int const i = i0 + ti;
     int const j = j0 + tj;
-    bool const own = kWhole ? (i < p.g.n0 - 1) && (j < p.g.n1 - 1) : tj < t.h;
+    bool const own = tj < t.h;
 
     StageCells<kStagePerThread<TX, TY>> cells;
     if (STAGE == kStageAsync) {
-        cells = stage_cells<T, TX, TY>(p, t, i0, j0);
+        cells = stage_cells<TX, TY>(p, t, i0, j0);
     }
 
     __syncthreads(); // the previous item's readers of slots and fluxes are done
     if (STAGE == kStageTma) {
         // planes kb-1, kb, kb+1 -> slots 0, 1, 2 (kb+1 <= ke always)
         if (tid == 0) {
-            issue_plane<T, TX, TY, NSLOT>(smem, c.bars, 0, maps, i0, j0, kb - 1);
-            issue_plane<T, TX, TY, NSLOT>(smem, c.bars, 1, maps, i0, j0, kb);
-            issue_plane<T, TX, TY, NSLOT>(smem, c.bars, 2, maps, i0, j0, kb + 1);
+            issue_plane<TX, TY, NSLOT>(smem, c.bars, 0, maps, i0, j0, kb - 1);
+            issue_plane<TX, TY, NSLOT>(smem, c.bars, 1, maps, i0, j0, kb);
+            issue_plane<TX, TY, NSLOT>(smem, c.bars, 2, maps, i0, j0, kb + 1);
         }
         c.inflight |= 7u;
-        c.timed_out |= !wait_slot<T, NSLOT>(c, 0);
-        c.timed_out |= !wait_slot<T, NSLOT>(c, 1);
+        c.timed_out |= !wait_slot<NSLOT>(c, 0);
+        c.timed_out |= !wait_slot<NSLOT>(c, 1);
     } else if constexpr (STAGE == kStageAsync) {
         for (int s = 0; s < NSLOT; ++s) {
-            issue_plane_async<T, TX, TY, NSLOT>(smem, s, p, cells, kb - 1 + s);
+            issue_plane_async<TX, TY, NSLOT>(smem, s, p, cells, kb - 1 + s);
         }
         asm volatile("cp.async.wait_all;" ::: "memory");
         __syncthreads();
     } else {
-        load_plane<T, TX, TY, NSLOT, MODE, COMP>(smem, 0, p, t, i0, j0, kb - 1);
-        load_plane<T, TX, TY, NSLOT, MODE, COMP>(smem, 1, p, t, i0, j0, kb);
+        load_plane<TX, TY, NSLOT>(smem, 0, p, t, i0, j0, kb - 1);
+        load_plane<TX, TY, NSLOT>(smem, 1, p, t, i0, j0, kb);
         __syncthreads();
     }
     // z face below the chunk's first plane, kept in registers in global
     // axes (the z face frame has n = mx2, t1 = mx0, t2 = mx1)
-    T zlo[5] = {T(0), T(0), T(0), T(0), T(0)};
-    if (kWhole || own) {
-        Flux<T> const f0 = hllc_flux(load_side<T, L::PLANE_PAD>(slot_field<T, TX, TY, NSLOT>(smem, 0, 0), center, 2),
-                                     load_side<T, L::PLANE_PAD>(slot_field<T, TX, TY, NSLOT>(smem, 1, 0), center, 2));
+    double zlo[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+    if (own) {
+        Flux<double> const f0 = hllc_flux(load_side<L::PLANE_PAD>(slot_field<TX, TY, NSLOT>(smem, 0, 0), center, 2),
+                                     load_side<L::PLANE_PAD>(slot_field<TX, TY, NSLOT>(smem, 1, 0), center, 2));
         zlo[0] = f0.d;
         zlo[1] = f0.e;
         zlo[2] = f0.t1;
@@ -414,23 +362,23 @@ __device__ __forceinline__ bool tile_item(TileCtx<T>& c, FluxParams<T> const& p,
     if (STAGE == kStageTma) {
         if (kb + 2 <= ke) {
             if (tid == 0) {
-                issue_plane<T, TX, TY, NSLOT>(smem, c.bars, 0, maps, i0, j0, kb + 2);
+                issue_plane<TX, TY, NSLOT>(smem, c.bars, 0, maps, i0, j0, kb + 2);
             }
             c.inflight |= 1u;
         }
     } else if constexpr (STAGE == kStageAsync) {
         if (kb + 2 <= ke) {
-            issue_plane_async<T, TX, TY, NSLOT>(smem, 0, p, cells, kb + 2);
+            issue_plane_async<TX, TY, NSLOT>(smem, 0, p, cells, kb + 2);
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     }
-    int const nfx = (t.w + 1) * t.h; // FP64: the faces of each family
+    int const nfx = (t.w + 1) * t.h; // the faces of each family
     int const nfy = t.w * (t.h + 1);
     int const nface = nfx + nfy + t.w * t.h;
 
-    // FP64 step: the next step's CFL wavespeed is screened (WaveScreen); the
+    // fused step: the next step's CFL wavespeed is screened (WaveScreen); the
     // running max carries over from the CTA's previous item of the same grid
-    constexpr bool kScreen = sizeof(T) == 8 && MODE == kModeStep;
+    constexpr bool kScreen = MODE == kModeStep;
     WaveScreen screen(p.gamma, p.invdx0, p.invdx1, p.invdx2);
     screen.run = c.wrun;
 
@@ -438,79 +386,39 @@ __device__ __forceinline__ bool tile_item(TileCtx<T>& c, FluxParams<T> const& p,
         int const cur = (k - kb + 1) % NSLOT;
         int const nxt = (k - kb + 2) % NSLOT;
         // this cell's conservative state, fetched while the faces are solved
-        T u[5];
-        T ulo[5] = {T(0), T(0), T(0), T(0), T(0)};
+        double u[5];
         long long const o = p.g.at(i, j, k);
         if (own) {
 #pragma unroll
             for (int f = 0; f < 5; ++f) {
                 u[f] = p.cons_in.f[f][o];
-                if (COMP == kCompHiLo) {
-                    ulo[f] = p.lo_in.f[f][o];
-                }
             }
         }
         if (STAGE == kStageTma) {
-            c.timed_out |= !wait_slot<T, NSLOT>(c, nxt);
+            c.timed_out |= !wait_slot<NSLOT>(c, nxt);
         } else if (STAGE == kStageLoad) {
-            load_plane<T, TX, TY, NSLOT, MODE, COMP>(smem, nxt, p, t, i0, j0, k + 1);
+            load_plane<TX, TY, NSLOT>(smem, nxt, p, t, i0, j0, k + 1);
             __syncthreads();
         }
 
         // ---- face phase
-        T const* qc = slot_field<T, TX, TY, NSLOT>(smem, cur, 0);
-        T const* qn = slot_field<T, TX, TY, NSLOT>(smem, nxt, 0);
-        if constexpr (sizeof(T) == 8) {
-            // FP64 (bound by the FP64 pipe): one index space over the three
-            // families; each face's family, left cell and right cell are
-            // chosen by selects, so a warp that straddles two families still
-            // runs the HLLC once
-            for (int f = tid; f < nface; f += L::NT) {
-                bool const is_x = f < nfx;
-                bool const is_y = !is_x && f < nfx + nfy;
-                int const g = is_x ? f : (is_y ? f - nfx : f - nfx - nfy);
-                int const gj = div_runtime(g, is_x ? t.mw1 : t.mw);
-                int const gi = g - gj * (is_x ? t.w + 1 : t.w);
-                int const a = (is_y ? gj : gj + 1) * L::HX + (is_x ? gi : gi + 1);
-                int const dir = is_x ? 0 : (is_y ? 1 : 2);
-                T const* const qr = is_x || is_y ? qc : qn;
-                int const ar = a + (is_x ? 1 : (is_y ? L::HX : 0));
-                store_flux(is_x ? fx : (is_y ? fy : fz), is_x ? L::NFX : (is_y ? L::NFY : L::NFZ), g, dir,
-                           hllc_flux(load_side<T, L::PLANE_PAD>(qc, a, dir), load_side<T, L::PLANE_PAD>(qr, ar, dir)));
-            }
-        } else {
-            // FP32 (bound by instruction issue, where the selects above cost
-            // more than they save): each family in its own warp-aligned
-            // index range, with compile-time axes
-            for (int f = tid; f < L::NFACE_W; f += L::NT) {
-                if (f < L::NFX_W) {
-                    if (f < L::NFX) {
-                        int const fj = f / (TX + 1);
-                        int const fi = f % (TX + 1);
-                        int const a = (fj + 1) * L::HX + fi;
-                        store_flux(fx, L::NFX, f, 0,
-                                   hllc_flux(load_side<T, L::PLANE_PAD>(qc, a, 0),
-                                             load_side<T, L::PLANE_PAD>(qc, a + 1, 0)));
-                    }
-                } else if (f < L::NFX_W + L::NFY_W) {
-                    int const g = f - L::NFX_W;
-                    if (g < L::NFY) {
-                        int const fj = g / TX;
-                        int const fi = g % TX;
-                        int const a = fj * L::HX + fi + 1;
-                        store_flux(fy, L::NFY, g, 1,
-                                   hllc_flux(load_side<T, L::PLANE_PAD>(qc, a, 1),
-                                             load_side<T, L::PLANE_PAD>(qc, a + L::HX, 1)));
-                    }
-                } else {
-                    int const g = f - L::NFX_W - L::NFY_W; // < NFZ
-                    int const fj = g / TX;
-                    int const fi = g % TX;
-                    int const a = (fj + 1) * L::HX + fi + 1;
-                    store_flux(fz, L::NFZ, g, 2,
-                               hllc_flux(load_side<T, L::PLANE_PAD>(qc, a, 2), load_side<T, L::PLANE_PAD>(qn, a, 2)));
-                }
-            }
+        double const* qc = slot_field<TX, TY, NSLOT>(smem, cur, 0);
+        double const* qn = slot_field<TX, TY, NSLOT>(smem, nxt, 0);
+        // one index space over the three families; each face's family, left
+        // cell and right cell are chosen by selects, so a warp that straddles
+        // two families still runs the HLLC once
+        for (int f = tid; f < nface; f += L::NT) {
+            bool const is_x = f < nfx;
+            bool const is_y = !is_x && f < nfx + nfy;
+            int const g = is_x ? f : (is_y ? f - nfx : f - nfx - nfy);
+            int const gj = div_runtime(g, is_x ? t.mw1 : t.mw);
+            int const gi = g - gj * (is_x ? t.w + 1 : t.w);
+            int const a = (is_y ? gj : gj + 1) * L::HX + (is_x ? gi : gi + 1);
+            int const dir = is_x ? 0 : (is_y ? 1 : 2);
+            double const* const qr = is_x || is_y ? qc : qn;
+            int const ar = a + (is_x ? 1 : (is_y ? L::HX : 0));
+            store_flux(is_x ? fx : (is_y ? fy : fz), is_x ? L::NFX : (is_y ? L::NFY : L::NFZ), g, dir,
+                       hllc_flux(load_side<L::PLANE_PAD>(qc, a, dir), load_side<L::PLANE_PAD>(qr, ar, dir)));
         }
         if (__syncthreads_or(c.timed_out)) {
             return false;
@@ -519,112 +427,66 @@ __device__ __forceinline__ bool tile_item(TileCtx<T>& c, FluxParams<T> const& p,
         if (STAGE == kStageTma) {
             if (k + 3 <= ke) {
                 if (tid == 0) {
-                    issue_plane<T, TX, TY, NSLOT>(smem, c.bars, cur, maps, i0, j0, k + 3);
+                    issue_plane<TX, TY, NSLOT>(smem, c.bars, cur, maps, i0, j0, k + 3);
                 }
                 c.inflight |= 1u << cur;
             }
         } else if constexpr (STAGE == kStageAsync) {
             if (k + 3 <= ke) {
-                issue_plane_async<T, TX, TY, NSLOT>(smem, cur, p, cells, k + 3);
+                issue_plane_async<TX, TY, NSLOT>(smem, cur, p, cells, k + 3);
             }
             asm volatile("cp.async.commit_group;" ::: "memory");
         }
 
         // ---- cell phase
-        T fza[5];
+        double fza[5];
 #pragma unroll
         for (int f = 0; f < 5; ++f) {
             fza[f] = fz[f * L::NFZ + tid];
         }
-        T wv[4] = {T(0), T(0), T(0), T(0)}; // FP64 step: the new cs, v0, v1, v2, for the screened wavespeed
+        double wv[4] = {0.0, 0.0, 0.0, 0.0}; // fused step: the new cs, v0, v1, v2, for the screened wavespeed
         if (own) {
-            int const tw = kWhole ? TX : t.w;
-            int const xl = tj * (tw + 1) + ti;
-            int const yb = tj * tw + ti;
+            int const xl = tj * (t.w + 1) + ti;
+            int const yb = tj * t.w + ti;
 #pragma unroll
             for (int f = 0; f < 5; ++f) {
-                if (COMP == kCompNone) {
-                    T const ax = fx[f * L::NFX + xl + 1] - fx[f * L::NFX + xl];
-                    T const ay = fy[f * L::NFY + yb + tw] - fy[f * L::NFY + yb];
-                    T const az = fza[f] - zlo[f];
-                    u[f] = u[f] - k0 * ax - k1 * ay - k2 * az;
-                } else {
-                    // cons + six signed face terms, summed without
-                    // intermediate rounding error (TwoProduct + TwoSum),
-                    // then rounded once
-                    T sum = u[f];
-                    T err = ulo[f];
-                    compensated_add(sum, err, -k0, fx[f * L::NFX + xl + 1]);
-                    compensated_add(sum, err, k0, fx[f * L::NFX + xl]);
-                    compensated_add(sum, err, -k1, fy[f * L::NFY + yb + TX]);
-                    compensated_add(sum, err, k1, fy[f * L::NFY + yb]);
-                    compensated_add(sum, err, -k2, fza[f]);
-                    compensated_add(sum, err, k2, zlo[f]);
-                    u[f] = sum + err;
-                    ulo[f] = err - (u[f] - sum);
-                }
+                double const ax = fx[f * L::NFX + xl + 1] - fx[f * L::NFX + xl];
+                double const ay = fy[f * L::NFY + yb + t.w] - fy[f * L::NFY + yb];
+                double const az = fza[f] - zlo[f];
+                u[f] = u[f] - k0 * ax - k1 * ay - k2 * az;
             }
 #pragma unroll
             for (int f = 0; f < 5; ++f) {
                 p.cons_out.f[f][o] = u[f];
-                if (COMP == kCompHiLo) {
-                    p.lo_out.f[f][o] = ulo[f];
-                }
             }
-            if (MODE == kModeStep || MODE == kModeStepCons) {
+            if constexpr (MODE == kModeStep) {
                 // cons_to_prim of the new state (cons_to_prim.hpp:26-31)
-                T const r = rcp_faithful(u[0]); // FP32: correctly rounded
-                T const v0 = u[2] * r;
-                T const v1 = u[3] * r;
-                T const v2 = u[4] * r;
-                T pr;
-                if (MODE == kModeStep) {
-                    T const mv = u[2] * v0 + u[3] * v1 + u[4] * v2; // |m|^2 / rho
-                    pr = p.gm1 * u[1] - p.half_gm1 * mv;              // (gamma-1)(e - |m|^2/(2 rho))
-                } else {
-                    pr = cons_pressure<COMP>(u[0], u[1], u[2], u[3], u[4], r, p.gm1, COMP == kCompHiLo ? ulo : nullptr);
+                double const r = rcp_faithful(u[0]);
+                double const v0 = u[2] * r;
+                double const v1 = u[3] * r;
+                double const v2 = u[4] * r;
+                double const mv = u[2] * v0 + u[3] * v1 + u[4] * v2;   // |m|^2 / rho
+                double const pr = p.gm1 * u[1] - p.half_gm1 * mv;      // (gamma-1)(e - |m|^2/(2 rho))
+                double const cs = fast_sound_speed((p.gamma * r) * pr);
+                p.h_out[o] = u[1] + pr; // staged as e + p at the next step
+                p.prim_out.f[0][o] = u[0];
+                p.prim_out.f[1][o] = pr;
+                p.prim_out.f[2][o] = v0;
+                p.prim_out.f[3][o] = v1;
+                p.prim_out.f[4][o] = v2;
+                if (p.prim_rec.f[0] != nullptr) { // a second copy, for a recording caller
+                    p.prim_rec.f[0][o] = u[0];
+                    p.prim_rec.f[1][o] = pr;
+                    p.prim_rec.f[2][o] = v0;
+                    p.prim_rec.f[3][o] = v1;
+                    p.prim_rec.f[4][o] = v2;
                 }
-                T const cs = fast_sound_speed((p.gamma * r) * pr);
-                if (MODE == kModeStep) {
-                    if constexpr (sizeof(T) == 8) {
-                        if (p.h_out != nullptr) {
-                            p.h_out[o] = u[1] + pr; // staged by TMA at the next step
-                        }
-                    }
-                    p.prim_out.f[0][o] = u[0];
-                    p.prim_out.f[1][o] = pr;
-                    p.prim_out.f[2][o] = v0;
-                    p.prim_out.f[3][o] = v1;
-                    p.prim_out.f[4][o] = v2;
-                    if (p.prim_rec.f[0] != nullptr) { // a second copy, for a recording caller
-                        p.prim_rec.f[0][o] = u[0];
-                        p.prim_rec.f[1][o] = pr;
-                        p.prim_rec.f[2][o] = v0;
-                        p.prim_rec.f[3][o] = v1;
-                        p.prim_rec.f[4][o] = v2;
-                    }
-                    p.cs_out[o] = cs;
-                }
-                if constexpr (kScreen) {
-                    wv[0] = cs;
-                    wv[1] = v0;
-                    wv[2] = v1;
-                    wv[3] = v2;
-                    c.bad |= !(finite_positive(u[0]) && finite_positive(pr)); // the wavespeed is checked below
-                } else {
-                    // next step's CFL wavespeed (time_step.hpp:28-33)
-                    // (cubic cells: one product instead of three)
-                    T const invdt = cubic ? (T(3) * cs + abs_(v0) + abs_(v1) + abs_(v2)) * p.invdx0
-                                          : (cs + abs_(v0)) * p.invdx0 + (cs + abs_(v1)) * p.invdx1 +
-                                                    (cs + abs_(v2)) * p.invdx2;
-                    if constexpr (sizeof(T) == 4) {
-                        c.wmaxf = fmaxf(c.wmaxf, invdt); // NaN never wins (fmaxf returns the other operand)
-                    } else {
-                        long long const key = wave_key(invdt);
-                        c.wkey = key > c.wkey ? key : c.wkey;
-                    }
-                    c.bad |= !cell_ok(u[0], pr, invdt);
-                }
+                p.cs_out[o] = cs;
+                wv[0] = cs;
+                wv[1] = v0;
+                wv[2] = v1;
+                wv[3] = v2;
+                c.bad |= !(finite_positive(u[0]) && finite_positive(pr)); // the wavespeed is checked below
             }
         }
         if constexpr (kScreen) {
@@ -634,7 +496,7 @@ __device__ __forceinline__ bool tile_item(TileCtx<T>& c, FluxParams<T> const& p,
             // Every lane of the warp is here (the screen is warp-collective);
             // a non-finite wavespeed always takes the FP64 branch.
             if (screen.step_exact_needed(own, wv[0], wv[1], wv[2], wv[3], cubic)) {
-                T const invdt = cubic ? (T(3) * wv[0] + abs_(wv[1]) + abs_(wv[2]) + abs_(wv[3])) * p.invdx0
+                double const invdt = cubic ? (3.0 * wv[0] + abs_(wv[1]) + abs_(wv[2]) + abs_(wv[3])) * p.invdx0
                                       : (wv[0] + abs_(wv[1])) * p.invdx0 + (wv[0] + abs_(wv[2])) * p.invdx1 +
                                                 (wv[0] + abs_(wv[3])) * p.invdx2;
                 long long const key = wave_key(invdt);
@@ -658,17 +520,13 @@ __device__ __forceinline__ bool tile_item(TileCtx<T>& c, FluxParams<T> const& p,
 
 // Block-wide max of the threads' wavespeed keys into *wmax, and the
 // non-physical flag into *status; clears the per-thread values.
-template <class T, int NT>
-__device__ __forceinline__ void flush_wavespeed(TileCtx<T>& c, unsigned long long* wmax, int* status)
+template <int NT>
+__device__ __forceinline__ void flush_wavespeed(TileCtx& c, unsigned long long* wmax, int* status)
 {
     __shared__ long long warp_best[NT / 32];
     __shared__ int any_bad;
     int const tid = threadIdx.x;
     long long w = c.wkey;
-    if constexpr (sizeof(T) == 4) {
-        long long const kf = wave_key(c.wmaxf);
-        w = kf > w ? kf : w;
-    }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         long long const v = __shfl_xor_sync(0xffffffffu, w, o);
@@ -699,19 +557,18 @@ __device__ __forceinline__ void flush_wavespeed(TileCtx<T>& c, unsigned long lon
     }
     c.wkey = 0;
     c.wrun = 0u; // the next item may be another grid's
-    c.wmaxf = 0.0f;
     c.bad = false;
 }
 
-template <class T, int TX, int TY, int NSLOT>
-__device__ __forceinline__ TileCtx<T> make_ctx(unsigned char* smem_dyn)
+template <int TX, int TY, int NSLOT>
+__device__ __forceinline__ TileCtx make_ctx(unsigned char* smem_dyn)
 {
-    using L = TileLayout<T, TX, TY, NSLOT>;
+    using L = TileLayout<TX, TY, NSLOT>;
     // TMA destinations must sit on 128-byte boundaries of the shared window
     unsigned char* raw = smem_dyn + ((128u - (smem_u32(smem_dyn) & 127u)) & 127u);
-    TileCtx<T> c;
+    TileCtx c;
     c.bars = reinterpret_cast<unsigned long long*>(raw);
-    c.smem = reinterpret_cast<T*>(raw + L::MBAR_BYTES);
+    c.smem = reinterpret_cast<double*>(raw + L::MBAR_BYTES);
     c.fx = c.smem + L::FX_OFF;
     c.fy = c.smem + L::FY_OFF;
     c.fz = c.smem + L::FZ_OFF;
@@ -720,22 +577,20 @@ __device__ __forceinline__ TileCtx<T> make_ctx(unsigned char* smem_dyn)
     c.timed_out = false;
     c.wkey = 0;
     c.wrun = 0u;
-    c.wmaxf = 0.0f;
     c.bad = false;
     return c;
 }
 
-template <class T, int TX, int TY, int MODE, int STAGE, int COMP>
-__global__ void __launch_bounds__(TX* TY) flux_tile_kernel(const __grid_constant__ FluxParams<T> p,
+template <int TX, int TY, int MODE, int STAGE>
+__global__ void __launch_bounds__(TX* TY, 2) flux_tile_kernel(const __grid_constant__ FluxParams<double> p,
                                                            const __grid_constant__ TmaMaps maps)
 {
-    static_assert(COMP == kCompNone || (sizeof(T) == 4 && MODE == kModeStepCons), "compensation is for the FP32 step");
     constexpr int NSLOT = kStageSlots<STAGE>;
     extern __shared__ __align__(128) unsigned char smem_dyn[];
-    TileCtx<T> c = make_ctx<T, TX, TY, NSLOT>(smem_dyn);
-    T const dtodv = dt_over_dv(p);
+    TileCtx c = make_ctx<TX, TY, NSLOT>(smem_dyn);
+    double const dtodv = dt_over_dv(p);
     // cons -= dt/dv * sum_d ds_d (F_R - F_L), coefficients folded
-    T const k0 = dtodv * p.ds0, k1 = dtodv * p.ds1, k2 = dtodv * p.ds2;
+    double const k0 = dtodv * p.ds0, k1 = dtodv * p.ds1, k2 = dtodv * p.ds2;
 
     if (STAGE == kStageTma) {
         if (threadIdx.x == 0) {
@@ -747,29 +602,20 @@ __global__ void __launch_bounds__(TX* TY) flux_tile_kernel(const __grid_constant
         __syncthreads();
     }
 
-    if constexpr (sizeof(T) == 8) {
-        // CTA b's share of all tiles' planes, counted tile by tile: a run of
-        // planes up one tile, and on into the next
-        int const iz = p.g.n2 - 2;
-        long long w = static_cast<long long>(p.nwork) * blockIdx.x / gridDim.x;
-        long long const end = static_cast<long long>(p.nwork) * (blockIdx.x + 1) / gridDim.x;
-        while (w < end) {
-            int const tile = static_cast<int>(w) / iz;
-            int const k = static_cast<int>(w) - tile * iz;
-            int const run = static_cast<int>(min(end - w, static_cast<long long>(iz - k)));
-            if (!tile_item<T, TX, TY, MODE, STAGE, COMP>(c, p, maps, k0, k1, k2, tile % p.tiles_x, tile / p.tiles_x,
-                                                         1 + k, 1 + k + run)) {
-                break;
-            }
-            w += run;
+    // CTA b's share of all tiles' planes, counted tile by tile: a run of
+    // planes up one tile, and on into the next
+    int const iz = p.g.n2 - 2;
+    int w = static_cast<int>(static_cast<long long>(p.nwork) * blockIdx.x / gridDim.x);
+    int const end = static_cast<int>(static_cast<long long>(p.nwork) * (blockIdx.x + 1) / gridDim.x);
+    while (w < end) {
+        int const tile = w / iz;
+        int const k = w - tile * iz;
+        int const run = min(end - w, iz - k);
+        if (!tile_item<TX, TY, MODE, STAGE>(c, p, maps, k0, k1, k2, tile % p.tiles_x, tile / p.tiles_x, 1 + k,
+                                               1 + k + run)) {
+            break;
         }
-    } else {
-        int const tiles_xy = p.tiles_x * p.tiles_y;
-        for (int w = blockIdx.x; w < p.nwork; w += gridDim.x) {
-            int const kb = 1 + w / tiles_xy * p.kchunk;
-            tile_item<T, TX, TY, MODE, STAGE, COMP>(c, p, maps, k0, k1, k2, w % p.tiles_x, (w / p.tiles_x) % p.tiles_y,
-                                                    kb, min(kb + p.kchunk, p.g.n2 - 1));
-        }
+        w += run;
     }
 
     if (STAGE == kStageTma && __syncthreads_or(c.timed_out)) {
@@ -780,14 +626,14 @@ __global__ void __launch_bounds__(TX* TY) flux_tile_kernel(const __grid_constant
         }
         for (int s = 0; s < NSLOT; ++s) {
             if (c.inflight & (1u << s)) {
-                wait_slot<T, NSLOT>(c, s);
+                wait_slot<NSLOT>(c, s);
             }
         }
         step_done(p); // the launch still counts this CTA, so the next launch starts from zero
         return;
     }
-    if (MODE == kModeStep || MODE == kModeStepCons) {
-        flush_wavespeed<T, TX * TY>(c, p.wmax, p.status);
+    if (MODE == kModeStep) {
+        flush_wavespeed<TX * TY>(c, p.wmax, p.status);
         step_done(p);
     }
 }
@@ -796,19 +642,17 @@ __global__ void __launch_bounds__(TX* TY) flux_tile_kernel(const __grid_constant
 // (grid, tile, chunk) items from a global queue (largest grids first),
 // copies the item's grid parameters to shared memory and runs the same tile
 // engine; each item's wavespeed goes to its own grid's accumulator, so every
-// grid keeps its own dt.  No TMA (grids of any shape): the FP64 state stages
-// by cp.async, the FP32 states by plain loads.
-template <class T, int TX, int TY, int MODE, int COMP>
-__global__ void __launch_bounds__(TX* TY) flux_batch_kernel(const __grid_constant__ BatchParams<T> b)
+// grid keeps its own dt.  Staging by cp.async (grids of any shape).
+template <int TX, int TY>
+__global__ void __launch_bounds__(TX* TY) flux_batch_kernel(const __grid_constant__ BatchParams<double> b)
 {
-    constexpr int STAGE = sizeof(T) == 8 ? kStageAsync : kStageLoad;
-    constexpr int NSLOT = kStageSlots<STAGE>;
+    constexpr int NSLOT = kStageSlots<kStageAsync>;
     constexpr int NT = TX * TY;
-    static_assert(sizeof(FluxParams<T>) % 4 == 0, "parameter copy in 4-byte words");
+    static_assert(sizeof(FluxParams<double>) % 4 == 0, "parameter copy in 4-byte words");
     extern __shared__ __align__(128) unsigned char smem_dyn[];
-    __shared__ __align__(16) FluxParams<T> gp;
+    __shared__ __align__(16) FluxParams<double> gp;
     __shared__ int s_item;
-    TileCtx<T> c = make_ctx<T, TX, TY, NSLOT>(smem_dyn);
+    TileCtx c = make_ctx<TX, TY, NSLOT>(smem_dyn);
     int const tid = threadIdx.x;
     for (;;) {
         __syncthreads(); // everyone is done with the previous item's parameters
@@ -821,16 +665,16 @@ __global__ void __launch_bounds__(TX* TY) flux_batch_kernel(const __grid_constan
             break;
         }
         int4 const it = b.items[item];
-        for (int w = tid; w < static_cast<int>(sizeof(FluxParams<T>) / 4); w += NT) {
+        for (int w = tid; w < static_cast<int>(sizeof(FluxParams<double>) / 4); w += NT) {
             reinterpret_cast<int*>(&gp)[w] = reinterpret_cast<const int*>(&b.grids[it.x])[w];
         }
         __syncthreads();
-        T const dtodv = dt_over_dv(gp);
-        T const k0 = dtodv * gp.ds0, k1 = dtodv * gp.ds1, k2 = dtodv * gp.ds2;
+        double const dtodv = dt_over_dv(gp);
+        double const k0 = dtodv * gp.ds0, k1 = dtodv * gp.ds1, k2 = dtodv * gp.ds2;
         int const kb = 1 + it.w * gp.kchunk;
-        tile_item<T, TX, TY, MODE, STAGE, COMP>(c, gp, TmaMaps{}, k0, k1, k2, it.y, it.z, kb,
-                                                min(kb + gp.kchunk, gp.g.n2 - 1));
-        flush_wavespeed<T, NT>(c, gp.wmax, gp.status);
+        tile_item<TX, TY, kModeStep, kStageAsync>(c, gp, TmaMaps{}, k0, k1, k2, it.y, it.z, kb,
+                                                     min(kb + gp.kchunk, gp.g.n2 - 1));
+        flush_wavespeed<NT>(c, gp.wmax, gp.status);
         item_done(gp);
     }
     batch_cta_done(b);
@@ -960,21 +804,12 @@ __global__ void finalize_dt_kernel(SimScalars* s, T cfl, int add_time, const dou
     }
 }
 
-// The single-grid tile, at most.  FP64: 16x16 columns, whose 800 faces per
-// plane fill exactly 25 warp-passes (a 32x8 tile's 808 need 26) with the same
-// 256 threads, 18x18 TMA boxes and two resident CTAs per SM.  (A 16x8 kernel
-// with four CTAs of 128 threads per SM measured 33.2 ms a 512^3 step against
-// 32.9, and no better on small grids.)  FP32 (the state
-// with stored low words; the other FP32 states run the column engine):
-// 32x8, measured faster there (26.9 against 21.9 Gcell/s at 512^3).
-template <class T>
-struct StepTile {
-    static constexpr int X = 16, Y = 16;
-};
-template <>
-struct StepTile<float> {
-    static constexpr int X = 32, Y = 8;
-};
+// The single-grid tile, at most: 16x16 columns, whose 800 faces per plane
+// fill exactly 25 warp-passes (a 32x8 tile's 808 need 26) with the same 256
+// threads, 18x18 TMA boxes and two resident CTAs per SM.  (A 16x8 kernel with
+// four CTAs of 128 threads per SM measured 33.2 ms a 512^3 step against 32.9,
+// and no better on small grids.)
+constexpr int kStepTX = 16, kStepTY = 16;
 
 // Tiles per axis of a single-grid FP64 launch.
 struct TilePlan {
@@ -996,13 +831,12 @@ struct TilePlan {
 // 48^3 97 -> 46, 64^3 97 -> 86, 99 x 128 x 75 311 -> 270.
 TilePlan choose_tiles(int ix, int iy, int iz, int sms, int per_sm, bool step, int q)
 {
-    constexpr int kTX = StepTile<double>::X, kTY = StepTile<double>::Y;
     constexpr double kInstr = 9.0e-3, kWait2 = 1.1, kWait1 = 1.6; // us
     int const units = (ix + q - 1) / q;
     TilePlan best{};
     double best_us = 1e300;
     int last_nx = 0;
-    for (int w = kTX / q; w >= 1; --w) {
+    for (int w = kStepTX / q; w >= 1; --w) {
         int const nx = (units + w - 1) / w;
         int const tw = (units + nx - 1) / nx * q;
         if (nx == last_nx) {
@@ -1010,7 +844,7 @@ TilePlan choose_tiles(int ix, int iy, int iz, int sms, int per_sm, bool step, in
         }
         last_nx = nx;
         int last_ny = 0;
-        for (int h = kTY; h >= 1; --h) {
+        for (int h = kStepTY; h >= 1; --h) {
             int const ny = (iy + h - 1) / h;
             int const th = (iy + ny - 1) / ny;
             if (ny == last_ny) {
@@ -1035,80 +869,62 @@ TilePlan choose_tiles(int ix, int iy, int iz, int sms, int per_sm, bool step, in
     return best;
 }
 
-template <class T, int MODE, int STAGE, int COMP>
+template <int MODE, int STAGE>
 struct FluxKernel {
-    static constexpr int TX = StepTile<T>::X, TY = StepTile<T>::Y;
-    using L = TileLayout<T, TX, TY, kStageSlots<STAGE>>;
-    static auto fn() { return flux_tile_kernel<T, TX, TY, MODE, STAGE, COMP>; }
-};
+    using L = TileLayout<kStepTX, kStepTY, kStageSlots<STAGE>>;
+    static auto fn() { return flux_tile_kernel<kStepTX, kStepTY, MODE, STAGE>; }
 
-// Opts the kernel into its dynamic shared memory size and returns its
-// resident CTAs per SM.  Called outside any stream capture (by the entry
-// points before they enqueue work), and cheap to repeat.
-template <class T, int MODE, int STAGE, int COMP>
-cudaError_t configure_flux_impl(int* per_sm)
-{
-    using K = FluxKernel<T, MODE, STAGE, COMP>;
-    auto kern = K::fn();
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(K::L::BYTES));
-    if (e != cudaSuccess) {
-        return e;
+    // Opts the kernel into its dynamic shared memory size and returns its
+    // resident CTAs per SM.  Called outside any stream capture (by the entry
+    // points before they enqueue work), and cheap to repeat.
+    static cudaError_t configure(int* per_sm)
+    {
+        cudaError_t e = cudaFuncSetAttribute(fn(), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             static_cast<int>(L::BYTES));
+        if (e != cudaSuccess) {
+            return e;
+        }
+        int n = 0;
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn(), L::NT, L::BYTES);
+        if (e != cudaSuccess) {
+            return e;
+        }
+        *per_sm = n < 1 ? 1 : n;
+        return cudaSuccess;
     }
-    int n = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, K::L::NT, K::L::BYTES);
-    if (e != cudaSuccess) {
-        return e;
-    }
-    *per_sm = n < 1 ? 1 : n;
-    return cudaSuccess;
-}
 
-template <class T, int MODE, int STAGE, int COMP>
-cudaError_t launch_flux_impl(FluxParams<T> p, TmaMaps const& maps, int sms, cudaStream_t s)
-{
-    using K = FluxKernel<T, MODE, STAGE, COMP>;
-    int const per_sm = p.per_sm > 0 ? p.per_sm : 1;
-    int const ix = p.g.n0 - 2;
-    int const iy = p.g.n1 - 2;
-    int const iz = p.g.n2 - 2;
-    if (ix <= 0 || iy <= 0 || iz <= 0) {
-        return cudaSuccess; // no interior cell
-    }
-    long long const slots = static_cast<long long>(sms) * per_sm;
-    if constexpr (sizeof(T) == 8) {
+    static cudaError_t launch(FluxParams<double> p, TmaMaps const& maps, int sms, cudaStream_t s)
+    {
+        int const per_sm = p.per_sm > 0 ? p.per_sm : 1;
+        int const ix = p.g.n0 - 2;
+        int const iy = p.g.n1 - 2;
+        int const iz = p.g.n2 - 2;
+        if (ix <= 0 || iy <= 0 || iz <= 0) {
+            return cudaSuccess; // no interior cell
+        }
         int const q = STAGE == kStageTma ? 2 : 1;
         TilePlan const plan = choose_tiles(ix, iy, iz, sms, per_sm, MODE == kModeStep, q);
         p.sx = split_tiles(ix, plan.nx, q);
         p.sy = split_tiles(iy, plan.ny, 1);
         p.tiles_x = plan.nx;
         p.tiles_y = plan.ny;
-        p.kchunk = 1; // the kernel divides the planes themselves among its CTAs
-    } else {
-        p.tiles_x = (ix + K::TX - 1) / K::TX;
-        p.tiles_y = (iy + K::TY - 1) / K::TY;
-        p.kchunk = choose_kchunk(p.tiles_x * p.tiles_y, iz, slots);
+        p.nwork = plan.nx * plan.ny * iz;
+        long long const slots = static_cast<long long>(sms) * per_sm;
+        int const grid = static_cast<int>(slots < p.nwork ? slots : p.nwork);
+        fn()<<<grid, L::NT, L::BYTES, s>>>(p, maps);
+        return cudaGetLastError();
     }
-    int const kchunks = (iz + p.kchunk - 1) / p.kchunk;
-    long long const nwork = static_cast<long long>(p.tiles_x) * p.tiles_y * kchunks;
-    p.nwork = static_cast<int>(nwork);
-    long long grid = slots;
-    if (grid > nwork) {
-        grid = nwork;
-    }
-    K::fn()<<<static_cast<int>(grid), K::L::NT, K::L::BYTES, s>>>(p, maps);
-    return cudaGetLastError();
-}
+};
 
-// Tile shapes the batch kernel is built for (the autotuner picks one).  For
-// FP32 states without low words the 32 x 8 shape runs the column engine.
+// Tile shapes of the batch (the autotuner picks one); the FP32 states' column
+// engine has those of 256 columns.
 constexpr int kBatchShapes[][2] = {{32, 8}, {16, 8}, {16, 16}};
 constexpr int kNumBatchShapes = 3;
 
-template <class T, int TX, int TY, int MODE, int COMP>
+template <int TX, int TY>
 struct BatchKernel {
-    using L = TileLayout<T, TX, TY, kStageSlots<(sizeof(T) == 8 ? kStageAsync : kStageLoad)>>;
-    static auto fn() { return flux_batch_kernel<T, TX, TY, MODE, COMP>; }
+    using L = TileLayout<TX, TY, kStageSlots<kStageAsync>>;
+    static auto fn() { return flux_batch_kernel<TX, TY>; }
     static cudaError_t configure(int* per_sm)
     {
         auto kern = fn();
@@ -1122,27 +938,12 @@ struct BatchKernel {
         *per_sm = n < 1 ? 1 : n;
         return e;
     }
-    static cudaError_t launch(BatchParams<T> const& b, int grid, cudaStream_t s)
+    static cudaError_t launch(BatchParams<double> const& b, int grid, cudaStream_t s)
     {
         fn()<<<grid, L::NT, L::BYTES, s>>>(b);
         return cudaGetLastError();
     }
 };
-
-template <class T, int MODE, int COMP>
-cudaError_t batch_dispatch(int shape, BatchParams<T> const* b, int grid, int* per_sm, cudaStream_t s)
-{
-    if constexpr (sizeof(T) == 4 && COMP != kCompHiLo) {
-        if (shape == 0) { // the column engine
-            return launch_batch_f32col(COMP, b, grid, per_sm, s);
-        }
-    }
-    switch (shape) {
-    case 0: return b ? BatchKernel<T, 32, 8, MODE, COMP>::launch(*b, grid, s) : BatchKernel<T, 32, 8, MODE, COMP>::configure(per_sm);
-    case 1: return b ? BatchKernel<T, 16, 8, MODE, COMP>::launch(*b, grid, s) : BatchKernel<T, 16, 8, MODE, COMP>::configure(per_sm);
-    default: return b ? BatchKernel<T, 16, 16, MODE, COMP>::launch(*b, grid, s) : BatchKernel<T, 16, 16, MODE, COMP>::configure(per_sm);
-    }
-}
 
 } // namespace
 
@@ -1152,6 +953,7 @@ void batch_shape(int shape, int* tx, int* ty)
     *tx = kBatchShapes[shape][0];
     *ty = kBatchShapes[shape][1];
 }
+bool batch_shape_built(int shape, bool f64) { return f64 || kBatchShapes[shape][0] * kBatchShapes[shape][1] == 256; }
 
 // b == nullptr: configure (dynamic shared memory opt-in) and report the
 // resident CTAs per SM; otherwise launch `grid` persistent CTAs.
@@ -1159,13 +961,13 @@ template <class T>
 cudaError_t launch_flux_batch(int shape, int comp, BatchParams<T> const* b, int grid, int* per_sm, cudaStream_t s)
 {
     if constexpr (sizeof(T) == sizeof(double)) {
-        return batch_dispatch<double, kModeStep, kCompNone>(shape, b, grid, per_sm, s);
-    } else {
-        switch (comp) {
-        case kCompSum: return batch_dispatch<float, kModeStepCons, kCompSum>(shape, b, grid, per_sm, s);
-        case kCompHiLo: return batch_dispatch<float, kModeStepCons, kCompHiLo>(shape, b, grid, per_sm, s);
-        default: return batch_dispatch<float, kModeStepCons, kCompNone>(shape, b, grid, per_sm, s);
+        switch (shape) {
+        case 0: return b ? BatchKernel<32, 8>::launch(*b, grid, s) : BatchKernel<32, 8>::configure(per_sm);
+        case 1: return b ? BatchKernel<16, 8>::launch(*b, grid, s) : BatchKernel<16, 8>::configure(per_sm);
+        default: return b ? BatchKernel<16, 16>::launch(*b, grid, s) : BatchKernel<16, 16>::configure(per_sm);
         }
+    } else {
+        return launch_batch_f32col(comp, kBatchShapes[shape][0], b, grid, per_sm, s);
     }
 }
 
@@ -1180,21 +982,21 @@ struct FluxDispatch<double> {
     static cudaError_t configure(int mode, bool tma, int /*comp*/, int* per_sm)
     {
         if (mode == kModeStep) {
-            return tma ? configure_flux_impl<double, kModeStep, kStageTma, kCompNone>(per_sm)
-                       : configure_flux_impl<double, kModeStep, kStageAsync, kCompNone>(per_sm);
+            return tma ? FluxKernel<kModeStep, kStageTma>::configure(per_sm)
+                       : FluxKernel<kModeStep, kStageAsync>::configure(per_sm);
         }
-        return configure_flux_impl<double, kModeGodunov, kStageLoad, kCompNone>(per_sm);
+        return FluxKernel<kModeGodunov, kStageLoad>::configure(per_sm);
     }
     static cudaError_t launch(FluxParams<double> const& p, TmaMaps const* maps, int mode, int /*comp*/, int sms,
                               cudaStream_t s)
     {
         if (mode == kModeStep) {
             if (maps != nullptr) {
-                return launch_flux_impl<double, kModeStep, kStageTma, kCompNone>(p, *maps, sms, s);
+                return FluxKernel<kModeStep, kStageTma>::launch(p, *maps, sms, s);
             }
-            return launch_flux_impl<double, kModeStep, kStageAsync, kCompNone>(p, TmaMaps{}, sms, s);
+            return FluxKernel<kModeStep, kStageAsync>::launch(p, TmaMaps{}, sms, s);
         }
-        return launch_flux_impl<double, kModeGodunov, kStageLoad, kCompNone>(p, TmaMaps{}, sms, s);
+        return FluxKernel<kModeGodunov, kStageLoad>::launch(p, TmaMaps{}, sms, s);
     }
 };
 
@@ -1202,28 +1004,12 @@ template <>
 struct FluxDispatch<float> {
     static cudaError_t configure(int mode, bool /*tma*/, int comp, int* per_sm)
     {
-        if (mode == kModeStep) {
-            // the stored low words do not fit the column engine's registers: the
-            // double-float state keeps the shared-memory tile engine
-            switch (comp) {
-            case kCompSum: return configure_step_f32col(kCompSum, per_sm);
-            case kCompHiLo: return configure_flux_impl<float, kModeStepCons, kStageLoad, kCompHiLo>(per_sm);
-            default: return configure_step_f32col(kCompNone, per_sm);
-            }
-        }
-        return configure_flux_impl<float, kModeGodunov, kStageLoad, kCompNone>(per_sm);
+        return mode == kModeStep ? configure_step_f32col(comp, per_sm) : cudaSuccess;
     }
     static cudaError_t launch(FluxParams<float> const& p, TmaMaps const* /*maps*/, int mode, int comp, int sms,
                               cudaStream_t s)
     {
-        if (mode == kModeStep) {
-            switch (comp) {
-            case kCompSum: return launch_step_f32col(p, kCompSum, sms, s);
-            case kCompHiLo: return launch_flux_impl<float, kModeStepCons, kStageLoad, kCompHiLo>(p, TmaMaps{}, sms, s);
-            default: return launch_step_f32col(p, kCompNone, sms, s);
-            }
-        }
-        return launch_flux_impl<float, kModeGodunov, kStageLoad, kCompNone>(p, TmaMaps{}, sms, s);
+        return mode == kModeStep ? launch_step_f32col(p, comp, sms, s) : launch_godunov_f32(p, sms, s);
     }
 };
 
@@ -1268,8 +1054,8 @@ cudaError_t launch_finalize_dt(SimScalars* sc, T cfl, int add_time, cudaStream_t
     return cudaGetLastError();
 }
 
-int flux_tile_x() { return StepTile<double>::X; } // the FP64 step's TMA boxes
-int flux_tile_y() { return StepTile<double>::Y; }
+int flux_tile_x() { return kStepTX; } // the FP64 step's TMA boxes
+int flux_tile_y() { return kStepTY; }
 
 template cudaError_t configure_flux<double>(int, bool, int, int*);
 template cudaError_t configure_flux<float>(int, bool, int, int*);

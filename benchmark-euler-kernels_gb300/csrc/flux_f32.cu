@@ -1,6 +1,5 @@
-// The FP32 states' fused step on the column engine, single grid and batch.
-// (The FP64 step and the per-operator godunov run on the tile engine of
-// flux.cu; the FP32 state with stored low words does too.)
+// The column engine: the FP32 states' fused step, single grid and batch, and
+// the per-operator FP32 godunov.  (FP64 runs on the tile engine of flux.cu.)
 #include "euler_device.cuh"
 #include "kernels.h"
 #include "step_common.cuh"
@@ -11,28 +10,37 @@ namespace {
 
 // ------------------------------------------------- FP32 step, column engine
 // The fused step of the FP32 states (cons only in HBM) with a regular
-// face-per-thread mapping.  Thread (ti, tj) of a 32 x 8 CTA owns the column
-// (i0 + ti, j0 + tj) and marches it up z, keeping its cell's primitive state
-// of planes k and k+1 in registers.  Per plane it solves
+// face-per-thread mapping.  Thread (ti, tj) of a 256-column CTA (32 x 8,
+// 16 x 16 or 8 x 32) owns the column (i0 + ti, j0 + tj) and marches it up z,
+// keeping its cell's primitive state of planes k and k+1 in registers.  Per
+// plane it solves
 //   x: the face on its cell's left  (the right one is lane+1's, by shuffle;
-//      the tile's 8 right boundary faces are solved by the first 8 lanes of
-//      one warp and read by lane 31 from shared memory: solved in lane 31 of
-//      every warp, each would cost its warp a whole extra HLLC of issue),
+//      the tile's right boundary faces are solved by the first lanes of one
+//      warp, a row each, and read by the rows' last lanes from shared memory:
+//      solved in those lanes, each would cost its warp a whole extra HLLC of
+//      issue),
 //   y: the face below its cell      (the one above is the next row's, through
-//      shared memory; row 7 also solves the tile's top boundary faces),
+//      shared memory; the last row also solves the tile's top boundary faces),
 //   z: the face above its cell      (both sides in registers; the face below
 //      is the previous plane's).
 // Shared memory holds two slots of primitive tiles with their halo rings
 // (for the y and boundary neighbours): plane k's, read by the faces, and
-// plane k+1's, whose halo ring (threads 0..79) is staged meanwhile, so that
+// plane k+1's, whose halo ring (threads 0..NHALO-1) is staged meanwhile, so that
 // no halo conversion stands between a plane's own staging and its barrier.
 // The y fluxes and the right boundary fluxes go through shared memory too.
 // Cons of plane k+2 (own cell) and k+2 (halo ring) are prefetched with
-// cp.async a plane before they are converted.
+// cp.async a plane before they are converted; the own cell's stay in a ring
+// of three planes for the update, which in registers cost spills.
 //
-// Plain (kCompNone) and compensated (kCompSum) FP32 states; the state with
-// stored low words (kCompHiLo) keeps the shared-memory tile engine, whose
-// register budget fits them.
+// It is bound by instruction issue.  Measured (one step): compensated state
+// 70 Gcell/s at 512^3 and 67 at 256^3, plain 74 and 72, double-float 37 (27
+// on the shared-memory tile engine it had before), operator 72 (40 before).
+//
+// The state is plain FP32 (kCompNone), compensated (kCompSum), or
+// double-float (kCompHiLo: a low word per field, which only the update reads;
+// it arrives by cp.async while the faces are solved).  The per-operator
+// godunov (kCompOperator) stages the caller's prim instead of cons, updates
+// the caller's cons in place and computes no wavespeed.
 //
 // The compensated update rounds once at the scale of the state.  The state
 // word is FP32, so its own rounding, 0.5 ulp of cons per step, is the floor
@@ -53,19 +61,32 @@ namespace {
 // 256^3): the state's own rounding and the FP32 fluxes dominate it.
 namespace f32col {
 
-constexpr int TX = 32;
-constexpr int TY = 8;
-constexpr int NT = TX * TY;
-constexpr int HX = TX + 2;
-constexpr int HY = TY + 2;
-constexpr int PLANE = HX * HY; // 340
-constexpr int NHALO = 2 * TY + 2 * TX; // 80: left, right columns, bottom, top rows
-// The warp whose first TY lanes solve the tile's right boundary x faces: one
-// without halo staging (threads 0..NHALO-1) and other than the top row's warp
-// (which solves the top boundary y faces), so that no warp solves more than
-// one extra face per plane.
-constexpr int kRightWarp = 3;
-static_assert(kRightWarp * 32 >= NHALO && kRightWarp < TY - 1 && TY <= 32, "right boundary warp");
+constexpr int NT = 256;          // threads of a CTA, one column each
+constexpr int kCompOperator = 3; // the per-operator godunov
+
+// A tile of TX columns along x; a warp holds 32 / TX rows of it.
+template <int TX_>
+struct Tile {
+    static constexpr int TX = TX_;
+    static constexpr int TY = NT / TX;
+    static constexpr int HX = TX + 2;
+    static constexpr int HY = TY + 2;
+    static constexpr int PLANE = HX * HY;
+    static constexpr int NHALO = 2 * TY + 2 * TX; // left, right columns, bottom, top rows
+    // The warp whose first TY lanes solve the tile's right boundary x faces:
+    // one without halo staging (threads 0..NHALO-1) and other than the top
+    // row's warp (which solves the top boundary y faces), so that no warp
+    // solves more than one extra face per plane.
+    static constexpr int kRightWarp = 3;
+    static_assert(kRightWarp * 32 >= NHALO && kRightWarp < NT / 32 - 1 && TY <= 32 && 32 % TX == 0, "right boundary warp");
+};
+
+// The fields the engine stages: the state's cons, or the operator's prim.
+template <int COMP>
+__device__ __forceinline__ CBundle<float> const& staged(FluxParams<float> const& p)
+{
+    return COMP == kCompOperator ? p.prim : p.cons_in;
+}
 
 struct Prim7 {
     float d, p, u[3], c, e; // e: e + p, as the HLLC takes it
@@ -100,16 +121,19 @@ __device__ __forceinline__ void to_global(Flux<float> const& f, int dir, float* 
 
 // Pressure (gamma-1) (e - m.u / 2) of an FP32 conservative cell from its
 // velocities u = m / rho: the kinetic energy as m.u instead of |m|^2 / rho
-// saves the product by 1/(2 rho).  Compensated states redo the subtraction
+// saves the product by 1/(2 rho).  (Sums of products are written as the fma
+// they become here and below, so that every kernel of the engine gives the
+// same bits whatever the compiler contracts.)  Compensated states redo the subtraction
 // in FP64 where it lost more than 8 bits (pressure_f64_rescue).
 template <int COMP>
-__device__ __forceinline__ float col_pressure(Raw5 const& r, float u0, float u1, float u2, float ir, float gm1)
+__device__ __forceinline__ float col_pressure(Raw5 const& r, float u0, float u1, float u2, float ir, float gm1,
+                                              const float* lo = nullptr)
 {
-    float const eint = r.e - 0.5f * (r.m[0] * u0 + r.m[1] * u1 + r.m[2] * u2);
+    float const eint = fmaf(-0.5f, fmaf(r.m[2], u2, fmaf(r.m[1], u1, __fmul_rn(r.m[0], u0))), r.e);
     if (COMP == kCompNone || eint > kLowPressure * r.e) {
         return gm1 * eint;
     }
-    return pressure_f64_rescue(r.d, r.e, r.m[0], r.m[1], r.m[2], ir, gm1, nullptr);
+    return pressure_f64_rescue(r.d, r.e, r.m[0], r.m[1], r.m[2], ir, gm1, COMP == kCompHiLo ? lo : nullptr);
 }
 
 // Primitive state, sound speed and e + p of an FP32 conservative cell.  1/rho
@@ -120,7 +144,26 @@ template <int COMP>
 __device__ __forceinline__ Prim7 prim_of(Raw5 const& r, FluxParams<float> const& p)
 {
     Prim7 q;
-    float const ir = rcp_approx(r.d);
+    if constexpr (COMP == kCompOperator) {
+        // r holds prim (d, p, u).  The sound speed gamma p / sqrt(gamma p d):
+        // the hardware reciprocal square root and one Newton step, within
+        // 1.5 ulps of the correctly rounded sqrt(gamma p / d).
+        q.d = r.d;
+        q.p = r.e;
+        q.u[0] = r.m[0];
+        q.u[1] = r.m[1];
+        q.u[2] = r.m[2];
+        float const gp = p.gamma * r.e;
+        float const z = gp * r.d;
+        float const y = rsqrt_approx(z);
+        q.c = gp * fmaf(0.5f * y, fmaf(-z * y, y, 1.0f), y);
+        float const uu = fmaf(r.m[2], r.m[2], fmaf(r.m[1], r.m[1], __fmul_rn(r.m[0], r.m[0])));
+        q.e = __fadd_rn(fmaf(r.e, p.inv_gm1, __fmul_rn(0.5f * r.d, uu)), r.e);
+        return q;
+    }
+    // The double-float state keeps the correctly rounded 1/rho (one FMA pair
+    // more): its low words make the conversion's own rounding visible.
+    float const ir = COMP == kCompHiLo ? rcp_rn(r.d) : rcp_approx(r.d);
     q.d = r.d;
     q.u[0] = r.m[0] * ir;
     q.u[1] = r.m[1] * ir;
@@ -131,8 +174,10 @@ __device__ __forceinline__ Prim7 prim_of(Raw5 const& r, FluxParams<float> const&
     return q;
 }
 
-// A benign state for cells outside the array (no face touching one is used).
-__device__ __forceinline__ Raw5 outside() { return Raw5{1.0f, 2.5f, {0.0f, 0.0f, 0.0f}}; }
+// Keeps the compiler from turning field pointer + running offset into a
+// running 64-bit pointer per field, which would hold up to 20 registers.
+__device__ __forceinline__ void opaque(unsigned& o) { asm("" : "+r"(o)); }
+__device__ __forceinline__ void opaque(long long& o) { asm("" : "+l"(o)); }
 
 // Element offset of cell (i, j, k) in the type Off: unsigned (32-bit
 // arithmetic, one instruction fewer per address) when the grid has fewer
@@ -144,20 +189,19 @@ __device__ __forceinline__ Off cell_offset(Geom const& g, int i, int j, int k)
            static_cast<Off>(g.s2) * static_cast<Off>(k);
 }
 
+// A cell past the array's last ghost layer (a tile overhanging the grid)
+// takes the state of the nearest ghost cell: physical values, read without a
+// branch, and no face that touches such a cell is used.
 template <class Off>
-__device__ __forceinline__ Raw5 load_raw(FluxParams<float> const& p, int i, int j, int k)
+__device__ __forceinline__ Off clamped_offset(Geom const& g, int i, int j, int k)
 {
-    if (i >= p.g.n0 || j >= p.g.n1) {
-        return outside();
-    }
-    Off const o = cell_offset<Off>(p.g, i, j, k);
-    Raw5 r;
-    r.d = __ldg(p.cons_in.f[0] + o);
-    r.e = __ldg(p.cons_in.f[1] + o);
-    r.m[0] = __ldg(p.cons_in.f[2] + o);
-    r.m[1] = __ldg(p.cons_in.f[3] + o);
-    r.m[2] = __ldg(p.cons_in.f[4] + o);
-    return r;
+    return cell_offset<Off>(g, min(i, g.n0 - 1), min(j, g.n1 - 1), k);
+}
+
+template <class Off>
+__device__ __forceinline__ Raw5 load_raw(CBundle<float> const& src, Off o)
+{
+    return Raw5{__ldg(src.f[0] + o), __ldg(src.f[1] + o), {__ldg(src.f[2] + o), __ldg(src.f[3] + o), __ldg(src.f[4] + o)}};
 }
 
 // Asynchronous 4-byte global->shared copies (cp.async): the prefetched cons
@@ -172,18 +216,23 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 // All of this thread's copy groups but the last committed one have landed.
 __device__ __forceinline__ void cp_async_wait_all_but_last() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
 
-// Starts copying the cons of cell (i, j, k) to dst[f * stride].  A cell past
-// the array's last ghost layer (a tile overhanging the grid) takes the state
-// of the nearest ghost cell: physical values, read without a branch, and no
-// face that touches such a cell is used.
+// Starts copying the fields src of the cell at offset o to dst[f * stride].
 template <class Off>
-__device__ __forceinline__ void prefetch_raw(float* dst, int stride, FluxParams<float> const& p, int i, int j, int k)
+__device__ __forceinline__ void prefetch_raw(float* dst, int stride, CBundle<float> const& src, Off o)
 {
-    Off const o = cell_offset<Off>(p.g, min(i, p.g.n0 - 1), min(j, p.g.n1 - 1), k);
 #pragma unroll
     for (int f = 0; f < 5; ++f) {
-        cp_async4(dst + f * stride, p.cons_in.f[f] + o);
+        cp_async4(dst + f * stride, src.f[f] + o);
     }
+}
+
+__device__ __forceinline__ void write_raw(float* dst, int stride, Raw5 const& r)
+{
+    dst[0] = r.d;
+    dst[stride] = r.e;
+    dst[2 * stride] = r.m[0];
+    dst[3 * stride] = r.m[1];
+    dst[4 * stride] = r.m[2];
 }
 
 __device__ __forceinline__ Raw5 read_raw(float const* src, int stride)
@@ -191,8 +240,10 @@ __device__ __forceinline__ Raw5 read_raw(float const* src, int stride)
     return Raw5{src[0], src[stride], {src[2 * stride], src[3 * stride], src[4 * stride]}};
 }
 
+template <int W>
 __device__ __forceinline__ void halo_cell(int h, int& hx, int& hy)
 {
+    constexpr int TX = Tile<W>::TX, TY = Tile<W>::TY, HX = Tile<W>::HX, HY = Tile<W>::HY;
     if (h < TY) {
         hx = 0;
         hy = 1 + h;
@@ -212,18 +263,21 @@ __device__ __forceinline__ void halo_cell(int h, int& hx, int& hy)
 // (u2, c, e + p, -), written and read with two vector accesses (STS.128 and
 // LDS.128) instead of seven scalar ones.  Consecutive lanes touch
 // consecutive words, so the accesses are free of bank conflicts.
+template <int W>
 struct SlotPlane {
-    float4 a[PLANE];
-    float4 b[PLANE];
+    float4 a[Tile<W>::PLANE];
+    float4 b[Tile<W>::PLANE];
 };
 
-__device__ __forceinline__ void put(SlotPlane& q, int idx, Prim7 const& v)
+template <int W>
+__device__ __forceinline__ void put(SlotPlane<W>& q, int idx, Prim7 const& v)
 {
     q.a[idx] = make_float4(v.d, v.p, v.u[0], v.u[1]);
     q.b[idx] = make_float4(v.u[2], v.c, v.e, v.e);
 }
 
-__device__ __forceinline__ Prim7 get(SlotPlane const& q, int idx)
+template <int W>
+__device__ __forceinline__ Prim7 get(SlotPlane<W> const& q, int idx)
 {
     float4 const a = q.a[idx];
     float4 const b = q.b[idx];
@@ -280,74 +334,133 @@ __device__ __forceinline__ float2 comp_update2(float2 u, float2 xl, float2 xr, f
     return __fadd2_rn(s, sub2(err, nP));
 }
 
+// The double-float update of two fields: u + lo plus the six signed face
+// terms, accumulated without rounding error in any product (TwoProduct) or
+// running sum (TwoSum), the errors collected in lo; then one rounding of each
+// word.  compensated_add's operations on two fields at once.
+__device__ __forceinline__ void comp_add2(float2& sum, float2& err, float2 k, float2 nk, float2 f)
+{
+    float2 const prod = __fmul2_rn(k, f);
+    float2 const nprod_err = __ffma2_rn(nk, f, prod); // -(k f - prod)
+    float2 const s = __fadd2_rn(sum, prod);
+    float2 const bb = sub2(s, sum);
+    float2 const sum_err = __fadd2_rn(sub2(sum, sub2(s, bb)), sub2(prod, bb));
+    sum = s;
+    err = __fadd2_rn(err, sub2(sum_err, nprod_err));
+}
+
+__device__ __forceinline__ void hilo_update2(float2& u, float2& lo, float2 xl, float2 xr, float2 yb, float2 yt, float2 zl,
+                                             float2 zh, float k0, float k1, float k2)
+{
+    float2 const p0 = make_float2(k0, k0), n0 = make_float2(-k0, -k0);
+    float2 const p1 = make_float2(k1, k1), n1 = make_float2(-k1, -k1);
+    float2 const p2 = make_float2(k2, k2), n2 = make_float2(-k2, -k2);
+    float2 sum = u;
+    float2 err = lo;
+    comp_add2(sum, err, n0, p0, xr);
+    comp_add2(sum, err, p0, n0, xl);
+    comp_add2(sum, err, n1, p1, yt);
+    comp_add2(sum, err, p1, n1, yb);
+    comp_add2(sum, err, n2, p2, zh);
+    comp_add2(sum, err, p2, n2, zl);
+    u = __fadd2_rn(sum, err);
+    lo = sub2(err, sub2(u, sum));
+}
+
+template <int COMP, int W>
 struct ColShared {
-    SlotPlane slot[2];
+    static constexpr int TY = Tile<W>::TY, NHALO = Tile<W>::NHALO;
+    SlotPlane<W> slot[2];
     float4 yflux_a[NT]; // the y face below each cell
     float yflux_b[NT];
     float4 xflux_ra[TY]; // the tile's right boundary x faces
     float xflux_rb[TY];
-    float raw_own[5 * NT];     // own column, two planes ahead
+    float raw_own[3][5 * NT];  // own column's staged fields: planes k, k+1, k+2 in turn
     float raw_halo[5 * NHALO]; // halo ring, one plane ahead
+    float raw_lo[COMP == kCompHiLo ? 5 * NT : 1]; // own column's low words of the current plane
     long long warp_best[NT / 32];
     int any_bad;
 };
 
-// One work item: interior planes [kb, ke) of the 32 x 8 column tile (tx, ty),
-// kb = 1 + kc * kchunk, with update coefficients k0..k2 (UNIFORM: cubic cells, k0..k2
-// all equal and 1/dx_d too).  BRANCHED: the cell update sits inside the
+// One work item: interior planes [kb, ke) of the column tile (tx, ty), with
+// update coefficients k0..k2 (UNIFORM: cubic cells, k0..k2 all equal and
+// 1/dx_d too).  BRANCHED: the cell update sits inside the
 // interior test (the batch) rather than beside it (the single grid).
 // Accumulates this thread's max wavespeed and non-physical flag.
-template <int COMP, bool UNIFORM, class Off, bool BRANCHED>
+template <int COMP, int W, bool UNIFORM, class Off, bool BRANCHED>
 __device__ __forceinline__ void col_item(FluxParams<float> const& p, float k0, float k1, float k2, int tx, int ty,
-                                         int kc, ColShared& sh, float& wmaxf, bool& bad)
+                                         int kb, int ke, ColShared<COMP, W>& sh, float& wmaxf, bool& bad)
 {
+    constexpr int TX = Tile<W>::TX, TY = Tile<W>::TY, HX = Tile<W>::HX, NHALO = Tile<W>::NHALO;
+    constexpr int kRightWarp = Tile<W>::kRightWarp;
+    CBundle<float> const& src = staged<COMP>(p);
     int const tid = threadIdx.x;
-    int const ti = tid % TX; // == lane
-    int const tj = tid / TX; // == warp
+    int const ti = tid % TX;
+    int const tj = tid / TX;
     int const own_idx = (tj + 1) * HX + ti + 1;
-    int hhx = 0, hhy = 0;
-    if (tid < NHALO) {
-        halo_cell(tid, hhx, hhy);
-    }
     int const i0 = 1 + tx * TX;
     int const j0 = 1 + ty * TY;
-    int const kb = 1 + kc * p.kchunk;
-    int const ke = min(kb + p.kchunk, p.g.n2 - 1);
-    int const i = i0 + ti;
-    int const j = j0 + tj;
-    bool const own = (i < p.g.n0 - 1) && (j < p.g.n1 - 1);
+    bool const own = (i0 + ti < p.g.n0 - 1) && (j0 + tj < p.g.n1 - 1);
+    // offsets of the thread's own cell and of its halo cell, kept running
+    // from plane to plane
+    Off const s2 = static_cast<Off>(p.g.s2);
+    Off o = clamped_offset<Off>(p.g, i0 + ti, j0 + tj, kb);
+    Off ho = 0;
+    int halo_idx = 0;
+    if (tid < NHALO) {
+        int hx, hy;
+        halo_cell<W>(tid, hx, hy);
+        halo_idx = hy * HX + hx;
+        ho = clamped_offset<Off>(p.g, i0 - 1 + hx, j0 - 1 + hy, kb);
+    }
 
     // prologue: plane kb of the halo ring staged, kb+1 on its way; planes
     // kb-1 (z face below), kb, kb+1 of the own column
     if (tid < NHALO) {
-        prefetch_raw<Off>(sh.raw_halo + tid, NHALO, p, i0 - 1 + hhx, j0 - 1 + hhy, kb);
+        prefetch_raw(sh.raw_halo + tid, NHALO, src, ho);
         cp_async_wait_all();
-        put(sh.slot[0], hhy * HX + hhx, prim_of<COMP>(read_raw(sh.raw_halo + tid, NHALO), p));
+        put(sh.slot[0], halo_idx, prim_of<COMP>(read_raw(sh.raw_halo + tid, NHALO), p));
+        ho += s2;
         if (kb + 1 < ke) {
-            prefetch_raw<Off>(sh.raw_halo + tid, NHALO, p, i0 - 1 + hhx, j0 - 1 + hhy, kb + 1);
+            prefetch_raw(sh.raw_halo + tid, NHALO, src, ho);
         }
     }
     cp_async_commit();
-    Raw5 const rb = load_raw<Off>(p, i, j, kb - 1);
-    Raw5 rk = load_raw<Off>(p, i, j, kb);
-    Raw5 rn = load_raw<Off>(p, i, j, kb + 1); // kb + 1 <= ke <= n2 - 1
-    Prim7 q0 = prim_of<COMP>(rk, p);
-    Prim7 q1 = prim_of<COMP>(rn, p);
+    Raw5 const rb = load_raw(src, o - s2);
+    Raw5 const r0 = load_raw(src, o);
+    Raw5 const r1 = load_raw(src, o + s2); // kb + 1 <= ke <= n2 - 1
+    if constexpr (COMP != kCompOperator) {
+        write_raw(sh.raw_own[0] + tid, NT, r0);
+        write_raw(sh.raw_own[1] + tid, NT, r1);
+    }
+    Prim7 q0 = prim_of<COMP>(r0, p);
+    Prim7 q1 = prim_of<COMP>(r1, p);
+    float* raw_k = sh.raw_own[0] + tid; // this thread's words of plane k, and of plane k+2
+    float* raw_n = sh.raw_own[2] + tid;
     float zlo[5];
     to_global(hllc_flux(side_of(prim_of<COMP>(rb, p), 2), side_of(q0, 2)), 2, zlo);
-    Off o = cell_offset<Off>(p.g, min(i, p.g.n0 - 1), min(j, p.g.n1 - 1), kb);
 
     // Unrolled twice: the plane-to-plane register rotation (q0 <- q1,
-    // rk <- rn, zlo <- fzh) becomes renaming instead of moves, and the slot
-    // of each copy is a constant.
+    // zlo <- fzh) becomes renaming instead of moves, and the slot of each
+    // copy is a constant.
 #pragma unroll 2
     for (int k = kb; k < ke; ++k) {
-        SlotPlane& q = sh.slot[(k - kb) & 1];
+        SlotPlane<W>& q = sh.slot[(k - kb) & 1];
         // stage plane k: the own cell (its halo ring was staged a plane ahead)
         put(q, own_idx, q0);
         // own column plane k+2, consumed at the end of this plane
         if (k + 2 <= ke) {
-            prefetch_raw<Off>(sh.raw_own + tid, NT, p, i, j, k + 2);
+            prefetch_raw(raw_n, NT, src, o + 2 * s2);
+        }
+        if constexpr (COMP == kCompHiLo) { // and the low words of plane k, consumed by this plane's update
+            prefetch_raw(sh.raw_lo + tid, NT, p.lo_in, o);
+        }
+        float cons[5]; // the operator's cons, in flight while the faces are solved
+        if (COMP == kCompOperator && own) {
+#pragma unroll
+            for (int f = 0; f < 5; ++f) {
+                cons[f] = p.cons_in.f[f][o];
+            }
         }
         cp_async_commit();
         __syncthreads(); // plane k staged
@@ -356,9 +469,11 @@ __device__ __forceinline__ void col_item(FluxParams<float> const& p, float k0, f
         // plane's second barrier)
         if (tid < NHALO && k + 1 < ke) {
             cp_async_wait_all_but_last(); // the halo copies of plane k+1 landed (own k+2 may be in flight)
-            put(sh.slot[(k + 1 - kb) & 1], hhy * HX + hhx, prim_of<COMP>(read_raw(sh.raw_halo + tid, NHALO), p));
+            put(sh.slot[(k + 1 - kb) & 1], halo_idx, prim_of<COMP>(read_raw(sh.raw_halo + tid, NHALO), p));
+            ho += s2;
+            opaque(ho);
             if (k + 2 < ke) {
-                prefetch_raw<Off>(sh.raw_halo + tid, NHALO, p, i0 - 1 + hhx, j0 - 1 + hhy, k + 2);
+                prefetch_raw(sh.raw_halo + tid, NHALO, src, ho);
             }
         }
         cp_async_commit();
@@ -376,11 +491,12 @@ __device__ __forceinline__ void col_item(FluxParams<float> const& p, float k0, f
         for (int f = 0; f < 5; ++f) {
             fxr[f] = __shfl_down_sync(0xffffffffu, fxl[f], 1);
         }
-        if (tj == kRightWarp && ti < TY) { // the tile's right boundary faces, one per row
-            int const c = (ti + 1) * HX + TX;
+        int const lane = tid % 32;
+        if (tid / 32 == kRightWarp && lane < TY) { // the tile's right boundary faces, one per row
+            int const c = (lane + 1) * HX + TX;
             float t[5];
             to_global(hllc_flux(side_of(get(q, c), 0), side_of(get(q, c + 1), 0)), 0, t);
-            put_flux(sh.xflux_ra, sh.xflux_rb, ti, t);
+            put_flux(sh.xflux_ra, sh.xflux_rb, lane, t);
         }
         if (tj == TY - 1) { // the tile's top boundary faces
             to_global(hllc_flux(side_of(q0, 1), side_of(get(q, own_idx + HX), 1)), 1, fyt);
@@ -392,7 +508,7 @@ __device__ __forceinline__ void col_item(FluxParams<float> const& p, float k0, f
         }
         {
             float xr[5];
-            get_flux(sh.xflux_ra, sh.xflux_rb, tj, xr); // one broadcast read per warp
+            get_flux(sh.xflux_ra, sh.xflux_rb, tj, xr); // one broadcast read per row
 #pragma unroll
             for (int f = 0; f < 5; ++f) {
                 fxr[f] = ti == TX - 1 ? xr[f] : fxr[f];
@@ -406,7 +522,35 @@ __device__ __forceinline__ void col_item(FluxParams<float> const& p, float k0, f
         // whose tiles overhang its small grids more often, keeps the branch
         // (measured 4 % faster there).
         if (!BRANCHED || own) {
-            float u[5] = {rk.d, rk.e, rk.m[0], rk.m[1], rk.m[2]};
+            float u[5];
+            float lo[COMP == kCompHiLo ? 5 : 1];
+#pragma unroll
+            for (int f = 0; f < 5; ++f) {
+                u[f] = COMP == kCompOperator ? cons[f] : raw_k[f * NT];
+            }
+            if constexpr (COMP == kCompHiLo) {
+                cp_async_wait_all_but_last(); // the low words of plane k landed (and own k+2)
+                Raw5 const rl = read_raw(sh.raw_lo + tid, NT);
+                lo[0] = rl.d;
+                lo[1] = rl.e;
+                lo[2] = rl.m[0];
+                lo[3] = rl.m[1];
+                lo[4] = rl.m[2];
+#pragma unroll
+                for (int f = 0; f < 5; f += 2) { // (d, e), (m0, m1), (m2, -)
+                    int const h = f + 1 < 5 ? f + 1 : f;
+                    float2 uu = make_float2(u[f], u[h]), ll = make_float2(lo[f], lo[h]);
+                    hilo_update2(uu, ll, make_float2(fxl[f], fxl[h]), make_float2(fxr[f], fxr[h]),
+                                 make_float2(fyb[f], fyb[h]), make_float2(fyt[f], fyt[h]), make_float2(zlo[f], zlo[h]),
+                                 make_float2(fzh[f], fzh[h]), k0, k1, k2);
+                    u[f] = uu.x;
+                    lo[f] = ll.x;
+                    if (h != f) {
+                        u[h] = uu.y;
+                        lo[h] = ll.y;
+                    }
+                }
+            }
             constexpr bool kPaired = COMP == kCompSum && UNIFORM;
             if (kPaired) { // fields (d, e) and (m0, m1) in pairs, m2 below
                 float2 const kk = make_float2(k0, k0), nk = make_float2(-k0, -k0);
@@ -421,9 +565,10 @@ __device__ __forceinline__ void col_item(FluxParams<float> const& p, float k0, f
                 }
             }
 #pragma unroll
-            for (int f = kPaired ? 4 : 0; f < 5; ++f) {
-                if (COMP == kCompNone) {
-                    u[f] = u[f] - k0 * (fxr[f] - fxl[f]) - k1 * (fyt[f] - fyb[f]) - k2 * (fzh[f] - zlo[f]);
+            for (int f = COMP == kCompHiLo ? 5 : (kPaired ? 4 : 0); f < 5; ++f) {
+                if (COMP == kCompNone || COMP == kCompOperator) {
+                    u[f] = fmaf(-k2, __fsub_rn(fzh[f], zlo[f]),
+                                fmaf(-k1, __fsub_rn(fyt[f], fyb[f]), fmaf(-k0, __fsub_rn(fxr[f], fxl[f]), u[f])));
                 } else if (UNIFORM) {
                     // _rn intrinsics: no product may be fused into the sums
                     // the TwoSum and TwoProduct take apart
@@ -452,41 +597,51 @@ __device__ __forceinline__ void col_item(FluxParams<float> const& p, float k0, f
 #pragma unroll
                 for (int f = 0; f < 5; ++f) {
                     p.cons_out.f[f][o] = u[f];
+                    if (COMP == kCompHiLo) {
+                        p.lo_out.f[f][o] = lo[f];
+                    }
                 }
             }
+            if constexpr (COMP != kCompOperator) {
             // next step's CFL wavespeed of the new state (time_step.hpp:28-33);
             // on cubic cells (3 cs + |v0| + |v1| + |v2|) / dx, one product
             Raw5 const nr{u[0], u[1], {u[2], u[3], u[4]}};
-            float const r = rcp_approx(u[0]);
+            float const r = COMP == kCompHiLo ? rcp_rn(u[0]) : rcp_approx(u[0]);
             float const v0 = u[2] * r, v1 = u[3] * r, v2 = u[4] * r;
-            float const pr = col_pressure<COMP>(nr, v0, v1, v2, r, p.gm1);
+            float const pr = col_pressure<COMP>(nr, v0, v1, v2, r, p.gm1, lo);
             float const cs = fast_sound_speed((p.gamma * r) * pr);
-            float const invdt = UNIFORM ? (3.0f * cs + fabsf(v0) + fabsf(v1) + fabsf(v2)) * p.invdx0
-                                        : (cs + fabsf(v0)) * p.invdx0 + (cs + fabsf(v1)) * p.invdx1 +
-                                                  (cs + fabsf(v2)) * p.invdx2;
+            float const invdt =
+                    UNIFORM ? __fmul_rn(__fadd_rn(__fadd_rn(fmaf(3.0f, cs, fabsf(v0)), fabsf(v1)), fabsf(v2)), p.invdx0)
+                            : fmaf(__fadd_rn(cs, fabsf(v2)), p.invdx2,
+                                   fmaf(__fadd_rn(cs, fabsf(v1)), p.invdx1, __fmul_rn(__fadd_rn(cs, fabsf(v0)), p.invdx0)));
             wmaxf = own ? fmaxf(wmaxf, invdt) : wmaxf; // NaN never wins
             bad |= own && !cell_ok(u[0], pr, invdt);
+            }
         }
         // march: plane k+1 becomes the current plane
 #pragma unroll
         for (int f = 0; f < 5; ++f) {
             zlo[f] = fzh[f];
         }
-        rk = rn;
         q0 = q1;
         if (k + 2 <= ke) {
             cp_async_wait_all_but_last(); // the own copies of plane k+2 landed
-            rn = read_raw(sh.raw_own + tid, NT);
-            q1 = prim_of<COMP>(rn, p);
+            q1 = prim_of<COMP>(read_raw(raw_n, NT), p);
         }
-        o += static_cast<Off>(p.g.s2);
+        // the slots in turn: k <- k+1, k+1 <- k+2, and plane k's is free
+        float* const end = sh.raw_own[2] + tid;
+        raw_n = raw_k;
+        raw_k = raw_k == end ? sh.raw_own[0] + tid : raw_k + 5 * NT;
+        o += s2;
+        opaque(o);
     }
     __syncthreads(); // the slots are restaged by the next item
 }
 
 // Block max of the threads' wavespeeds into *wmax (ordered bits, one
 // atomicMax per CTA) and the non-physical flag into *status; clears both.
-__device__ __forceinline__ void col_flush(ColShared& sh, float& wmaxf, bool& bad, unsigned long long* wmax,
+template <int COMP, int W>
+__device__ __forceinline__ void col_flush(ColShared<COMP, W>& sh, float& wmaxf, bool& bad, unsigned long long* wmax,
                                           int* status)
 {
     int const tid = threadIdx.x;
@@ -523,33 +678,45 @@ __device__ __forceinline__ void col_flush(ColShared& sh, float& wmaxf, bool& bad
     bad = false;
 }
 
-template <int COMP, bool UNIFORM, class Off>
-__global__ void __launch_bounds__(NT, 3) f32_step_kernel(const __grid_constant__ FluxParams<float> p)
+// CTAs per SM the registers are cut for.
+template <int COMP>
+constexpr int kColPerSM = COMP == kCompHiLo ? 2 : 3;
+
+// One launch over a single grid: the fused step, or the operator.
+template <int COMP, int W, bool UNIFORM, class Off>
+__global__ void __launch_bounds__(NT, kColPerSM<COMP>) f32_step_kernel(const __grid_constant__ FluxParams<float> p)
 {
-    static_assert(COMP == kCompNone || COMP == kCompSum, "low-word states use the tile engine");
-    __shared__ __align__(16) ColShared sh;
+    __shared__ __align__(16) ColShared<COMP, W> sh;
     float const dtodv = dt_over_dv(p);
     float const k0 = dtodv * p.ds0, k1 = dtodv * p.ds1, k2 = dtodv * p.ds2; // UNIFORM: all equal
     float wmaxf = 0.0f;
     bool bad = false;
-    int const tiles_xy = p.tiles_x * p.tiles_y;
+    // (chunk, tile) items, tiles fastest: the CTAs at work at one time hold
+    // neighbouring tiles of one chunk, whose halos they share in L2.  The
+    // chunks (p.kchunk of them) are even to a plane.
+    int const iz = p.g.n2 - 2;
+    int const tiles = p.tiles_x * p.tiles_y;
     for (int w = blockIdx.x; w < p.nwork; w += gridDim.x) {
-        col_item<COMP, UNIFORM, Off, false>(p, k0, k1, k2, w % p.tiles_x, (w / p.tiles_x) % p.tiles_y, w / tiles_xy, sh, wmaxf,
-                                bad);
+        int const chunk = w / tiles;
+        int const tile = w - chunk * tiles;
+        int const kb = 1 + static_cast<int>(static_cast<long long>(chunk) * iz / p.kchunk);
+        int const ke = 1 + static_cast<int>(static_cast<long long>(chunk + 1) * iz / p.kchunk);
+        col_item<COMP, W, UNIFORM, Off, false>(p, k0, k1, k2, tile % p.tiles_x, tile / p.tiles_x, kb, ke, sh, wmaxf, bad);
     }
-    col_flush(sh, wmaxf, bad, p.wmax, p.status);
-    step_done(p);
+    if constexpr (COMP != kCompOperator) {
+        col_flush(sh, wmaxf, bad, p.wmax, p.status);
+        step_done(p);
+    }
 }
 
 // The column engine over a batch: CTAs pop (grid, tile x, tile y, chunk)
 // items from the queue, as flux_batch_kernel does; each item's wavespeed goes
 // to its own grid.  Grids of cubic cells take the cubic update and wavespeed.
-template <int COMP, class Off>
-__global__ void __launch_bounds__(NT, 3) f32_batch_kernel(const __grid_constant__ BatchParams<float> b)
+template <int COMP, int W, class Off>
+__global__ void __launch_bounds__(NT, kColPerSM<COMP>) f32_batch_kernel(const __grid_constant__ BatchParams<float> b)
 {
-    static_assert(COMP == kCompNone || COMP == kCompSum, "low-word states use the tile engine");
     static_assert(sizeof(FluxParams<float>) % 4 == 0, "parameter copy in 4-byte words");
-    __shared__ __align__(16) ColShared sh;
+    __shared__ __align__(16) ColShared<COMP, W> sh;
     __shared__ __align__(16) FluxParams<float> gp;
     __shared__ int s_item;
     int const tid = threadIdx.x;
@@ -572,10 +739,12 @@ __global__ void __launch_bounds__(NT, 3) f32_batch_kernel(const __grid_constant_
         __syncthreads();
         float const dtodv = dt_over_dv(gp);
         float const k0 = dtodv * gp.ds0, k1 = dtodv * gp.ds1, k2 = dtodv * gp.ds2;
+        int const kb = 1 + it.w * gp.kchunk;
+        int const ke = min(kb + gp.kchunk, gp.g.n2 - 1);
         if (gp.ds0 == gp.ds1 && gp.ds1 == gp.ds2 && gp.invdx0 == gp.invdx1 && gp.invdx1 == gp.invdx2) {
-            col_item<COMP, true, Off, true>(gp, k0, k1, k2, it.y, it.z, it.w, sh, wmaxf, bad);
+            col_item<COMP, W, true, Off, true>(gp, k0, k1, k2, it.y, it.z, kb, ke, sh, wmaxf, bad);
         } else {
-            col_item<COMP, false, Off, true>(gp, k0, k1, k2, it.y, it.z, it.w, sh, wmaxf, bad);
+            col_item<COMP, W, false, Off, true>(gp, k0, k1, k2, it.y, it.z, kb, ke, sh, wmaxf, bad);
         }
         col_flush(sh, wmaxf, bad, gp.wmax, gp.status);
         item_done(gp);
@@ -592,66 +761,118 @@ template <int COMP>
 cudaError_t configure_f32col(int* per_sm)
 {
     int n = 0;
-    cudaError_t const e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, f32col::f32_step_kernel<COMP, false, long long>,
-                                                                        f32col::NT, 0);
+    cudaError_t const e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+            &n, f32col::f32_step_kernel<COMP, 32, false, long long>, f32col::NT, 0);
     *per_sm = n < 1 ? 1 : n;
     return e;
 }
 
-template <int COMP>
-cudaError_t launch_f32col(FluxParams<float> p, int sms, cudaStream_t s)
+// Tile width and chunks of planes of a single-grid launch.
+// Width: the fewest tiles, a 16-column tile counted 2 % and an 8-column one
+// 12 % dearer than a 32-column one (measured at 512^3: -2 to 8 % and 10 to
+// 15 %), and 32-column tiles 6 % dearer where they leave a remainder (200^3,
+// compensated state: 166 us a step in 32-wide tiles, 142 in 16-wide).
+// Chunks: about three items per CTA slot, in chunks of 8 to 64 planes -- with
+// fewer items the SMs are not full, longer chunks let neighbouring CTAs drift
+// apart and lose the halos they share in L2, shorter ones pay the plane and a
+// half that an item costs besides its own too often -- and, within half of
+// that count, the one with the least work on the busiest SM.  A grid with
+// fewer tiles than SMs is cut finer, to one item per SM.  Within 5 % of the
+// best count tried on grids of 64^3 to 512^3.  Against 32-wide tiles in chunks of
+// at least 8 planes (compensated state, a step): 99 x 128 x 75 43 -> 30 us,
+// 200 x 147 x 131 93 -> 83, 200^3 172 -> 142, 16^3 15 -> 8.
+struct ColPlan {
+    int width, chunks;
+};
+
+ColPlan choose_columns(int ix, int iy, int iz, int sms, int per_sm)
+{
+    ColPlan best{32, 1};
+    double least = 1e300;
+    long long tiles = 1;
+    for (int tx : {32, 16, 8}) {
+        int const ty = f32col::NT / tx;
+        long long const n = static_cast<long long>((ix + tx - 1) / tx) * ((iy + ty - 1) / ty);
+        double const cost = n * (tx == 32 ? (ix % 32 == 0 ? 1.0 : 1.06) : (tx == 16 ? 1.02 : 1.12));
+        if (cost < least) {
+            least = cost;
+            best.width = tx;
+            tiles = n;
+        }
+    }
+    long long const slots = static_cast<long long>(sms) * per_sm;
+    long long planes = tiles * iz / (3 * slots);
+    planes = planes < 8 ? 8 : (planes > 64 ? 64 : planes);
+    int const aim = static_cast<int>((iz + planes - 1) / planes);
+    long long lo = aim * 2 / 3 > 0 ? aim * 2 / 3 : 1;
+    long long hi = aim * 3 / 2 > sms / tiles ? aim * 3 / 2 : sms / tiles;
+    hi = hi < iz ? (hi > lo ? hi : lo) : iz;
+    long long fewest = 0x7fffffffffffffffLL;
+    for (long long c = lo; c <= hi; ++c) {
+        long long const cost = (tiles * c + sms - 1) / sms * (2 * ((iz + c - 1) / c) + 3);
+        if (cost < fewest) {
+            fewest = cost;
+            best.chunks = static_cast<int>(c);
+        }
+    }
+    return best;
+}
+
+template <int COMP, int W, class Off>
+cudaError_t launch_f32col_as(FluxParams<float> p, int chunks, int sms, cudaStream_t s)
 {
     int const per_sm = p.per_sm > 0 ? p.per_sm : 1;
     int const ix = p.g.n0 - 2;
     int const iy = p.g.n1 - 2;
-    int const iz = p.g.n2 - 2;
-    if (ix <= 0 || iy <= 0 || iz <= 0) {
-        return cudaSuccess; // no interior cell
-    }
-    p.tiles_x = (ix + f32col::TX - 1) / f32col::TX;
-    p.tiles_y = (iy + f32col::TY - 1) / f32col::TY;
+    p.tiles_x = (ix + f32col::Tile<W>::TX - 1) / f32col::Tile<W>::TX;
+    p.tiles_y = (iy + f32col::Tile<W>::TY - 1) / f32col::Tile<W>::TY;
     long long const slots = static_cast<long long>(sms) * per_sm;
-    if (p.kchunk <= 0) {
-        p.kchunk = choose_kchunk(p.tiles_x * p.tiles_y, iz, slots);
-    }
-    int const kchunks = (iz + p.kchunk - 1) / p.kchunk;
-    long long const nwork = static_cast<long long>(p.tiles_x) * p.tiles_y * kchunks;
-    p.nwork = static_cast<int>(nwork);
-    long long const grid = slots < nwork ? slots : nwork;
+    p.kchunk = chunks;
+    p.nwork = p.tiles_x * p.tiles_y * chunks;
+    int const grid = static_cast<int>(slots < p.nwork ? slots : p.nwork);
     // cubic cells: equal face areas give equal update coefficients dt/dv * ds_d,
     // and equal 1/dx_d the one-product wavespeed
-    bool const uniform = p.ds0 == p.ds1 && p.ds1 == p.ds2 && p.invdx0 == p.invdx1 && p.invdx1 == p.invdx2;
-    if (p.g.ncell() <= kNarrowCells) {
-        if (uniform) {
-            f32col::f32_step_kernel<COMP, true, unsigned><<<static_cast<int>(grid), f32col::NT, 0, s>>>(p);
-        } else {
-            f32col::f32_step_kernel<COMP, false, unsigned><<<static_cast<int>(grid), f32col::NT, 0, s>>>(p);
-        }
-    } else if (uniform) {
-        f32col::f32_step_kernel<COMP, true, long long><<<static_cast<int>(grid), f32col::NT, 0, s>>>(p);
+    if (p.ds0 == p.ds1 && p.ds1 == p.ds2 && p.invdx0 == p.invdx1 && p.invdx1 == p.invdx2) {
+        f32col::f32_step_kernel<COMP, W, true, Off><<<grid, f32col::NT, 0, s>>>(p);
     } else {
-        f32col::f32_step_kernel<COMP, false, long long><<<static_cast<int>(grid), f32col::NT, 0, s>>>(p);
+        f32col::f32_step_kernel<COMP, W, false, Off><<<grid, f32col::NT, 0, s>>>(p);
     }
     return cudaGetLastError();
 }
 
-// The column engine as the 32 x 8 shape of the FP32 batch (states without low words).
 template <int COMP>
-struct ColBatchKernel {
-    static cudaError_t configure(int* per_sm)
-    {
-        int n = 0;
-        cudaError_t const e =
-                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, f32col::f32_batch_kernel<COMP, long long>, f32col::NT, 0);
-        *per_sm = n < 1 ? 1 : n;
-        return e;
+cudaError_t launch_f32col(FluxParams<float> const& p, int sms, cudaStream_t s)
+{
+    if (p.g.n0 <= 2 || p.g.n1 <= 2 || p.g.n2 <= 2) {
+        return cudaSuccess; // no interior cell
     }
-    static cudaError_t launch(BatchParams<float> const& b, int grid, cudaStream_t s)
+    ColPlan const plan = choose_columns(p.g.n0 - 2, p.g.n1 - 2, p.g.n2 - 2, sms, p.per_sm > 0 ? p.per_sm : 1);
+    if (p.g.ncell() > kNarrowCells) { // 64-bit offsets are built for one width
+        return launch_f32col_as<COMP, 32, long long>(p, plan.chunks, sms, s);
+    }
+    switch (plan.width) {
+    case 8: return launch_f32col_as<COMP, 8, unsigned>(p, plan.chunks, sms, s);
+    case 16: return launch_f32col_as<COMP, 16, unsigned>(p, plan.chunks, sms, s);
+    default: return launch_f32col_as<COMP, 32, unsigned>(p, plan.chunks, sms, s);
+    }
+}
+
+// The column engine as the 32 x 8 and 16 x 16 shapes of the FP32 batch.
+template <int COMP, int W>
+struct ColBatchKernel {
+    static cudaError_t run(BatchParams<float> const* b, int grid, int* per_sm, cudaStream_t s)
     {
-        if (b.max_cells <= kNarrowCells) {
-            f32col::f32_batch_kernel<COMP, unsigned><<<grid, f32col::NT, 0, s>>>(b);
+        if (b == nullptr) {
+            int n = 0;
+            cudaError_t const e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+                    &n, f32col::f32_batch_kernel<COMP, W, long long>, f32col::NT, 0);
+            *per_sm = n < 1 ? 1 : n;
+            return e;
+        }
+        if (b->max_cells <= kNarrowCells) {
+            f32col::f32_batch_kernel<COMP, W, unsigned><<<grid, f32col::NT, 0, s>>>(*b);
         } else {
-            f32col::f32_batch_kernel<COMP, long long><<<grid, f32col::NT, 0, s>>>(b);
+            f32col::f32_batch_kernel<COMP, W, long long><<<grid, f32col::NT, 0, s>>>(*b);
         }
         return cudaGetLastError();
     }
@@ -661,20 +882,40 @@ struct ColBatchKernel {
 
 cudaError_t configure_step_f32col(int comp, int* per_sm)
 {
-    return comp == kCompSum ? configure_f32col<kCompSum>(per_sm) : configure_f32col<kCompNone>(per_sm);
+    switch (comp) {
+    case kCompSum: return configure_f32col<kCompSum>(per_sm);
+    case kCompHiLo: return configure_f32col<kCompHiLo>(per_sm);
+    default: return configure_f32col<kCompNone>(per_sm);
+    }
 }
 
 cudaError_t launch_step_f32col(FluxParams<float> const& p, int comp, int sms, cudaStream_t s)
 {
-    return comp == kCompSum ? launch_f32col<kCompSum>(p, sms, s) : launch_f32col<kCompNone>(p, sms, s);
+    switch (comp) {
+    case kCompSum: return launch_f32col<kCompSum>(p, sms, s);
+    case kCompHiLo: return launch_f32col<kCompHiLo>(p, sms, s);
+    default: return launch_f32col<kCompNone>(p, sms, s);
+    }
 }
 
-cudaError_t launch_batch_f32col(int comp, BatchParams<float> const* b, int grid, int* per_sm, cudaStream_t s)
+cudaError_t launch_godunov_f32(FluxParams<float> const& p, int sms, cudaStream_t s)
 {
-    if (comp == kCompSum) {
-        return b ? ColBatchKernel<kCompSum>::launch(*b, grid, s) : ColBatchKernel<kCompSum>::configure(per_sm);
+    FluxParams<float> q = p;
+    cudaError_t const e = configure_f32col<f32col::kCompOperator>(&q.per_sm);
+    return e != cudaSuccess ? e : launch_f32col<f32col::kCompOperator>(q, sms, s);
+}
+
+cudaError_t launch_batch_f32col(int comp, int tx, BatchParams<float> const* b, int grid, int* per_sm, cudaStream_t s)
+{
+    bool const w = tx == 32;
+    switch (comp) {
+    case kCompSum:
+        return w ? ColBatchKernel<kCompSum, 32>::run(b, grid, per_sm, s) : ColBatchKernel<kCompSum, 16>::run(b, grid, per_sm, s);
+    case kCompHiLo:
+        return w ? ColBatchKernel<kCompHiLo, 32>::run(b, grid, per_sm, s) : ColBatchKernel<kCompHiLo, 16>::run(b, grid, per_sm, s);
+    default:
+        return w ? ColBatchKernel<kCompNone, 32>::run(b, grid, per_sm, s) : ColBatchKernel<kCompNone, 16>::run(b, grid, per_sm, s);
     }
-    return b ? ColBatchKernel<kCompNone>::launch(*b, grid, s) : ColBatchKernel<kCompNone>::configure(per_sm);
 }
 
 } // namespace eulr

@@ -12,12 +12,10 @@ namespace eulr {
 
 constexpr int kModeGodunov = 0; // per-operator godunov: cons updated in place from prim
 constexpr int kModeStep = 1;    // fused step: ping-pong buffers, next-step CFL reduction
-constexpr int kModeStepCons = 2; // fused step whose state is cons only (FP32): prim rebuilt on chip
 
 // Update arithmetic of the fused FP32 step.
 constexpr int kCompNone = 0;  // plain: cons -= sum of the six face terms, FP32
-constexpr int kCompSum = 1;   // compensated: one rounding at the state's scale (column engine: axis
-                              // differences + TwoProduct/TwoSum; tile engine: error-free sum of six terms)
+constexpr int kCompSum = 1;   // compensated: one rounding at the state's scale (axis differences + TwoProduct/TwoSum)
 constexpr int kCompHiLo = 2;  // compensated with a stored low word: cons = hi + lo (double-float)
 
 // Device scalars of a simulation.
@@ -156,9 +154,11 @@ cudaError_t launch_godunov_exact(CBundle<T> prim, Bundle<T> cons, Geom g, T gamm
 int flux_tile_x();
 int flux_tile_y();
 
-// Multi-grid batch (batch.cu): tile-shape variants of the batch kernel.
+// Multi-grid batch (batch.cu): tile-shape variants of the batch kernel; the
+// FP32 states have the 32 x 8 and 16 x 16 ones.
 int batch_shape_count();
 void batch_shape(int shape, int* tx, int* ty);
+bool batch_shape_built(int shape, bool f64);
 template <class T>
 cudaError_t launch_flux_batch(int shape, int comp, BatchParams<T> const* b, int grid, int* per_sm, cudaStream_t s);
 template <class T>
@@ -166,11 +166,12 @@ cudaError_t launch_ghost_shell(GhostParams<T> p, int sms, cudaStream_t s);
 template <class T>
 cudaError_t launch_finalize_dt(SimScalars* sc, T cfl, int add_time, cudaStream_t s, const double* dt_seq = nullptr);
 
-// The FP32 step on the column engine (flux_f32.cu), comp kCompNone or kCompSum.
+// The FP32 states' step and the FP32 godunov on the column engine (flux_f32.cu).
 cudaError_t configure_step_f32col(int comp, int* per_sm);
 cudaError_t launch_step_f32col(FluxParams<float> const& p, int comp, int sms, cudaStream_t s);
+cudaError_t launch_godunov_f32(FluxParams<float> const& p, int sms, cudaStream_t s);
 // b == nullptr: configure and report resident CTAs per SM; otherwise launch.
-cudaError_t launch_batch_f32col(int comp, BatchParams<float> const* b, int grid, int* per_sm, cudaStream_t s);
+cudaError_t launch_batch_f32col(int comp, int tx, BatchParams<float> const* b, int grid, int* per_sm, cudaStream_t s);
 
 cudaError_t launch_fma_probe(int kind, int blocks, int iters, float* sink, cudaStream_t s);
 template <class T>

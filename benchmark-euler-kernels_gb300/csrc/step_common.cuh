@@ -1,4 +1,4 @@
-// Device helpers shared by the FP64/FP32 tile engine (flux.cu) and the FP32
+// Device helpers shared by the FP64 tile engine (flux.cu) and the FP32
 // column engine (flux_f32.cu).  Internal to the library.
 #pragma once
 
@@ -51,7 +51,7 @@ __device__ __forceinline__ float cons_pressure(float d, float e, float m0, float
 template <int COMP>
 __device__ __forceinline__ double cons_pressure(double, double, double, double, double, double, double, const double*)
 {
-    return 0.0;
+    return 0.0; // FP64 states store prim: no caller reads this
 }
 
 // Sound speed sqrt(gamma p / rho), faithful: fewer FP64 instructions than a
@@ -74,20 +74,6 @@ __device__ __forceinline__ bool cell_ok(float d, float pr, float invdt)
 {
     return d > 0.0f && pr > 0.0f && invdt <= 3.0e38f;
 }
-
-// sum + err += k*f without rounding error in the product (TwoProduct via
-// FMA) or in the running sum (Knuth's TwoSum); the errors collect in err.
-__device__ __forceinline__ void compensated_add(float& sum, float& err, float k, float f)
-{
-    float const prod = k * f;
-    float const prod_err = fmaf(k, f, -prod);
-    float const s = sum + prod;
-    float const bb = s - sum;
-    float const sum_err = (sum - (s - bb)) + (prod - bb);
-    sum = s;
-    err += sum_err + prod_err;
-}
-__device__ __forceinline__ void compensated_add(double&, double&, double, double) {}
 
 // dt/dv, from the device dt when there is one (godunov.hpp:37 with the
 // cfl * dt of euler_simulation.cpp:65), evaluated in double.
@@ -187,31 +173,6 @@ __device__ __forceinline__ void batch_cta_done(BatchParams<T> const& b)
         *b.head = 0u;
         *b.exited = 0u;
     }
-}
-
-// Chunk length (planes per work item) that balances the persistent grid:
-// the step lasts as long as its busiest CTA, while each extra chunk costs
-// one more z face row and two more staged planes (about 1/(3 kchunk) of a
-// chunk's work).  Scores every length from 8 to 64 by
-//   (planes / (resident CTAs x planes of the busiest CTA)) x (1 - 1/(3 kchunk))
-// and keeps the best.
-inline int choose_kchunk(int columns, int iz, long long slots)
-{
-    int best = 64;
-    double best_score = -1.0;
-    for (int kc = 8; kc <= 64; ++kc) {
-        long long const chunks = (iz + kc - 1) / kc;
-        long long const items = chunks * columns;
-        long long const rounds = (items + slots - 1) / slots; // items of the busiest CTA
-        double const busiest = static_cast<double>(rounds) * kc;
-        double const score = (static_cast<double>(iz) * columns / (static_cast<double>(slots) * busiest)) *
-                             (1.0 - 1.0 / (3.0 * kc));
-        if (score > best_score + 1e-9) {
-            best_score = score;
-            best = kc;
-        }
-    }
-    return best;
 }
 
 // ------------------------------------------ exact max wavespeed, screened

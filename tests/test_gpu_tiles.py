@@ -54,3 +54,44 @@ def test_batch_tiles_equal_single_grid(cuda, euler, oracle_lib):
             s.advance(4)
             ps, cs = s.state_numpy()
         assert np.array_equal(pb, ps) and np.array_equal(cb, cs), shape
+
+
+@pytest.mark.parametrize("precision", ["f32", "f32c", "f32c_hilo"])
+def test_fp32_columns_match_oracle_and_batch(cuda, euler, oracle_lib, precision):
+    """The FP32 column engine at its tile widths and chunk edges.  Against the FP64 oracle after four steps: 4 steps
+    of at most about 20 roundings (2^-24) each at a field's scale, 5e-6 of it; the batch's bits equal the single
+    grid's."""
+    O = oracle_lib
+    dx = (0.11, 0.07, 0.13)
+    grids = [(*s, 1.4, *dx) for s in SHAPES]
+    prims = [O.random_prim(*s, seed=31 + i) for i, s in enumerate(SHAPES)]
+    with euler.Batch(grids, cfl=0.4, precision=precision) as b:
+        for g, p in enumerate(prims):
+            b.set_prim(g, p)
+        b.advance(4)
+        batch = [b.state_numpy(g)[1] for g in range(len(grids))]
+    for shape, p0, cb in zip(SHAPES, prims, batch):
+        pref, cref = p0.copy(), O.prim_to_cons(p0, 1.4)
+        O.simulate(pref, cref, 1.4, dx, 0.4, 4)
+        with euler.Simulation(*shape, 1.4, dx, 0.4, precision=precision) as s:
+            s.set_prim(p0)
+            s.advance(4)
+            assert s.status() == 0
+            cons = s.state_numpy()[1]
+        assert max(rel_linf(cons, cref)) <= 5e-6, shape
+        assert np.array_equal(cb, cons), shape
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+def test_fp32_godunov_matches_oracle(cuda, euler, oracle_lib, shape):
+    """The per-operator FP32 godunov against the FP64 oracle on the same FP32 inputs, cubic and uneven cells: the
+    operator's bar, 2e-5 of each field's scale."""
+    O = oracle_lib
+    p32 = O.random_prim(*shape, seed=sum(shape)).astype(np.float32)
+    for dx in ((0.11, 0.07, 0.13), (0.1, 0.1, 0.1)):
+        pg = cuda.from_numpy(p32).cuda()
+        cg = euler.prim_to_cons(pg, 1.4)
+        c0 = cg.cpu().numpy().astype(np.float64)
+        euler.godunov(pg, cg, 1.4, dx, 0.01)
+        ref = O.godunov(p32.astype(np.float64), c0, 1.4, dx, 0.01)
+        assert max(rel_linf(cg.cpu().numpy(), ref)) <= 2e-5
