@@ -376,18 +376,52 @@ int step_direct(eulr_batch* b)
     return after_step(b, dir);
 }
 
-// dt of grid g's loaded state (copy 0), its clock and status zeroed.
-int prepare_grid(eulr_batch* b, int g)
+// FP32: copy 1 gets copy 0's ghost cons, whose max invdt is kept for every
+// later step (the ghost layer never changes).
+int ghost_copy_f32(eulr_batch* b, int g)
+{
+    GridState const& G = b->grids[g];
+    GhostParams<float> q{};
+    q.g = G.g;
+    q.cons_in = cbundle_of<float>(G.cons[0]);
+    q.cons_out = bundle_of<float>(G.cons[1]);
+    if (b->comp == kCompHiLo) {
+        q.lo_in = cbundle_of<float>(G.lo[0]);
+        q.lo_out = bundle_of<float>(G.lo[1]);
+    }
+    q.comp = b->comp;
+    q.gamma = static_cast<float>(G.gamma);
+    q.gm1 = q.gamma - 1.0f;
+    q.invdx0 = 1.0f / static_cast<float>(G.dx[0]);
+    q.invdx1 = 1.0f / static_cast<float>(G.dx[1]);
+    q.invdx2 = 1.0f / static_cast<float>(G.dx[2]);
+    q.wmax = &b->sc[g].ghost_wmax;
+    B_CUDA(launch_ghost_shell<float>(q, b->sms, b->stream), "ghost shell");
+    return EULR_SUCCESS;
+}
+
+// Grid g's copy 0 from FP64 prim on the device (the caller's arrays, or copy
+// 0's own for the FP64 state): state, first dt, clock and status, ghost layer.
+// FP64: keep_cons takes cons as it is instead of deriving it from prim.
+int load_grid(eulr_batch* b, int g, const double* const* prim64, bool keep_cons = false)
 {
     GridState& G = b->grids[g];
     long long const n = G.g.ncell();
     B_CUDA(cudaMemsetAsync(&b->sc[g], 0, sizeof(SimScalars), b->stream), "cudaMemsetAsync");
     if (is_f64(b)) {
+        CBundle<double> pv;
+        Bundle<double> copy{};
+        for (int f = 0; f < 5; ++f) {
+            pv.f[f] = prim64[f];
+        }
+        if (pv.f[0] != G.prim[0][0]) {
+            copy = bundle_of<double>(G.prim[0]);
+        }
         // sound speed and first wavespeed as a loaded simulation computes them
-        B_CUDA(launch_load_prim<double>(cbundle_of<double>(G.prim[0]), Bundle<double>{}, static_cast<double*>(G.cs[0]),
-                                        n, G.gamma, 1.0 / G.dx[0], 1.0 / G.dx[1], 1.0 / G.dx[2], &b->sc[g].wmax,
-                                        b->sms, b->stream, static_cast<double*>(G.h[0]),
-                                        static_cast<const double*>(G.cons[0][1])),
+        B_CUDA(launch_load_prim(pv, keep_cons ? Bundle<double>{} : bundle_of<double>(G.cons[0]), copy,
+                                static_cast<double*>(G.cs[0]), static_cast<double*>(G.h[0]),
+                                static_cast<const double*>(G.cons[0][1]), n, G.gamma, 1.0 / G.dx[0], 1.0 / G.dx[1],
+                                1.0 / G.dx[2], &b->sc[g].wmax, b->sms, b->stream),
                "load");
         B_CUDA(launch_finalize_dt<double>(&b->sc[g], b->cfl, 0, b->stream), "finalize");
         // copy 1's ghost layer once (after the first dt, which the loaded
@@ -395,63 +429,45 @@ int prepare_grid(eulr_batch* b, int g)
         B_TRY(ghost_copy(b, g, 0, 1));
         G.ghost_fix = true;
     } else {
-        float const gm = static_cast<float>(G.gamma);
-        B_CUDA(launch_invdt_max_cons(cbundle_of<float>(G.cons[0]), n, gm, 1.0f / static_cast<float>(G.dx[0]),
-                                     1.0f / static_cast<float>(G.dx[1]), 1.0f / static_cast<float>(G.dx[2]),
-                                     b->comp != kCompNone ? 1 : 0, &b->sc[g].wmax, b->sms, b->stream),
-               "invdt");
-        B_CUDA(launch_finalize_dt<float>(&b->sc[g], static_cast<float>(b->cfl), 0, b->stream), "finalize");
-        // the ghost layer never changes: copy 1 gets copy 0's ghost cons once, and its
-        // max invdt is kept for every later step
-        GhostParams<float> q{};
-        q.g = G.g;
-        q.cons_in = cbundle_of<float>(G.cons[0]);
-        q.cons_out = bundle_of<float>(G.cons[1]);
-        if (b->comp == kCompHiLo) {
-            q.lo_in = cbundle_of<float>(G.lo[0]);
-            q.lo_out = bundle_of<float>(G.lo[1]);
+        ToF32Params p{};
+        for (int f = 0; f < 5; ++f) {
+            p.prim.f[f] = prim64[f];
         }
-        q.comp = b->comp;
-        q.gamma = gm;
-        q.gm1 = gm - 1.0f;
-        q.invdx0 = 1.0f / static_cast<float>(G.dx[0]);
-        q.invdx1 = 1.0f / static_cast<float>(G.dx[1]);
-        q.invdx2 = 1.0f / static_cast<float>(G.dx[2]);
-        q.wmax = &b->sc[g].ghost_wmax;
-        B_CUDA(launch_ghost_shell<float>(q, b->sms, b->stream), "ghost shell");
+        p.hi = bundle_of<float>(G.cons[0]);
+        if (b->comp == kCompHiLo) {
+            p.lo = bundle_of<float>(G.lo[0]);
+        }
+        p.n = n;
+        p.gamma = G.gamma;
+        p.ix0 = 1.0f / static_cast<float>(G.dx[0]);
+        p.ix1 = 1.0f / static_cast<float>(G.dx[1]);
+        p.ix2 = 1.0f / static_cast<float>(G.dx[2]);
+        p.comp = b->comp;
+        p.fp32_cons = b->precision == EULR_PRECISION_F32 ? 1 : 0;
+        p.wmax = &b->sc[g].wmax;
+        B_CUDA(launch_state_to_f32(p, b->sms, b->stream), "state conversion");
+        B_CUDA(launch_finalize_dt<float>(&b->sc[g], static_cast<float>(b->cfl), 0, b->stream), "finalize");
+        B_TRY(ghost_copy_f32(b, g));
     }
     G.loaded = true;
     return EULR_SUCCESS;
 }
 
-// Loads FP64 prim (device pointers) into grid g's copy 0.
-int load_grid(eulr_batch* b, int g, double* const* prim64)
+// Grid g's clock, dt and ghost layers as its load left them, from copy 0.
+int rewind_grid(eulr_batch* b, int g)
 {
     GridState& G = b->grids[g];
-    long long const n = G.g.ncell();
     if (is_f64(b)) {
-        for (int f = 0; f < 5; ++f) {
-            B_CUDA(cudaMemcpyAsync(G.prim[0][f], prim64[f], n * sizeof(double), cudaMemcpyDefault, b->stream),
-                   "copy in");
-        }
-        double const gm1 = G.gamma - 1.0;
-        B_CUDA(launch_prim_to_cons<double>(cbundle_of<double>(G.prim[0]), bundle_of<double>(G.cons[0]), n, gm1,
-                                           1.0 / gm1, b->sms, b->stream),
-               "prim_to_cons");
-    } else {
-        CBundle<double> pv, cv{};
-        for (int f = 0; f < 5; ++f) {
-            pv.f[f] = prim64[f];
-        }
-        Bundle<float> lo{};
-        if (b->comp == kCompHiLo) {
-            lo = bundle_of<float>(G.lo[0]);
-        }
-        B_CUDA(launch_state_to_f32(pv, cv, bundle_of<float>(G.cons[0]), lo, n, G.gamma,
-                                   b->precision == EULR_PRECISION_F32 ? 1 : 0, b->sms, b->stream),
-               "state conversion");
+        return load_grid(b, g, reinterpret_cast<const double* const*>(G.prim[0]), true);
     }
-    return prepare_grid(b, g);
+    B_CUDA(cudaMemsetAsync(&b->sc[g], 0, sizeof(SimScalars), b->stream), "cudaMemsetAsync");
+    float const gm = static_cast<float>(G.gamma);
+    B_CUDA(launch_invdt_max_cons(cbundle_of<float>(G.cons[0]), G.g.ncell(), gm, 1.0f / static_cast<float>(G.dx[0]),
+                                 1.0f / static_cast<float>(G.dx[1]), 1.0f / static_cast<float>(G.dx[2]),
+                                 b->comp != kCompNone ? 1 : 0, &b->sc[g].wmax, b->sms, b->stream),
+           "invdt");
+    B_CUDA(launch_finalize_dt<float>(&b->sc[g], static_cast<float>(b->cfl), 0, b->stream), "finalize");
+    return ghost_copy_f32(b, g);
 }
 
 // Temporary FP64 fields for one grid's conversions.
@@ -662,11 +678,17 @@ int eulr_batch_set_prim_f64(eulr_batch* b, int grid, eulr_prim_cf64 prim)
     }
     long long const n = b->grids[grid].g.ncell();
     Staging st;
-    B_TRY(make_staging(n, st, 5));
-    for (int f = 0; f < 5; ++f) {
-        B_CUDA(cudaMemcpyAsync(st.f[f], src[f], n * sizeof(double), cudaMemcpyDefault, b->stream), "copy in");
+    const double* from[5];
+    if (device_fields(reinterpret_cast<const void* const*>(src), 5, n * sizeof(double), b->device, true, false)) {
+        std::copy(src, src + 5, from); // read in place
+    } else {
+        B_TRY(make_staging(n, st, 5));
+        for (int f = 0; f < 5; ++f) {
+            B_CUDA(cudaMemcpyAsync(st.f[f], src[f], n * sizeof(double), cudaMemcpyDefault, b->stream), "copy in");
+            from[f] = st.f[f];
+        }
     }
-    B_TRY(load_grid(b, grid, st.f));
+    B_TRY(load_grid(b, grid, from));
     B_CUDA(cudaStreamSynchronize(b->stream), "cudaStreamSynchronize");
     return EULR_SUCCESS;
 }
@@ -681,14 +703,16 @@ int eulr_batch_init_step(eulr_batch* b, int grid, double c, double rho_in, doubl
     }
     GridState& G = b->grids[grid];
     Staging st;
-    B_TRY(make_staging(G.g.ncell(), st, 5));
     Bundle<double> pw;
+    if (!is_f64(b)) {
+        B_TRY(make_staging(G.g.ncell(), st, 5));
+    }
     for (int f = 0; f < 5; ++f) {
-        pw.f[f] = st.f[f];
+        pw.f[f] = is_f64(b) ? static_cast<double*>(G.prim[0][f]) : st.f[f];
     }
     B_CUDA(launch_init_step(pw, G.g, G.dx[0], G.dx[1], G.dx[2], c, rho_in, p_in, rho_out, p_out, b->sms, b->stream),
            "init_step");
-    B_TRY(load_grid(b, grid, st.f));
+    B_TRY(load_grid(b, grid, pw.f));
     B_CUDA(cudaStreamSynchronize(b->stream), "cudaStreamSynchronize");
     return EULR_SUCCESS;
 }
@@ -745,7 +769,7 @@ int eulr_batch_autotune(eulr_batch* b, int trial_steps, int* shape_out, int* kch
     B_TRY(build_items(b, best_shape, best_kc));
     // the trials advanced the clocks and dt: restore them from copy 0
     for (int g = 0; g < static_cast<int>(b->grids.size()); ++g) {
-        B_TRY(prepare_grid(b, g));
+        B_TRY(rewind_grid(b, g));
     }
     B_CUDA(cudaMemsetAsync(b->d_head, 0, 2 * sizeof(unsigned), b->stream), "cudaMemsetAsync"); // head, exited
     B_CUDA(cudaStreamSynchronize(b->stream), "cudaStreamSynchronize");
@@ -831,12 +855,22 @@ int eulr_batch_get_state_f64(eulr_batch* b, int grid, eulr_prim_f64 prim, eulr_c
         B_CUDA(cudaStreamSynchronize(b->stream), "cudaStreamSynchronize");
         return EULR_SUCCESS;
     }
-    Staging st;
-    B_TRY(make_staging(n, st, 10));
-    Bundle<double> pw, cw;
+    // this device's arrays are written by the conversion itself, others
+    // through temporary FP64 fields
+    void* all[10];
     for (int i = 0; i < 5; ++i) {
-        pw.f[i] = st.f[i];
-        cw.f[i] = st.f[5 + i];
+        all[i] = pf[i];
+        all[5 + i] = cf[i];
+    }
+    bool const direct = device_fields(all, 10, bytes, b->device, false, true);
+    Staging st;
+    Bundle<double> pw, cw;
+    if (!direct) {
+        B_TRY(make_staging(n, st, 10));
+    }
+    for (int i = 0; i < 5; ++i) {
+        pw.f[i] = direct || pf[i] == nullptr ? pf[i] : st.f[i];
+        cw.f[i] = direct || cf[i] == nullptr ? cf[i] : st.f[5 + i];
     }
     CBundle<float> lo{};
     if (b->comp == kCompHiLo) {
@@ -844,7 +878,7 @@ int eulr_batch_get_state_f64(eulr_batch* b, int grid, eulr_prim_f64 prim, eulr_c
     }
     B_CUDA(launch_state_from_f32(cbundle_of<float>(G.cons[b->cur]), lo, pw, cw, n, G.gamma, b->sms, b->stream),
            "state conversion");
-    for (int i = 0; i < 5; ++i) {
+    for (int i = 0; i < 5 && !direct; ++i) {
         if (pf[i] != nullptr) {
             B_CUDA(cudaMemcpyAsync(pf[i], pw.f[i], bytes, cudaMemcpyDefault, b->stream), "copy out");
         }

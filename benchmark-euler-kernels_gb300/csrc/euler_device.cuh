@@ -251,6 +251,17 @@ __device__ __forceinline__ float pressure_f32c(float d, float e, float m0, float
     return pressure_f64_rescue(d, e, m0, m1, m2, r, gm1, lo);
 }
 
+// invdt of one cell of a cons-only FP32 state, with the pressure the fused
+// FP32 step uses (compensated states rescue low-pressure cells in FP64).
+__device__ __forceinline__ float cons_invdt_f32(float d, float e, float m0, float m1, float m2, float gamma, float gm1,
+                                                float ix0, float ix1, float ix2, bool compensated)
+{
+    float const r = 1.0f / d;
+    float const pr = compensated ? pressure_f32c(d, e, m0, m1, m2, r, gm1, nullptr)
+                                 : gm1 * (e - (0.5f * r) * (m0 * m0 + m1 * m1 + m2 * m2));
+    return cell_invdt_exact(d, pr, m0 * r, m1 * r, m2 * r, gamma, ix0, ix1, ix2);
+}
+
 // ------------------------------------------------------------------ HLLC
 // One side of a face in the face's frame: normal velocity un, tangential
 // velocities ut1/ut2 (in the cyclic order of the axes after the normal), sound

@@ -127,12 +127,12 @@ cudaError_t launch_cons_to_prim(CBundle<T> cons, Bundle<T> prim, long long n, T 
 template <class T>
 cudaError_t launch_time_step(CBundle<T> prim, long long n, T gamma, T ix0, T ix1, T ix2, T* partials,
                              int max_partials, unsigned int* counter, T* dt_out, int sms, cudaStream_t s);
-// prim_to_cons (when cons.f[0] is set), the stored sound speed and the exact
-// first max wavespeed in one pass.
-template <class T>
-cudaError_t launch_load_prim(CBundle<T> prim, Bundle<T> cons, T* cs, long long n, T gamma, T ix0, T ix1, T ix2,
-                             unsigned long long* wmax, int sms, cudaStream_t s, T* h = nullptr,
-                             const T* e_in = nullptr);
+// prim_to_cons (when cons.f[0] is set), the stored sound speed and e + p, the
+// exact first max wavespeed, and (when copy.f[0] is set) a copy of prim, in one
+// pass.
+cudaError_t launch_load_prim(CBundle<double> prim, Bundle<double> cons, Bundle<double> copy, double* cs, double* h,
+                             const double* e_in, long long n, double gamma, double ix0, double ix1, double ix2,
+                             unsigned long long* wmax, int sms, cudaStream_t s);
 // out = a + b elementwise, rounded once (the FP64 state's e + p after a restore).
 cudaError_t launch_add_fields(const double* a, const double* b, double* out, long long n, int sms, cudaStream_t s);
 cudaError_t launch_init_step(Bundle<double> prim, Geom g, double dx0, double dx1, double dx2, double c,
@@ -176,8 +176,24 @@ cudaError_t launch_batch_f32col(int comp, int tx, BatchParams<float> const* b, i
 cudaError_t launch_fma_probe(int kind, int blocks, int iters, float* sink, cudaStream_t s);
 template <class T>
 cudaError_t launch_totals(CBundle<T> cons, CBundle<T> lo, Geom g, double* work, cudaStream_t s);
-cudaError_t launch_state_to_f32(CBundle<double> prim, CBundle<double> cons, Bundle<float> hi, Bundle<float> lo,
-                                long long n, double gamma, int fp32_cons, int sms, cudaStream_t s);
+// True when every field that is not NULL (and, when all_set, every field) is
+// 8-byte aligned memory of this device, whole within one allocation, and no
+// two of them overlap when they are written: a kernel may then read or write
+// them in place of a copy.
+bool device_fields(const void* const* f, int count, size_t bytes, int device, bool all_set, bool written);
+// An FP64 state converted to an FP32 one (conversion and max invdt in one pass).
+struct ToF32Params {
+    CBundle<double> prim, cons; // cons unset: prim_to_cons of prim
+    Bundle<float> hi, lo;       // lo unset: no low words
+    long long n;
+    double gamma;
+    float ix0, ix1, ix2;
+    int comp;      // kComp* of the state: how its wavespeed takes the pressure
+    int fp32_cons; // plain FP32 state: prim rounded first, prim_to_cons in FP32
+    unsigned long long* wmax;
+};
+cudaError_t launch_state_to_f32(ToF32Params const& p, int sms, cudaStream_t s);
+// The FP64 fields that are set, from an FP32 state.
 cudaError_t launch_state_from_f32(CBundle<float> hi, CBundle<float> lo, Bundle<double> prim, Bundle<double> cons,
                                   long long n, double gamma, int sms, cudaStream_t s);
 

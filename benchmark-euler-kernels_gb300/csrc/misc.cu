@@ -3,6 +3,11 @@
 #include "euler_device.cuh"
 #include "kernels.h"
 
+#include <cudaTypedefs.h>
+
+#include <cstdint>
+#include <mutex>
+
 namespace eulr {
 
 namespace {
@@ -124,71 +129,96 @@ cudaError_t launch_totals(CBundle<T> cons, CBundle<T> lo, Geom g, double* work, 
 // `fp32_cons` (plain FP32 mode) cons is instead prim_to_cons of the prim
 // rounded to FP32, computed in FP32 as the reference's real_t = float build
 // does.
-__global__ void __launch_bounds__(256) state_to_f32_kernel(CBundle<double> prim, CBundle<double> cons, Bundle<float> hi,
-                                                           Bundle<float> lo, long long n, double gamma, int fp32_cons)
+// The max invdt of the new state is taken in the same pass: FP64 conversions
+// bound it, and the FP32 wavespeed is nearly free beside them.
+__global__ void __launch_bounds__(256) state_to_f32_kernel(const __grid_constant__ ToF32Params p)
 {
-    double const gm1 = gamma - 1.0;
+    double const gm1 = p.gamma - 1.0;
     double const rgm1 = 1.0 / gm1;
-    float const gm1f = static_cast<float>(gamma) - 1.0f;
+    float const gammaf = static_cast<float>(p.gamma);
+    float const gm1f = gammaf - 1.0f;
     float const rgm1f = 1.0f / gm1f;
-    for (long long c = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; c < n;
+    float local = 0.0f;
+    for (long long c = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; c < p.n;
          c += static_cast<long long>(gridDim.x) * blockDim.x) {
-        if (fp32_cons) {
+        float h[5];
+        if (p.fp32_cons) {
             float q[5];
 #pragma unroll
             for (int f = 0; f < 5; ++f) {
-                q[f] = static_cast<float>(prim.f[f][c]);
+                q[f] = static_cast<float>(p.prim.f[f][c]);
             }
             float const int_e = div_by_rcp(q[1], gm1f, rgm1f);
             float const ke =
                     mul_rn(mul_rn(q[0], add_rn(add_rn(mul_rn(q[2], q[2]), mul_rn(q[3], q[3])), mul_rn(q[4], q[4]))),
                            0.5f);
-            hi.f[0][c] = q[0];
-            hi.f[1][c] = add_rn(ke, int_e);
-            hi.f[2][c] = mul_rn(q[0], q[2]);
-            hi.f[3][c] = mul_rn(q[0], q[3]);
-            hi.f[4][c] = mul_rn(q[0], q[4]);
-            continue;
-        }
-        double u[5];
-        if (cons.f[0] != nullptr) {
-#pragma unroll
-            for (int f = 0; f < 5; ++f) {
-                u[f] = cons.f[f][c];
-            }
+            h[0] = q[0];
+            h[1] = add_rn(ke, int_e);
+            h[2] = mul_rn(q[0], q[2]);
+            h[3] = mul_rn(q[0], q[3]);
+            h[4] = mul_rn(q[0], q[4]);
         } else {
-            double q[5];
+            double u[5];
+            if (p.cons.f[0] != nullptr) {
+#pragma unroll
+                for (int f = 0; f < 5; ++f) {
+                    u[f] = p.cons.f[f][c];
+                }
+            } else {
+                double q[5];
+#pragma unroll
+                for (int f = 0; f < 5; ++f) {
+                    q[f] = p.prim.f[f][c];
+                }
+                double const int_e = div_by_rcp(q[1], gm1, rgm1);
+                double const ke = half_exact(
+                        mul_rn(q[0], add_rn(add_rn(mul_rn(q[2], q[2]), mul_rn(q[3], q[3])), mul_rn(q[4], q[4]))));
+                u[0] = q[0];
+                u[1] = add_rn(ke, int_e);
+                u[2] = mul_rn(q[0], q[2]);
+                u[3] = mul_rn(q[0], q[3]);
+                u[4] = mul_rn(q[0], q[4]);
+            }
 #pragma unroll
             for (int f = 0; f < 5; ++f) {
-                q[f] = prim.f[f][c];
+                h[f] = static_cast<float>(u[f]);
+                if (p.lo.f[0] != nullptr) {
+                    p.lo.f[f][c] = static_cast<float>(u[f] - static_cast<double>(h[f]));
+                }
             }
-            double const int_e = div_by_rcp(q[1], gm1, rgm1);
-            double const ke =
-                    mul_rn(mul_rn(q[0], add_rn(add_rn(mul_rn(q[2], q[2]), mul_rn(q[3], q[3])), mul_rn(q[4], q[4]))),
-                           0.5);
-            u[0] = q[0];
-            u[1] = add_rn(ke, int_e);
-            u[2] = mul_rn(q[0], q[2]);
-            u[3] = mul_rn(q[0], q[3]);
-            u[4] = mul_rn(q[0], q[4]);
         }
 #pragma unroll
         for (int f = 0; f < 5; ++f) {
-            float const h = static_cast<float>(u[f]);
-            hi.f[f][c] = h;
-            if (lo.f[0] != nullptr) {
-                lo.f[f][c] = static_cast<float>(u[f] - static_cast<double>(h));
-            }
+            p.hi.f[f][c] = h[f];
         }
+        float const v = cons_invdt_f32(h[0], h[1], h[2], h[3], h[4], gammaf, gm1f, p.ix0, p.ix1, p.ix2,
+                                       p.comp != kCompNone);
+        local = (v > local) ? v : local;
+    }
+    __shared__ float warp_best[8];
+    local = warp_max(local);
+    if ((threadIdx.x & 31) == 0) {
+        warp_best[threadIdx.x >> 5] = local;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        float b = warp_best[0];
+        for (int w = 1; w < static_cast<int>(blockDim.x >> 5); ++w) {
+            b = (warp_best[w] > b) ? warp_best[w] : b;
+        }
+        atomicMax(p.wmax, order_bits(b));
     }
 }
 
 // Cons-only FP32 simulation state -> FP64: cons = hi (+ lo) in FP64 and prim
-// = cons_to_prim of it in FP64 (the reference's formula, cons_to_prim.hpp).
+// = cons_to_prim of it in FP64 (the reference's formula, cons_to_prim.hpp);
+// only the fields that are set.
 __global__ void __launch_bounds__(256) state_from_f32_kernel(CBundle<float> hi, CBundle<float> lo, Bundle<double> prim,
                                                              Bundle<double> cons, long long n, double gamma)
 {
     double const gm1 = gamma - 1.0;
+    bool const want_prim = prim.f[0] != nullptr || prim.f[1] != nullptr || prim.f[2] != nullptr ||
+                           prim.f[3] != nullptr || prim.f[4] != nullptr;
     for (long long c = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; c < n;
          c += static_cast<long long>(gridDim.x) * blockDim.x) {
         double u[5];
@@ -198,18 +228,20 @@ __global__ void __launch_bounds__(256) state_from_f32_kernel(CBundle<float> hi, 
             if (lo.f[0] != nullptr) {
                 u[f] += static_cast<double>(lo.f[f][c]);
             }
-            if (cons.f[0] != nullptr) {
+            if (cons.f[f] != nullptr) {
                 cons.f[f][c] = u[f];
             }
         }
-        if (prim.f[0] != nullptr) {
-            double pr, v0, v1, v2;
-            cons_to_prim_exact(u[0], u[1], u[2], u[3], u[4], gm1, pr, v0, v1, v2);
-            prim.f[0][c] = u[0];
-            prim.f[1][c] = pr;
-            prim.f[2][c] = v0;
-            prim.f[3][c] = v1;
-            prim.f[4][c] = v2;
+        if (want_prim) {
+            double q[5];
+            q[0] = u[0];
+            cons_to_prim_exact(u[0], u[1], u[2], u[3], u[4], gm1, q[1], q[2], q[3], q[4]);
+#pragma unroll
+            for (int f = 0; f < 5; ++f) {
+                if (prim.f[f] != nullptr) {
+                    prim.f[f][c] = q[f];
+                }
+            }
         }
     }
 }
@@ -221,11 +253,55 @@ static int grid256(long long n, int sms)
     return static_cast<int>(b < 1 ? 1 : (b < cap ? b : cap));
 }
 
-cudaError_t launch_state_to_f32(CBundle<double> prim, CBundle<double> cons, Bundle<float> hi, Bundle<float> lo,
-                                long long n, double gamma, int fp32_cons, int sms, cudaStream_t s)
+cudaError_t launch_state_to_f32(ToF32Params const& p, int sms, cudaStream_t s)
 {
-    state_to_f32_kernel<<<grid256(n, sms), 256, 0, s>>>(prim, cons, hi, lo, n, gamma, fp32_cons);
+    state_to_f32_kernel<<<grid256(p.n, sms), 256, 0, s>>>(p);
     return cudaGetLastError();
+}
+
+bool device_fields(const void* const* f, int count, size_t bytes, int device, bool all_set, bool written)
+{
+    // cuMemGetAddressRange from the driver, looked up once through the runtime
+    static std::once_flag once;
+    static PFN_cuMemGetAddressRange_v3020 range = nullptr;
+    std::call_once(once, [] {
+        void* p = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPointByVersion("cuMemGetAddressRange", &p, 3020, cudaEnableDefault, &q) == cudaSuccess &&
+            q == cudaDriverEntryPointSuccess) {
+            range = reinterpret_cast<PFN_cuMemGetAddressRange_v3020>(p);
+        }
+    });
+    if (range == nullptr) {
+        return false;
+    }
+    for (int i = 0; i < count; ++i) {
+        if (f[i] == nullptr) {
+            if (all_set) {
+                return false;
+            }
+            continue;
+        }
+        auto const a = reinterpret_cast<std::uintptr_t>(f[i]);
+        cudaPointerAttributes at{};
+        if (cudaPointerGetAttributes(&at, f[i]) != cudaSuccess) {
+            (void)cudaGetLastError();
+            return false;
+        }
+        CUdeviceptr base = 0;
+        size_t size = 0;
+        if (at.type != cudaMemoryTypeDevice || at.device != device || a % sizeof(double) != 0 ||
+            range(&base, &size, static_cast<CUdeviceptr>(a)) != CUDA_SUCCESS || a - base + bytes > size) {
+            return false;
+        }
+        for (int j = 0; written && j < i; ++j) {
+            auto const b = reinterpret_cast<std::uintptr_t>(f[j]);
+            if (f[j] != nullptr && a < b + bytes && b < a + bytes) {
+                return false;
+            }
+        }
+    }
+    return true;
 }
 
 cudaError_t launch_state_from_f32(CBundle<float> hi, CBundle<float> lo, Bundle<double> prim, Bundle<double> cons,

@@ -173,8 +173,7 @@ __global__ void __launch_bounds__(256) time_step_kernel(CBundle<T> prim, long lo
     }
 }
 
-// Max invdt over all cells of a cons-only FP32 state, with the pressure the
-// fused FP32 step uses (compensated states rescue low-pressure cells in FP64).
+// Max invdt over all cells of a cons-only FP32 state.
 __global__ void __launch_bounds__(256) invdt_max_cons_kernel(CBundle<float> cons, long long n, float gamma, float ix0,
                                                              float ix1, float ix2, int comp, unsigned long long* wmax)
 {
@@ -182,15 +181,8 @@ __global__ void __launch_bounds__(256) invdt_max_cons_kernel(CBundle<float> cons
     float const gm1 = gamma - 1.0f;
     for (long long c = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; c < n;
          c += static_cast<long long>(gridDim.x) * blockDim.x) {
-        float const d = cons.f[0][c];
-        float const e = cons.f[1][c];
-        float const m0 = cons.f[2][c];
-        float const m1 = cons.f[3][c];
-        float const m2 = cons.f[4][c];
-        float const r = 1.0f / d;
-        float const pr = comp ? pressure_f32c(d, e, m0, m1, m2, r, gm1, nullptr)
-                              : gm1 * (e - (0.5f * r) * (m0 * m0 + m1 * m1 + m2 * m2));
-        float const v = cell_invdt_exact(d, pr, m0 * r, m1 * r, m2 * r, gamma, ix0, ix1, ix2);
+        float const v = cons_invdt_f32(cons.f[0][c], cons.f[1][c], cons.f[2][c], cons.f[3][c], cons.f[4][c], gamma, gm1, ix0,
+                                       ix1, ix2, comp);
         local = (v > local) ? v : local;
     }
     __shared__ float warp_best[8];
@@ -209,21 +201,23 @@ __global__ void __launch_bounds__(256) invdt_max_cons_kernel(CBundle<float> cons
 }
 
 // Loading a primitive state into an FP64 simulation or batch grid, in one
-// pass:
+// pass (bound by the FP64 pipe, so what it also moves is nearly free):
+//  * prim itself when copy is set -- the caller's device arrays are read in
+//    place, not copied first (10.9 GB of traffic less at 514^3);
 //  * cons = prim_to_cons(prim) when cons is set, bit-identical to
 //    prim_to_cons_kernel;
 //  * the stored sound speed in the form the fused step stores it
 //    (fast_sound_speed of (gamma/rho) p, faithful), so a loaded state and a
-//    stepped one carry the same kind of value;
+//    stepped one carry the same kind of value, and e + p;
 //  * the EXACT max wavespeed of time_step.hpp:28-33 for the first dt, with
 //    the exact per-cell value evaluated only where WaveScreen says it can be
 //    the max.
-template <class T>
-__global__ void __launch_bounds__(256) load_prim_kernel(CBundle<T> prim, Bundle<T> cons, T* cs, long long n, T gamma,
-                                                        T gm1, T rgm1, T ix0, T ix1, T ix2, unsigned long long* wmax,
-                                                        T* h, const T* e_in)
+__global__ void __launch_bounds__(256) load_prim_kernel(CBundle<double> prim, Bundle<double> cons, Bundle<double> copy,
+                                                        double* cs, double* h, const double* e_in, long long n,
+                                                        double gamma, double gm1, double rgm1, double ix0, double ix1,
+                                                        double ix2, unsigned long long* wmax)
 {
-    T local = T(0);
+    double local = 0.0;
     WaveScreen screen(gamma, ix0, ix1, ix2);
     int const lane = threadIdx.x & 31;
     long long const stride = static_cast<long long>(gridDim.x) * blockDim.x;
@@ -232,51 +226,48 @@ __global__ void __launch_bounds__(256) load_prim_kernel(CBundle<T> prim, Bundle<
          base += stride) {
         long long const c = base + lane;
         bool const valid = c < n;
-        T d = T(1), p = T(1), u0 = T(0), u1 = T(0), u2 = T(0);
+        double d = 1.0, p = 1.0, u0 = 0.0, u1 = 0.0, u2 = 0.0;
         if (valid) {
             d = prim.f[0][c];
             p = prim.f[1][c];
             u0 = prim.f[2][c];
             u1 = prim.f[3][c];
             u2 = prim.f[4][c];
+            if (copy.f[0] != nullptr) {
+                copy.f[0][c] = d;
+                copy.f[1][c] = p;
+                copy.f[2][c] = u0;
+                copy.f[3][c] = u1;
+                copy.f[4][c] = u2;
+            }
             if (cons.f[0] != nullptr) {
-                T const int_e = div_by_rcp(p, gm1, rgm1);
-                T const ke = half_exact(mul_rn(d, add_rn(add_rn(mul_rn(u0, u0), mul_rn(u1, u1)), mul_rn(u2, u2))));
-                T const e = add_rn(ke, int_e);
+                double const int_e = div_by_rcp(p, gm1, rgm1);
+                double const ke = half_exact(mul_rn(d, add_rn(add_rn(mul_rn(u0, u0), mul_rn(u1, u1)), mul_rn(u2, u2))));
+                double const e = add_rn(ke, int_e);
                 cons.f[0][c] = d;
                 cons.f[1][c] = e;
                 cons.f[2][c] = mul_rn(d, u0);
                 cons.f[3][c] = mul_rn(d, u1);
                 cons.f[4][c] = mul_rn(d, u2);
-                if (h != nullptr) {
-                    h[c] = add_rn(e, p);
-                }
-            } else if (h != nullptr) {
+                h[c] = add_rn(e, p);
+            } else {
                 h[c] = add_rn(e_in[c], p);
             }
+            cs[c] = sqrt_quotient_faithful(gamma * p, d); // 1/rho is not needed here
         }
-        bool cand = valid;
-        if constexpr (sizeof(T) == 8) {
-            if (valid) {
-                cs[c] = sqrt_quotient_faithful(gamma * p, d); // 1/rho is not needed here
-            }
-            cand = screen.exact_needed(valid, d, p, u0, u1, u2);
-        } else if (valid) {
-            cs[c] = sqrt_rn(div_rn(mul_rn(gamma, p), d));
-        }
-        if (cand) {
-            T const v = cell_invdt_exact(d, p, u0, u1, u2, gamma, ix0, ix1, ix2);
+        if (screen.exact_needed(valid, d, p, u0, u1, u2)) {
+            double const v = cell_invdt_exact(d, p, u0, u1, u2, gamma, ix0, ix1, ix2);
             local = (v > local) ? v : local; // NaN never wins
         }
     }
-    __shared__ T warp_best[8];
+    __shared__ double warp_best[8];
     local = warp_max(local);
     if (lane == 0) {
         warp_best[threadIdx.x >> 5] = local;
     }
     __syncthreads();
     if (threadIdx.x == 0) {
-        T b = warp_best[0];
+        double b = warp_best[0];
         for (int w = 1; w < static_cast<int>(blockDim.x >> 5); ++w) {
             b = (warp_best[w] > b) ? warp_best[w] : b;
         }
@@ -354,13 +345,13 @@ cudaError_t launch_time_step(CBundle<T> prim, long long n, T gamma, T ix0, T ix1
     return cudaGetLastError();
 }
 
-template <class T>
-cudaError_t launch_load_prim(CBundle<T> prim, Bundle<T> cons, T* cs, long long n, T gamma, T ix0, T ix1, T ix2,
-                             unsigned long long* wmax, int sms, cudaStream_t s, T* h, const T* e_in)
+cudaError_t launch_load_prim(CBundle<double> prim, Bundle<double> cons, Bundle<double> copy, double* cs, double* h,
+                             const double* e_in, long long n, double gamma, double ix0, double ix1, double ix2,
+                             unsigned long long* wmax, int sms, cudaStream_t s)
 {
-    T const gm1 = gamma - T(1);
-    load_prim_kernel<T><<<grid_for(n, sms), 256, 0, s>>>(prim, cons, cs, n, gamma, gm1, T(1) / gm1, ix0, ix1, ix2,
-                                                          wmax, h, e_in);
+    double const gm1 = gamma - 1.0;
+    load_prim_kernel<<<grid_for(n, sms), 256, 0, s>>>(prim, cons, copy, cs, h, e_in, n, gamma, gm1, 1.0 / gm1, ix0, ix1,
+                                                      ix2, wmax);
     return cudaGetLastError();
 }
 
@@ -398,9 +389,7 @@ cudaError_t launch_invdt_max_cons(CBundle<float> cons, long long n, float gamma,
     template cudaError_t launch_prim_to_cons<T>(CBundle<T>, Bundle<T>, long long, T, T, int, cudaStream_t);  \
     template cudaError_t launch_cons_to_prim<T>(CBundle<T>, Bundle<T>, long long, T, int, cudaStream_t);     \
     template cudaError_t launch_time_step<T>(CBundle<T>, long long, T, T, T, T, T*, int, unsigned int*, T*,  \
-                                             int, cudaStream_t);                                             \
-    template cudaError_t launch_load_prim<T>(CBundle<T>, Bundle<T>, T*, long long, T, T, T, T, unsigned long long*,    \
-                                             int, cudaStream_t, T*, const T*);
+                                             int, cudaStream_t);
 
 EULR_INSTANTIATE_POINTWISE(double)
 EULR_INSTANTIATE_POINTWISE(float)

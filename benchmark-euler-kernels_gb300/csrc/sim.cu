@@ -370,41 +370,66 @@ int step_direct(eulr_sim* s, cudaEvent_t* ev = nullptr)
     return after_step(s);
 }
 
-// After a state was loaded into copy 0: sound speed (FP64 state), dt of the
-// state, zeroed clock and status.
-// Resets the clocks of copy 0 and computes its first dt.  FP64: with
-// derive_cons, cons = prim_to_cons(prim) is computed in the same pass as the
-// sound speed and the wavespeed (launch_load_prim); otherwise cons is taken
-// as loaded.
-int prepare_loaded(eulr_sim* s, bool derive_cons = false)
+// Resets the clocks of a state being loaded into copy 0.
+int reset_clocks(eulr_sim* s)
 {
     s->cur = 0;
     s->host_steps = 0;
     SIM_CUDA(cudaMemsetAsync(s->sc, 0, sizeof(SimScalars), s->stream), "cudaMemsetAsync");
-    if (is_f64(s)) {
-        CBundle<double> pv = cbundle_of<double>(s->prim[0]);
-        Bundle<double> cv{};
-        if (derive_cons) {
-            cv = bundle_of<double>(s->cons[0]);
-        }
-        SIM_CUDA(launch_load_prim<double>(pv, cv, static_cast<double*>(s->cs[0]), ncell(s), s->gamma, 1.0 / s->dx[0],
-                                          1.0 / s->dx[1], 1.0 / s->dx[2], &s->sc->wmax, s->sms, s->stream,
-                                          static_cast<double*>(s->h[0]),
-                                          derive_cons ? nullptr : static_cast<const double*>(s->cons[0][1])),
-                 "load launch");
-        SIM_CUDA(launch_finalize_dt<double>(s->sc, s->cfl, 0, s->stream), "finalize launch");
-        SIM_TRY(set_ghost_layer(s)); // after the first dt, which the loaded ghost prim sets
-    } else {
-        float const g = static_cast<float>(s->gamma);
-        SIM_CUDA(launch_invdt_max_cons(cbundle_of<float>(s->cons[0]), ncell(s), g, 1.0f / static_cast<float>(s->dx[0]),
-                                       1.0f / static_cast<float>(s->dx[1]), 1.0f / static_cast<float>(s->dx[2]),
-                                       s->comp != kCompNone ? 1 : 0, &s->sc->wmax, s->sms, s->stream),
-                 "invdt launch");
-        SIM_CUDA(launch_finalize_dt<float>(s->sc, static_cast<float>(s->cfl), 0, s->stream), "finalize launch");
-        // the ghost layer, once for every later step: copy 1 gets copy 0's ghost cons
-        SIM_CUDA(launch_ghost_shell<float>(ghost_params<float>(s, 0, 1, &s->sc->ghost_wmax), s->sms, s->stream),
-                 "ghost shell launch");
+    return EULR_SUCCESS;
+}
+
+// The FP64 state of copy 0 from prim (the caller's device arrays, copied in
+// the same pass, or copy 0's own): the sound speed, e + p, the first dt and
+// the ghost layer; with derive_cons also cons = prim_to_cons(prim), else cons
+// is taken as loaded.
+int load_f64(eulr_sim* s, CBundle<double> prim, bool derive_cons)
+{
+    SIM_TRY(reset_clocks(s));
+    Bundle<double> cv{}, copy{};
+    if (derive_cons) {
+        cv = bundle_of<double>(s->cons[0]);
     }
+    if (prim.f[0] != s->prim[0][0]) {
+        copy = bundle_of<double>(s->prim[0]);
+    }
+    SIM_CUDA(launch_load_prim(prim, cv, copy, static_cast<double*>(s->cs[0]), static_cast<double*>(s->h[0]),
+                              static_cast<const double*>(s->cons[0][1]), ncell(s), s->gamma, 1.0 / s->dx[0],
+                              1.0 / s->dx[1], 1.0 / s->dx[2], &s->sc->wmax, s->sms, s->stream),
+             "load launch");
+    SIM_CUDA(launch_finalize_dt<double>(s->sc, s->cfl, 0, s->stream), "finalize launch");
+    SIM_TRY(set_ghost_layer(s)); // after the first dt, which the loaded ghost prim sets
+    s->loaded = true;
+    return EULR_SUCCESS;
+}
+
+// An FP32 state's copy 0 from FP64 prim (and cons, or NULL to derive it) on
+// the device, with its first dt and ghost layer.
+int load_f32(eulr_sim* s, const double* const* prim64, const double* const* cons64)
+{
+    SIM_TRY(reset_clocks(s));
+    ToF32Params p{};
+    for (int i = 0; i < 5; ++i) {
+        p.prim.f[i] = prim64[i];
+        p.cons.f[i] = cons64 != nullptr ? cons64[i] : nullptr;
+    }
+    p.hi = bundle_of<float>(s->cons[0]);
+    if (s->comp == kCompHiLo) {
+        p.lo = bundle_of<float>(s->lo[0]);
+    }
+    p.n = ncell(s);
+    p.gamma = s->gamma;
+    p.ix0 = 1.0f / static_cast<float>(s->dx[0]);
+    p.ix1 = 1.0f / static_cast<float>(s->dx[1]);
+    p.ix2 = 1.0f / static_cast<float>(s->dx[2]);
+    p.comp = s->comp;
+    p.fp32_cons = s->precision == EULR_PRECISION_F32 ? 1 : 0;
+    p.wmax = &s->sc->wmax;
+    SIM_CUDA(launch_state_to_f32(p, s->sms, s->stream), "state conversion");
+    SIM_CUDA(launch_finalize_dt<float>(s->sc, static_cast<float>(s->cfl), 0, s->stream), "finalize launch");
+    // the ghost layer, once for every later step: copy 1 gets copy 0's ghost cons
+    SIM_CUDA(launch_ghost_shell<float>(ghost_params<float>(s, 0, 1, &s->sc->ghost_wmax), s->sms, s->stream),
+             "ghost shell launch");
     s->loaded = true;
     return EULR_SUCCESS;
 }
@@ -444,33 +469,32 @@ int copy_in(eulr_sim* s, void* const* dst, const double* const* src)
     return EULR_SUCCESS;
 }
 
-// Load FP64 prim (and cons, or nullptr to derive it) already on the device
-// into an FP32 state's copy 0.
-int load_f32(eulr_sim* s, double* const* prim64, double* const* cons64)
-{
-    CBundle<double> pv, cv;
-    for (int i = 0; i < 5; ++i) {
-        pv.f[i] = prim64[i];
-        cv.f[i] = cons64 != nullptr ? cons64[i] : nullptr;
-    }
-    Bundle<float> lo{};
-    if (s->comp == kCompHiLo) {
-        lo = bundle_of<float>(s->lo[0]);
-    }
-    SIM_CUDA(launch_state_to_f32(pv, cv, bundle_of<float>(s->cons[0]), lo, ncell(s), s->gamma,
-                                 s->precision == EULR_PRECISION_F32 ? 1 : 0, s->sms, s->stream),
-             "state conversion");
-    return EULR_SUCCESS;
-}
-
+// The caller's arrays are read in place where they are this device's memory
+// and copied in first (FP32 states: to temporary FP64 fields) where not.
 int set_state_impl(eulr_sim* s, const double* const* prim, const double* const* cons)
 {
+    size_t const bytes = static_cast<size_t>(ncell(s)) * sizeof(double);
+    bool const direct = device_fields(reinterpret_cast<const void* const*>(prim), 5, bytes, s->device, true, false) &&
+                        (cons == nullptr ||
+                         device_fields(reinterpret_cast<const void* const*>(cons), 5, bytes, s->device, true, false));
     if (is_f64(s)) {
-        SIM_TRY(copy_in(s, s->prim[0], prim));
+        CBundle<double> pv = cbundle_of<double>(s->prim[0]);
+        if (direct) {
+            for (int i = 0; i < 5; ++i) {
+                pv.f[i] = prim[i];
+            }
+        } else {
+            SIM_TRY(copy_in(s, s->prim[0], prim));
+        }
         if (cons != nullptr) {
             SIM_TRY(copy_in(s, s->cons[0], cons));
         }
-        return prepare_loaded(s, cons == nullptr);
+        return load_f64(s, pv, cons == nullptr);
+    }
+    if (direct) {
+        SIM_TRY(load_f32(s, prim, cons));
+        SIM_CUDA(cudaStreamSynchronize(s->stream), "cudaStreamSynchronize"); // the arrays are the caller's again
+        return EULR_SUCCESS;
     }
     Staging st;
     SIM_TRY(make_staging(s, st, cons != nullptr ? 10 : 5));
@@ -485,7 +509,6 @@ int set_state_impl(eulr_sim* s, const double* const* prim, const double* const* 
         SIM_TRY(copy_in(s, cd, cons));
     }
     SIM_TRY(load_f32(s, st.f, cons != nullptr ? st.f + 5 : nullptr));
-    SIM_TRY(prepare_loaded(s));
     SIM_CUDA(cudaStreamSynchronize(s->stream), "cudaStreamSynchronize"); // staging is freed next
     return EULR_SUCCESS;
 }
@@ -729,7 +752,7 @@ int eulr_sim_init_implode(eulr_sim* s)
         SIM_CUDA(launch_init_implode<double>(bundle_of<double>(s->prim[0]), s->g, s->dx[0], s->dx[1], s->dx[2], s->sms,
                                              s->stream),
                  "init_implode");
-        return prepare_loaded(s, true);
+        return load_f64(s, cbundle_of<double>(s->prim[0]), true);
     }
     // FP32 states: the FP64 implosion state, converted on the device
     Staging st;
@@ -740,7 +763,6 @@ int eulr_sim_init_implode(eulr_sim* s)
     }
     SIM_CUDA(launch_init_implode<double>(pw, s->g, s->dx[0], s->dx[1], s->dx[2], s->sms, s->stream), "init_implode");
     SIM_TRY(load_f32(s, st.f, nullptr));
-    SIM_TRY(prepare_loaded(s));
     SIM_CUDA(cudaStreamSynchronize(s->stream), "cudaStreamSynchronize");
     return EULR_SUCCESS;
 }
@@ -812,12 +834,22 @@ int eulr_sim_get_state_f64(eulr_sim* s, eulr_prim_f64 prim, eulr_cons_f64 cons)
         SIM_CUDA(cudaStreamSynchronize(s->stream), "cudaStreamSynchronize");
         return EULR_SUCCESS;
     }
-    Staging st;
-    SIM_TRY(make_staging(s, st, 10));
-    Bundle<double> pw, cw;
+    // this device's arrays are written by the conversion itself, others
+    // through temporary FP64 fields
+    void* all[10];
     for (int i = 0; i < 5; ++i) {
-        pw.f[i] = st.f[i];
-        cw.f[i] = st.f[5 + i];
+        all[i] = pf[i];
+        all[5 + i] = cf[i];
+    }
+    bool const direct = device_fields(all, 10, bytes, s->device, false, true);
+    Staging st;
+    Bundle<double> pw, cw;
+    if (!direct) {
+        SIM_TRY(make_staging(s, st, 10));
+    }
+    for (int i = 0; i < 5; ++i) {
+        pw.f[i] = direct || pf[i] == nullptr ? pf[i] : st.f[i];
+        cw.f[i] = direct || cf[i] == nullptr ? cf[i] : st.f[5 + i];
     }
     CBundle<float> lo{};
     if (s->comp == kCompHiLo) {
@@ -826,7 +858,7 @@ int eulr_sim_get_state_f64(eulr_sim* s, eulr_prim_f64 prim, eulr_cons_f64 cons)
     SIM_CUDA(launch_state_from_f32(cbundle_of<float>(s->cons[s->cur]), lo, pw, cw, ncell(s), s->gamma, s->sms,
                                    s->stream),
              "state conversion");
-    for (int i = 0; i < 5; ++i) {
+    for (int i = 0; i < 5 && !direct; ++i) {
         if (pf[i] != nullptr) {
             SIM_CUDA(cudaMemcpyAsync(pf[i], pw.f[i], bytes, cudaMemcpyDefault, s->stream), "copy out");
         }
