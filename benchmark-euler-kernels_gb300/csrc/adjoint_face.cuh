@@ -103,50 +103,15 @@ struct FaceBar {
 
 EULR_ADJ_FN void zero(FaceBar& b) { b.r = b.p = b.un = b.t1 = b.t2 = 0.0; }
 
-// Subsonic star-state branch of the upwind side q (hllc.hpp:78-102 with
-// S = S_q): for the cotangent (gd, ge, gn, gt1, gt2) of the face flux it SETS
-// gus (d/d ustar), gps (d/d pstar) and bq (d/d q's primitives) and returns
-// d/d S_q.  a = S_q - un_q, iY = 1/(S_q - ustar).
-EULR_ADJ_FN double star_branch_bar(FaceSide const& q, double a, double iY, double ustar, double pstar, double gd,
-                                   double ge, double gn, double gt1, double gt2, double inv_gm1, double& gus,
-                                   double& gps, FaceBar& bq)
+// One side's share of d flux / d ustar at ustar == 0 (a = S - un of the side,
+// iS = 1/S): there the flux's mass and energy terms are b d and b E with
+// b = a ustar/(S - ustar) and E = e + p + S d w, w = ustar - un.
+EULR_ADJ_FN double tie_side_bar(FaceSide const& q, double a, double S, double iS, double gd, double ge, double gt1,
+                                double gt2)
 {
-    // forward: ratio = (S - un)/(S - ustar), d_o = ratio rho, etot_o = ratio e + X/(S - ustar),
-    // X = pstar ustar - p un; fluxes m = d_o ustar; (m, (etot_o + pstar) ustar, m ustar + pstar, m t1, m t2)
-    double const r = a * iY;
-    double const X = pstar * ustar - q.p * q.un;
-    double const Xy = X * iY;
-    double const d_o = r * q.r;
-    double const eo = r * q.e + Xy;
-    double const m = d_o * ustar;
-    double const gm = gd + gn * ustar + gt1 * q.t1 + gt2 * q.t2;
-    double const gE = ge * ustar;           // d/d etot_o
-    double const gdo = gm * ustar;          // d/d d_o
-    double const gr = gdo * q.r + gE * q.e; // d/d ratio
-    double const geq = gE * r;              // d/d e (side total energy)
-    double const gX = gE * iY;
-    double const gY = -(gE * Xy + gr * r) * iY; // d/d (S - ustar)
-    double const ga = gr * iY;                  // d/d (S - un)
-    gps = gn + ge * ustar + gX * ustar;
-    gus = gn * m + ge * (eo + pstar) + gm * d_o + gX * pstar - gY;
-    bq.r = gdo * r + geq * q.ke;
-    bq.p = geq * inv_gm1 - gX * q.un;
-    bq.un = geq * (q.r * q.un) - gX * q.p - ga;
-    bq.t1 = gt1 * m + geq * (q.r * q.t1);
-    bq.t2 = gt2 * m + geq * (q.r * q.t2);
-    return gY + ga;
-}
-
-// star_branch_bar at ustar == 0 (iS = 1/S_Q): returns the branch's d/d ustar;
-// its d/d pstar is gn and it adds nothing to bq or d/d S_Q.
-EULR_ADJ_FN double tie_branch_bar(FaceSide const& q, double a, double iS, double pstar, double gd, double ge,
-                                  double gt1, double gt2)
-{
-    double const r = a * iS;
-    double const d_o = r * q.r;
-    double const eo = r * q.e - (q.p * q.un) * iS;
-    double const gm = gd + gt1 * q.t1 + gt2 * q.t2;
-    return ge * (eo + pstar) + gm * d_o;
+    double const E = (q.e + q.p) - S * (q.r * q.un);
+    double const gb = (gd + gt1 * q.t1 + gt2 * q.t2) * q.r + ge * E;
+    return gb * (a * iS);
 }
 
 // Transposed HLLC flux of one face (hllc.hpp:50-105).  The cotangent of the
@@ -155,37 +120,41 @@ EULR_ADJ_FN double tie_branch_bar(FaceSide const& q, double a, double iS, double
 // ds into (dd, ..., dt2) and ds is not read.  SETS the cotangents of the two
 // sides' primitive states, bL and bR.
 //
+// What is transposed is the flux in the forward step's form (hllc_flux in
+// euler_device.cuh), which is the reference's in exact arithmetic:
+//   A = cmax + max(u_L - u_R, 0), G = A (d_L + d_R),
+//   n = A (d_L u_L + d_R u_R) - (p_R - p_L), ustar = n/G,
+//   and with the upwind side's S = u + a, a = -+A, w = ustar - u and
+//   b = a ustar/(S - ustar):  mass d b, energy b (e + p + S d w), normal
+//   momentum d b ustar + p + a d w, tangential d b t.
+// One acoustic speed in place of two wave speeds and two impedances: about 83
+// FP64 instructions a face where the form with both took 103.  The pressure
+// term is the upwind side's, p_q + rc_q (ustar - un_q): the reference's mean
+// of the two sides' values is the same function wherever ustar = num/den.
+//
 // Written for SIMT: the upwind side q (L when ustar > 0) is selected field by
 // field instead of branching on it, so a warp whose faces point both ways
 // runs the star branch once, not twice; only the rare supersonic faces and
-// the ustar == 0 ties take their own paths.  pstar is differentiated in its
-// upwind form p_q + rc_q (ustar - un_q): the reference's mean of the two
-// sides' values is the same function wherever ustar = num/den (their
-// difference is (num - ustar den)/2), so the total derivative is the same.
+// the ustar == 0 ties take their own paths.
 template <bool UNIT = false>
 EULR_ADJ_FN void hllc_bar(FaceSide const& L, FaceSide const& R, double dd, double de, double dn, double dt1,
                           double dt2, double ds, double inv_gm1, FaceBar& bL, FaceBar& bR)
 {
-    // S_L = min(un_L, un_R) - max(c_L, c_R), S_R = max(un_L, un_R) + max(c_L, c_R)
     long long const kuL = adj_key(L.un), kuR = adj_key(R.un);
     long long const kcL = adj_key(L.c), kcR = adj_key(R.c);
     bool const u_lt = kuL < kuR;
     bool const u_gt = kuR < kuL;
     bool const c_lt = kcL < kcR;
     bool const c_gt = kcR < kcL;
-    double const umin = u_gt ? R.un : L.un;
-    double const umax = u_lt ? R.un : L.un;
     double const cmax = c_lt ? R.c : L.c;
-    double const SL = umin - cmax;
-    double const SR = umax + cmax;
-    double const aL = SL - L.un;
-    double const aR = SR - R.un;
-    double const rcL = L.r * aL;
-    double const rcR = R.r * aR;
-    double const num = (R.p - L.p) + rcL * L.un - rcR * R.un;
-    double const den = rcL - rcR; // rcL <= 0 <= rcR: den < 0, so ustar > 0 exactly when num < 0
-    bool const left = adj_neg(num);
-    bool const tie = adj_zero(num);
+    double const du = L.un - R.un;
+    double const A = cmax + (u_gt ? du : 0.0);
+    double const D = L.r + R.r;
+    double const G = A * D;
+    double const mom = L.r * L.un + R.r * R.un;
+    double const n = A * mom - (R.p - L.p); // G > 0, so ustar has the sign of n
+    bool const left = adj_pos(n);
+    bool const tie = adj_zero(n);
     double const gd = UNIT ? dd : ds * dd;
     double const ge = UNIT ? de : ds * de;
     double const gn = UNIT ? dn : ds * dn;
@@ -200,19 +169,21 @@ EULR_ADJ_FN void hllc_bar(FaceSide const& L, FaceSide const& R, double dd, doubl
     q.t2 = left ? L.t2 : R.t2;
     q.e = left ? L.e : R.e;
     q.ke = left ? L.ke : R.ke;
-    double const qrc = left ? rcL : rcR;
+    double const a = left ? -A : A; // S - un
+    double const S = q.un + a;
 
     FaceBar bq;
-    if (adj_pos(SL) || adj_neg(SR)) {
-        // S_L * S_R > 0: the flux is the upwind side's physical flux
+    if (left ? adj_pos(S) : adj_neg(S)) {
+        // supersonic: the flux is the upwind side's physical flux
         double const m = q.r * q.un;
         double const gm = gd + gn * q.un + gt1 * q.t1 + gt2 * q.t2;
-        double const geq = ge * q.un;
-        bq.un = gn * m + ge * (q.e + q.p) + gm * q.r + geq * (q.r * q.un);
-        bq.r = gm * q.un + geq * q.ke;
-        bq.p = gn + ge * q.un + geq * inv_gm1;
-        bq.t1 = gt1 * m + geq * (q.r * q.t1);
-        bq.t2 = gt2 * m + geq * (q.r * q.t2);
+        double const gE = ge * q.un;
+        double const gEd = gE * q.r;
+        bq.un = gn * m + ge * (q.e + q.p) + gm * q.r + gE * m;
+        bq.r = gm * q.un + gE * q.ke;
+        bq.p = gn + gE + gE * inv_gm1;
+        bq.t1 = gt1 * m + gEd * q.t1;
+        bq.t2 = gt2 * m + gEd * q.t2;
         bL.r = left ? bq.r : 0.0;
         bL.p = left ? bq.p : 0.0;
         bL.un = left ? bq.un : 0.0;
@@ -226,46 +197,58 @@ EULR_ADJ_FN void hllc_bar(FaceSide const& L, FaceSide const& R, double dd, doubl
         return;
     }
 
-    double inv_den, ustar, gus, gps, gS;
+    double iG, ustar, gus, ga;
     if (tie) {
-        // ustar == 0: the mean of the two star branches, each taking half of
-        // the cotangent.  With ustar = 0 the mass flux m = d_o ustar
-        // vanishes, and so does every cotangent that carries a factor ustar:
-        // each branch adds only its mass and energy terms to d/d ustar and
-        // half of gn to d/d pstar (star_branch_bar with ustar = 0).  One
-        // reciprocal gives 1/den, 1/S_L and 1/S_R.
+        // ustar == 0: the mean of the two branches, each taking half of the
+        // cotangent.  b and the mass flux vanish, so each side adds only its
+        // b's derivative; the pressure term p + a d w (q's) is as elsewhere.
+        // One reciprocal gives 1/G, 1/S_L and 1/S_R.
+        double const SL = L.un - A;
+        double const SR = R.un + A;
         double const P = SL * SR;
-        double const Rr = adj_rcp(den * P);
-        inv_den = P * Rr;
+        double const Rr = adj_rcp(G * P);
+        iG = P * Rr;
         ustar = 0.0;
-        double const pstar = q.p - qrc * q.un; // both sides' values agree at num == 0
         double const hd = adj_half(gd), he = adj_half(ge), ht1 = adj_half(gt1), ht2 = adj_half(gt2);
-        gus = tie_branch_bar(L, aL, (den * SR) * Rr, pstar, hd, he, ht1, ht2) +
-              tie_branch_bar(R, aR, (den * SL) * Rr, pstar, hd, he, ht1, ht2);
-        gps = gn;
-        gS = 0.0;
-        bq.r = 0.0;
-        bq.p = 0.0;
-        bq.un = 0.0;
+        double const gw = q.r * (gn * a);
+        gus = tie_side_bar(L, -A, SL, (G * SR) * Rr, hd, he, ht1, ht2) +
+              tie_side_bar(R, A, SR, (G * SL) * Rr, hd, he, ht1, ht2) + gw;
+        ga = -gn * (q.r * q.un);
+        bq.r = -(gn * a) * q.un;
+        bq.p = gn;
+        bq.un = -gw;
         bq.t1 = 0.0;
         bq.t2 = 0.0;
     } else {
-        // One reciprocal gives 1/den and 1/(S - ustar): with Z = S den - num,
-        // S - ustar = Z/den, so 1/den = Z R and 1/(S - ustar) = den^2 R for R = 1/(den Z).
-        double const Z = (left ? SL : SR) * den - num;
-        double const Rr = adj_rcp(den * Z);
-        inv_den = Z * Rr;
-        double const iY0 = (den * den) * Rr;
-        ustar = num * inv_den;
-        double const pstar = q.p + qrc * (ustar - q.un);
-        gS = star_branch_bar(q, left ? aL : aR, iY0, ustar, pstar, gd, ge, gn, gt1, gt2, inv_gm1, gus, gps, bq);
+        double const M = S * G - n; // G (S - ustar)
+        double const Rr = adj_rcp(G * M);
+        double const nR = n * Rr;
+        iG = M * Rr;
+        ustar = nR * M;
+        double const iu = nR * G;       // ustar/(S - ustar)
+        double const y = G * (G * Rr);  // 1/(S - ustar)
+        double const b = a * iu;
+        double const w = ustar - q.un;
+        double const dw = q.r * w;
+        double const m = q.r * b;
+        double const E = S * dw + (q.e + q.p);
+        double const gm = gd + gn * ustar + gt1 * q.t1 + gt2 * q.t2; // d/d (d b)
+        double const gb = gm * q.r + ge * E;                         // d/d b
+        double const gE = ge * b;                                    // d/d E
+        double const K = gE * S + gn * a;                            // d/d (d w)
+        double const gw = q.r * K;
+        double const gby = gb * y;
+        double const gS = gE * dw - gby * b; // db/dS = -b y
+        ga = gn * dw + gb * iu + gS;         // S = un + a
+        gus = gn * m + gw + gby * (a + b);   // db/dustar = (a + b) y
+        double const gEd = gE * q.r;
+        bq.r = gm * b + K * w + gE * q.ke;
+        bq.p = gn + gE + gE * inv_gm1;
+        bq.un = gS - gw + gEd * q.un;
+        bq.t1 = gt1 * m + gEd * q.t1;
+        bq.t2 = gt2 * m + gEd * q.t2;
     }
 
-    // pstar = p_q + rc_q (ustar - un_q)
-    bq.p += gps;
-    bq.un -= gps * qrc;
-    gus += gps * qrc;
-    double const grcq = gps * (ustar - q.un);
     // to the upwind side
     bL.r = left ? bq.r : 0.0;
     bL.p = left ? bq.p : 0.0;
@@ -277,35 +260,26 @@ EULR_ADJ_FN void hllc_bar(FaceSide const& L, FaceSide const& R, double dd, doubl
     bR.un = left ? 0.0 : bq.un;
     bR.t1 = left ? 0.0 : bq.t1;
     bR.t2 = left ? 0.0 : bq.t2;
-    double grcL = left ? grcq : 0.0;
-    double grcR = left ? 0.0 : grcq;
-    double gSL = left ? gS : 0.0;
-    double gSR = left ? 0.0 : gS;
-    // ustar = num / den
-    double const gnum = gus * inv_den;
-    double const gden = -gnum * ustar;
-    bR.p += gnum;
-    bL.p -= gnum;
-    grcL += gnum * L.un + gden;
-    grcR -= gnum * R.un + gden;
-    bL.un += gnum * rcL;
-    bR.un -= gnum * rcR;
-    // rc = rho (S - un)
-    bL.r += grcL * aL;
-    bR.r += grcR * aR;
-    double const gaL = grcL * L.r;
-    double const gaR = grcR * R.r;
-    gSL += gaL;
-    gSR += gaR;
-    bL.un -= gaL;
-    bR.un -= gaR;
-    // S_L = umin - cmax, S_R = umax + cmax (equal un: half to each side)
-    double const hs = adj_half(gSL + gSR);
-    bL.un += u_lt ? gSL : (u_gt ? gSR : hs);
-    bR.un += u_lt ? gSR : (u_gt ? gSL : hs);
-    double const gc = gSR - gSL;
-    double const gcL = c_lt ? 0.0 : (c_gt ? gc : adj_half(gc));
-    double const gcR = gc - gcL;
+    // ustar = n / G
+    double const gN = gus * iG;
+    double const gG = -gN * ustar;
+    bL.p += gN;
+    bR.p -= gN;
+    // n's momentum sum and G's density sum
+    double const gmom = gN * A;
+    double const gD = gG * A;
+    bL.r += gmom * L.un + gD;
+    bR.r += gmom * R.un + gD;
+    bL.un += gmom * L.r;
+    bR.un += gmom * R.r;
+    double const gA = gN * mom + gG * D + (left ? -ga : ga);
+    // A = cmax + max(u_L - u_R, 0) (equal: half to each side)
+    double const half_gA = adj_half(gA);
+    double const gdu = u_gt ? gA : (u_lt ? 0.0 : half_gA);
+    bL.un += gdu;
+    bR.un -= gdu;
+    double const gcL = c_lt ? 0.0 : (c_gt ? gA : half_gA);
+    double const gcR = gA - gcL;
     bL.p += gcL * L.cp;
     bL.r += gcL * L.cr;
     bR.p += gcR * R.cp;
