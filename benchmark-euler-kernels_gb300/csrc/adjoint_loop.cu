@@ -19,6 +19,9 @@
 //   segment prims (k-1) x 5
 //   cbar 5, prim0_bar 5, final prim_bar 5, final prim 5
 //   reverse-step workspace kAdjWorkFields
+//   the steps' lengths (nsteps doubles), written by the forward pass's steps
+//   themselves and read by the recompute's
+// No step waits for the host: neither pass synchronizes before its end.
 #include "euler_gb300.h"
 #include "kernels.h"
 
@@ -59,6 +62,11 @@ struct eulr_adjoint {
     double* primN(int f) const { return at(tail() + 15 + f); }
     void* work() const { return at(tail() + 20); }
     size_t nfields() const { return tail() + 20 + kAdjWorkFields; }
+    double* dt_dev() const { return at(nfields()); } // after the fields
+    size_t bytes() const
+    {
+        return field * nfields() + ((static_cast<size_t>(nsteps) * sizeof(double) + 255) & ~static_cast<size_t>(255));
+    }
 };
 
 namespace {
@@ -197,7 +205,7 @@ int eulr_adjoint_create(int n0, int n1, int n2, double gamma, double dx0, double
         e = cudaDeviceGetAttribute(&a->sms, cudaDevAttrMultiProcessorCount, a->device);
     }
     if (e == cudaSuccess) {
-        e = cudaMalloc(&a->slab, a->field * a->nfields());
+        e = cudaMalloc(&a->slab, a->bytes());
     }
     if (e != cudaSuccess) {
         st = cfail(e, "eulr_adjoint_create");
@@ -244,9 +252,12 @@ int eulr_adjoint_forward(eulr_adjoint* a, eulr_prim_cf64 prim0, const double* dt
             }
             a->dts[static_cast<size_t>(n)] = dts[n];
         }
-        ADJ_TRY(eulr_sim_set_dt_sequence(a->sim, a->dts.data(), a->nsteps));
+        ADJ_CUDA(cudaMemcpyAsync(a->dt_dev(), a->dts.data(), a->dts.size() * sizeof(double), cudaMemcpyHostToDevice,
+                                 a->stream),
+                 "copy time steps");
+        ADJ_TRY(eulr::sim_time_steps(a->sim, a->dt_dev(), a->nsteps, nullptr));
     } else {
-        ADJ_TRY(eulr_sim_set_dt_sequence(a->sim, nullptr, 0));
+        ADJ_TRY(eulr::sim_time_steps(a->sim, nullptr, 0, a->dt_dev()));
     }
     ADJ_TRY(eulr_sim_set_prim_f64(a->sim, prim0));
     Span span;
@@ -259,16 +270,7 @@ int eulr_adjoint_forward(eulr_adjoint* a, eulr_prim_cf64 prim0, const double* dt
         ADJ_TRY(eulr::sim_snapshot(a->sim, dst, 11));
         int const s0 = c * a->every;
         int const s1 = s0 + a->every < a->nsteps ? s0 + a->every : a->nsteps;
-        if (fixed) {
-            ADJ_TRY(eulr_sim_advance(a->sim, s1 - s0));
-        } else {
-            for (int n = s0; n < s1; ++n) {
-                double next = 0.0;
-                ADJ_TRY(eulr_sim_time(a->sim, nullptr, &next, nullptr));
-                a->dts[static_cast<size_t>(n)] = next;
-                ADJ_TRY(eulr_sim_advance(a->sim, 1));
-            }
-        }
+        ADJ_TRY(eulr_sim_advance(a->sim, s1 - s0));
     }
     ADJ_CUDA(cudaEventRecord(span.b, a->stream), "cudaEventRecord");
     double* fin[5];
@@ -280,7 +282,16 @@ int eulr_adjoint_forward(eulr_adjoint* a, eulr_prim_cf64 prim0, const double* dt
     ADJ_TRY(eulr_sim_get_state_f64(a->sim, prim_final, eulr_cons_f64{nullptr, nullptr, nullptr, nullptr, nullptr}));
     a->fwd_ms = span.ms();
     if (!fixed) { // the recompute replays the recorded steps
-        ADJ_TRY(eulr_sim_set_dt_sequence(a->sim, a->dts.data(), a->nsteps));
+        ADJ_CUDA(cudaMemcpyAsync(a->dts.data(), a->dt_dev(), a->dts.size() * sizeof(double), cudaMemcpyDeviceToHost,
+                                 a->stream),
+                 "copy time steps");
+        ADJ_CUDA(cudaStreamSynchronize(a->stream), "cudaStreamSynchronize");
+        for (double const dt : a->dts) {
+            if (!std::isfinite(dt) || !(dt > 0.0)) {
+                return fail(EULR_ERR_INVALID_VALUE, "dt sequence entries must be finite and > 0");
+            }
+        }
+        ADJ_TRY(eulr::sim_time_steps(a->sim, a->dt_dev(), a->nsteps, nullptr));
     }
     a->have_forward = true;
     return EULR_SUCCESS;
@@ -341,6 +352,9 @@ int eulr_adjoint_backward(eulr_adjoint* a, eulr_prim_cf64 prim_final_bar, eulr_p
             src[f] = a->ckpt(c, f);
         }
         ADJ_TRY(eulr::sim_restore(a->sim, src, s0));
+        if (s1 - s0 > 1) {
+            ADJ_TRY(eulr::sim_record_ghosts(a->sim, a->seg(1, 0), a->field / sizeof(double), s1 - s0 - 1));
+        }
         // prim of steps s0+1 .. s1-1, written by the recomputing step kernels
         // themselves (prim of step s0 is the checkpoint's)
         for (int n = s0 + 1; n < s1; ++n) {

@@ -680,6 +680,46 @@ __global__ void __launch_bounds__(TX* TY) flux_batch_kernel(const __grid_constan
     batch_cta_done(b);
 }
 
+// Cells of the ghost layer (all cells of a grid without interior), and the
+// offset of the c-th of them.
+__host__ __device__ inline long long ghost_cells(Geom const& g)
+{
+    if (g.n0 < 3 || g.n1 < 3 || g.n2 < 3) {
+        return g.ncell();
+    }
+    return 2 * g.s2 + (2LL * g.n0 + 2LL * (g.n1 - 2)) * (g.n2 - 2);
+}
+
+__device__ __forceinline__ long long ghost_offset(Geom const& g, long long c)
+{
+    long long const plane = g.s2;
+    if (g.n0 < 3 || g.n1 < 3 || g.n2 < 3) {
+        return c;
+    }
+    if (c < 2 * plane) {
+        return (c < plane) ? c : c - plane + plane * (g.n2 - 1);
+    }
+    // grids hold < 2^31 cells: the ring index fits 32-bit division
+    long long const ring = 2LL * g.n0 + 2LL * (g.n1 - 2);
+    unsigned const r0 = static_cast<unsigned>(c - 2 * plane);
+    unsigned const q = r0 / static_cast<unsigned>(ring);
+    int const k = 1 + static_cast<int>(q);
+    int const r = static_cast<int>(r0 - q * static_cast<unsigned>(ring));
+    int i, j;
+    if (r < g.n0) {
+        i = r;
+        j = 0;
+    } else if (r < 2 * g.n0) {
+        i = r - g.n0;
+        j = g.n1 - 1;
+    } else {
+        int const r2 = r - 2 * g.n0;
+        j = 1 + r2 / 2;
+        i = (r2 & 1) ? g.n0 - 1 : 0;
+    }
+    return g.at(i, j, k);
+}
+
 // Ghost shell of the step's output: cons copied, prim = cons_to_prim(cons)
 // (bit-identical to the reference's cons_to_prim over ghosts,
 // cons_to_prim.hpp:26-27), sound speed and CFL contribution.
@@ -687,38 +727,11 @@ template <class T>
 __device__ __forceinline__ void ghost_shell_body(GhostParams<T> const& p)
 {
     Geom const g = p.g;
-    bool const all = (g.n0 < 3) || (g.n1 < 3) || (g.n2 < 3);
-    long long const plane = g.s2;
-    long long const ring = 2LL * g.n0 + 2LL * (g.n1 - 2);
-    long long const total = all ? g.ncell() : 2 * plane + ring * (g.n2 - 2);
+    long long const total = ghost_cells(g);
     T wmax = T(0);
     for (long long c = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; c < total;
          c += static_cast<long long>(gridDim.x) * blockDim.x) {
-        long long o;
-        if (all) {
-            o = c;
-        } else if (c < 2 * plane) {
-            o = (c < plane) ? c : c - plane + plane * (g.n2 - 1);
-        } else {
-            // grids hold < 2^31 cells: the ring index fits 32-bit division
-            unsigned const r0 = static_cast<unsigned>(c - 2 * plane);
-            unsigned const q = r0 / static_cast<unsigned>(ring);
-            int const k = 1 + static_cast<int>(q);
-            int const r = static_cast<int>(r0 - q * static_cast<unsigned>(ring));
-            int i, j;
-            if (r < g.n0) {
-                i = r;
-                j = 0;
-            } else if (r < 2 * g.n0) {
-                i = r - g.n0;
-                j = g.n1 - 1;
-            } else {
-                int const r2 = r - 2 * g.n0;
-                j = 1 + r2 / 2;
-                i = (r2 & 1) ? g.n0 - 1 : 0;
-            }
-            o = g.at(i, j, k);
-        }
+        long long const o = ghost_offset(g, c);
         T const d = p.cons_in.f[0][o];
         T const e = p.cons_in.f[1][o];
         T const m0 = p.cons_in.f[2][o];
@@ -756,13 +769,6 @@ __device__ __forceinline__ void ghost_shell_body(GhostParams<T> const& p)
             p.prim_out.f[2][o] = u0;
             p.prim_out.f[3][o] = u1;
             p.prim_out.f[4][o] = u2;
-            if (p.prim_rec.f[0] != nullptr) {
-                p.prim_rec.f[0][o] = d;
-                p.prim_rec.f[1][o] = pr;
-                p.prim_rec.f[2][o] = u0;
-                p.prim_rec.f[3][o] = u1;
-                p.prim_rec.f[4][o] = u2;
-            }
             p.cs_out[o] = sqrt_rn(div_rn(mul_rn(p.gamma, pr), d));
         }
         T v;
@@ -796,11 +802,28 @@ __global__ void __launch_bounds__(256) ghost_shell_kernel(GhostParams<T> p)
     ghost_shell_body(p);
 }
 
+__global__ void __launch_bounds__(256) ghost_prim_kernel(CBundle<double> prim, Geom g, double* base, size_t field,
+                                                         int count)
+{
+    long long const total = ghost_cells(g);
+    for (long long c = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; c < total;
+         c += static_cast<long long>(gridDim.x) * blockDim.x) {
+        long long const o = ghost_offset(g, c);
+#pragma unroll
+        for (int f = 0; f < 5; ++f) {
+            double const v = prim.f[f][o];
+            for (int b = 0; b < count; ++b) {
+                base[(static_cast<size_t>(b) * 5 + f) * field + o] = v;
+            }
+        }
+    }
+}
+
 template <class T>
-__global__ void finalize_dt_kernel(SimScalars* s, T cfl, int add_time, const double* dt_seq)
+__global__ void finalize_dt_kernel(SimScalars* s, T cfl, int add_time, const double* dt_seq, double* dt_log)
 {
     if (threadIdx.x == 0 && blockIdx.x == 0) {
-        finalize_one(s, cfl, add_time, dt_seq);
+        finalize_one(s, cfl, add_time, dt_seq, dt_log);
     }
 }
 
@@ -1025,32 +1048,31 @@ cudaError_t launch_flux(FluxParams<T> p, TmaMaps const* maps, int mode, int comp
     return FluxDispatch<T>::launch(p, maps, mode, comp, sms, s);
 }
 
-template <class T>
-cudaError_t launch_ghost_shell(GhostParams<T> p, int sms, cudaStream_t s)
+static int ghost_blocks(Geom const& g, int sms)
 {
-    Geom const& g = p.g;
-    long long total;
-    if (g.n0 < 3 || g.n1 < 3 || g.n2 < 3) {
-        total = g.ncell();
-    } else {
-        total = 2 * g.s2 + (2LL * g.n0 + 2LL * (g.n1 - 2)) * (g.n2 - 2);
-    }
-    long long blocks = (total + 255) / 256;
+    long long const blocks = (ghost_cells(g) + 255) / 256;
     long long const cap = static_cast<long long>(sms) * 8;
-    if (blocks > cap) {
-        blocks = cap;
-    }
-    if (blocks < 1) {
-        blocks = 1;
-    }
-    ghost_shell_kernel<T><<<static_cast<int>(blocks), 256, 0, s>>>(p);
+    return static_cast<int>(blocks < 1 ? 1 : (blocks < cap ? blocks : cap));
+}
+
+cudaError_t launch_ghost_prim(CBundle<double> prim, Geom g, double* base, size_t field, int count, int sms,
+                              cudaStream_t s)
+{
+    ghost_prim_kernel<<<ghost_blocks(g, sms), 256, 0, s>>>(prim, g, base, field, count);
     return cudaGetLastError();
 }
 
 template <class T>
-cudaError_t launch_finalize_dt(SimScalars* sc, T cfl, int add_time, cudaStream_t s, const double* dt_seq)
+cudaError_t launch_ghost_shell(GhostParams<T> p, int sms, cudaStream_t s)
 {
-    finalize_dt_kernel<T><<<1, 32, 0, s>>>(sc, cfl, add_time, dt_seq);
+    ghost_shell_kernel<T><<<ghost_blocks(p.g, sms), 256, 0, s>>>(p);
+    return cudaGetLastError();
+}
+
+template <class T>
+cudaError_t launch_finalize_dt(SimScalars* sc, T cfl, int add_time, cudaStream_t s, const double* dt_seq, double* dt_log)
+{
+    finalize_dt_kernel<T><<<1, 32, 0, s>>>(sc, cfl, add_time, dt_seq, dt_log);
     return cudaGetLastError();
 }
 
@@ -1063,7 +1085,7 @@ template cudaError_t launch_flux<double>(FluxParams<double>, TmaMaps const*, int
 template cudaError_t launch_flux<float>(FluxParams<float>, TmaMaps const*, int, int, int, cudaStream_t);
 template cudaError_t launch_ghost_shell<double>(GhostParams<double>, int, cudaStream_t);
 template cudaError_t launch_ghost_shell<float>(GhostParams<float>, int, cudaStream_t);
-template cudaError_t launch_finalize_dt<double>(SimScalars*, double, int, cudaStream_t, const double*);
-template cudaError_t launch_finalize_dt<float>(SimScalars*, float, int, cudaStream_t, const double*);
+template cudaError_t launch_finalize_dt<double>(SimScalars*, double, int, cudaStream_t, const double*, double*);
+template cudaError_t launch_finalize_dt<float>(SimScalars*, float, int, cudaStream_t, const double*, double*);
 
 } // namespace eulr

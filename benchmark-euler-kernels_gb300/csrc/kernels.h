@@ -73,6 +73,7 @@ struct FluxParams {
     double cfl;
     const double* dt_seq;       // if set: step n uses dt = dt_seq[n] (a fixed sequence, CFL not applied)
     const long long* step_dev;  // the step index n (SimScalars::steps)
+    double* dt_log;             // if set: step n's length goes to dt_log[n]
     CBundle<T> lo_in;    // compensated FP32 state: low words of cons (comp == 2)
     Bundle<T> lo_out;
     T invdx0, invdx1, invdx2;
@@ -110,9 +111,8 @@ struct GhostParams {
     Bundle<T> lo_out;
     int comp;         // kComp* of a cons-only FP32 state (prim_out unset)
     Bundle<T> prim_out;
-    Bundle<T> prim_rec; // when set: a second copy of prim_out
     T* cs_out;
-    T* h_out;           // when set (FP64 state): e + p
+    T* h_out;         // when set (FP64 state): e + p
     T gamma, gm1;
     T invdx0, invdx1, invdx2;
     unsigned long long* wmax;
@@ -133,8 +133,24 @@ cudaError_t launch_time_step(CBundle<T> prim, long long n, T gamma, T ix0, T ix1
 cudaError_t launch_load_prim(CBundle<double> prim, Bundle<double> cons, Bundle<double> copy, double* cs, double* h,
                              const double* e_in, long long n, double gamma, double ix0, double ix1, double ix2,
                              unsigned long long* wmax, int sms, cudaStream_t s);
-// out = a + b elementwise, rounded once (the FP64 state's e + p after a restore).
-cudaError_t launch_add_fields(const double* a, const double* b, double* out, long long n, int sms, cudaStream_t s);
+// Copies count (<= 11) fields of n doubles, 256-byte aligned and padded, in
+// one launch.  With h set, also h = field 1 + field 6 (the FP64 state's e + p
+// when the fields are prim, cons, sound speed), and with sc set, *sc = the
+// scalars of a state restored at `step`.
+struct CopyFieldsParams {
+    const double* src[11];
+    double* dst[11];
+    int count;
+    long long n;
+    double* h;
+    SimScalars* sc;
+    long long step;
+};
+cudaError_t launch_copy_fields(CopyFieldsParams const& p, int sms, cudaStream_t s);
+// The ghost layer of prim copied into `count` bundles whose fields lie
+// `field` doubles apart, bundle after bundle, from base.
+cudaError_t launch_ghost_prim(CBundle<double> prim, Geom g, double* base, size_t field, int count, int sms,
+                              cudaStream_t s);
 cudaError_t launch_init_step(Bundle<double> prim, Geom g, double dx0, double dx1, double dx2, double c,
                              double rho_in, double p_in, double rho_out, double p_out, int sms, cudaStream_t s);
 // max invdt over all cells of a cons-only FP32 state (compensated: FP64
@@ -164,7 +180,8 @@ cudaError_t launch_flux_batch(int shape, int comp, BatchParams<T> const* b, int 
 template <class T>
 cudaError_t launch_ghost_shell(GhostParams<T> p, int sms, cudaStream_t s);
 template <class T>
-cudaError_t launch_finalize_dt(SimScalars* sc, T cfl, int add_time, cudaStream_t s, const double* dt_seq = nullptr);
+cudaError_t launch_finalize_dt(SimScalars* sc, T cfl, int add_time, cudaStream_t s, const double* dt_seq = nullptr,
+                               double* dt_log = nullptr);
 
 // The FP32 states' step and the FP32 godunov on the column engine (flux_f32.cu).
 cudaError_t configure_step_f32col(int comp, int* per_sm);
@@ -235,6 +252,7 @@ cudaError_t launch_prim_to_cons_adjoint(CBundle<double> prim, CBundle<double> cb
 // copy.  sim_snapshot copies the first nfields of them to device memory (on
 // the simulation's stream, asynchronously); sim_restore loads all 11 into the
 // first copy and sets the step counter (which indexes a fixed dt sequence).
+// Both are one launch on the simulation's stream.
 int sim_snapshot(eulr_sim* s, double* const* dst, int nfields);
 // Records msg as the last error (eulr_last_error) and returns status.
 int sim_fail(int status, const char* msg);
@@ -242,7 +260,15 @@ int sim_restore(eulr_sim* s, const double* const* src, long long step);
 // The stream the simulation's work runs on (its own when created with NULL).
 cudaStream_t sim_stream(eulr_sim* s);
 // One step of a loaded FP64 simulation (as eulr_sim_advance(s, 1)) whose
-// kernels also write the new prim (every cell) into dst[0..4].
+// kernel also writes the new prim of interior cells into dst[0..4]; the ghost
+// layers, the same after every step but none, are sim_record_ghosts'.
 int sim_advance_recording(eulr_sim* s, double* const* dst);
+// The ghost prim of every later step into count bundles (see
+// launch_ghost_prim); after a load or restore.
+int sim_record_ghosts(eulr_sim* s, double* base, size_t field, int count);
+// Time steps from a device array the caller keeps (n > 0; unchecked), or CFL
+// steps (seq NULL); each step's length logged to `log` when set.  Applies to
+// the steps enqueued next.
+int sim_time_steps(eulr_sim* s, double* seq, long long n, double* log);
 
 } // namespace eulr

@@ -355,17 +355,41 @@ cudaError_t launch_load_prim(CBundle<double> prim, Bundle<double> cons, Bundle<d
     return cudaGetLastError();
 }
 
-__global__ void __launch_bounds__(256) add_fields_kernel(const double* a, const double* b, double* out, long long n)
+// Bound by HBM: 16-byte accesses, each thread's loads of every field in
+// flight before its stores.  A state's 11 fields in one launch instead of a
+// copy each (64^3: 11 launches of about 2.5 us for 8 us of traffic).
+__global__ void __launch_bounds__(256) copy_fields_kernel(const __grid_constant__ CopyFieldsParams p)
 {
-    for (long long c = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; c < n;
+    if (p.sc != nullptr && blockIdx.x == 0 && threadIdx.x == 0) {
+        SimScalars v{};
+        v.steps = p.step;
+        *p.sc = v;
+    }
+    long long const pairs = (p.n + 1) / 2; // fields are padded to 256 bytes
+    for (long long c = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; c < pairs;
          c += static_cast<long long>(gridDim.x) * blockDim.x) {
-        out[c] = __dadd_rn(a[c], b[c]);
+        double2 v[11];
+#pragma unroll
+        for (int f = 0; f < 11; ++f) {
+            if (f < p.count) {
+                v[f] = reinterpret_cast<const double2*>(p.src[f])[c];
+            }
+        }
+#pragma unroll
+        for (int f = 0; f < 11; ++f) {
+            if (f < p.count) {
+                reinterpret_cast<double2*>(p.dst[f])[c] = v[f];
+            }
+        }
+        if (p.h != nullptr) {
+            reinterpret_cast<double2*>(p.h)[c] = make_double2(__dadd_rn(v[6].x, v[1].x), __dadd_rn(v[6].y, v[1].y));
+        }
     }
 }
 
-cudaError_t launch_add_fields(const double* a, const double* b, double* out, long long n, int sms, cudaStream_t s)
+cudaError_t launch_copy_fields(CopyFieldsParams const& p, int sms, cudaStream_t s)
 {
-    add_fields_kernel<<<grid_for(n, sms), 256, 0, s>>>(a, b, out, n);
+    copy_fields_kernel<<<grid_for((p.n + 1) / 2, sms), 256, 0, s>>>(p);
     return cudaGetLastError();
 }
 

@@ -20,8 +20,7 @@
 // therefore writes copy 1's ghost layer once (cons copied, prim and sound
 // speed from cons, their max wavespeed kept in ghost_wmax, which every dt
 // includes); copy 0 keeps the loaded ghost prim for the first step and gets
-// the round trip once, right after it.  The recording steps of the adjoint
-// (a second prim output) still rebuild the output's ghost layer each step.
+// the round trip once, right after it.
 // Two steps (A->B, B->A) are captured once into a CUDA graph and replayed.
 //
 // Precisions: EULR_PRECISION_F64 (FP64 state and arithmetic),
@@ -107,7 +106,11 @@ struct eulr_sim {
     TmaMaps maps[2] = {}; // descriptors of copy 0 and copy 1 as step input
     bool loaded = false;
     cudaGraphExec_t graph = nullptr;
-    double* dt_seq = nullptr;  // device copy of a fixed dt sequence (owned), or null
+    double* dt_seq = nullptr;  // device copy of a fixed dt sequence, or null
+    bool own_dt_seq = false;   // allocated here (eulr_sim_set_dt_sequence)
+    double* dt_log = nullptr;  // device array of the steps' lengths (a recording caller's), or null
+    double* graph_seq = nullptr; // dt_seq and dt_log the graph was captured with
+    double* graph_log = nullptr;
     long long dt_seq_len = 0;
     long long host_steps = 0;  // steps taken since the state was loaded (host-side count)
     double* rec[5] = {};       // set only inside sim_advance_recording: a second prim output
@@ -233,9 +236,6 @@ GhostParams<T> ghost_params(eulr_sim* s, int in, int out, unsigned long long* wm
         gp.prim_out = bundle_of<T>(s->prim[out]);
         gp.cs_out = static_cast<T*>(s->cs[out]);
         gp.h_out = static_cast<T*>(s->h[out]);
-        if (s->rec[0] != nullptr) {
-            gp.prim_rec = bundle_of<T>(reinterpret_cast<void* const*>(s->rec));
-        }
     }
     gp.comp = s->comp;
     gp.gamma = gamma;
@@ -250,11 +250,10 @@ GhostParams<T> ghost_params(eulr_sim* s, int in, int out, unsigned long long* wm
 // One fused step from copy `in` to copy `1-in`: one launch of the step
 // kernel, which also finalizes the step (next dt, clock).  With `ev` (4
 // events) the launches are bracketed for per-kernel timing (ghost layer,
-// step, finalize; the first and last are empty except when recording or on
-// grids without interior cells).  Ghost layers are set at load (see the top
-// of this file); recording steps rebuild the output's ghost layer, which
-// writes its prim into the recording too.  A grid without interior cells
-// launches no step kernel: a finalize launch takes its step.
+// step, finalize; the first is empty, the last too except on grids without
+// interior cells).  Ghost layers are set at load (see the top of this file).
+// A grid without interior cells launches no step kernel: a finalize launch
+// takes its step.
 template <class T>
 int enqueue_step_t(eulr_sim* s, int in, cudaEvent_t* ev)
 {
@@ -267,10 +266,6 @@ int enqueue_step_t(eulr_sim* s, int in, cudaEvent_t* ev)
     bool const has_lo = s->comp == kCompHiLo;
     if (ev != nullptr) {
         SIM_CUDA(cudaEventRecord(ev[0], s->stream), "cudaEventRecord");
-    }
-    if (is_f64(s) && s->rec[0] != nullptr) {
-        SIM_CUDA(launch_ghost_shell<T>(ghost_params<T>(s, in, out, &s->sc->wmax), s->sms, s->stream),
-                 "ghost shell launch");
     }
 
     FluxParams<T> p{};
@@ -304,6 +299,7 @@ int enqueue_step_t(eulr_sim* s, int in, cudaEvent_t* ev)
     p.cfl = s->cfl;
     p.dt_seq = s->dt_seq;
     p.step_dev = &s->sc->steps;
+    p.dt_log = s->dt_log;
     p.invdx0 = ix0;
     p.invdx1 = ix1;
     p.invdx2 = ix2;
@@ -322,7 +318,8 @@ int enqueue_step_t(eulr_sim* s, int in, cudaEvent_t* ev)
         SIM_CUDA(cudaEventRecord(ev[2], s->stream), "cudaEventRecord");
     }
     if (!interior) {
-        SIM_CUDA(launch_finalize_dt<T>(s->sc, static_cast<T>(s->cfl), 1, s->stream, s->dt_seq), "finalize launch");
+        SIM_CUDA(launch_finalize_dt<T>(s->sc, static_cast<T>(s->cfl), 1, s->stream, s->dt_seq, s->dt_log),
+                 "finalize launch");
     }
     if (ev != nullptr) {
         SIM_CUDA(cudaEventRecord(ev[3], s->stream), "cudaEventRecord");
@@ -354,9 +351,8 @@ int after_step(eulr_sim* s)
     if (s->ghost_fix) {
         int const in = s->cur;     // the copy the step wrote
         int const out = 1 - in;    // the copy it read
-        GhostParams<double> q = ghost_params<double>(s, in, out, &s->sc->ghost_wmax);
-        q.prim_rec = Bundle<double>{}; // a recording step has recorded its own ghost layer
-        SIM_CUDA(launch_ghost_shell<double>(q, s->sms, s->stream), "ghost shell launch");
+        SIM_CUDA(launch_ghost_shell<double>(ghost_params<double>(s, in, out, &s->sc->ghost_wmax), s->sms, s->stream),
+                 "ghost shell launch");
         s->ghost_fix = false;
     }
     return EULR_SUCCESS;
@@ -523,11 +519,14 @@ int sim_snapshot(eulr_sim* s, double* const* dst, int nfields)
     if (!is_f64(s) || !s->loaded || nfields < 1 || nfields > 11) {
         return eulr::sim_fail(EULR_ERR_INVALID_ARGUMENT, "snapshot needs a loaded FP64 simulation and 1..11 fields");
     }
-    size_t const bytes = static_cast<size_t>(ncell(s)) * sizeof(double);
+    CopyFieldsParams p{};
+    p.count = nfields;
+    p.n = ncell(s);
     for (int f = 0; f < nfields; ++f) {
-        void const* src = f < 5 ? s->prim[s->cur][f] : (f < 10 ? s->cons[s->cur][f - 5] : s->cs[s->cur]);
-        SIM_CUDA(cudaMemcpyAsync(dst[f], src, bytes, cudaMemcpyDeviceToDevice, s->stream), "snapshot copy");
+        p.src[f] = static_cast<const double*>(f < 5 ? s->prim[s->cur][f] : (f < 10 ? s->cons[s->cur][f - 5] : s->cs[s->cur]));
+        p.dst[f] = dst[f];
     }
+    SIM_CUDA(launch_copy_fields(p, s->sms, s->stream), "snapshot copy");
     return EULR_SUCCESS;
 }
 
@@ -557,26 +556,51 @@ int sim_advance_recording(eulr_sim* s, double* const* dst)
     return EULR_SUCCESS;
 }
 
+int sim_record_ghosts(eulr_sim* s, double* base, size_t field, int count)
+{
+    SIM_TRY(check_sim(s));
+    if (!is_f64(s) || !s->loaded || !s->ghost_fix) {
+        return eulr::sim_fail(EULR_ERR_INVALID_ARGUMENT, "ghost recording needs an FP64 simulation just loaded");
+    }
+    // copy 1 holds the ghost layer of every step but the loaded one's
+    SIM_CUDA(launch_ghost_prim(cbundle_of<double>(s->prim[1]), s->g, base, field, count, s->sms, s->stream),
+             "ghost recording");
+    return EULR_SUCCESS;
+}
+
+int sim_time_steps(eulr_sim* s, double* seq, long long n, double* log)
+{
+    SIM_TRY(check_sim(s));
+    if (s->own_dt_seq) {
+        SIM_CUDA(cudaStreamSynchronize(s->stream), "cudaStreamSynchronize");
+        cudaFree(s->dt_seq);
+        s->own_dt_seq = false;
+    }
+    s->dt_seq = seq;
+    s->dt_seq_len = seq != nullptr ? n : 0;
+    s->dt_log = log;
+    return EULR_SUCCESS;
+}
+
 int sim_restore(eulr_sim* s, const double* const* src, long long step)
 {
     SIM_TRY(check_sim(s));
     if (!is_f64(s) || step < 0) {
         return eulr::sim_fail(EULR_ERR_INVALID_ARGUMENT, "restore needs an FP64 simulation and a step >= 0");
     }
-    size_t const bytes = static_cast<size_t>(ncell(s)) * sizeof(double);
+    CopyFieldsParams p{};
+    p.count = 11;
+    p.n = ncell(s);
     for (int f = 0; f < 11; ++f) {
-        void* dst = f < 5 ? s->prim[0][f] : (f < 10 ? s->cons[0][f - 5] : s->cs[0]);
-        SIM_CUDA(cudaMemcpyAsync(dst, src[f], bytes, cudaMemcpyDeviceToDevice, s->stream), "restore copy");
+        p.src[f] = src[f];
+        p.dst[f] = static_cast<double*>(f < 5 ? s->prim[0][f] : (f < 10 ? s->cons[0][f - 5] : s->cs[0]));
     }
-    SimScalars h{};
-    h.steps = step;
-    SIM_CUDA(cudaMemcpyAsync(s->sc, &h, sizeof(h), cudaMemcpyHostToDevice, s->stream), "restore scalars");
+    p.h = static_cast<double*>(s->h[0]);
+    p.sc = s->sc;
+    p.step = step;
+    SIM_CUDA(launch_copy_fields(p, s->sms, s->stream), "restore copy");
     s->cur = 0;
-    SIM_CUDA(launch_add_fields(static_cast<const double*>(s->cons[0][1]), static_cast<const double*>(s->prim[0][1]),
-                               static_cast<double*>(s->h[0]), ncell(s), s->sms, s->stream),
-             "restore e + p");
     SIM_TRY(set_ghost_layer(s));
-    SIM_CUDA(cudaStreamSynchronize(s->stream), "cudaStreamSynchronize"); // h is a stack value
     s->host_steps = step;
     s->loaded = true;
     return EULR_SUCCESS;
@@ -717,7 +741,7 @@ int eulr_sim_destroy(eulr_sim* s)
     if (s->slab != nullptr) {
         cudaFree(s->slab);
     }
-    if (s->dt_seq != nullptr) {
+    if (s->own_dt_seq) {
         cudaFree(s->dt_seq);
     }
     if (s->own_stream && s->stream != nullptr) {
@@ -789,7 +813,13 @@ int eulr_sim_advance(eulr_sim* s, int nsteps)
         SIM_TRY(step_direct(s));
         --left;
     }
+    if (left >= 2 && s->graph != nullptr && (s->graph_seq != s->dt_seq || s->graph_log != s->dt_log)) {
+        cudaGraphExecDestroy(s->graph); // the captured launches carry other time steps
+        s->graph = nullptr;
+    }
     if (left >= 2 && s->graph == nullptr) {
+        s->graph_seq = s->dt_seq;
+        s->graph_log = s->dt_log;
         cudaGraph_t graph = nullptr;
         SIM_CUDA(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal), "cudaStreamBeginCapture");
         int const st0 = enqueue_step(s, 0);
@@ -942,13 +972,15 @@ int eulr_sim_set_dt_sequence(eulr_sim* s, const double* dts, long long n)
         }
     }
     SIM_CUDA(cudaStreamSynchronize(s->stream), "cudaStreamSynchronize");
-    if (s->dt_seq != nullptr) {
+    if (s->own_dt_seq) {
         cudaFree(s->dt_seq);
-        s->dt_seq = nullptr;
-        s->dt_seq_len = 0;
     }
+    s->dt_seq = nullptr;
+    s->dt_seq_len = 0;
+    s->own_dt_seq = false;
     if (n > 0) {
         SIM_CUDA(cudaMalloc(&s->dt_seq, sizeof(double) * n), "cudaMalloc(dt sequence)");
+        s->own_dt_seq = true;
         SIM_CUDA(cudaMemcpy(s->dt_seq, dts, sizeof(double) * n, cudaMemcpyHostToDevice), "copy dt sequence");
         s->dt_seq_len = n;
     }

@@ -95,7 +95,8 @@ __device__ __forceinline__ T dt_over_dv(FluxParams<T> const& p)
 // accumulator is read with a volatile load: other CTAs of the same launch
 // raised it by atomics, and a cached copy must not answer.
 template <class T>
-__device__ __forceinline__ void finalize_one(SimScalars* s, T cfl, int add_time, const double* dt_seq = nullptr)
+__device__ __forceinline__ void finalize_one(SimScalars* s, T cfl, int add_time, const double* dt_seq = nullptr,
+                                             double* dt_log = nullptr)
 {
     if (add_time) {
         // the step just taken, cfl*dt (or the fixed dt), added with separate
@@ -104,6 +105,9 @@ __device__ __forceinline__ void finalize_one(SimScalars* s, T cfl, int add_time,
                                               : (sizeof(T) == 8 ? __dmul_rn(static_cast<double>(cfl), s->dt)
                                                                 : static_cast<double>(cfl * static_cast<T>(s->dt)));
         s->t = __dadd_rn(s->t, step);
+        if (dt_log != nullptr) {
+            dt_log[s->steps] = step;
+        }
         s->steps += 1;
     }
     unsigned long long const w = *reinterpret_cast<volatile unsigned long long*>(&s->wmax);
@@ -129,7 +133,7 @@ __device__ __forceinline__ void step_done(FluxParams<T> const& p)
     __threadfence();
     if (atomicAdd(&p.fin->done, 1u) == gridDim.x - 1) {
         __threadfence();
-        finalize_one(p.fin, static_cast<T>(p.cfl), 1, p.dt_seq);
+        finalize_one(p.fin, static_cast<T>(p.cfl), 1, p.dt_seq, p.dt_log);
         p.fin->done = 0u;
     }
 }
