@@ -39,6 +39,7 @@
 #include "kernels.h"
 #include "step_common.cuh"
 
+#include <algorithm>
 #include <cfloat>
 
 namespace eulr {
@@ -834,27 +835,34 @@ __global__ void finalize_dt_kernel(SimScalars* s, T cfl, int add_time, const dou
 // and no better on small grids.)
 constexpr int kStepTX = 16, kStepTY = 16;
 
-// Tiles per axis of a single-grid FP64 launch.
-struct TilePlan {
-    int nx, ny;
-};
+} // namespace
 
-// Picks them by the time of the busiest SM.  The kernel divides all tiles'
+// Picks the tiles by the time of the busiest SM.  The kernel divides all tiles'
 // planes evenly among its CTAs, so with U planes in all on G CTAs, r of them
 // on an SM, each solves m = ceil(U/G) planes of cost c and the z faces below
 // its first plane, z: the SM's FP64 pipe is busy r (m c + z), and every plane
 // adds a wait that its neighbour does not cover (its barriers and its last,
-// partly filled pass of faces).  c and z count FP64 warp instructions, 27 a
-// face and 49 a cell of the step (30 of the operator's update, and 15 a cell
-// that it stages), each holding its SM for 9.0 ns; the wait measured
+// partly filled pass of faces).  c and z count FP64 warp instructions, each
+// holding its SM for 9.0 ns; the wait measured
 // 1.1 us a plane with two CTAs on the SM and 1.6 us with one.  Whole
 // 16 x 16 tiles are the best for large grids (256^3: 4.14 ms a step, 4.42 in
 // 16 x 8), smaller ones where their number leaves SMs idle.  Against whole
 // 16 x 16 tiles in chunks of at least 8 planes: 16^3 97 -> 12.5 us a step,
 // 48^3 97 -> 46, 64^3 97 -> 86, 99 x 128 x 75 311 -> 270.
-TilePlan choose_tiles(int ix, int iy, int iz, int sms, int per_sm, bool step, int q)
+TilePlan choose_tiles(int ix, int iy, int iz, int sms, int per_sm, int face, int cell, int stage, int q)
 {
     constexpr double kInstr = 9.0e-3, kWait2 = 1.1, kWait1 = 1.6; // us
+    // the last answer of this thread: a loop over one grid asks the same
+    // again, and the search takes a few microseconds
+    struct Asked {
+        int key[9];
+        TilePlan plan;
+    };
+    thread_local Asked last{};
+    int const key[9] = {ix, iy, iz, sms, per_sm, face, cell, stage, q};
+    if (std::equal(key, key + 9, last.key)) {
+        return last.plan;
+    }
     int const units = (ix + q - 1) / q;
     TilePlan best{};
     double best_us = 1e300;
@@ -876,44 +884,35 @@ TilePlan choose_tiles(int ix, int iy, int iz, int sms, int per_sm, bool step, in
             last_ny = ny;
             int const faces = (tw + 1) * th + tw * (th + 1) + tw * th;
             int const rows = (tw * th + 31) / 32;
-            int const c = 27 * ((faces + 31) / 32) +
-                          (step ? 49 * rows : 30 * rows + 15 * (((tw + 2) * (th + 2) + 31) / 32));
+            int const c = face * ((faces + 31) / 32) + cell * rows + stage * (((tw + 2) * (th + 2) + 31) / 32);
             long long const u = static_cast<long long>(nx) * ny * iz;
             long long const ctas = u < static_cast<long long>(sms) * per_sm ? u : static_cast<long long>(sms) * per_sm;
             long long const r = (ctas + sms - 1) / sms;
             long long const m = (u + ctas - 1) / ctas;
-            double const us = m * (r * c * kInstr + (r > 1 ? kWait2 : kWait1)) + r * 27 * rows * kInstr;
+            double const us = m * (r * c * kInstr + (r > 1 ? kWait2 : kWait1)) + r * face * rows * kInstr;
             if (us < best_us * (1.0 - 1e-9)) {
                 best_us = us;
                 best = TilePlan{nx, ny};
             }
         }
     }
+    std::copy(key, key + 9, last.key);
+    last.plan = best;
     return best;
 }
+
+namespace {
 
 template <int MODE, int STAGE>
 struct FluxKernel {
     using L = TileLayout<kStepTX, kStepTY, kStageSlots<STAGE>>;
     static auto fn() { return flux_tile_kernel<kStepTX, kStepTY, MODE, STAGE>; }
 
-    // Opts the kernel into its dynamic shared memory size and returns its
-    // resident CTAs per SM.  Called outside any stream capture (by the entry
-    // points before they enqueue work), and cheap to repeat.
+    // Resident CTAs per SM.  Called outside any stream capture (by the entry
+    // points before they enqueue work).
     static cudaError_t configure(int* per_sm)
     {
-        cudaError_t e = cudaFuncSetAttribute(fn(), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             static_cast<int>(L::BYTES));
-        if (e != cudaSuccess) {
-            return e;
-        }
-        int n = 0;
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn(), L::NT, L::BYTES);
-        if (e != cudaSuccess) {
-            return e;
-        }
-        *per_sm = n < 1 ? 1 : n;
-        return cudaSuccess;
+        return resident_ctas<flux_tile_kernel<kStepTX, kStepTY, MODE, STAGE>>(L::NT, static_cast<int>(L::BYTES), per_sm);
     }
 
     static cudaError_t launch(FluxParams<double> p, TmaMaps const& maps, int sms, cudaStream_t s)
@@ -926,7 +925,10 @@ struct FluxKernel {
             return cudaSuccess; // no interior cell
         }
         int const q = STAGE == kStageTma ? 2 : 1;
-        TilePlan const plan = choose_tiles(ix, iy, iz, sms, per_sm, MODE == kModeStep, q);
+        // FP64 instructions: 27 a face; the step's 49 a cell, or the operator's
+        // 30 a cell and 15 a staged one
+        TilePlan const plan = MODE == kModeStep ? choose_tiles(ix, iy, iz, sms, per_sm, 27, 49, 0, q)
+                                                : choose_tiles(ix, iy, iz, sms, per_sm, 27, 30, 15, q);
         p.sx = split_tiles(ix, plan.nx, q);
         p.sy = split_tiles(iy, plan.ny, 1);
         p.tiles_x = plan.nx;

@@ -760,11 +760,7 @@ constexpr long long kNarrowCells = 0xffffffffLL;
 template <int COMP>
 cudaError_t configure_f32col(int* per_sm)
 {
-    int n = 0;
-    cudaError_t const e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-            &n, f32col::f32_step_kernel<COMP, 32, false, long long>, f32col::NT, 0);
-    *per_sm = n < 1 ? 1 : n;
-    return e;
+    return resident_ctas<f32col::f32_step_kernel<COMP, 32, false, long long>>(f32col::NT, 0, per_sm);
 }
 
 // Tile width and chunks of planes of a single-grid launch.

@@ -4,6 +4,8 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 
+#include <atomic>
+
 #include "euler_device.cuh"
 
 struct eulr_sim;
@@ -47,6 +49,48 @@ inline TileSplit split_tiles(int n, int parts, int q)
 {
     int const units = (n + q - 1) / q;
     return TileSplit{n, parts, units / parts, units % parts, q};
+}
+
+// Tiles per axis of a launch whose CTAs share all tiles' planes evenly, for a
+// kernel of tiles up to 16 x 16 bound by the FP64 pipe (choose_tiles in
+// flux.cu): face, cell and stage are the FP64 instructions of a face, of a
+// cell's update and of a staged cell.
+struct TilePlan {
+    int nx, ny;
+};
+TilePlan choose_tiles(int ix, int iy, int iz, int sms, int per_sm, int face, int cell, int stage, int q);
+
+// Opts Kernel into `bytes` of dynamic shared memory and returns its resident
+// CTAs per SM for blocks of `threads`, once per device: asked on every call
+// it cost a small operator 3 us.  Not during stream capture's first call.
+template <auto Kernel>
+cudaError_t resident_ctas(int threads, int bytes, int* per_sm)
+{
+    constexpr int kDevices = 64;
+    static std::atomic<int> known[kDevices];
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) {
+        return e;
+    }
+    int n = dev < kDevices ? known[dev].load(std::memory_order_acquire) : 0;
+    if (n == 0) {
+        if (bytes > 0) {
+            e = cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+        }
+        if (e == cudaSuccess) {
+            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, Kernel, threads, bytes);
+        }
+        if (e != cudaSuccess) {
+            return e;
+        }
+        n = n < 1 ? 1 : n;
+        if (dev < kDevices) {
+            known[dev].store(n, std::memory_order_release);
+        }
+    }
+    *per_sm = n;
+    return cudaSuccess;
 }
 
 // TMA descriptors of the seven staged fields (d, p, u0, u1, u2, c, e) of the

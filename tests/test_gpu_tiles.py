@@ -95,3 +95,30 @@ def test_fp32_godunov_matches_oracle(cuda, euler, oracle_lib, shape):
         euler.godunov(pg, cg, 1.4, dx, 0.01)
         ref = O.godunov(p32.astype(np.float64), c0, 1.4, dx, 0.01)
         assert max(rel_linf(cg.cpu().numpy(), ref)) <= 2e-5
+
+
+def _bits(a):
+    return a.view(np.uint64 if a.dtype == np.float64 else np.uint32)
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("shape", SHAPES + [(258, 162, 130)])
+def test_exact_godunov_tiles_bit_identical(cuda, euler, oracle_lib, dtype, shape):
+    """The bit-identical godunov at tile edges, on random states with patches of gas at rest (zero numerators of the
+    shared-reciprocal quotients), signed zeros, and cells out of the quotients' mid range; the last shape is large
+    enough for FP32's whole-tile kernel.  Every bit, the signs of zeros included."""
+    O = oracle_lib
+    n0, n1, n2 = shape
+    prim = O.random_prim(n0, n1, n2, seed=n0 + n1 + n2).astype(dtype)
+    prim[1, : n2 // 2 + 1] = 1.0
+    prim[2:, : n2 // 2 + 1] = 0.0
+    prim[2:, : n2 // 4 + 1] = -0.0
+    prim[2:, -1] *= dtype(1e25 if dtype == np.float32 else 1e150) ** dtype(0.5)  # out of the mid range, squares finite
+    cons = O.prim_to_cons(prim, 1.4)
+    dx, dt = (0.11, 0.07, 0.13), 1e-3
+    ref = O.godunov(prim, cons, 1.4, dx, dt)
+    cg = cuda.from_numpy(cons.copy()).cuda()
+    euler.godunov(cuda.from_numpy(prim).cuda(), cg, 1.4, dx, dt, exact=True)
+    got = cg.cpu().numpy()
+    same = (_bits(got) == _bits(ref)) | (np.isnan(got) & np.isnan(ref))
+    assert same.all(), (int((~same).sum()), got[~same][:4], ref[~same][:4])
