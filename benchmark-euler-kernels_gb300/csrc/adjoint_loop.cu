@@ -75,6 +75,7 @@ int fail(int status, const char* msg) { return eulr::sim_fail(status, msg); }
 
 int cfail(cudaError_t e, const char* what)
 {
+    (void)cudaGetLastError(); // reported here: a later launch's check must not find it again
     char buf[256];
     std::snprintf(buf, sizeof(buf), "%s: %s", what, cudaGetErrorString(e));
     return fail(e == cudaErrorMemoryAllocation ? EULR_ERR_OUT_OF_MEMORY : EULR_ERR_CUDA, buf);

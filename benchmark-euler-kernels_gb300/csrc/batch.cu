@@ -37,6 +37,7 @@ size_t pad256(size_t b) { return (b + 255) & ~static_cast<size_t>(255); }
 
 int cfail(cudaError_t e, const char* what)
 {
+    (void)cudaGetLastError(); // reported here: a later launch's check must not find it again
     char buf[400];
     std::snprintf(buf, sizeof(buf), "%s: %s", what, cudaGetErrorString(e));
     return eulr::sim_fail(e == cudaErrorMemoryAllocation ? EULR_ERR_OUT_OF_MEMORY : EULR_ERR_CUDA, buf);

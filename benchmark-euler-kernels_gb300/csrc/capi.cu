@@ -36,6 +36,7 @@ int fail(int status, const char* fmt, ...)
 
 int cuda_fail(cudaError_t e, const char* what)
 {
+    (void)cudaGetLastError(); // reported here: a later launch's check must not find it again
     if (e == cudaErrorMemoryAllocation) {
         return fail(EULR_ERR_OUT_OF_MEMORY, "%s: %s", what, cudaGetErrorString(e));
     }
