@@ -138,9 +138,18 @@ def check(status: int) -> None:
 
 
 # ------------------------------------------------------------ tensor helpers
+# An operator's call on a small grid is host work: the C entry point takes 3-4
+# us, so these helpers build no tensor views and no stream objects (16^3: 20 us
+# a call with them).
+_torch_module = None
+
+
 def _torch():
-    import torch
-    return torch
+    global _torch_module
+    if _torch_module is None:
+        import torch
+        _torch_module = torch
+    return _torch_module
 
 
 def bundle(t) -> Bundle5:
@@ -148,8 +157,9 @@ def bundle(t) -> Bundle5:
     if hasattr(t, "data_ptr"):
         if not t.is_contiguous() or t.dim() != 4 or t.shape[0] != 5:
             raise ValueError("a bundle is a contiguous tensor of shape (5, n2, n1, n0)")
-        step = t[0].numel() * t.element_size()
+        step = t.numel() // 5 * t.element_size()
         base = t.data_ptr()
+        return Bundle5(base, base + step, base + 2 * step, base + 3 * step, base + 4 * step)
     else:
         if not t.flags.c_contiguous or t.ndim != 4 or t.shape[0] != 5:
             raise ValueError("a bundle is a C-contiguous array of shape (5, n2, n1, n0)")
@@ -163,7 +173,7 @@ def null_bundle() -> Bundle5:
 
 
 def dims(t) -> tuple[int, int, int]:
-    n2, n1, n0 = t.shape[1:]
+    _, n2, n1, n0 = t.shape
     return int(n0), int(n1), int(n2)
 
 
@@ -176,51 +186,58 @@ def _sfx(t) -> str:
     raise TypeError(f"unsupported dtype {t.dtype}")
 
 
-def _stream(stream=None):
+_raw_stream = None  # the current device's current stream as an integer, once CUDA is up
+
+
+def _stream(stream=None) -> int:
+    global _raw_stream
+    if stream is not None:
+        return stream.cuda_stream
+    if _raw_stream is not None:
+        return _raw_stream()
     torch = _torch()
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return ctypes.c_void_p(s.cuda_stream)
+    s = torch.cuda.current_stream().cuda_stream  # initializes CUDA
+    get, device = getattr(torch._C, "_cuda_getCurrentRawStream", None), getattr(torch._C, "_cuda_getDevice", None)
+    if get is not None and device is not None:
+        _raw_stream = lambda: get(device())  # noqa: E731
+    return s
 
 
-def _scalar(sfx):
-    return _D if sfx == "f64" else _F
+_operators: dict = {}  # (entry point, suffix) -> its C function
+
+
+def _operator(name: str, sfx: str):
+    fn = _operators.get((name, sfx))
+    if fn is None:
+        fn = _operators[name, sfx] = getattr(load(), f"eulr_{name}_{sfx}")
+    return fn
 
 
 def init_implode(n0, n1, n2, dx, dtype=None, device="cuda", stream=None):
     torch = _torch()
     dtype = dtype or torch.float64
     prim = torch.empty((5, n2, n1, n0), dtype=dtype, device=device)
-    sfx = _sfx(prim)
-    c = _scalar(sfx)
-    check(getattr(load(), f"eulr_init_implode_{sfx}")(bundle(prim), n0, n1, n2, c(dx[0]), c(dx[1]), c(dx[2]),
-                                                       _stream(stream)))
+    check(_operator("init_implode", _sfx(prim))(bundle(prim), n0, n1, n2, dx[0], dx[1], dx[2], _stream(stream)))
     return prim
 
 
 def prim_to_cons(prim, gamma, out=None, stream=None):
     cons = out if out is not None else _torch().empty_like(prim)
-    sfx = _sfx(prim)
-    check(getattr(load(), f"eulr_prim_to_cons_{sfx}")(bundle(prim), bundle(cons), *dims(prim),
-                                                       _scalar(sfx)(gamma), _stream(stream)))
+    check(_operator("prim_to_cons", _sfx(prim))(bundle(prim), bundle(cons), *dims(prim), gamma, _stream(stream)))
     return cons
 
 
 def cons_to_prim(cons, gamma, out=None, stream=None):
     prim = out if out is not None else _torch().empty_like(cons)
-    sfx = _sfx(cons)
-    check(getattr(load(), f"eulr_cons_to_prim_{sfx}")(bundle(cons), bundle(prim), *dims(cons),
-                                                       _scalar(sfx)(gamma), _stream(stream)))
+    check(_operator("cons_to_prim", _sfx(cons))(bundle(cons), bundle(prim), *dims(cons), gamma, _stream(stream)))
     return prim
 
 
 def time_step(prim, gamma, dx, out=None, stream=None):
     """Device scalar tensor holding time_step(prim) (not multiplied by CFL)."""
-    torch = _torch()
-    dt = out if out is not None else torch.empty((), dtype=prim.dtype, device=prim.device)
-    sfx = _sfx(prim)
-    c = _scalar(sfx)
-    check(getattr(load(), f"eulr_time_step_{sfx}")(bundle(prim), *dims(prim), c(gamma), c(dx[0]), c(dx[1]),
-                                                    c(dx[2]), ctypes.c_void_p(dt.data_ptr()), _stream(stream)))
+    dt = out if out is not None else _torch().empty((), dtype=prim.dtype, device=prim.device)
+    check(_operator("time_step", _sfx(prim))(bundle(prim), *dims(prim), gamma, dx[0], dx[1], dx[2], dt.data_ptr(),
+                                             _stream(stream)))
     return dt
 
 
@@ -230,21 +247,20 @@ def godunov(prim, cons, gamma, dx, dt, stream=None, exact=False):
     (tensor, cfl)).  exact=True: bit-identical to the reference
     (eulr_godunov_exact_*; a float dt only)."""
     sfx = _sfx(prim)
-    c = _scalar(sfx)
     if exact:
         if isinstance(dt, tuple):
             raise ValueError("the exact godunov takes dt as a number")
-        check(getattr(load(), f"eulr_godunov_exact_{sfx}")(bundle(prim), bundle(cons), *dims(prim), c(gamma),
-                                                            c(dx[0]), c(dx[1]), c(dx[2]), c(dt), _stream(stream)))
-        return cons
-    if isinstance(dt, tuple):
+        check(_operator("godunov_exact", sfx)(bundle(prim), bundle(cons), *dims(prim), gamma, dx[0], dx[1], dx[2], dt,
+                                              _stream(stream)))
+    elif isinstance(dt, tuple):
+        if sfx != "f64":
+            raise ctypes.ArgumentError("a device dt needs FP64 bundles")
         dt_t, cfl = dt
-        check(load().eulr_godunov_devdt_f64(bundle(prim), bundle(cons), *dims(prim), c(gamma), c(dx[0]),
-                                            c(dx[1]), c(dx[2]), ctypes.c_void_p(dt_t.data_ptr()), c(cfl),
-                                            _stream(stream)))
+        check(_operator("godunov_devdt", "f64")(bundle(prim), bundle(cons), *dims(prim), gamma, dx[0], dx[1], dx[2],
+                                                dt_t.data_ptr(), cfl, _stream(stream)))
     else:
-        check(getattr(load(), f"eulr_godunov_{sfx}")(bundle(prim), bundle(cons), *dims(prim), c(gamma), c(dx[0]),
-                                                      c(dx[1]), c(dx[2]), c(dt), _stream(stream)))
+        check(_operator("godunov", sfx)(bundle(prim), bundle(cons), *dims(prim), gamma, dx[0], dx[1], dx[2], dt,
+                                        _stream(stream)))
     return cons
 
 
