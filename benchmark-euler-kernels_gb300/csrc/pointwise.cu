@@ -16,6 +16,10 @@
 
 namespace eulr {
 
+// Cells whose loads a thread of a memory-bound pass has in flight.
+template <class T>
+constexpr int kCellsInFlight = sizeof(T) == 8 ? 2 : 4;
+
 // ------------------------------------------------------------ init_implode
 // init_implode.hpp:24-44.  Cell centres are computed in double (the literal 0.5
 // promotes (i-1) to double) and rounded to T, as in the reference's float
@@ -44,27 +48,56 @@ __global__ void __launch_bounds__(256) init_implode_kernel(Bundle<T> prim, Geom 
     }
 }
 
+// One pass over n cells from five fields to five others.  FP32 is bound by
+// HBM: a thread has four cells' loads in flight (256^3: 125 -> 115 us, 6.0 TB/s).
+// FP64 is bound by its arithmetic and takes one cell at a time.
+template <class T, class Cell>
+__device__ __forceinline__ void pointwise_pass(CBundle<T> const& in, Bundle<T> const& out, long long n, Cell cell)
+{
+    constexpr int kCells = sizeof(T) == 8 ? 1 : kCellsInFlight<T>;
+    long long const stride = static_cast<long long>(gridDim.x) * blockDim.x;
+    for (long long base = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; base < n; base += kCells * stride) {
+        T a[kCells][5];
+#pragma unroll
+        for (int u = 0; u < kCells; ++u) {
+            long long const c = base + u * stride;
+            if (c < n) {
+#pragma unroll
+                for (int f = 0; f < 5; ++f) {
+                    a[u][f] = in.f[f][c];
+                }
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < kCells; ++u) {
+            long long const c = base + u * stride;
+            if (c < n) {
+                T b[5];
+                cell(a[u], b);
+#pragma unroll
+                for (int f = 0; f < 5; ++f) {
+                    out.f[f][c] = b[f];
+                }
+            }
+        }
+    }
+}
+
 // ------------------------------------------------------------ prim_to_cons
 // prim_to_cons.hpp:20-32 with to_cons (euler_arrays.hpp:56-64):
 //   e = d*((u0*u0 + u1*u1) + u2*u2)/2 + p/(gamma-1),  m_i = d*u_i.
 template <class T>
 __global__ void __launch_bounds__(256) prim_to_cons_kernel(CBundle<T> prim, Bundle<T> cons, long long n, T gm1, T rgm1)
 {
-    for (long long c = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; c < n;
-         c += static_cast<long long>(gridDim.x) * blockDim.x) {
-        T const d = prim.f[0][c];
-        T const p = prim.f[1][c];
-        T const u0 = prim.f[2][c];
-        T const u1 = prim.f[3][c];
-        T const u2 = prim.f[4][c];
-        T const int_e = div_by_rcp(p, gm1, rgm1);
-        T const ke = half_exact(mul_rn(d, add_rn(add_rn(mul_rn(u0, u0), mul_rn(u1, u1)), mul_rn(u2, u2))));
-        cons.f[0][c] = d;
-        cons.f[1][c] = add_rn(ke, int_e);
-        cons.f[2][c] = mul_rn(d, u0);
-        cons.f[3][c] = mul_rn(d, u1);
-        cons.f[4][c] = mul_rn(d, u2);
-    }
+    pointwise_pass(prim, cons, n, [=](T const* q, T* u) {
+        T const int_e = div_by_rcp(q[1], gm1, rgm1);
+        T const ke = half_exact(mul_rn(q[0], add_rn(add_rn(mul_rn(q[2], q[2]), mul_rn(q[3], q[3])), mul_rn(q[4], q[4]))));
+        u[0] = q[0];
+        u[1] = add_rn(ke, int_e);
+        u[2] = mul_rn(q[0], q[2]);
+        u[3] = mul_rn(q[0], q[3]);
+        u[4] = mul_rn(q[0], q[4]);
+    });
 }
 
 // ------------------------------------------------------------ cons_to_prim
@@ -74,76 +107,53 @@ __global__ void __launch_bounds__(256) prim_to_cons_kernel(CBundle<T> prim, Bund
 template <class T>
 __global__ void __launch_bounds__(256) cons_to_prim_kernel(CBundle<T> cons, Bundle<T> prim, long long n, T gm1)
 {
-    for (long long c = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; c < n;
-         c += static_cast<long long>(gridDim.x) * blockDim.x) {
-        T const d = cons.f[0][c];
-        T p, u0, u1, u2;
-        cons_to_prim_exact(d, cons.f[1][c], cons.f[2][c], cons.f[3][c], cons.f[4][c], gm1, p, u0, u1, u2);
-        prim.f[0][c] = d;
-        prim.f[1][c] = p;
-        prim.f[2][c] = u0;
-        prim.f[3][c] = u1;
-        prim.f[4][c] = u2;
-    }
+    pointwise_pass(cons, prim, n, [=](T const* u, T* q) {
+        q[0] = u[0];
+        cons_to_prim_exact(u[0], u[1], u[2], u[3], u[4], gm1, q[1], q[2], q[3], q[4]);
+    });
 }
 
 // --------------------------------------------------------------- time_step
 // time_step.hpp:22-39.  The reference takes min over cells of 1/invdt; since
 // correctly rounded division is monotonic, min_c RN(1/x_c) = RN(1/max_c x_c),
 // so the kernel reduces max(invdt) (exact, order-free) and divides once.
-// FP64: the max is screened (WaveScreen), so the kernel reads 40 B per cell
-// and issues FP64 instructions only for the few cells evaluated exactly; the
-// dt is still the reference's bit for bit.  NaN never wins (the reference's Kokkos::min
+// The max is screened (WaveScreen, CflRecord), so the kernel reads each cell
+// and evaluates its exact wavespeed only where it can be the max; the dt is
+// still the reference's bit for bit.  Bound by HBM (256^3: FP64 167 -> 114 us,
+// 6.1 TB/s; FP32, which took every exact wavespeed, 90 -> 62).  NaN never wins (the reference's Kokkos::min
 // skips it) and an all-zero grid returns the reduction identity T's max, as
 // the reference's Min reducer does.
 template <class T>
 __global__ void __launch_bounds__(256) time_step_kernel(CBundle<T> prim, long long n, T gamma, T ix0, T ix1, T ix2,
-                                                        T* partials, unsigned int* counter, T* dt_out)
+                                                        ScreenArgs a, T* partials, unsigned int* counter, T* dt_out)
 {
-    T local = T(0);
-    if constexpr (sizeof(T) == 8) {
-        WaveScreen screen(gamma, ix0, ix1, ix2);
-        int const lane = threadIdx.x & 31;
-        long long const stride = static_cast<long long>(gridDim.x) * blockDim.x;
-        // warp-uniform trip count: every lane of a warp runs every iteration
-        for (long long base = blockIdx.x * static_cast<long long>(blockDim.x) + (threadIdx.x & ~31); base < n;
-             base += stride) {
-            long long const c = base + lane;
-            bool const valid = c < n;
-            T d = T(1), p = T(1), u0 = T(0), u1 = T(0), u2 = T(0);
-            if (valid) {
-                d = prim.f[0][c];
-                p = prim.f[1][c];
-                u0 = prim.f[2][c];
-                u1 = prim.f[3][c];
-                u2 = prim.f[4][c];
-            }
-            if (screen.exact_needed(valid, d, p, u0, u1, u2)) {
-                T const v = cell_invdt_exact(d, p, u0, u1, u2, gamma, ix0, ix1, ix2);
-                local = (v > local) ? v : local;
+    WaveScreen const screen(a.gamma, a.ix0, a.ix1, a.ix2);
+    CflRecord<T> record;
+    // several cells' loads in flight at a time
+    constexpr int kCells = kCellsInFlight<T>;
+    long long const stride = static_cast<long long>(gridDim.x) * blockDim.x;
+    for (long long base = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; base < n; base += kCells * stride) {
+        T q[kCells][5];
+#pragma unroll
+        for (int u = 0; u < kCells; ++u) {
+            long long const c = base + u * stride < n ? base + u * stride : base; // loaded without a branch
+#pragma unroll
+            for (int f = 0; f < 5; ++f) {
+                q[u][f] = prim.f[f][c];
             }
         }
-    } else {
-        for (long long c = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; c < n;
-             c += static_cast<long long>(gridDim.x) * blockDim.x) {
-            T const v = cell_invdt_exact(prim.f[0][c], prim.f[1][c], prim.f[2][c], prim.f[3][c], prim.f[4][c], gamma,
-                                         ix0, ix1, ix2);
-            local = (v > local) ? v : local;
+#pragma unroll
+        for (int u = 0; u < kCells; ++u) {
+            if (base + u * stride < n) {
+                record.offer(screen, q[u][0], q[u][1], q[u][2], q[u][3], q[u][4], gamma, ix0, ix1, ix2);
+            }
         }
     }
-    __shared__ T warp_best[8];
+    record.finish(gamma, ix0, ix1, ix2);
     __shared__ bool is_last;
-    local = warp_max(local);
-    if ((threadIdx.x & 31) == 0) {
-        warp_best[threadIdx.x >> 5] = local;
-    }
-    __syncthreads();
+    T const mine = block_max(record.local);
     if (threadIdx.x == 0) {
-        T b = warp_best[0];
-        for (int w = 1; w < static_cast<int>(blockDim.x >> 5); ++w) {
-            b = (warp_best[w] > b) ? warp_best[w] : b;
-        }
-        partials[blockIdx.x] = b;
+        partials[blockIdx.x] = mine;
         __threadfence();
         unsigned int const done = atomicAdd(counter, 1u);
         is_last = (done == gridDim.x - 1);
@@ -157,16 +167,8 @@ __global__ void __launch_bounds__(256) time_step_kernel(CBundle<T> prim, long lo
             T const v = __ldcg(&partials[w]);
             b = (v > b) ? v : b;
         }
-        b = warp_max(b);
-        if ((threadIdx.x & 31) == 0) {
-            warp_best[threadIdx.x >> 5] = b;
-        }
-        __syncthreads();
+        T const m = block_max(b);
         if (threadIdx.x == 0) {
-            T m = warp_best[0];
-            for (int w = 1; w < static_cast<int>(blockDim.x >> 5); ++w) {
-                m = (warp_best[w] > m) ? warp_best[w] : m;
-            }
             *dt_out = (m > T(0)) ? rcp_rn(m) : (sizeof(T) == 8 ? T(DBL_MAX) : T(FLT_MAX));
             *counter = 0u;
         }
@@ -215,63 +217,44 @@ __global__ void __launch_bounds__(256) invdt_max_cons_kernel(CBundle<float> cons
 __global__ void __launch_bounds__(256) load_prim_kernel(CBundle<double> prim, Bundle<double> cons, Bundle<double> copy,
                                                         double* cs, double* h, const double* e_in, long long n,
                                                         double gamma, double gm1, double rgm1, double ix0, double ix1,
-                                                        double ix2, unsigned long long* wmax)
+                                                        double ix2, ScreenArgs a, unsigned long long* wmax)
 {
-    double local = 0.0;
-    WaveScreen screen(gamma, ix0, ix1, ix2);
-    int const lane = threadIdx.x & 31;
-    long long const stride = static_cast<long long>(gridDim.x) * blockDim.x;
-    // warp-uniform trip count: every lane of a warp runs every iteration
-    for (long long base = blockIdx.x * static_cast<long long>(blockDim.x) + (threadIdx.x & ~31); base < n;
-         base += stride) {
-        long long const c = base + lane;
-        bool const valid = c < n;
-        double d = 1.0, p = 1.0, u0 = 0.0, u1 = 0.0, u2 = 0.0;
-        if (valid) {
-            d = prim.f[0][c];
-            p = prim.f[1][c];
-            u0 = prim.f[2][c];
-            u1 = prim.f[3][c];
-            u2 = prim.f[4][c];
-            if (copy.f[0] != nullptr) {
-                copy.f[0][c] = d;
-                copy.f[1][c] = p;
-                copy.f[2][c] = u0;
-                copy.f[3][c] = u1;
-                copy.f[4][c] = u2;
-            }
-            if (cons.f[0] != nullptr) {
-                double const int_e = div_by_rcp(p, gm1, rgm1);
-                double const ke = half_exact(mul_rn(d, add_rn(add_rn(mul_rn(u0, u0), mul_rn(u1, u1)), mul_rn(u2, u2))));
-                double const e = add_rn(ke, int_e);
-                cons.f[0][c] = d;
-                cons.f[1][c] = e;
-                cons.f[2][c] = mul_rn(d, u0);
-                cons.f[3][c] = mul_rn(d, u1);
-                cons.f[4][c] = mul_rn(d, u2);
-                h[c] = add_rn(e, p);
-            } else {
-                h[c] = add_rn(e_in[c], p);
-            }
-            cs[c] = sqrt_quotient_faithful(gamma * p, d); // 1/rho is not needed here
+    WaveScreen const screen(a.gamma, a.ix0, a.ix1, a.ix2);
+    CflRecord<double> record;
+    for (long long c = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; c < n;
+         c += static_cast<long long>(gridDim.x) * blockDim.x) {
+        double const d = prim.f[0][c];
+        double const p = prim.f[1][c];
+        double const u0 = prim.f[2][c];
+        double const u1 = prim.f[3][c];
+        double const u2 = prim.f[4][c];
+        if (copy.f[0] != nullptr) {
+            copy.f[0][c] = d;
+            copy.f[1][c] = p;
+            copy.f[2][c] = u0;
+            copy.f[3][c] = u1;
+            copy.f[4][c] = u2;
         }
-        if (screen.exact_needed(valid, d, p, u0, u1, u2)) {
-            double const v = cell_invdt_exact(d, p, u0, u1, u2, gamma, ix0, ix1, ix2);
-            local = (v > local) ? v : local; // NaN never wins
+        if (cons.f[0] != nullptr) {
+            double const int_e = div_by_rcp(p, gm1, rgm1);
+            double const ke = half_exact(mul_rn(d, add_rn(add_rn(mul_rn(u0, u0), mul_rn(u1, u1)), mul_rn(u2, u2))));
+            double const e = add_rn(ke, int_e);
+            cons.f[0][c] = d;
+            cons.f[1][c] = e;
+            cons.f[2][c] = mul_rn(d, u0);
+            cons.f[3][c] = mul_rn(d, u1);
+            cons.f[4][c] = mul_rn(d, u2);
+            h[c] = add_rn(e, p);
+        } else {
+            h[c] = add_rn(e_in[c], p);
         }
+        cs[c] = sqrt_quotient_faithful(gamma * p, d); // 1/rho is not needed here
+        record.offer(screen, d, p, u0, u1, u2, gamma, ix0, ix1, ix2);
     }
-    __shared__ double warp_best[8];
-    local = warp_max(local);
-    if (lane == 0) {
-        warp_best[threadIdx.x >> 5] = local;
-    }
-    __syncthreads();
+    record.finish(gamma, ix0, ix1, ix2);
+    double const mine = block_max(record.local);
     if (threadIdx.x == 0) {
-        double b = warp_best[0];
-        for (int w = 1; w < static_cast<int>(blockDim.x >> 5); ++w) {
-            b = (warp_best[w] > b) ? warp_best[w] : b;
-        }
-        atomicMax(wmax, order_bits(b));
+        atomicMax(wmax, static_cast<unsigned long long>(dbits(mine)));
     }
 }
 
@@ -313,6 +296,12 @@ static int grid_for(long long n, int sms)
 }
 
 template <class T>
+static ScreenArgs screen_args(T gamma, T ix0, T ix1, T ix2)
+{
+    return ScreenArgs{static_cast<float>(gamma), static_cast<float>(ix0), static_cast<float>(ix1), static_cast<float>(ix2)};
+}
+
+template <class T>
 cudaError_t launch_init_implode(Bundle<T> prim, Geom g, double dx0, double dx1, double dx2, int sms, cudaStream_t s)
 {
     init_implode_kernel<T><<<grid_for(g.ncell(), sms), 256, 0, s>>>(prim, g, dx0, dx1, dx2);
@@ -337,11 +326,12 @@ template <class T>
 cudaError_t launch_time_step(CBundle<T> prim, long long n, T gamma, T ix0, T ix1, T ix2, T* partials,
                              int max_partials, unsigned int* counter, T* dt_out, int sms, cudaStream_t s)
 {
-    int grid = grid_for(n, sms);
+    int grid = grid_for((n + kCellsInFlight<T> - 1) / kCellsInFlight<T>, sms);
     if (grid > max_partials) {
         grid = max_partials;
     }
-    time_step_kernel<T><<<grid, 256, 0, s>>>(prim, n, gamma, ix0, ix1, ix2, partials, counter, dt_out);
+    time_step_kernel<T><<<grid, 256, 0, s>>>(prim, n, gamma, ix0, ix1, ix2, screen_args(gamma, ix0, ix1, ix2), partials,
+                                             counter, dt_out);
     return cudaGetLastError();
 }
 
@@ -351,7 +341,7 @@ cudaError_t launch_load_prim(CBundle<double> prim, Bundle<double> cons, Bundle<d
 {
     double const gm1 = gamma - 1.0;
     load_prim_kernel<<<grid_for(n, sms), 256, 0, s>>>(prim, cons, copy, cs, h, e_in, n, gamma, gm1, 1.0 / gm1, ix0, ix1,
-                                                      ix2, wmax);
+                                                      ix2, screen_args(gamma, ix0, ix1, ix2), wmax);
     return cudaGetLastError();
 }
 

@@ -188,17 +188,19 @@ __device__ __forceinline__ void batch_cta_done(BatchParams<T> const& b)
 // from the doubles' high words on the integer pipe (the mantissa truncated to
 // 20 bits, a relative error in (-2^-20, 0]) and the rest runs on the FP32
 // pipe.  Where rho, p and gamma p/rho lie in [1e-30, 1e30] and the estimate
-// is at most 1e30, its relative error is below 2^-20 + 5 * 2^-24 to first
-// order: p/rho carries under 2^-20 (both truncations go toward zero), the
-// square root halves it, |u| carries under 2^-20, and gamma, 1/dx and eight
-// FP32 operations add 2^-24 each along any path.  Two estimates can thus
-// misorder cells by at most 2.7 * 2^-20 relative, 42 FP32 ulps; a cell is
-// evaluated exactly when its estimate is within 128 ulps of the warp's
-// running max of estimates.  Every other cell -- NaN, infinite or
-// out-of-range values -- is always evaluated exactly.  So the cell holding
-// the exact max is always evaluated, and the max of the exact values over
-// the evaluated cells is the exact max.  The evaluated cells are essentially
-// each warp's running-max records: a few per ten thousand on random states.
+// is at most 1e30, its relative error is below 2^-20 + 2^-21 + 5 * 2^-24 to
+// first order: p/rho carries under 2^-20 (both truncations go toward zero),
+// the square root halves it, |u| carries under 2^-20, the hardware's
+// approximations of the reciprocal and the reciprocal square root under 2^-22
+// each, and gamma, 1/dx and eight FP32 operations add 2^-24 each along any
+// path.  Two estimates can thus misorder cells by at most 3.7 * 2^-20
+// relative, 59 FP32 ulps; a cell is
+// evaluated exactly when its estimate is within 128 ulps of the running max of
+// estimates (a thread's own and then its block's, CflRecord; a warp's in the
+// fused step).  Every other cell -- NaN, infinite or out-of-range values -- is
+// always evaluated exactly.  So the cell holding the exact max is always
+// evaluated, and the max of the exact values over the evaluated cells is the
+// exact max.
 struct WaveScreen {
     float g, ix0, ix1, ix2;
     bool on;        // gamma and 1/dx in FP32's safe range: screening is sound
@@ -216,31 +218,47 @@ struct WaveScreen {
         return __uint_as_float((hi & 0x80000000u) | mag);
     }
 
-    __device__ __forceinline__ WaveScreen(double gamma, double x0, double x1, double x2)
-        : g(static_cast<float>(gamma)), ix0(static_cast<float>(x0)), ix1(static_cast<float>(x1)),
-          ix2(static_cast<float>(x2)), run(0u)
+    __device__ __forceinline__ WaveScreen(float gamma, float x0, float x1, float x2)
+        : g(gamma), ix0(x0), ix1(x1), ix2(x2), run(0u)
     {
         on = in_range(g) && in_range(ix0) && in_range(ix1) && in_range(ix2);
     }
+    __device__ __forceinline__ WaveScreen(double gamma, double x0, double x1, double x2)
+        : WaveScreen(static_cast<float>(gamma), static_cast<float>(x0), static_cast<float>(x1), static_cast<float>(x2))
+    {
+    }
 
-    // Warp-collective (all 32 lanes call it together): true when this lane's
-    // cell (if valid) needs its exact wavespeed.
-    __device__ __forceinline__ bool exact_needed(bool valid, double d, double p, double u0, double u1, double u2)
+    // Bit pattern of a cell's estimate, and whether the estimate's bound
+    // holds for it.
+    __device__ __forceinline__ unsigned estimate(double d, double p, double u0, double u1, double u2, bool& sure) const
     {
         float const d32 = high_word_float(d);
         float const p32 = high_word_float(p);
-        float const x32 = __fdiv_rn(g * p32, d32);
-        float const c32 = __fsqrt_rn(x32);
+        float const x32 = g * p32 * rcp_approx(d32);
+        float const c32 = x32 * rsqrt_approx(x32);
         float const v32 = (c32 + fabsf(high_word_float(u0))) * ix0 + (c32 + fabsf(high_word_float(u1))) * ix1 +
                           (c32 + fabsf(high_word_float(u2))) * ix2;
-        bool const sure = on && in_range(d32) && in_range(p32) && in_range(x32) && v32 <= 1e30f;
-        unsigned const key = (valid && sure) ? __float_as_uint(v32) : 0u;
-        unsigned const m = __reduce_max_sync(0xffffffffu, key);
-        run = m > run ? m : run;
-        return valid && (!sure || key + 128u >= run);
+        sure = on && in_range(d32) && in_range(p32) && in_range(x32) && v32 <= 1e30f;
+        return __float_as_uint(v32);
     }
 
-    // The fused FP64 step's form (warp-collective as well).  The step has the
+    // The same for FP32 cells, whose wavespeed takes a correctly rounded
+    // quotient and square root: the hardware's approximations, each within
+    // 2^-22, put the estimate within 2^-21 + 6 * 2^-24 of the true value and
+    // the exact expression's own roundings add 6 * 2^-24, so two estimates
+    // misorder exact values by at most 28 ulps.
+    __device__ __forceinline__ unsigned estimate(float d, float p, float u0, float u1, float u2, bool& sure) const
+    {
+        float const x = g * p * rcp_approx(d);
+        float const c = x * rsqrt_approx(x);
+        float const v = (c + fabsf(u0)) * ix0 + (c + fabsf(u1)) * ix1 + (c + fabsf(u2)) * ix2;
+        sure = on && in_range(d) && in_range(p) && in_range(x) && v <= 1e30f;
+        return __float_as_uint(v);
+    }
+
+    // The fused FP64 step's form (warp-collective: all 32 lanes call it
+    // together): true when this lane's cell, if valid, needs its exact
+    // wavespeed.  The step has the
     // new state's faithful sound speed cs and its velocities, and its
     // wavespeed is (3 cs + |v0| + |v1| + |v2|) / dx on cubic cells, else
     // sum_d (cs + |v_d|) / dx_d.  The estimate truncates cs and |v_d| (each
@@ -262,6 +280,115 @@ struct WaveScreen {
         unsigned const m = __reduce_max_sync(0xffffffffu, key);
         run = m > run ? m : run;
         return valid && (!sure || key + 128u >= run);
+    }
+};
+
+// gamma and 1/dx in FP32, converted on the host: four conversions a thread
+// would go through the FP64 pipe.
+struct ScreenArgs {
+    float gamma, ix0, ix1, ix2;
+};
+
+// Block max of non-negative values, in thread 0; on the integer pipe.
+__device__ __forceinline__ double block_max(double v)
+{
+    __shared__ long long best[32];
+    long long b = dbits(v);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        long long const w = __shfl_xor_sync(0xffffffffu, b, o);
+        b = w > b ? w : b;
+    }
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) {
+        best[threadIdx.x >> 5] = b;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < static_cast<int>(blockDim.x >> 5); ++w) {
+            b = best[w] > b ? best[w] : b;
+        }
+    }
+    return __longlong_as_double(b);
+}
+__device__ __forceinline__ float block_max(float v)
+{
+    __shared__ unsigned best[32];
+    unsigned b = __reduce_max_sync(0xffffffffu, __float_as_uint(v));
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) {
+        best[threadIdx.x >> 5] = b;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < static_cast<int>(blockDim.x >> 5); ++w) {
+            b = best[w] > b ? best[w] : b;
+        }
+    }
+    return __uint_as_float(b);
+}
+
+__device__ __forceinline__ bool same_bits(double a, double b) { return dbits(a) == dbits(b); }
+__device__ __forceinline__ bool same_bits(float a, float b) { return __float_as_uint(a) == __float_as_uint(b); }
+
+// A thread's cells offered one by one: keeps the one with the largest
+// estimate and drops those that it outranks by more than the band, so that a
+// pass over the grid evaluates the exact wavespeed about once per block (the
+// warps' own running maxima, as the fused step takes them, cost a pass at
+// 129 x 96 x 73 more than its memory traffic: 46 us, 17 this way).  Cells within
+// the band of the kept one are evaluated at once, bit-equal ones skipped.
+template <class T>
+struct CflRecord {
+    unsigned best = 0u; // the kept cell's estimate; 0: none
+    T d = T(1), p = T(1), u0 = T(0), u1 = T(0), u2 = T(0);
+    T local = T(0); // max over the cells evaluated
+
+    __device__ __forceinline__ void take(T v) { local = v > local ? v : local; } // NaN never wins
+
+    // ix: 1/dx in T, as the exact expression takes them
+    __device__ __forceinline__ void offer(WaveScreen const& screen, T cd, T cp, T c0, T c1, T c2, T gamma, T ix0, T ix1,
+                                          T ix2)
+    {
+        bool sure;
+        unsigned const key = screen.estimate(cd, cp, c0, c1, c2, sure);
+        if (!sure || key <= 256u) { // out of the estimate's range, or too small for a band in ulps
+            take(cell_invdt_exact(cd, cp, c0, c1, c2, gamma, ix0, ix1, ix2));
+            return;
+        }
+        if (key + 128u < best) {
+            return;
+        }
+        if (best + 128u >= key) {
+            if (same_bits(cd, d) && same_bits(cp, p) && same_bits(c0, u0) && same_bits(c1, u1) && same_bits(c2, u2)) {
+                return;
+            }
+            take(cell_invdt_exact(d, p, u0, u1, u2, gamma, ix0, ix1, ix2)); // the kept cell; the new one is kept
+        }
+        best = key;
+        d = cd;
+        p = cp;
+        u0 = c0;
+        u1 = c1;
+        u2 = c2;
+    }
+
+    // Block-collective: the exact wavespeed of the kept cells within the band
+    // of the block's largest estimate.
+    __device__ __forceinline__ void finish(T gamma, T ix0, T ix1, T ix2)
+    {
+        __shared__ unsigned top;
+        if (threadIdx.x == 0) {
+            top = 0u;
+        }
+        __syncthreads();
+        unsigned const w = __reduce_max_sync(0xffffffffu, best);
+        if ((threadIdx.x & 31) == 0) {
+            atomicMax(&top, w);
+        }
+        __syncthreads();
+        if (best != 0u && best + 128u >= top) {
+            take(cell_invdt_exact(d, p, u0, u1, u2, gamma, ix0, ix1, ix2));
+        }
     }
 };
 
