@@ -120,8 +120,8 @@ EULR_ADJ_FN double tie_side_bar(FaceSide const& q, double a, double S, double iS
 // ds into (dd, ..., dt2) and ds is not read.  SETS the cotangents of the two
 // sides' primitive states, bL and bR.
 //
-// What is transposed is the flux in the forward step's form (hllc_flux in
-// euler_device.cuh), which is the reference's in exact arithmetic:
+// What is transposed is the flux in the forward step's form (hllc_upwind
+// in euler_device.cuh), which is the reference's in exact arithmetic:
 //   A = cmax + max(u_L - u_R, 0), G = A (d_L + d_R),
 //   n = A (d_L u_L + d_R u_R) - (p_R - p_L), ustar = n/G,
 //   and with the upwind side's S = u + a, a = -+A, w = ustar - u and

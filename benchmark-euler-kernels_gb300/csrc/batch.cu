@@ -194,6 +194,8 @@ int upload_params(eulr_batch* b)
             p.ds0 = static_cast<T>(G.dx[1] * G.dx[2]);
             p.ds1 = static_cast<T>(G.dx[2] * G.dx[0]);
             p.ds2 = static_cast<T>(G.dx[0] * G.dx[1]);
+            p.rs1 = p.ds1 / p.ds0;
+            p.rs2 = p.ds2 / p.ds0;
             p.dv = G.dx[0] * G.dx[1] * G.dx[2];
             p.dt_dev = &b->sc[g].dt;
             p.cfl = b->cfl;

@@ -277,6 +277,13 @@ struct Flux {
     T d, e, n, t1, t2;
 };
 
+// One side of a face of the FP64 kernels: what decides the face's flux, with
+// the normal momentum mn = d un and h = e + p; the tangential momenta are
+// read where the flux is used.
+struct StagedSide {
+    double d, p, un, mn, c, h;
+};
+
 // ------------------------------------------------- integer-pipe predicates
 // On GB300 an FP64 compare, min or max takes a full slot of the FP64 pipe
 // (1/64 of the FP32 rate); the same decisions taken on the bit patterns run
@@ -337,8 +344,9 @@ __device__ __forceinline__ bool finite_positive(double x)
 // function:
 //  * one acoustic speed.  S_L = min(u) - cmax and S_R = max(u) + cmax give
 //    S_L - u_L = -A and S_R - u_R = A with the same
-//    A = cmax + max(u_L - u_R, 0), so with D = d_L + d_R and G = A D
-//      ustar = n / G,  n = A (d_L u_L + d_R u_R) - (p_R - p_L),
+//    A = cmax + max(u_L - u_R, 0), so with D = d_L + d_R, G = A D and the
+//    momenta m = d u
+//      ustar = n / G,  n = A (m_L + m_R) - (p_R - p_L),
 //    and only the upwind side's wave speed S = u -+ A is formed: the face is
 //    supersonic exactly when S has the sign of ustar.
 //  * ustar and 1/(S - ustar) = G/M, M = S G - n, come from ONE reciprocal
@@ -350,39 +358,46 @@ __device__ __forceinline__ bool finite_positive(double x)
 //    upwind one is used.
 //  * with a = S - u = -+A, w = ustar - u and b = a ustar/(S - ustar) the
 //    flux is
-//      mass    d_star ustar                = d b,
+//      mass                d_star ustar    = b d,
+//      tangential momentum mass u_t        = b m_t,
 //      energy  (e_star + pstar) ustar      = b ((e + p) + S d w),
-//      normal momentum                     = mass ustar + p + a d w,
+//      normal momentum                     = b d ustar + p + a d w,
 //    because e_star + pstar = [a e + pstar ustar - p u + pstar (S - ustar)]/(S - ustar)
 //                           = [a (e + p) + S (pstar - p)]/(S - ustar)
-//    and pstar - p = a d w.
+//    and pstar - p = a d w, with d w = d ustar - m.
 //  * in the supersonic case the reference's ratio (S-u)/(S-u) is exactly 1
 //    and its energy correction exactly 0: ustar := u and b := u (so w = 0)
 //    give the upwind state's own flux with two selects.
 //  * min/max and the sign tests run on the integer pipe (order_key etc.).
+// So four of the five fluxes are b times a value of the upwind side, and the
+// FP64 kernels never form them: the face keeps b, h = (e + p) + S d w and the
+// normal momentum's flux, the side is the sign of b, and each cell adds b d,
+// b m_t and b h to its update with one fma each.
 // Every sum of products is written as the fma it becomes, so that all kernels
 // that inline this give a face the same bits whatever the compiler contracts.
-// 27 FP64 instructions and a reciprocal seed a face, against 30 and a seed
-// with both wave speeds, both impedances and 1/(S - ustar) formed: FP64
-// instructions set the FP64 kernels' time on this GPU.  Results agree with
-// the reference to a few ulps per face; against quadruple precision the mass,
-// energy and tangential fluxes' rms error is 0.7-0.8 of that other form's and
-// the normal momentum's 0.9-1.1 of it.
-__device__ __forceinline__ Flux<double> hllc_flux(Side<double> const& L, Side<double> const& R)
+// 22 FP64 instructions and a reciprocal seed a face, against 27 and a seed
+// with all five fluxes formed from velocities: FP64 instructions set the FP64
+// kernels' time on this GPU.
+struct UpwindFlux {
+    double b;  // carries d, m_t and h of its upwind side: the left one where b > 0
+    double h;  // e + p of that side plus S d w
+    double fn; // flux of the normal momentum
+};
+
+__device__ __forceinline__ UpwindFlux hllc_upwind(StagedSide const& L, StagedSide const& R)
 {
     double const cmax = (dbits(L.c) > dbits(R.c)) ? L.c : R.c; // sound speeds are >= 0
     double const du = L.un - R.un;
     double const A = cmax + (dbits(du) < 0 ? 0.0 : du);
     double const G = A * (L.d + R.d);
-    double const n = fma_rn(A, fma_rn(L.d, L.un, mul_rn(R.d, R.un)), sub_rn(L.p, R.p));
+    double const n = fma_rn(A, L.mn + R.mn, sub_rn(L.p, R.p));
 
     bool const left = dbits(n) > 0; // ustar > 0 (G > 0)
     double const qd = left ? L.d : R.d;
     double const qp = left ? L.p : R.p;
     double const qun = left ? L.un : R.un;
-    double const qut1 = left ? L.ut1 : R.ut1;
-    double const qut2 = left ? L.ut2 : R.ut2;
-    double const qh = left ? L.e : R.e; // e + p of the upwind side
+    double const qmn = left ? L.mn : R.mn;
+    double const qh = left ? L.h : R.h;
     // a = -A on the left, A on the right: the sign bit, on the integer pipe
     double const a = __longlong_as_double(dbits(A) ^ (left ? static_cast<long long>(0x8000000000000000ull) : 0LL));
 
@@ -392,19 +407,17 @@ __device__ __forceinline__ Flux<double> hllc_flux(Side<double> const& L, Side<do
     // S = -0 cannot occur (a is not zero), so the sign bit decides
     bool const supersonic = left ? dbits(S) > 0 : dbits(S) < 0;
     double const ustar = supersonic ? qun : nR * M;
-    double const b = supersonic ? qun : a * (nR * G);
-    double const dw = mul_rn(qd, sub_rn(ustar, qun));
+    double const dus = mul_rn(qd, ustar);
+    double const dw = fma_rn(qd, ustar, -qmn);
 
-    Flux<double> f;
-    f.d = qd * b;
-    f.e = b * fma_rn(S, dw, qh);
-    f.n = fma_rn(f.d, ustar, fma_rn(a, dw, qp));
-    f.t1 = f.d * qut1;
-    f.t2 = f.d * qut2;
+    UpwindFlux f;
+    f.b = supersonic ? qun : a * (nR * G);
+    f.h = fma_rn(S, dw, qh);
+    f.fn = fma_rn(f.b, dus, fma_rn(a, dw, qp));
     return f;
 }
 
-// FP32 version (real_t = float operators): same algebra, FP32 min/max and
+// FP32 version: the same algebra with all five fluxes formed, FP32 min/max and
 // the hardware reciprocal.
 __device__ __forceinline__ Flux<float> hllc_flux(Side<float> const& L, Side<float> const& R)
 {

@@ -7,34 +7,48 @@
 // is chosen for the grid (choose_tiles), and all tiles' planes are divided
 // evenly among a resident grid of CTAs, a run of planes each.  Batch: chunks
 // of planes popped from a queue.  A CTA marches up its run one plane at a
-// time through a ring of plane slots in shared memory, each slot holding the 7 face inputs (d, p, u0, u1, u2, c, e) of a
-// (TX+2) x (TY+2) plane with its one-cell halo.  Per plane:
+// time through a ring of plane slots in shared memory, each slot holding ten
+// values (d, p, u0, u1, u2, c, e + p, m0, m1, m2) of a (TX+2) x (TY+2) plane
+// with its one-cell halo.  Per plane:
 //   1. face phase -- every x face and y face of plane k and every z face
 //      between planes k and k+1 is solved ONCE (the reference solves each
 //      interior face twice, once from each side, godunov.hpp:48-82).  The
 //      FP64 pipe is the bound: the x, y and z faces share one index space
 //      of exactly the tile's faces, and each face's family, cells and axis
-//      permutation are chosen by selects, so a warp whose lanes straddle two
-//      families still runs the HLLC once -- the 800 faces of a 16x16 tile
-//      take exactly 25 warp-passes.  Fluxes go to shared memory in global axes;
-//   2. cell phase -- each thread owns one column cell and applies
-//      cons -= dt/dv * sum_d ds_d (F_R - F_L) (godunov.hpp:84-90) with the
-//      face-area and dt/dv factors folded into three coefficients.  The z
-//      face below the cell is carried in registers from the previous plane.
+//      are chosen by selects, so a warp whose lanes straddle two families
+//      still runs the HLLC once -- the 800 faces of a 16x16 tile take exactly
+//      25 warp-passes.  Three numbers a face go to shared memory
+//      (hllc_upwind), b scaled by the ratio of the face's area to an x
+//      face's where the areas differ;
+//   2. cell phase -- each thread owns one column cell and forms div F of its
+//      six faces, each term b times d, m or h of the face's upwind side, read
+//      from the slots; then cons -= dt/dv ds_0 div F (godunov.hpp:84-90), one
+//      rounding at the state's scale.  What the z face below the cell carries
+//      stays in registers from the previous plane.
+// 22 FP64 instructions a face and 32 a cell's update, where forming all five
+// fluxes at the face took 27 and 30; m staged besides u is what saves them
+// (loading 512^3 and 4 steps: 141.0 -> 133.7 ms; 20 steps of 24 batched grids
+// 36.5 -> 34.5; prim_to_cons, godunov, cons_to_prim and time_step of 256^3
+// 5.36 -> 5.12; the rounding error of a step 0.6 of the other form's against
+// quadruple precision, 1.0 where pressure outweighs
+// momentum).
 // The fused step then finishes the cell on chip: cons_to_prim, sound speed
 // and the next step's CFL max-wavespeed, reduced warp -> block -> one
 // atomicMax per CTA, so dt never leaves the device.
 //
-// Staging: in the fused FP64 step the seven input fields of a plane slot are
+// Staging: in the fused FP64 step the ten input fields of a plane slot are
 // fetched into a ring of three slots, two planes ahead of the plane being
 // solved: by TMA (cp.async.bulk.tensor, one 18x18x1 box per field, each slot
 // completing on its own mbarrier) where the row pitch is a multiple of 16
 // bytes, else and in the batch by 8-byte cp.async (20 steps of a
 // 99 x 128 x 75 grid, odd pitch: 7.0 -> 5.9 ms against synchronous loads and
-// whole tiles).  The per-operator godunov (arbitrary caller pointers, values
-// computed while staged) stages with plain cooperative loads instead.  Every mbarrier wait is bounded: a wait that runs out sets
-// bit 1 of the status word, waits (bounded) for the copies still in flight
-// and ends the CTA.
+// whole tiles).  A slot is refilled once its plane's cell phase is over and
+// has the whole next plane to land.  The per-operator godunov (arbitrary
+// caller pointers, values computed while staged) and the first step of a
+// state whose cons the caller gave besides prim (its momenta need not be
+// d u) stage with plain cooperative loads instead.  Every mbarrier wait is
+// bounded: a wait that runs out sets bit 1 of the status word, waits
+// (bounded) for the copies still in flight and ends the CTA.
 #include "euler_device.cuh"
 #include "kernels.h"
 #include "step_common.cuh"
@@ -52,7 +66,7 @@ constexpr int kWaitTries = 1 << 20; // mbarrier.try_wait attempts before giving 
 enum Staging {
     kStageTma,   // fused FP64 step, row pitch a multiple of 16 bytes: TMA boxes, ring of three slots
     kStageAsync, // fused FP64 step, any pitch, and the batch: 8-byte cp.async, the same ring
-    kStageLoad,  // values are computed while staged (per-operator godunov): plain loads, two slots
+    kStageLoad,  // values are computed while staged (per-operator godunov, FluxParams::own_momenta): plain loads, two slots
 };
 template <int STAGE>
 constexpr int kStageSlots = STAGE == kStageLoad ? 2 : 3;
@@ -71,9 +85,9 @@ struct TileLayout {
     // shared memory, in double elements after a 128-byte mbarrier block
     static constexpr int Q_ELEMS = NSLOT * kFields * PLANE_PAD;
     static constexpr int FX_OFF = Q_ELEMS;
-    static constexpr int FY_OFF = FX_OFF + 5 * NFX;
-    static constexpr int FZ_OFF = FY_OFF + 5 * NFY;
-    static constexpr int ELEMS = FZ_OFF + 5 * NFZ;
+    static constexpr int FY_OFF = FX_OFF + 3 * NFX;
+    static constexpr int FZ_OFF = FY_OFF + 3 * NFY;
+    static constexpr int ELEMS = FZ_OFF + 3 * NFZ;
     static constexpr int MBAR_BYTES = 128;
     // + 128 bytes of slack to align the dynamic region to 128 bytes at run time
     static constexpr size_t BYTES = 128 + MBAR_BYTES + sizeof(double) * static_cast<size_t>(ELEMS);
@@ -197,7 +211,7 @@ __device__ __forceinline__ void issue_plane_async(double* smem, int slot, FluxPa
             long long const o = s.src[r] + plane;
 #pragma unroll
             for (int f = 0; f < kFields; ++f) {
-                const double* const src = (f < 5 ? p.prim.f[f] : (f == 5 ? p.cs : p.h)) + o;
+                const double* const src = (f < 5 ? p.prim.f[f] : (f == 5 ? p.cs : (f == 6 ? p.h : p.cons_in.f[f - 5]))) + o;
                 asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(
                                      base + static_cast<unsigned>((f * L::PLANE_PAD + s.dst[r]) * sizeof(double))),
                              "l"(src)
@@ -207,9 +221,10 @@ __device__ __forceinline__ void issue_plane_async(double* smem, int slot, FluxPa
     }
 }
 
-// Stage plane k of the tile and its halo for the per-operator godunov with
-// plain loads: prim as it is, the sound speed and e + p derived from it.
-template <int TX, int TY, int NSLOT>
+// Stage plane k of the tile and its halo with plain loads: prim as it is and
+// the momenta d u.  Per-operator godunov: the sound speed and e + p derived
+// from prim; step: as stored.
+template <int TX, int TY, int NSLOT, int MODE>
 __device__ __forceinline__ void load_plane(double* smem, int slot, FluxParams<double> const& p, TileDims const& t, int i0, int j0,
                                            int k)
 {
@@ -226,54 +241,71 @@ __device__ __forceinline__ void load_plane(double* smem, int slot, FluxParams<do
         double const u0 = __ldg(p.prim.f[2] + o);
         double const u1 = __ldg(p.prim.f[3] + o);
         double const u2 = __ldg(p.prim.f[4] + o);
+        double const m0 = d * u0;
+        double const m1 = d * u1;
+        double const m2 = d * u2;
         q[0 * L::PLANE_PAD + c] = d;
         q[1 * L::PLANE_PAD + c] = pr;
         q[2 * L::PLANE_PAD + c] = u0;
         q[3 * L::PLANE_PAD + c] = u1;
         q[4 * L::PLANE_PAD + c] = u2;
-        // sqrt(gamma p / rho) from one reciprocal square root, and
-        // e + p = p gamma/(gamma-1) + (rho/2) |u|^2 with the halving on the
-        // integer pipe: 4 FP64 instructions and a seed fewer per staged cell
-        // than 1/rho, a square root and e formed before p is added
-        q[5 * L::PLANE_PAD + c] = sqrt_quotient_faithful(p.gamma * pr, d);
-        q[6 * L::PLANE_PAD + c] = pr * (p.inv_gm1 + 1.0) + half_exact(d) * (u0 * u0 + u1 * u1 + u2 * u2);
+        q[7 * L::PLANE_PAD + c] = m0;
+        q[8 * L::PLANE_PAD + c] = m1;
+        q[9 * L::PLANE_PAD + c] = m2;
+        if (MODE == kModeStep) {
+            q[5 * L::PLANE_PAD + c] = __ldg(p.cs + o);
+            q[6 * L::PLANE_PAD + c] = __ldg(p.h + o);
+        } else {
+            // sqrt(gamma p / rho) from one reciprocal square root, and
+            // e + p = p gamma/(gamma-1) + m.u / 2 with the halving on the
+            // integer pipe
+            q[5 * L::PLANE_PAD + c] = sqrt_quotient_faithful(p.gamma * pr, d);
+            q[6 * L::PLANE_PAD + c] = pr * (p.inv_gm1 + 1.0) + half_exact(m0 * u0 + m1 * u1 + m2 * u2);
+        }
     }
 }
 
 template <int PLANE_PAD>
-__device__ __forceinline__ Side<double> load_side(double const* q, int c, int dir)
+__device__ __forceinline__ StagedSide load_side(double const* q, int c, int dir)
 {
-    int const d1 = dir == 2 ? 0 : dir + 1; // the axes after the normal, cyclically
-    int const d2 = dir == 0 ? 2 : dir - 1;
-    Side<double> s;
+    StagedSide s;
     s.d = q[0 * PLANE_PAD + c];
     s.p = q[1 * PLANE_PAD + c];
     s.un = q[(2 + dir) * PLANE_PAD + c];
-    s.ut1 = q[(2 + d1) * PLANE_PAD + c];
-    s.ut2 = q[(2 + d2) * PLANE_PAD + c];
+    s.mn = q[(7 + dir) * PLANE_PAD + c];
     s.c = q[5 * PLANE_PAD + c];
-    s.e = q[6 * PLANE_PAD + c];
+    s.h = q[6 * PLANE_PAD + c];
     return s;
 }
 
-__device__ __forceinline__ void store_flux(double* out, int stride, int idx, int dir, Flux<double> const& f)
+// What a face carries into the cells beside it: its flux (b scaled by the
+// ratio of its area to an x face's) and d and the momenta of its upwind side.
+struct FaceTerms {
+    double b, h, fn, d, m0, m1, m2;
+};
+
+template <int PLANE_PAD>
+__device__ __forceinline__ FaceTerms face_terms(double const* f, int stride, int idx, double const* q, int left, int right)
 {
-    int const d1 = dir == 2 ? 0 : dir + 1;
-    int const d2 = dir == 0 ? 2 : dir - 1;
-    out[0 * stride + idx] = f.d;
-    out[1 * stride + idx] = f.e;
-    out[(2 + dir) * stride + idx] = f.n;
-    out[(2 + d1) * stride + idx] = f.t1;
-    out[(2 + d2) * stride + idx] = f.t2;
+    FaceTerms t;
+    t.b = f[idx];
+    t.h = f[stride + idx];
+    t.fn = f[2 * stride + idx];
+    double const* const u = q + (dbits(t.b) > 0 ? left : right);
+    t.d = u[0 * PLANE_PAD];
+    t.m0 = u[7 * PLANE_PAD];
+    t.m1 = u[8 * PLANE_PAD];
+    t.m2 = u[9 * PLANE_PAD];
+    return t;
 }
 
 // Per-CTA state of the tile engine that lives across work items.
 struct TileCtx {
     unsigned long long* bars; // one mbarrier per slot (TMA ring)
     double* smem;                  // plane slots
-    double* fx;                    // x-face fluxes (5 fields)
-    double* fy;                    // y-face fluxes
-    double* fz;                    // z-face fluxes
+    double* fx;                    // x faces' b, h and fn (UpwindFlux)
+    double* fy;                    // y faces'
+    double* fz;                    // z faces'
     unsigned phase;           // bit s: parity of slot s's next completion (TMA ring)
     unsigned inflight;        // bit s: a TMA into slot s has not been waited for
     bool timed_out;           // a bounded mbarrier wait ran out
@@ -291,18 +323,19 @@ __device__ __forceinline__ bool wait_slot(TileCtx& c, int s)
     return ok;
 }
 
-// One work item: interior planes [kb, ke) of tile (tx, ty), with update
-// coefficients k0..k2 (dt/dv times the face areas).  Tiles are at most
+// One work item: interior planes [kb, ke) of tile (tx, ty), with the update
+// coefficient k0 (dt/dv times an x face's area).  Tiles are at most
 // TX x TY cells, cut evenly out of the grid (p.sx, p.sy), so a warp solves no
 // face and updates no cell that is not the grid's.  Returns false when a staged plane never arrived.
 template <int TX, int TY, int MODE, int STAGE>
-__device__ __forceinline__ bool tile_item(TileCtx& c, FluxParams<double> const& p, TmaMaps const& maps, double k0, double k1,
-                                          double k2, int tx, int ty, int kb, int ke)
+__device__ __forceinline__ bool tile_item(TileCtx& c, FluxParams<double> const& p, TmaMaps const& maps, double k0, int tx,
+                                          int ty, int kb, int ke)
 {
     constexpr int NSLOT = kStageSlots<STAGE>;
     using L = TileLayout<TX, TY, NSLOT>;
     int const tid = threadIdx.x;
     bool const cubic = p.invdx0 == p.invdx1 && p.invdx1 == p.invdx2;
+    bool const equal_areas = p.rs1 == 1.0 && p.rs2 == 1.0;
     double* const smem = c.smem;
     double* const fx = c.fx;
     double* const fy = c.fy;
@@ -341,21 +374,19 @@ __device__ __forceinline__ bool tile_item(TileCtx& c, FluxParams<double> const& 
         asm volatile("cp.async.wait_all;" ::: "memory");
         __syncthreads();
     } else {
-        load_plane<TX, TY, NSLOT>(smem, 0, p, t, i0, j0, kb - 1);
-        load_plane<TX, TY, NSLOT>(smem, 1, p, t, i0, j0, kb);
+        load_plane<TX, TY, NSLOT, MODE>(smem, 0, p, t, i0, j0, kb - 1);
+        load_plane<TX, TY, NSLOT, MODE>(smem, 1, p, t, i0, j0, kb);
         __syncthreads();
     }
-    // z face below the chunk's first plane, kept in registers in global
-    // axes (the z face frame has n = mx2, t1 = mx0, t2 = mx1)
-    double zlo[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+    // z face below the run's first plane, kept in registers
+    FaceTerms zlo{};
     if (own) {
-        Flux<double> const f0 = hllc_flux(load_side<L::PLANE_PAD>(slot_field<TX, TY, NSLOT>(smem, 0, 0), center, 2),
-                                     load_side<L::PLANE_PAD>(slot_field<TX, TY, NSLOT>(smem, 1, 0), center, 2));
-        zlo[0] = f0.d;
-        zlo[1] = f0.e;
-        zlo[2] = f0.t1;
-        zlo[3] = f0.t2;
-        zlo[4] = f0.n;
+        double const* const q0 = slot_field<TX, TY, NSLOT>(smem, 0, 0);
+        double const* const q1 = slot_field<TX, TY, NSLOT>(smem, 1, 0);
+        UpwindFlux const f0 = hllc_upwind(load_side<L::PLANE_PAD>(q0, center, 2), load_side<L::PLANE_PAD>(q1, center, 2));
+        double const* const u = (dbits(f0.b) > 0 ? q0 : q1) + center;
+        zlo = FaceTerms{equal_areas ? f0.b : f0.b * p.rs2, f0.h, f0.fn, u[0], u[7 * L::PLANE_PAD], u[8 * L::PLANE_PAD],
+                        u[9 * L::PLANE_PAD]};
     }
     if (__syncthreads_or(c.timed_out)) { // slot 0 is refilled next
         return false;
@@ -371,7 +402,6 @@ __device__ __forceinline__ bool tile_item(TileCtx& c, FluxParams<double> const& 
         if (kb + 2 <= ke) {
             issue_plane_async<TX, TY, NSLOT>(smem, 0, p, cells, kb + 2);
         }
-        asm volatile("cp.async.commit_group;" ::: "memory");
     }
     int const nfx = (t.w + 1) * t.h; // the faces of each family
     int const nfy = t.w * (t.h + 1);
@@ -387,18 +417,22 @@ __device__ __forceinline__ bool tile_item(TileCtx& c, FluxParams<double> const& 
         int const cur = (k - kb + 1) % NSLOT;
         int const nxt = (k - kb + 2) % NSLOT;
         // this cell's conservative state, fetched while the faces are solved
+        // (where density and momenta are staged from cons, only the energy)
         double u[5];
         long long const o = p.g.at(i, j, k);
         if (own) {
-#pragma unroll
-            for (int f = 0; f < 5; ++f) {
-                u[f] = p.cons_in.f[f][o];
+            u[1] = p.cons_in.f[1][o];
+            if (STAGE == kStageLoad) {
+                u[0] = p.cons_in.f[0][o];
+                u[2] = p.cons_in.f[2][o];
+                u[3] = p.cons_in.f[3][o];
+                u[4] = p.cons_in.f[4][o];
             }
         }
         if (STAGE == kStageTma) {
             c.timed_out |= !wait_slot<NSLOT>(c, nxt);
         } else if (STAGE == kStageLoad) {
-            load_plane<TX, TY, NSLOT>(smem, nxt, p, t, i0, j0, k + 1);
+            load_plane<TX, TY, NSLOT, MODE>(smem, nxt, p, t, i0, j0, k + 1);
             __syncthreads();
         }
 
@@ -418,44 +452,66 @@ __device__ __forceinline__ bool tile_item(TileCtx& c, FluxParams<double> const& 
             int const dir = is_x ? 0 : (is_y ? 1 : 2);
             double const* const qr = is_x || is_y ? qc : qn;
             int const ar = a + (is_x ? 1 : (is_y ? L::HX : 0));
-            store_flux(is_x ? fx : (is_y ? fy : fz), is_x ? L::NFX : (is_y ? L::NFY : L::NFZ), g, dir,
-                       hllc_flux(load_side<L::PLANE_PAD>(qc, a, dir), load_side<L::PLANE_PAD>(qr, ar, dir)));
+            UpwindFlux u = hllc_upwind(load_side<L::PLANE_PAD>(qc, a, dir), load_side<L::PLANE_PAD>(qr, ar, dir));
+            if (!equal_areas) {
+                u.b *= is_x ? 1.0 : (is_y ? p.rs1 : p.rs2);
+            }
+            double* const out = (is_x ? fx : (is_y ? fy : fz)) + g;
+            int const stride = is_x ? L::NFX : (is_y ? L::NFY : L::NFZ);
+            out[0] = u.b;
+            out[stride] = u.h;
+            out[2 * stride] = u.fn;
         }
         if (__syncthreads_or(c.timed_out)) {
             return false;
         }
-        // plane k is no longer read: refill its slot with plane k+3
-        if (STAGE == kStageTma) {
-            if (k + 3 <= ke) {
-                if (tid == 0) {
-                    issue_plane<TX, TY, NSLOT>(smem, c.bars, cur, maps, i0, j0, k + 3);
-                }
-                c.inflight |= 1u << cur;
-            }
-        } else if constexpr (STAGE == kStageAsync) {
-            if (k + 3 <= ke) {
-                issue_plane_async<TX, TY, NSLOT>(smem, cur, p, cells, k + 3);
-            }
-            asm volatile("cp.async.commit_group;" ::: "memory");
-        }
 
         // ---- cell phase
-        double fza[5];
-#pragma unroll
-        for (int f = 0; f < 5; ++f) {
-            fza[f] = fz[f * L::NFZ + tid];
-        }
+        FaceTerms zhi{};
         double wv[4] = {0.0, 0.0, 0.0, 0.0}; // fused step: the new cs, v0, v1, v2, for the screened wavespeed
         if (own) {
+            zhi = face_terms<L::PLANE_PAD>(fz, L::NFZ, tid, qc + center, 0, static_cast<int>(qn - qc));
             int const xl = tj * (t.w + 1) + ti;
             int const yb = tj * t.w + ti;
-#pragma unroll
-            for (int f = 0; f < 5; ++f) {
-                double const ax = fx[f * L::NFX + xl + 1] - fx[f * L::NFX + xl];
-                double const ay = fy[f * L::NFY + yb + t.w] - fy[f * L::NFY + yb];
-                double const az = fza[f] - zlo[f];
-                u[f] = u[f] - k0 * ax - k1 * ay - k2 * az;
+            FaceTerms const xlo = face_terms<L::PLANE_PAD>(fx, L::NFX, xl, qc + center, -1, 0);
+            FaceTerms const xhi = face_terms<L::PLANE_PAD>(fx, L::NFX, xl + 1, qc + center, 0, 1);
+            // div F in units of an x face's area: every term but the normal
+            // momenta's is b times a value of the face's upwind side
+            double rd = fma_rn(-xlo.b, xlo.d, mul_rn(xhi.b, xhi.d));
+            double re = fma_rn(-xlo.b, xlo.h, mul_rn(xhi.b, xhi.h));
+            double r0 = sub_rn(xhi.fn, xlo.fn);
+            double r1 = fma_rn(-xlo.b, xlo.m1, mul_rn(xhi.b, xhi.m1));
+            double r2 = fma_rn(-xlo.b, xlo.m2, mul_rn(xhi.b, xhi.m2));
+            FaceTerms const ylo = face_terms<L::PLANE_PAD>(fy, L::NFY, yb, qc + center, -L::HX, 0);
+            FaceTerms const yhi = face_terms<L::PLANE_PAD>(fy, L::NFY, yb + t.w, qc + center, 0, L::HX);
+            double const fy1 = sub_rn(yhi.fn, ylo.fn);
+            double const fz2 = sub_rn(zhi.fn, zlo.fn);
+            rd = fma_rn(-ylo.b, ylo.d, fma_rn(yhi.b, yhi.d, rd));
+            re = fma_rn(-ylo.b, ylo.h, fma_rn(yhi.b, yhi.h, re));
+            r0 = fma_rn(-ylo.b, ylo.m0, fma_rn(yhi.b, yhi.m0, r0));
+            r2 = fma_rn(-ylo.b, ylo.m2, fma_rn(yhi.b, yhi.m2, r2));
+            rd = fma_rn(-zlo.b, zlo.d, fma_rn(zhi.b, zhi.d, rd));
+            re = fma_rn(-zlo.b, zlo.h, fma_rn(zhi.b, zhi.h, re));
+            r0 = fma_rn(-zlo.b, zlo.m0, fma_rn(zhi.b, zhi.m0, r0));
+            r1 = fma_rn(-zlo.b, zlo.m1, fma_rn(zhi.b, zhi.m1, r1));
+            if (equal_areas) {
+                r1 = add_rn(r1, fy1);
+                r2 = add_rn(r2, fz2);
+            } else {
+                r1 = fma_rn(p.rs1, fy1, r1);
+                r2 = fma_rn(p.rs2, fz2, r2);
             }
+            if (STAGE != kStageLoad) {
+                u[0] = qc[center];
+                u[2] = qc[7 * L::PLANE_PAD + center];
+                u[3] = qc[8 * L::PLANE_PAD + center];
+                u[4] = qc[9 * L::PLANE_PAD + center];
+            }
+            u[0] = fma_rn(-k0, rd, u[0]);
+            u[1] = fma_rn(-k0, re, u[1]);
+            u[2] = fma_rn(-k0, r0, u[2]);
+            u[3] = fma_rn(-k0, r1, u[3]);
+            u[4] = fma_rn(-k0, r2, u[4]);
 #pragma unroll
             for (int f = 0; f < 5; ++f) {
                 p.cons_out.f[f][o] = u[f];
@@ -505,15 +561,23 @@ __device__ __forceinline__ bool tile_item(TileCtx& c, FluxParams<double> const& 
                 c.bad |= dbits(invdt) >= kInfBits;
             }
         }
-        // the z face above becomes the next plane's z face below
-#pragma unroll
-        for (int f = 0; f < 5; ++f) {
-            zlo[f] = fza[f];
-        }
+        zlo = zhi; // the z face above becomes the next plane's z face below
         if (STAGE == kStageAsync) {
-            asm volatile("cp.async.wait_group 1;" ::: "memory"); // plane k+2 landed (k+3 may be in flight)
+            asm volatile("cp.async.wait_all;" ::: "memory"); // plane k+2 landed
         }
-        __syncthreads(); // fluxes are rewritten by the next face phase
+        __syncthreads(); // the next face phase rewrites the fluxes, and plane k is no longer read:
+        if (STAGE == kStageTma) { // refill its slot with plane k+3
+            if (k + 3 <= ke) {
+                if (tid == 0) {
+                    issue_plane<TX, TY, NSLOT>(smem, c.bars, cur, maps, i0, j0, k + 3);
+                }
+                c.inflight |= 1u << cur;
+            }
+        } else if constexpr (STAGE == kStageAsync) {
+            if (k + 3 <= ke) {
+                issue_plane_async<TX, TY, NSLOT>(smem, cur, p, cells, k + 3);
+            }
+        }
     }
     c.wrun = screen.run;
     return !__syncthreads_or(c.timed_out);
@@ -590,8 +654,7 @@ __global__ void __launch_bounds__(TX* TY, 2) flux_tile_kernel(const __grid_const
     extern __shared__ __align__(128) unsigned char smem_dyn[];
     TileCtx c = make_ctx<TX, TY, NSLOT>(smem_dyn);
     double const dtodv = dt_over_dv(p);
-    // cons -= dt/dv * sum_d ds_d (F_R - F_L), coefficients folded
-    double const k0 = dtodv * p.ds0, k1 = dtodv * p.ds1, k2 = dtodv * p.ds2;
+    double const k0 = dtodv * p.ds0;
 
     if (STAGE == kStageTma) {
         if (threadIdx.x == 0) {
@@ -612,8 +675,7 @@ __global__ void __launch_bounds__(TX* TY, 2) flux_tile_kernel(const __grid_const
         int const tile = w / iz;
         int const k = w - tile * iz;
         int const run = min(end - w, iz - k);
-        if (!tile_item<TX, TY, MODE, STAGE>(c, p, maps, k0, k1, k2, tile % p.tiles_x, tile / p.tiles_x, 1 + k,
-                                               1 + k + run)) {
+        if (!tile_item<TX, TY, MODE, STAGE>(c, p, maps, k0, tile % p.tiles_x, tile / p.tiles_x, 1 + k, 1 + k + run)) {
             break;
         }
         w += run;
@@ -671,9 +733,8 @@ __global__ void __launch_bounds__(TX* TY) flux_batch_kernel(const __grid_constan
         }
         __syncthreads();
         double const dtodv = dt_over_dv(gp);
-        double const k0 = dtodv * gp.ds0, k1 = dtodv * gp.ds1, k2 = dtodv * gp.ds2;
         int const kb = 1 + it.w * gp.kchunk;
-        tile_item<TX, TY, kModeStep, kStageAsync>(c, gp, TmaMaps{}, k0, k1, k2, it.y, it.z, kb,
+        tile_item<TX, TY, kModeStep, kStageAsync>(c, gp, TmaMaps{}, dtodv * gp.ds0, it.y, it.z, kb,
                                                      min(kb + gp.kchunk, gp.g.n2 - 1));
         flush_wavespeed<NT>(c, gp.wmax, gp.status);
         item_done(gp);
@@ -925,10 +986,12 @@ struct FluxKernel {
             return cudaSuccess; // no interior cell
         }
         int const q = STAGE == kStageTma ? 2 : 1;
-        // FP64 instructions: 27 a face; the step's 49 a cell, or the operator's
-        // 30 a cell and 15 a staged one
-        TilePlan const plan = MODE == kModeStep ? choose_tiles(ix, iy, iz, sms, per_sm, 27, 49, 0, q)
-                                                : choose_tiles(ix, iy, iz, sms, per_sm, 27, 30, 15, q);
+        // FP64 instructions: 22 a face; the step's 51 a cell, or the operator's
+        // 32 a cell and 17 a staged one
+        TilePlan const plan = MODE == kModeStep ? choose_tiles(ix, iy, iz, sms, per_sm, 22, 51, 0, q)
+                                                : choose_tiles(ix, iy, iz, sms, per_sm, 22, 32, 17, q);
+        p.rs1 = p.ds1 / p.ds0;
+        p.rs2 = p.ds2 / p.ds0;
         p.sx = split_tiles(ix, plan.nx, q);
         p.sy = split_tiles(iy, plan.ny, 1);
         p.tiles_x = plan.nx;
@@ -1007,6 +1070,10 @@ struct FluxDispatch<double> {
     static cudaError_t configure(int mode, bool tma, int /*comp*/, int* per_sm)
     {
         if (mode == kModeStep) {
+            cudaError_t const e = FluxKernel<kModeStep, kStageLoad>::configure(per_sm);
+            if (e != cudaSuccess) {
+                return e;
+            }
             return tma ? FluxKernel<kModeStep, kStageTma>::configure(per_sm)
                        : FluxKernel<kModeStep, kStageAsync>::configure(per_sm);
         }
@@ -1016,6 +1083,9 @@ struct FluxDispatch<double> {
                               cudaStream_t s)
     {
         if (mode == kModeStep) {
+            if (p.own_momenta) {
+                return FluxKernel<kModeStep, kStageLoad>::launch(p, TmaMaps{}, sms, s);
+            }
             if (maps != nullptr) {
                 return FluxKernel<kModeStep, kStageTma>::launch(p, *maps, sms, s);
             }

@@ -93,10 +93,11 @@ cudaError_t resident_ctas(int threads, int bytes, int* per_sm)
     return cudaSuccess;
 }
 
-// TMA descriptors of the seven staged fields (d, p, u0, u1, u2, c, e) of the
-// step's input copy: 3D tensors (n0, n1, n2), boxes of (TX+2) x (TY+2) x 1.
+// TMA descriptors of the ten staged fields (d, p, u0, u1, u2, c, e + p, m0,
+// m1, m2) of the step's input copy: 3D tensors (n0, n1, n2), boxes of
+// (TX+2) x (TY+2) x 1.
 struct TmaMaps {
-    CUtensorMap m[7];
+    CUtensorMap m[10];
 };
 
 template <class T>
@@ -104,13 +105,14 @@ struct FluxParams {
     Geom g;
     CBundle<T> prim;     // read (with halo)
     const T* cs;         // step mode: stored sound speed of prim
-    CBundle<T> cons_in;  // read (centre; step mode also e with halo)
+    CBundle<T> cons_in;  // read (centre; FP64 step mode also the momenta with halo)
     Bundle<T> cons_out;  // written (interior); may equal cons_in in godunov mode
     Bundle<T> prim_out;  // step mode: cons_to_prim of the new state (interior)
     Bundle<T> prim_rec;  // step mode, when set: a second copy of prim_out (the adjoint's recompute)
     T* cs_out;           // step mode: sound speed of the new state (interior)
     T gamma, gm1, inv_gm1, half_gm1;
     T ds0, ds1, ds2;     // face areas dx1*dx2, dx2*dx0, dx0*dx1
+    T rs1, rs2;          // FP64: ds1/ds0 and ds2/ds0
     double dv;           // cell volume
     T dtodv;             // dt/dv when dt_dev is null
     const double* dt_dev; // if set: dt/dv = (cfl * *dt_dev) / dv, evaluated in double
@@ -127,6 +129,7 @@ struct FluxParams {
     TileSplit sx, sy;                    // FP64: the tiles along x and y
     int tiles_x, tiles_y, kchunk, nwork; // work decomposition (FP64 single grid: nwork planes of tiles, no chunks)
     int per_sm;                          // resident CTAs per SM (from configure_flux)
+    bool own_momenta;    // FP64 step mode: cons_in came with prim from the caller, not from it; the faces take d u
     SimScalars* fin;  // step mode, when set: the kernel finalizes the step itself (next dt, clock)
     T* h_out;         // FP64 step mode, when set: e + p of the new state (interior), the HLLC's
                       // energy-flux input, staged by TMA at the next step

@@ -116,6 +116,7 @@ struct eulr_sim {
     long long host_steps = 0;  // steps taken since the state was loaded (host-side count)
     double* rec[5] = {};       // set only inside sim_advance_recording: a second prim output
     bool ghost_fix = false;    // FP64: copy 0 still holds the loaded ghost prim; fixed after the next step
+    bool given_cons = false;   // FP64: copy 0 still holds a prim and a cons that were loaded each by itself
 };
 
 namespace {
@@ -206,9 +207,9 @@ void setup_tma(eulr_sim* s)
         return;
     }
     for (int c = 0; c < 2; ++c) {
-        void* f[7] = {s->prim[c][0], s->prim[c][1], s->prim[c][2], s->prim[c][3], s->prim[c][4], s->cs[c],
-                      s->h[c]};
-        for (int i = 0; i < 7; ++i) {
+        void* f[10] = {s->prim[c][0], s->prim[c][1], s->prim[c][2], s->prim[c][3], s->prim[c][4],
+                       s->cs[c],      s->h[c],       s->cons[c][2], s->cons[c][3], s->cons[c][4]};
+        for (int i = 0; i < 10; ++i) {
             if (!encode_field_map(&s->maps[c].m[i], f[i], s->g)) {
                 return;
             }
@@ -307,6 +308,7 @@ int enqueue_step_t(eulr_sim* s, int in, cudaEvent_t* ev)
     p.wmax = &s->sc->wmax;
     p.status = &s->sc->status;
     p.per_sm = s->per_sm;
+    p.own_momenta = s->given_cons;
     p.fin = s->sc;
     if (ev != nullptr) {
         SIM_CUDA(cudaEventRecord(ev[1], s->stream), "cudaEventRecord");
@@ -355,6 +357,7 @@ int after_step(eulr_sim* s)
         SIM_CUDA(launch_ghost_shell<double>(ghost_params<double>(s, in, out, &s->sc->ghost_wmax), s->sms, s->stream),
                  "ghost shell launch");
         s->ghost_fix = false;
+        s->given_cons = false;
     }
     return EULR_SUCCESS;
 }
@@ -396,6 +399,7 @@ int load_f64(eulr_sim* s, CBundle<double> prim, bool derive_cons)
              "load launch");
     SIM_CUDA(launch_finalize_dt<double>(s->sc, s->cfl, 0, s->stream), "finalize launch");
     SIM_TRY(set_ghost_layer(s)); // after the first dt, which the loaded ghost prim sets
+    s->given_cons = !derive_cons;
     s->loaded = true;
     return EULR_SUCCESS;
 }
@@ -602,6 +606,7 @@ int sim_restore(eulr_sim* s, const double* const* src, long long step)
     SIM_CUDA(launch_copy_fields(p, s->sms, s->stream), "restore copy");
     s->cur = 0;
     SIM_TRY(set_ghost_layer(s));
+    s->given_cons = false; // a snapshot's cons and prim belong together
     s->host_steps = step;
     s->loaded = true;
     return EULR_SUCCESS;

@@ -10,7 +10,7 @@
 namespace eulr {
 namespace {
 
-constexpr int kFields = 7; // face inputs of a staged cell: d, p, u0, u1, u2, c, e
+constexpr int kFields = 10; // staged values of a cell: d, p, u0, u1, u2, c, e + p, m0, m1, m2
 constexpr long long kInfBits = 0x7ff0000000000000LL;
 
 // g / D for 0 <= g < 2^12 and a compile-time 0 < D < 256, as one product and

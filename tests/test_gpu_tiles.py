@@ -56,6 +56,23 @@ def test_batch_tiles_equal_single_grid(cuda, euler, oracle_lib):
         assert np.array_equal(pb, ps) and np.array_equal(cb, cs), shape
 
 
+@pytest.mark.parametrize("shape", [(4, 3, 5), (19, 35, 5), (34, 21, 23)])
+def test_first_step_of_a_state_loaded_with_its_own_cons(cuda, euler, oracle_lib, shape):
+    """set_state with momenta that are not d u: the first step's faces take the velocities from prim, the update
+    starts from cons, as the operator does.  1e-12 of each field's scale, the bar of one step."""
+    O = oracle_lib
+    dx = (0.11, 0.07, 0.13)
+    prim0 = O.random_prim(*shape, seed=sum(shape))
+    cons0 = O.prim_to_cons(prim0, 1.4)
+    cons0[2:] += 0.2 * np.random.default_rng(5).standard_normal(cons0[2:].shape)
+    with euler.Simulation(*shape, 1.4, dx, 0.3) as s:
+        s.set_state(prim0, cons0)
+        s.advance(1)
+        dt = s.time()[0]
+        cons = s.state_numpy()[1]
+    assert max(rel_linf(cons, O.godunov(prim0, cons0.copy(), 1.4, dx, dt))) <= 1e-12
+
+
 @pytest.mark.parametrize("precision", ["f32", "f32c", "f32c_hilo"])
 def test_fp32_columns_match_oracle_and_batch(cuda, euler, oracle_lib, precision):
     """The FP32 column engine at its tile widths and chunk edges.  Against the FP64 oracle after four steps: 4 steps
