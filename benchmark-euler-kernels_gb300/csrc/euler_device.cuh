@@ -336,6 +336,73 @@ __device__ __forceinline__ bool finite_positive(double x)
     return b > 0 && b < 0x7ff0000000000000LL;
 }
 
+// ------------------------------------------- FP64 work on the integer pipes
+// a*b on the integer pipes: the 53 x 53-bit product of the significands in
+// four 32-bit multiplies, rounded to nearest (a tie away from zero, where the
+// FP64 multiply takes the even neighbour).  FP64 kernels leave 85 % of the
+// issue slots idle while the FP64 pipe is full, and one FP64 instruction
+// holds that pipe as long as about 60 issue slots last; this takes about 30.
+// (Products only: a 512^3 step 31.2 -> 27.4 ms with 22 of 127 FP64
+// instructions a cell replaced, and 24.4 with rcp_alu and ten more products.)
+// Operands with a magnitude outside [2^-255, 2^257) take the FP64 multiply,
+// except zeros.
+__device__ __forceinline__ double mul_alu(double a, double b)
+{
+    long long const ab = dbits(a), bb = dbits(b);
+    unsigned const a0 = static_cast<unsigned>(ab), a1 = static_cast<unsigned>(ab >> 32);
+    unsigned const b0 = static_cast<unsigned>(bb), b1 = static_cast<unsigned>(bb >> 32);
+    if (((2u * a1 - 0x60000000u) | (2u * b1 - 0x60000000u)) >= 0x40000000u) {
+        bool const finite = (a1 & 0x7ff00000u) != 0x7ff00000u && (b1 & 0x7ff00000u) != 0x7ff00000u;
+        if (finite && ((ab << 1) == 0 || (bb << 1) == 0)) {
+            return __longlong_as_double((ab ^ bb) & static_cast<long long>(0x8000000000000000ull));
+        }
+        return mul_rn(a, b);
+    }
+    unsigned const am = (a1 & 0xfffffu) | 0x100000u, bm = (b1 & 0xfffffu) | 0x100000u;
+    unsigned long long const t = static_cast<unsigned long long>(a0) * b0;
+    unsigned long long const u = static_cast<unsigned long long>(a0) * bm + (t >> 32);
+    unsigned long long const v = static_cast<unsigned long long>(am) * b0 + static_cast<unsigned>(u);
+    unsigned long long w = static_cast<unsigned long long>(am) * bm + (u >> 32) + (v >> 32);
+    // the product w : low word of v : low word of t has 106 bits (c = 1) or 105
+    unsigned const c = static_cast<unsigned>(w >> 41);
+    unsigned const x = static_cast<unsigned>(v);
+    unsigned const y = x + (0x80000u << c);
+    w += y < x ? 1u : 0u;
+    unsigned const lo = __funnelshift_r(y, static_cast<unsigned>(w), 20u + c);
+    unsigned const hi = __funnelshift_r(static_cast<unsigned>(w), static_cast<unsigned>(w >> 32), 20u + c) +
+                        (a1 & 0xfff00000u) + (b1 & 0xfff00000u) - 0x40000000u + (c << 20);
+    return __hiloint2double(static_cast<int>(hi), static_cast<int>(lo));
+}
+
+// 1/x on the integer pipes: an FP32 seed q of the significand's reciprocal,
+// its error E = 1 - f q exactly in 64-bit fixed point, and q (1 + E + E^2)
+// rounded to nearest: within 0.5001 ulp for a seed within two FP32 ulps.
+// Magnitudes outside [2^-255, 2^257) take rcp_faithful.
+__device__ __forceinline__ double rcp_alu(double x)
+{
+    long long const xb = dbits(x);
+    unsigned const x0 = static_cast<unsigned>(xb), x1 = static_cast<unsigned>(xb >> 32);
+    if (2u * x1 - 0x60000000u >= 0x40000000u) {
+        return rcp_faithful(x);
+    }
+    // f, the significand, to 24 bits; q / 2^24 in [1/2, 1)
+    unsigned const f24 = (((__funnelshift_l(x0, x1, 4) & 0xffffffu) + 1u) >> 1) + 0x3f800000u;
+    unsigned const seed = min(max(__float_as_uint(rcp_approx(__uint_as_float(f24))), 0x3f000000u), 0x3f7fffffu);
+    unsigned const q = (seed & 0x7fffffu) | 0x800000u;
+    // E in units of 2^-76, from f q modulo 2^64
+    unsigned long long const t = static_cast<unsigned long long>(x0) * q;
+    unsigned const u = ((x1 & 0xfffffu) | 0x100000u) * q + static_cast<unsigned>(t >> 32);
+    long long const e = -static_cast<long long>((static_cast<unsigned long long>(u) << 32) | static_cast<unsigned>(t));
+    int const eh = static_cast<int>(e >> 24);
+    long long const e2 = e + ((static_cast<long long>(eh) * eh) >> 28);
+    // q (1 + E + E^2) in units of 2^-53
+    unsigned long long const p = static_cast<unsigned long long>(q) * static_cast<unsigned>(e2);
+    long long const c = static_cast<long long>(static_cast<int>(q)) * static_cast<int>(e2 >> 32) + static_cast<long long>(p >> 32);
+    unsigned long long const g = (static_cast<unsigned long long>(q) << 29) + static_cast<unsigned long long>((c + 0x4000) >> 15);
+    unsigned const hi = static_cast<unsigned>(g >> 32) + 0x7fc00000u - (x1 & 0xfff00000u);
+    return __hiloint2double(static_cast<int>(hi), static_cast<int>(static_cast<unsigned>(g)));
+}
+
 // HLLC flux of hllc::operator() (euler_operators/hllc.hpp:50-105) in the face
 // frame: wave speeds (:64-68), acoustic star state (:70-76), upwind side by
 // the sign of ustar (:78-79), supersonic test S_L*S_R > 0 (:84-85), star
@@ -375,9 +442,9 @@ __device__ __forceinline__ bool finite_positive(double x)
 // b m_t and b h to its update with one fma each.
 // Every sum of products is written as the fma it becomes, so that all kernels
 // that inline this give a face the same bits whatever the compiler contracts.
-// 22 FP64 instructions and a reciprocal seed a face, against 27 and a seed
-// with all five fluxes formed from velocities: FP64 instructions set the FP64
-// kernels' time on this GPU.
+// 22 FP64 operations and a reciprocal seed a face, against 27 and a seed with
+// all five fluxes formed from velocities; the seven products and the
+// reciprocal run on the integer pipes (mul_alu, rcp_alu), which leaves 12.
 struct UpwindFlux {
     double b;  // carries d, m_t and h of its upwind side: the left one where b > 0
     double h;  // e + p of that side plus S d w
@@ -389,7 +456,7 @@ __device__ __forceinline__ UpwindFlux hllc_upwind(StagedSide const& L, StagedSid
     double const cmax = (dbits(L.c) > dbits(R.c)) ? L.c : R.c; // sound speeds are >= 0
     double const du = L.un - R.un;
     double const A = cmax + (dbits(du) < 0 ? 0.0 : du);
-    double const G = A * (L.d + R.d);
+    double const G = mul_alu(A, L.d + R.d);
     double const n = fma_rn(A, L.mn + R.mn, sub_rn(L.p, R.p));
 
     bool const left = dbits(n) > 0; // ustar > 0 (G > 0)
@@ -403,15 +470,15 @@ __device__ __forceinline__ UpwindFlux hllc_upwind(StagedSide const& L, StagedSid
 
     double const S = qun + a;
     double const M = fma_rn(S, G, -n); // G (S - ustar)
-    double const nR = n * rcp_faithful(G * M);
+    double const nR = mul_alu(n, rcp_alu(mul_alu(G, M)));
     // S = -0 cannot occur (a is not zero), so the sign bit decides
     bool const supersonic = left ? dbits(S) > 0 : dbits(S) < 0;
-    double const ustar = supersonic ? qun : nR * M;
-    double const dus = mul_rn(qd, ustar);
+    double const ustar = supersonic ? qun : mul_alu(nR, M);
+    double const dus = mul_alu(qd, ustar);
     double const dw = fma_rn(qd, ustar, -qmn);
 
     UpwindFlux f;
-    f.b = supersonic ? qun : a * (nR * G);
+    f.b = supersonic ? qun : mul_alu(a, mul_alu(nR, G));
     f.h = fma_rn(S, dw, qh);
     f.fn = fma_rn(f.b, dus, fma_rn(a, dw, qp));
     return f;

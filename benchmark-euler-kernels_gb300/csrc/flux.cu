@@ -25,30 +25,34 @@
 //      from the slots; then cons -= dt/dv ds_0 div F (godunov.hpp:84-90), one
 //      rounding at the state's scale.  What the z face below the cell carries
 //      stays in registers from the previous plane.
-// 22 FP64 instructions a face and 32 a cell's update, where forming all five
-// fluxes at the face took 27 and 30; m staged besides u is what saves them
-// (loading 512^3 and 4 steps: 141.0 -> 133.7 ms; 20 steps of 24 batched grids
-// 36.5 -> 34.5; prim_to_cons, godunov, cons_to_prim and time_step of 256^3
-// 5.36 -> 5.12; the rounding error of a step 0.6 of the other form's against
-// quadruple precision, 1.0 where pressure outweighs
-// momentum).
+// Forming all five fluxes at the face took 27 FP64 operations a face and 30 a
+// cell's update; this takes 22 and 32, with m staged besides u (loading 512^3
+// and 4 steps: 141.0 -> 133.7 ms; the rounding error of a step 0.6 of the
+// other form's against quadruple precision, 1.0 where pressure outweighs
+// momentum).  That filled the FP64 pipe (553 G instructions/s of about 560)
+// with 85 % of the issue slots idle, so plain products and reciprocals run on
+// the integer pipes (mul_alu, rcp_alu): 12 FP64 instructions stay of a face's
+// 22 and seed, 41 of a cell's 51, and with three CTAs on an SM (two plane
+// slots, 80 registers) a step of 512^3 took 24.2 ms where it took 31.0, the
+// operator godunov 25.5 where it took 31.6.
 // The fused step then finishes the cell on chip: cons_to_prim, sound speed
 // and the next step's CFL max-wavespeed, reduced warp -> block -> one
 // atomicMax per CTA, so dt never leaves the device.
 //
-// Staging: in the fused FP64 step the ten input fields of a plane slot are
-// fetched into a ring of three slots, two planes ahead of the plane being
-// solved: by TMA (cp.async.bulk.tensor, one 18x18x1 box per field, each slot
+// Staging: the ten fields of a plane slot are fetched into a ring of two
+// slots by TMA (cp.async.bulk.tensor, one 18x18x1 box per field, each slot
 // completing on its own mbarrier) where the row pitch is a multiple of 16
 // bytes, else and in the batch by 8-byte cp.async (20 steps of a
 // 99 x 128 x 75 grid, odd pitch: 7.0 -> 5.9 ms against synchronous loads and
-// whole tiles).  A slot is refilled once its plane's cell phase is over and
-// has the whole next plane to land.  The per-operator godunov (arbitrary
-// caller pointers, values computed while staged) and the first step of a
-// state whose cons the caller gave besides prim (its momenta need not be
-// d u) stage with plain cooperative loads instead.  Every mbarrier wait is
-// bounded: a wait that runs out sets bit 1 of the status word, waits
-// (bounded) for the copies still in flight and ends the CTA.
+// whole tiles).  A slot is refilled once its plane's cell phase is over, and
+// waited for before the next plane's first pass with z faces; the SM's other
+// CTAs cover what is left of the wait.  (Three slots leave room for two CTAs:
+// the same time a 512^3 step, 3.5 % more for 24 batched grids.)  The
+// per-operator godunov, and the first step of a state whose cons the caller
+// gave besides prim (its momenta need not be d u), copy what is stored the
+// same way and compute the rest in place.  Every mbarrier wait is bounded: a
+// wait that runs out sets bit 1 of the status word, waits (bounded) for the
+// copies still in flight and ends the CTA.
 #include "euler_device.cuh"
 #include "kernels.h"
 #include "step_common.cuh"
@@ -66,10 +70,9 @@ constexpr int kWaitTries = 1 << 20; // mbarrier.try_wait attempts before giving 
 enum Staging {
     kStageTma,   // fused FP64 step, row pitch a multiple of 16 bytes: TMA boxes, ring of three slots
     kStageAsync, // fused FP64 step, any pitch, and the batch: 8-byte cp.async, the same ring
-    kStageLoad,  // values are computed while staged (per-operator godunov, FluxParams::own_momenta): plain loads, two slots
+    kStageDerive, // only prim is stored (per-operator godunov, FluxParams::own_momenta): cp.async, the rest computed
 };
-template <int STAGE>
-constexpr int kStageSlots = STAGE == kStageLoad ? 2 : 3;
+constexpr int kSlots = 2; // plane slots of the ring
 
 template <int TX, int TY, int NSLOT>
 struct TileLayout {
@@ -196,13 +199,14 @@ __device__ __forceinline__ StageCells<kStagePerThread<TX, TY>> stage_cells(FluxP
     return s;
 }
 
-// Start copying plane k of the tile and its halo into `slot` (fused FP64
-// step: every staged value is stored, none is computed).
-template <int TX, int TY, int NSLOT>
+// Start copying plane k of the tile and its halo into `slot`: all ten values,
+// or those that derive_plane does not compute.
+template <int TX, int TY, int NSLOT, int MODE, int STAGE>
 __device__ __forceinline__ void issue_plane_async(double* smem, int slot, FluxParams<double> const& p,
                                                   StageCells<kStagePerThread<TX, TY>> const& s, int k)
 {
     using L = TileLayout<TX, TY, NSLOT>;
+    constexpr int NF = STAGE == kStageAsync ? kFields : (MODE == kModeStep ? 7 : 5);
     unsigned const base = smem_u32(slot_field<TX, TY, NSLOT>(smem, slot, 0));
     long long const plane = p.g.s2 * k;
 #pragma unroll
@@ -210,7 +214,7 @@ __device__ __forceinline__ void issue_plane_async(double* smem, int slot, FluxPa
         if (s.dst[r] >= 0) {
             long long const o = s.src[r] + plane;
 #pragma unroll
-            for (int f = 0; f < kFields; ++f) {
+            for (int f = 0; f < NF; ++f) {
                 const double* const src = (f < 5 ? p.prim.f[f] : (f == 5 ? p.cs : (f == 6 ? p.h : p.cons_in.f[f - 5]))) + o;
                 asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(
                                      base + static_cast<unsigned>((f * L::PLANE_PAD + s.dst[r]) * sizeof(double))),
@@ -221,46 +225,36 @@ __device__ __forceinline__ void issue_plane_async(double* smem, int slot, FluxPa
     }
 }
 
-// Stage plane k of the tile and its halo with plain loads: prim as it is and
-// the momenta d u.  Per-operator godunov: the sound speed and e + p derived
-// from prim; step: as stored.
+// The rest of a plane whose prim this thread has copied: the momenta d u and,
+// for the per-operator godunov, the sound speed and e + p.
 template <int TX, int TY, int NSLOT, int MODE>
-__device__ __forceinline__ void load_plane(double* smem, int slot, FluxParams<double> const& p, TileDims const& t, int i0, int j0,
-                                           int k)
+__device__ __forceinline__ void derive_plane(double* smem, int slot, FluxParams<double> const& p,
+                                             StageCells<kStagePerThread<TX, TY>> const& s)
 {
     using L = TileLayout<TX, TY, NSLOT>;
-    double* q = slot_field<TX, TY, NSLOT>(smem, slot, 0);
-    int const n = (t.w + 2) * (t.h + 2);
-    for (int cc = threadIdx.x; cc < n; cc += L::NT) {
-        int const hy = div_runtime(cc, t.mw2);
-        int const hx = cc - hy * (t.w + 2);
-        int const c = hy * L::HX + hx;
-        long long const o = p.g.at(i0 - 1 + hx, j0 - 1 + hy, k);
-        double const d = __ldg(p.prim.f[0] + o);
-        double const pr = __ldg(p.prim.f[1] + o);
-        double const u0 = __ldg(p.prim.f[2] + o);
-        double const u1 = __ldg(p.prim.f[3] + o);
-        double const u2 = __ldg(p.prim.f[4] + o);
-        double const m0 = d * u0;
-        double const m1 = d * u1;
-        double const m2 = d * u2;
-        q[0 * L::PLANE_PAD + c] = d;
-        q[1 * L::PLANE_PAD + c] = pr;
-        q[2 * L::PLANE_PAD + c] = u0;
-        q[3 * L::PLANE_PAD + c] = u1;
-        q[4 * L::PLANE_PAD + c] = u2;
-        q[7 * L::PLANE_PAD + c] = m0;
-        q[8 * L::PLANE_PAD + c] = m1;
-        q[9 * L::PLANE_PAD + c] = m2;
-        if (MODE == kModeStep) {
-            q[5 * L::PLANE_PAD + c] = __ldg(p.cs + o);
-            q[6 * L::PLANE_PAD + c] = __ldg(p.h + o);
-        } else {
-            // sqrt(gamma p / rho) from one reciprocal square root, and
-            // e + p = p gamma/(gamma-1) + m.u / 2 with the halving on the
-            // integer pipe
-            q[5 * L::PLANE_PAD + c] = sqrt_quotient_faithful(p.gamma * pr, d);
-            q[6 * L::PLANE_PAD + c] = pr * (p.inv_gm1 + 1.0) + half_exact(m0 * u0 + m1 * u1 + m2 * u2);
+#pragma unroll
+    for (int r = 0; r < kStagePerThread<TX, TY>; ++r) {
+        if (s.dst[r] >= 0) {
+            double* const q = slot_field<TX, TY, NSLOT>(smem, slot, 0) + s.dst[r];
+            double const d = q[0 * L::PLANE_PAD];
+            double const u0 = q[2 * L::PLANE_PAD];
+            double const u1 = q[3 * L::PLANE_PAD];
+            double const u2 = q[4 * L::PLANE_PAD];
+            double const m0 = mul_alu(d, u0);
+            double const m1 = mul_alu(d, u1);
+            double const m2 = mul_alu(d, u2);
+            q[7 * L::PLANE_PAD] = m0;
+            q[8 * L::PLANE_PAD] = m1;
+            q[9 * L::PLANE_PAD] = m2;
+            if (MODE != kModeStep) {
+                // sqrt(gamma p / rho) from one reciprocal square root, and
+                // e + p = p gamma/(gamma-1) + m.u / 2 with the halving on the
+                // integer pipe
+                double const pr = q[1 * L::PLANE_PAD];
+                q[5 * L::PLANE_PAD] = sqrt_quotient_faithful(p.gamma * pr, d);
+                q[6 * L::PLANE_PAD] =
+                        fma_rn(pr, p.h_over_p, half_exact(fma_rn(m2, u2, fma_rn(m1, u1, mul_alu(m0, u0)))));
+            }
         }
     }
 }
@@ -331,7 +325,7 @@ template <int TX, int TY, int MODE, int STAGE>
 __device__ __forceinline__ bool tile_item(TileCtx& c, FluxParams<double> const& p, TmaMaps const& maps, double k0, int tx,
                                           int ty, int kb, int ke)
 {
-    constexpr int NSLOT = kStageSlots<STAGE>;
+    constexpr int NSLOT = kSlots;
     using L = TileLayout<TX, TY, NSLOT>;
     int const tid = threadIdx.x;
     bool const cubic = p.invdx0 == p.invdx1 && p.invdx1 == p.invdx2;
@@ -352,30 +346,31 @@ __device__ __forceinline__ bool tile_item(TileCtx& c, FluxParams<double> const& 
     bool const own = tj < t.h;
 
     StageCells<kStagePerThread<TX, TY>> cells;
-    if (STAGE == kStageAsync) {
+    if (STAGE != kStageTma) {
         cells = stage_cells<TX, TY>(p, t, i0, j0);
     }
 
     __syncthreads(); // the previous item's readers of slots and fluxes are done
     if (STAGE == kStageTma) {
-        // planes kb-1, kb, kb+1 -> slots 0, 1, 2 (kb+1 <= ke always)
+        // planes kb-1 and kb -> slots 0 and 1
         if (tid == 0) {
-            issue_plane<TX, TY, NSLOT>(smem, c.bars, 0, maps, i0, j0, kb - 1);
-            issue_plane<TX, TY, NSLOT>(smem, c.bars, 1, maps, i0, j0, kb);
-            issue_plane<TX, TY, NSLOT>(smem, c.bars, 2, maps, i0, j0, kb + 1);
+            for (int s = 0; s < NSLOT; ++s) {
+                issue_plane<TX, TY, NSLOT>(smem, c.bars, s, maps, i0, j0, kb - 1 + s);
+            }
         }
-        c.inflight |= 7u;
+        c.inflight |= (1u << NSLOT) - 1u;
         c.timed_out |= !wait_slot<NSLOT>(c, 0);
         c.timed_out |= !wait_slot<NSLOT>(c, 1);
-    } else if constexpr (STAGE == kStageAsync) {
+    } else {
         for (int s = 0; s < NSLOT; ++s) {
-            issue_plane_async<TX, TY, NSLOT>(smem, s, p, cells, kb - 1 + s);
+            issue_plane_async<TX, TY, NSLOT, MODE, STAGE>(smem, s, p, cells, kb - 1 + s);
         }
         asm volatile("cp.async.wait_all;" ::: "memory");
-        __syncthreads();
-    } else {
-        load_plane<TX, TY, NSLOT, MODE>(smem, 0, p, t, i0, j0, kb - 1);
-        load_plane<TX, TY, NSLOT, MODE>(smem, 1, p, t, i0, j0, kb);
+        if (STAGE == kStageDerive) {
+            for (int s = 0; s < NSLOT; ++s) {
+                derive_plane<TX, TY, NSLOT, MODE>(smem, s, p, cells);
+            }
+        }
         __syncthreads();
     }
     // z face below the run's first plane, kept in registers
@@ -391,17 +386,13 @@ __device__ __forceinline__ bool tile_item(TileCtx& c, FluxParams<double> const& 
     if (__syncthreads_or(c.timed_out)) { // slot 0 is refilled next
         return false;
     }
-    if (STAGE == kStageTma) {
-        if (kb + 2 <= ke) {
-            if (tid == 0) {
-                issue_plane<TX, TY, NSLOT>(smem, c.bars, 0, maps, i0, j0, kb + 2);
-            }
-            c.inflight |= 1u;
+    if (STAGE == kStageTma) { // plane kb + 1 <= ke
+        if (tid == 0) {
+            issue_plane<TX, TY, NSLOT>(smem, c.bars, 0, maps, i0, j0, kb + 1);
         }
-    } else if constexpr (STAGE == kStageAsync) {
-        if (kb + 2 <= ke) {
-            issue_plane_async<TX, TY, NSLOT>(smem, 0, p, cells, kb + 2);
-        }
+        c.inflight |= 1u;
+    } else {
+        issue_plane_async<TX, TY, NSLOT, MODE, STAGE>(smem, 0, p, cells, kb + 1);
     }
     int const nfx = (t.w + 1) * t.h; // the faces of each family
     int const nfy = t.w * (t.h + 1);
@@ -422,27 +413,38 @@ __device__ __forceinline__ bool tile_item(TileCtx& c, FluxParams<double> const& 
         long long const o = p.g.at(i, j, k);
         if (own) {
             u[1] = p.cons_in.f[1][o];
-            if (STAGE == kStageLoad) {
+            if (STAGE == kStageDerive) {
                 u[0] = p.cons_in.f[0][o];
                 u[2] = p.cons_in.f[2][o];
                 u[3] = p.cons_in.f[3][o];
                 u[4] = p.cons_in.f[4][o];
             }
         }
-        if (STAGE == kStageTma) {
-            c.timed_out |= !wait_slot<NSLOT>(c, nxt);
-        } else if (STAGE == kStageLoad) {
-            load_plane<TX, TY, NSLOT, MODE>(smem, nxt, p, t, i0, j0, k + 1);
-            __syncthreads();
-        }
-
         // ---- face phase
         double const* qc = slot_field<TX, TY, NSLOT>(smem, cur, 0);
         double const* qn = slot_field<TX, TY, NSLOT>(smem, nxt, 0);
         // one index space over the three families; each face's family, left
         // cell and right cell are chosen by selects, so a warp that straddles
         // two families still runs the HLLC once
-        for (int f = tid; f < nface; f += L::NT) {
+        // The z faces come last: plane k + 1, copied since the previous plane's
+        // end, is waited for before the first pass that holds one.
+        bool staged = false;
+        for (int f = tid; f - tid < nface; f += L::NT) {
+            if (!staged && f - tid + L::NT > nfx + nfy) {
+                staged = true;
+                if (STAGE == kStageTma) {
+                    c.timed_out |= !wait_slot<NSLOT>(c, nxt);
+                } else {
+                    asm volatile("cp.async.wait_all;" ::: "memory");
+                    if (STAGE == kStageDerive) {
+                        derive_plane<TX, TY, NSLOT, MODE>(smem, nxt, p, cells);
+                    }
+                    __syncthreads();
+                }
+            }
+            if (f >= nface) {
+                break;
+            }
             bool const is_x = f < nfx;
             bool const is_y = !is_x && f < nfx + nfy;
             int const g = is_x ? f : (is_y ? f - nfx : f - nfx - nfy);
@@ -477,15 +479,19 @@ __device__ __forceinline__ bool tile_item(TileCtx& c, FluxParams<double> const& 
             FaceTerms const xhi = face_terms<L::PLANE_PAD>(fx, L::NFX, xl + 1, qc + center, 0, 1);
             // div F in units of an x face's area: every term but the normal
             // momenta's is b times a value of the face's upwind side
-            double rd = fma_rn(-xlo.b, xlo.d, mul_rn(xhi.b, xhi.d));
-            double re = fma_rn(-xlo.b, xlo.h, mul_rn(xhi.b, xhi.h));
+            double rd = fma_rn(-xlo.b, xlo.d, mul_alu(xhi.b, xhi.d));
+            double re = fma_rn(-xlo.b, xlo.h, mul_alu(xhi.b, xhi.h));
             double r0 = sub_rn(xhi.fn, xlo.fn);
-            double r1 = fma_rn(-xlo.b, xlo.m1, mul_rn(xhi.b, xhi.m1));
-            double r2 = fma_rn(-xlo.b, xlo.m2, mul_rn(xhi.b, xhi.m2));
             FaceTerms const ylo = face_terms<L::PLANE_PAD>(fy, L::NFY, yb, qc + center, -L::HX, 0);
             FaceTerms const yhi = face_terms<L::PLANE_PAD>(fy, L::NFY, yb + t.w, qc + center, 0, L::HX);
-            double const fy1 = sub_rn(yhi.fn, ylo.fn);
-            double const fz2 = sub_rn(zhi.fn, zlo.fn);
+            double r1 = sub_rn(yhi.fn, ylo.fn);
+            double r2 = sub_rn(zhi.fn, zlo.fn);
+            if (!equal_areas) {
+                r1 = mul_rn(r1, p.rs1);
+                r2 = mul_rn(r2, p.rs2);
+            }
+            r1 = fma_rn(-xlo.b, xlo.m1, fma_rn(xhi.b, xhi.m1, r1));
+            r2 = fma_rn(-xlo.b, xlo.m2, fma_rn(xhi.b, xhi.m2, r2));
             rd = fma_rn(-ylo.b, ylo.d, fma_rn(yhi.b, yhi.d, rd));
             re = fma_rn(-ylo.b, ylo.h, fma_rn(yhi.b, yhi.h, re));
             r0 = fma_rn(-ylo.b, ylo.m0, fma_rn(yhi.b, yhi.m0, r0));
@@ -494,14 +500,7 @@ __device__ __forceinline__ bool tile_item(TileCtx& c, FluxParams<double> const& 
             re = fma_rn(-zlo.b, zlo.h, fma_rn(zhi.b, zhi.h, re));
             r0 = fma_rn(-zlo.b, zlo.m0, fma_rn(zhi.b, zhi.m0, r0));
             r1 = fma_rn(-zlo.b, zlo.m1, fma_rn(zhi.b, zhi.m1, r1));
-            if (equal_areas) {
-                r1 = add_rn(r1, fy1);
-                r2 = add_rn(r2, fz2);
-            } else {
-                r1 = fma_rn(p.rs1, fy1, r1);
-                r2 = fma_rn(p.rs2, fz2, r2);
-            }
-            if (STAGE != kStageLoad) {
+            if (STAGE != kStageDerive) {
                 u[0] = qc[center];
                 u[2] = qc[7 * L::PLANE_PAD + center];
                 u[3] = qc[8 * L::PLANE_PAD + center];
@@ -518,13 +517,13 @@ __device__ __forceinline__ bool tile_item(TileCtx& c, FluxParams<double> const& 
             }
             if constexpr (MODE == kModeStep) {
                 // cons_to_prim of the new state (cons_to_prim.hpp:26-31)
-                double const r = rcp_faithful(u[0]);
-                double const v0 = u[2] * r;
-                double const v1 = u[3] * r;
-                double const v2 = u[4] * r;
-                double const mv = u[2] * v0 + u[3] * v1 + u[4] * v2;   // |m|^2 / rho
-                double const pr = p.gm1 * u[1] - p.half_gm1 * mv;      // (gamma-1)(e - |m|^2/(2 rho))
-                double const cs = fast_sound_speed((p.gamma * r) * pr);
+                double const r = rcp_alu(u[0]);
+                double const v0 = mul_alu(u[2], r);
+                double const v1 = mul_alu(u[3], r);
+                double const v2 = mul_alu(u[4], r);
+                double const mv = fma_rn(u[4], v2, fma_rn(u[3], v1, mul_alu(u[2], v0))); // |m|^2 / rho
+                double const pr = fma_rn(-p.half_gm1, mv, mul_alu(p.gm1, u[1])); // (gamma-1)(e - |m|^2/(2 rho))
+                double const cs = fast_sound_speed(mul_alu(mul_alu(p.gamma, r), pr));
                 p.h_out[o] = u[1] + pr; // staged as e + p at the next step
                 p.prim_out.f[0][o] = u[0];
                 p.prim_out.f[1][o] = pr;
@@ -562,20 +561,15 @@ __device__ __forceinline__ bool tile_item(TileCtx& c, FluxParams<double> const& 
             }
         }
         zlo = zhi; // the z face above becomes the next plane's z face below
-        if (STAGE == kStageAsync) {
-            asm volatile("cp.async.wait_all;" ::: "memory"); // plane k+2 landed
-        }
         __syncthreads(); // the next face phase rewrites the fluxes, and plane k is no longer read:
-        if (STAGE == kStageTma) { // refill its slot with plane k+3
-            if (k + 3 <= ke) {
+        if (k + 2 <= ke) { // refill its slot
+            if (STAGE == kStageTma) {
                 if (tid == 0) {
-                    issue_plane<TX, TY, NSLOT>(smem, c.bars, cur, maps, i0, j0, k + 3);
+                    issue_plane<TX, TY, NSLOT>(smem, c.bars, cur, maps, i0, j0, k + 2);
                 }
                 c.inflight |= 1u << cur;
-            }
-        } else if constexpr (STAGE == kStageAsync) {
-            if (k + 3 <= ke) {
-                issue_plane_async<TX, TY, NSLOT>(smem, cur, p, cells, k + 3);
+            } else {
+                issue_plane_async<TX, TY, NSLOT, MODE, STAGE>(smem, cur, p, cells, k + 2);
             }
         }
     }
@@ -647,10 +641,10 @@ __device__ __forceinline__ TileCtx make_ctx(unsigned char* smem_dyn)
 }
 
 template <int TX, int TY, int MODE, int STAGE>
-__global__ void __launch_bounds__(TX* TY, 2) flux_tile_kernel(const __grid_constant__ FluxParams<double> p,
+__global__ void __launch_bounds__(TX* TY, 3) flux_tile_kernel(const __grid_constant__ FluxParams<double> p,
                                                            const __grid_constant__ TmaMaps maps)
 {
-    constexpr int NSLOT = kStageSlots<STAGE>;
+    constexpr int NSLOT = kSlots;
     extern __shared__ __align__(128) unsigned char smem_dyn[];
     TileCtx c = make_ctx<TX, TY, NSLOT>(smem_dyn);
     double const dtodv = dt_over_dv(p);
@@ -707,9 +701,9 @@ __global__ void __launch_bounds__(TX* TY, 2) flux_tile_kernel(const __grid_const
 // engine; each item's wavespeed goes to its own grid's accumulator, so every
 // grid keeps its own dt.  Staging by cp.async (grids of any shape).
 template <int TX, int TY>
-__global__ void __launch_bounds__(TX* TY) flux_batch_kernel(const __grid_constant__ BatchParams<double> b)
+__global__ void __launch_bounds__(TX* TY, TX* TY == 256 ? 3 : 6) flux_batch_kernel(const __grid_constant__ BatchParams<double> b)
 {
-    constexpr int NSLOT = kStageSlots<kStageAsync>;
+    constexpr int NSLOT = kSlots;
     constexpr int NT = TX * TY;
     static_assert(sizeof(FluxParams<double>) % 4 == 0, "parameter copy in 4-byte words");
     extern __shared__ __align__(128) unsigned char smem_dyn[];
@@ -891,9 +885,7 @@ __global__ void finalize_dt_kernel(SimScalars* s, T cfl, int add_time, const dou
 
 // The single-grid tile, at most: 16x16 columns, whose 800 faces per plane
 // fill exactly 25 warp-passes (a 32x8 tile's 808 need 26) with the same 256
-// threads, 18x18 TMA boxes and two resident CTAs per SM.  (A 16x8 kernel with
-// four CTAs of 128 threads per SM measured 33.2 ms a 512^3 step against 32.9,
-// and no better on small grids.)
+// threads, 18x18 TMA boxes and three resident CTAs per SM.
 constexpr int kStepTX = 16, kStepTY = 16;
 
 } // namespace
@@ -902,14 +894,14 @@ constexpr int kStepTX = 16, kStepTY = 16;
 // planes evenly among its CTAs, so with U planes in all on G CTAs, r of them
 // on an SM, each solves m = ceil(U/G) planes of cost c and the z faces below
 // its first plane, z: the SM's FP64 pipe is busy r (m c + z), and every plane
-// adds a wait that its neighbour does not cover (its barriers and its last,
+// adds a wait that its neighbours do not cover (its barriers and its last,
 // partly filled pass of faces).  c and z count FP64 warp instructions, each
 // holding its SM for 9.0 ns; the wait measured
 // 1.1 us a plane with two CTAs on the SM and 1.6 us with one.  Whole
-// 16 x 16 tiles are the best for large grids (256^3: 4.14 ms a step, 4.42 in
-// 16 x 8), smaller ones where their number leaves SMs idle.  Against whole
-// 16 x 16 tiles in chunks of at least 8 planes: 16^3 97 -> 12.5 us a step,
-// 48^3 97 -> 46, 64^3 97 -> 86, 99 x 128 x 75 311 -> 270.
+// 16 x 16 tiles are the best for large grids, smaller ones where their number
+// leaves SMs idle.  Against whole 16 x 16 tiles in chunks of at least 8
+// planes: 16^3 97 -> 12.5 us a step, 48^3 97 -> 46, 64^3 97 -> 86,
+// 99 x 128 x 75 311 -> 270.
 TilePlan choose_tiles(int ix, int iy, int iz, int sms, int per_sm, int face, int cell, int stage, int q)
 {
     constexpr double kInstr = 9.0e-3, kWait2 = 1.1, kWait1 = 1.6; // us
@@ -966,7 +958,7 @@ namespace {
 
 template <int MODE, int STAGE>
 struct FluxKernel {
-    using L = TileLayout<kStepTX, kStepTY, kStageSlots<STAGE>>;
+    using L = TileLayout<kStepTX, kStepTY, kSlots>;
     static auto fn() { return flux_tile_kernel<kStepTX, kStepTY, MODE, STAGE>; }
 
     // Resident CTAs per SM.  Called outside any stream capture (by the entry
@@ -986,12 +978,14 @@ struct FluxKernel {
             return cudaSuccess; // no interior cell
         }
         int const q = STAGE == kStageTma ? 2 : 1;
-        // FP64 instructions: 22 a face; the step's 51 a cell, or the operator's
-        // 32 a cell and 17 a staged one
-        TilePlan const plan = MODE == kModeStep ? choose_tiles(ix, iy, iz, sms, per_sm, 22, 51, 0, q)
-                                                : choose_tiles(ix, iy, iz, sms, per_sm, 22, 32, 17, q);
+        // in FP64 instructions, the integer work beside them included: 16 a
+        // face; the step's 48 a cell, or the operator's 30 a cell and 17 a
+        // staged one
+        TilePlan const plan = MODE == kModeStep ? choose_tiles(ix, iy, iz, sms, per_sm, 16, 48, 0, q)
+                                                : choose_tiles(ix, iy, iz, sms, per_sm, 16, 30, 17, q);
         p.rs1 = p.ds1 / p.ds0;
         p.rs2 = p.ds2 / p.ds0;
+        p.h_over_p = p.inv_gm1 + 1.0;
         p.sx = split_tiles(ix, plan.nx, q);
         p.sy = split_tiles(iy, plan.ny, 1);
         p.tiles_x = plan.nx;
@@ -1011,7 +1005,7 @@ constexpr int kNumBatchShapes = 3;
 
 template <int TX, int TY>
 struct BatchKernel {
-    using L = TileLayout<TX, TY, kStageSlots<kStageAsync>>;
+    using L = TileLayout<TX, TY, kSlots>;
     static auto fn() { return flux_batch_kernel<TX, TY>; }
     static cudaError_t configure(int* per_sm)
     {
@@ -1070,28 +1064,28 @@ struct FluxDispatch<double> {
     static cudaError_t configure(int mode, bool tma, int /*comp*/, int* per_sm)
     {
         if (mode == kModeStep) {
-            cudaError_t const e = FluxKernel<kModeStep, kStageLoad>::configure(per_sm);
+            cudaError_t const e = FluxKernel<kModeStep, kStageDerive>::configure(per_sm);
             if (e != cudaSuccess) {
                 return e;
             }
             return tma ? FluxKernel<kModeStep, kStageTma>::configure(per_sm)
                        : FluxKernel<kModeStep, kStageAsync>::configure(per_sm);
         }
-        return FluxKernel<kModeGodunov, kStageLoad>::configure(per_sm);
+        return FluxKernel<kModeGodunov, kStageDerive>::configure(per_sm);
     }
     static cudaError_t launch(FluxParams<double> const& p, TmaMaps const* maps, int mode, int /*comp*/, int sms,
                               cudaStream_t s)
     {
         if (mode == kModeStep) {
             if (p.own_momenta) {
-                return FluxKernel<kModeStep, kStageLoad>::launch(p, TmaMaps{}, sms, s);
+                return FluxKernel<kModeStep, kStageDerive>::launch(p, TmaMaps{}, sms, s);
             }
             if (maps != nullptr) {
                 return FluxKernel<kModeStep, kStageTma>::launch(p, *maps, sms, s);
             }
             return FluxKernel<kModeStep, kStageAsync>::launch(p, TmaMaps{}, sms, s);
         }
-        return FluxKernel<kModeGodunov, kStageLoad>::launch(p, TmaMaps{}, sms, s);
+        return FluxKernel<kModeGodunov, kStageDerive>::launch(p, TmaMaps{}, sms, s);
     }
 };
 

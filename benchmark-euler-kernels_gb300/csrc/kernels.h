@@ -111,6 +111,7 @@ struct FluxParams {
     Bundle<T> prim_rec;  // step mode, when set: a second copy of prim_out (the adjoint's recompute)
     T* cs_out;           // step mode: sound speed of the new state (interior)
     T gamma, gm1, inv_gm1, half_gm1;
+    T h_over_p;          // FP64 godunov: gamma/(gamma-1)
     T ds0, ds1, ds2;     // face areas dx1*dx2, dx2*dx0, dx0*dx1
     T rs1, rs2;          // FP64: ds1/ds0 and ds2/ds0
     double dv;           // cell volume
