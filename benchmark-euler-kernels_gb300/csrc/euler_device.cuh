@@ -337,13 +337,28 @@ __device__ __forceinline__ bool finite_positive(double x)
 }
 
 // ------------------------------------------- FP64 work on the integer pipes
+// The FP64 unit's product, for the operands mul_alu does not take, zeros aside.
+// Out of line: inlined, it was predicated instead of branched around, and a
+// predicated-off FP64 instruction takes its slot of the pipe all the same.
+static __device__ __noinline__ double mul_rare(double a, double b)
+{
+    long long const ab = dbits(a), bb = dbits(b);
+    long long const inf = 0x7ff0000000000000LL;
+    if ((ab & inf) != inf && (bb & inf) != inf && ((ab << 1) == 0 || (bb << 1) == 0)) {
+        return __longlong_as_double((ab ^ bb) & static_cast<long long>(0x8000000000000000ull));
+    }
+    return mul_rn(a, b);
+}
+
 // a*b on the integer pipes: the 53 x 53-bit product of the significands in
 // four 32-bit multiplies, rounded to nearest (a tie away from zero, where the
 // FP64 multiply takes the even neighbour).  FP64 kernels leave 85 % of the
 // issue slots idle while the FP64 pipe is full, and one FP64 instruction
 // holds that pipe as long as about 60 issue slots last; this takes about 30.
-// (Products only: a 512^3 step 31.2 -> 27.4 ms with 22 of 127 FP64
-// instructions a cell replaced, and 24.4 with rcp_alu and ten more products.)
+// A step of 512^3 went from 31.2 ms to 27.4 with 22 of 127 FP64 instructions a
+// cell replaced by it, to 24.2 with rcp_alu and ten more products, to 23.9
+// with sqrt_alu and add_alu, and to 20.6 with the FP64 unit's forms out of
+// line.
 // Operands with a magnitude outside [2^-255, 2^257) take the FP64 multiply,
 // except zeros.
 __device__ __forceinline__ double mul_alu(double a, double b)
@@ -352,11 +367,7 @@ __device__ __forceinline__ double mul_alu(double a, double b)
     unsigned const a0 = static_cast<unsigned>(ab), a1 = static_cast<unsigned>(ab >> 32);
     unsigned const b0 = static_cast<unsigned>(bb), b1 = static_cast<unsigned>(bb >> 32);
     if (((2u * a1 - 0x60000000u) | (2u * b1 - 0x60000000u)) >= 0x40000000u) {
-        bool const finite = (a1 & 0x7ff00000u) != 0x7ff00000u && (b1 & 0x7ff00000u) != 0x7ff00000u;
-        if (finite && ((ab << 1) == 0 || (bb << 1) == 0)) {
-            return __longlong_as_double((ab ^ bb) & static_cast<long long>(0x8000000000000000ull));
-        }
-        return mul_rn(a, b);
+        return mul_rare(a, b);
     }
     unsigned const am = (a1 & 0xfffffu) | 0x100000u, bm = (b1 & 0xfffffu) | 0x100000u;
     unsigned long long const t = static_cast<unsigned long long>(a0) * b0;
@@ -374,6 +385,10 @@ __device__ __forceinline__ double mul_alu(double a, double b)
     return __hiloint2double(static_cast<int>(hi), static_cast<int>(lo));
 }
 
+static __device__ __noinline__ double rcp_rare(double x) { return rcp_faithful(x); }
+static __device__ __noinline__ double sqrt_rare(double x) { return sqrt_faithful(x); }
+static __device__ __noinline__ double add_rare(double a, double b) { return add_rn(a, b); }
+
 // 1/x on the integer pipes: an FP32 seed q of the significand's reciprocal,
 // its error E = 1 - f q exactly in 64-bit fixed point, and q (1 + E + E^2)
 // rounded to nearest: within 0.5001 ulp for a seed within two FP32 ulps.
@@ -383,7 +398,7 @@ __device__ __forceinline__ double rcp_alu(double x)
     long long const xb = dbits(x);
     unsigned const x0 = static_cast<unsigned>(xb), x1 = static_cast<unsigned>(xb >> 32);
     if (2u * x1 - 0x60000000u >= 0x40000000u) {
-        return rcp_faithful(x);
+        return rcp_rare(x);
     }
     // f, the significand, to 24 bits; q / 2^24 in [1/2, 1)
     unsigned const f24 = (((__funnelshift_l(x0, x1, 4) & 0xffffffu) + 1u) >> 1) + 0x3f800000u;
@@ -401,6 +416,63 @@ __device__ __forceinline__ double rcp_alu(double x)
     unsigned long long const g = (static_cast<unsigned long long>(q) << 29) + static_cast<unsigned long long>((c + 0x4000) >> 15);
     unsigned const hi = static_cast<unsigned>(g >> 32) + 0x7fc00000u - (x1 & 0xfff00000u);
     return __hiloint2double(static_cast<int>(hi), static_cast<int>(static_cast<unsigned>(g)));
+}
+
+// sqrt(x) on the integer pipes: s = f y from an FP32 seed y of 1/sqrt(f), cut
+// to 32 bits, the exact residual R = f - s^2 in 64-bit fixed point and
+// s + R y/2 (1 + (3/2 d - cut) y), d = R y/2: within 0.52 ulp for a seed
+// within two FP32 ulps.  Magnitudes outside [2^-255, 2^257), zeros and
+// negative values take sqrt_faithful.
+__device__ __forceinline__ double sqrt_alu(double x)
+{
+    long long const xb = dbits(x);
+    unsigned const x0 = static_cast<unsigned>(xb), x1 = static_cast<unsigned>(xb >> 32);
+    if (x1 - 0x30000000u >= 0x20000000u) {
+        return sqrt_rare(x);
+    }
+    // x = f 4^n with f in [1, 4), m = f 2^52; q / 2^24 in [1/2, 1)
+    unsigned const odd = (~x1 >> 20) & 1u;
+    unsigned long long const m = ((static_cast<unsigned long long>((x1 & 0xfffffu) | 0x100000u) << 32) | x0) << odd;
+    unsigned const f24 = (((__funnelshift_l(x0, x1, 4) & 0xffffffu) + 1u) >> 1) + 0x3f800000u + (odd << 23);
+    unsigned const seed = min(max(__float_as_uint(rsqrt_approx(__uint_as_float(f24))), 0x3f000000u), 0x3f7fffffu);
+    unsigned const q = (seed & 0x7fffffu) | 0x800000u;
+    unsigned long long const t = static_cast<unsigned long long>(static_cast<unsigned>(m)) * q;
+    unsigned long long const s = static_cast<unsigned long long>(static_cast<unsigned>(m >> 32)) * q + (t >> 32); // 2^-44
+    unsigned const sh = (s >> 45) != 0 ? 0xffffffffu : static_cast<unsigned>(s >> 13);                            // 2^-31
+    long long const res = static_cast<long long>((m << 10) - static_cast<unsigned long long>(sh) * sh);           // 2^-62
+    long long const d = (res >> 5) * static_cast<long long>(q);                                                   // 2^-82
+    int const dh = static_cast<int>(d >> 32);                                                                     // 2^-50
+    int const cut = static_cast<int>((static_cast<unsigned>(s) - (sh << 13)) << 6);                               // 2^-50
+    int const z = static_cast<int>((static_cast<long long>(dh) * (dh + (dh >> 1) - cut)) >> 40);                  // 2^-60
+    long long const z2 = static_cast<long long>(z) * static_cast<int>(q);                                         // 2^-84
+    unsigned long long const g = ((static_cast<unsigned long long>(sh) << 31) + static_cast<unsigned long long>(d >> 20) +
+                                  static_cast<unsigned long long>(z2 >> 22) + 512u) >> 10;                        // 2^-52
+    unsigned const hi = static_cast<unsigned>(g >> 32) + (((x1 >> 1) + 0x1ff80000u - (odd << 19)) & 0xfff00000u) - 0x100000u;
+    return __hiloint2double(static_cast<int>(hi), static_cast<int>(static_cast<unsigned>(g)));
+}
+
+// a + b on the integer pipes for a, b >= 0, rounded to nearest even as the
+// FP64 add.  Exponents 32 or more apart, and operands or sums out of the
+// normal range, take the FP64 add.
+__device__ __forceinline__ double add_alu(double a, double b)
+{
+    unsigned long long const x = static_cast<unsigned long long>(dbits(a)), y = static_cast<unsigned long long>(dbits(b));
+    unsigned long long const g = x > y ? x : y, l = x > y ? y : x;
+    unsigned const g1 = static_cast<unsigned>(g >> 32), l1 = static_cast<unsigned>(l >> 32), l0 = static_cast<unsigned>(l);
+    unsigned const d = (g1 >> 20) - (l1 >> 20);
+    if (d >= 32u || g1 >= 0x7fe00000u || l1 < 0x00100000u) {
+        return add_rare(a, b);
+    }
+    unsigned const lm = (l1 & 0xfffffu) | 0x100000u;
+    unsigned const rest = __funnelshift_r(0u, l0, d); // what the alignment shifts out
+    unsigned long long t = (g & 0xfffffffffffffull) + 0x10000000000000ull +
+                           ((static_cast<unsigned long long>(lm >> d) << 32) | __funnelshift_r(l0, lm, d));
+    unsigned const c = static_cast<unsigned>(t >> 53);
+    bool const tie = c != 0 ? (rest == 0u && (t & 1u) != 0) : rest == 0x80000000u;
+    t += c != 0 ? 1u : rest >> 31;
+    t >>= c;
+    t -= tie ? (t & 1u) : 0u;
+    return __longlong_as_double(static_cast<long long>(t + (static_cast<unsigned long long>((g1 >> 20) - 1u + c) << 52)));
 }
 
 // HLLC flux of hllc::operator() (euler_operators/hllc.hpp:50-105) in the face
@@ -443,8 +515,10 @@ __device__ __forceinline__ double rcp_alu(double x)
 // Every sum of products is written as the fma it becomes, so that all kernels
 // that inline this give a face the same bits whatever the compiler contracts.
 // 22 FP64 operations and a reciprocal seed a face, against 27 and a seed with
-// all five fluxes formed from velocities; the seven products and the
-// reciprocal run on the integer pipes (mul_alu, rcp_alu), which leaves 12.
+// all five fluxes formed from velocities; the seven products, the
+// reciprocal and the sum of the densities run on the integer pipes (mul_alu,
+// rcp_alu, add_alu), which leaves 11.  (A's sum there too measured 4 % slower
+// in the operator godunov and 1-2 % faster in the batch.)
 struct UpwindFlux {
     double b;  // carries d, m_t and h of its upwind side: the left one where b > 0
     double h;  // e + p of that side plus S d w
@@ -456,7 +530,7 @@ __device__ __forceinline__ UpwindFlux hllc_upwind(StagedSide const& L, StagedSid
     double const cmax = (dbits(L.c) > dbits(R.c)) ? L.c : R.c; // sound speeds are >= 0
     double const du = L.un - R.un;
     double const A = cmax + (dbits(du) < 0 ? 0.0 : du);
-    double const G = mul_alu(A, L.d + R.d);
+    double const G = mul_alu(A, add_alu(L.d, R.d));
     double const n = fma_rn(A, L.mn + R.mn, sub_rn(L.p, R.p));
 
     bool const left = dbits(n) > 0; // ustar > 0 (G > 0)

@@ -30,11 +30,12 @@
 // and 4 steps: 141.0 -> 133.7 ms; the rounding error of a step 0.6 of the
 // other form's against quadruple precision, 1.0 where pressure outweighs
 // momentum).  That filled the FP64 pipe (553 G instructions/s of about 560)
-// with 85 % of the issue slots idle, so plain products and reciprocals run on
-// the integer pipes (mul_alu, rcp_alu): 12 FP64 instructions stay of a face's
-// 22 and seed, 41 of a cell's 51, and with three CTAs on an SM (two plane
-// slots, 80 registers) a step of 512^3 took 24.2 ms where it took 31.0, the
-// operator godunov 25.5 where it took 31.6.
+// with 85 % of the issue slots idle, so products, reciprocals, square roots
+// and the sum of the densities run on the integer pipes (mul_alu, rcp_alu,
+// sqrt_alu, add_alu): 11 FP64 instructions stay of a face's 22 and seed, 34 of
+// a cell's 51 and two seeds.  With three CTAs on an SM (two plane slots, 80
+// registers) a step of 512^3 takes 20.6 ms where it took 31.0, the operator
+// godunov 21.1 where it took 31.6.
 // The fused step then finishes the cell on chip: cons_to_prim, sound speed
 // and the next step's CFL max-wavespeed, reduced warp -> block -> one
 // atomicMax per CTA, so dt never leaves the device.
@@ -251,7 +252,7 @@ __device__ __forceinline__ void derive_plane(double* smem, int slot, FluxParams<
                 // e + p = p gamma/(gamma-1) + m.u / 2 with the halving on the
                 // integer pipe
                 double const pr = q[1 * L::PLANE_PAD];
-                q[5 * L::PLANE_PAD] = sqrt_quotient_faithful(p.gamma * pr, d);
+                q[5 * L::PLANE_PAD] = sqrt_alu(mul_alu(mul_alu(p.gamma, pr), rcp_alu(d)));
                 q[6 * L::PLANE_PAD] =
                         fma_rn(pr, p.h_over_p, half_exact(fma_rn(m2, u2, fma_rn(m1, u1, mul_alu(m0, u0)))));
             }
@@ -317,6 +318,16 @@ __device__ __forceinline__ bool wait_slot(TileCtx& c, int s)
     return ok;
 }
 
+// a*b by a ratio of face areas.  The FP64 product is predicated on meshes of
+// equal areas, where it still takes its slots of the pipe; the integer one is
+// branched around, but its registers spill in the step (512^3: 20.6 ms a step
+// with the first, 20.8 with the second; godunov 22.2 and 21.1).
+template <int MODE>
+__device__ __forceinline__ double scaled(double a, double b)
+{
+    return MODE == kModeStep ? mul_rn(a, b) : mul_alu(a, b);
+}
+
 // One work item: interior planes [kb, ke) of tile (tx, ty), with the update
 // coefficient k0 (dt/dv times an x face's area).  Tiles are at most
 // TX x TY cells, cut evenly out of the grid (p.sx, p.sy), so a warp solves no
@@ -380,7 +391,7 @@ __device__ __forceinline__ bool tile_item(TileCtx& c, FluxParams<double> const& 
         double const* const q1 = slot_field<TX, TY, NSLOT>(smem, 1, 0);
         UpwindFlux const f0 = hllc_upwind(load_side<L::PLANE_PAD>(q0, center, 2), load_side<L::PLANE_PAD>(q1, center, 2));
         double const* const u = (dbits(f0.b) > 0 ? q0 : q1) + center;
-        zlo = FaceTerms{equal_areas ? f0.b : f0.b * p.rs2, f0.h, f0.fn, u[0], u[7 * L::PLANE_PAD], u[8 * L::PLANE_PAD],
+        zlo = FaceTerms{equal_areas ? f0.b : scaled<MODE>(f0.b, p.rs2), f0.h, f0.fn, u[0], u[7 * L::PLANE_PAD], u[8 * L::PLANE_PAD],
                         u[9 * L::PLANE_PAD]};
     }
     if (__syncthreads_or(c.timed_out)) { // slot 0 is refilled next
@@ -456,7 +467,7 @@ __device__ __forceinline__ bool tile_item(TileCtx& c, FluxParams<double> const& 
             int const ar = a + (is_x ? 1 : (is_y ? L::HX : 0));
             UpwindFlux u = hllc_upwind(load_side<L::PLANE_PAD>(qc, a, dir), load_side<L::PLANE_PAD>(qr, ar, dir));
             if (!equal_areas) {
-                u.b *= is_x ? 1.0 : (is_y ? p.rs1 : p.rs2);
+                u.b = scaled<MODE>(u.b, is_x ? 1.0 : (is_y ? p.rs1 : p.rs2));
             }
             double* const out = (is_x ? fx : (is_y ? fy : fz)) + g;
             int const stride = is_x ? L::NFX : (is_y ? L::NFY : L::NFZ);
@@ -487,8 +498,8 @@ __device__ __forceinline__ bool tile_item(TileCtx& c, FluxParams<double> const& 
             double r1 = sub_rn(yhi.fn, ylo.fn);
             double r2 = sub_rn(zhi.fn, zlo.fn);
             if (!equal_areas) {
-                r1 = mul_rn(r1, p.rs1);
-                r2 = mul_rn(r2, p.rs2);
+                r1 = scaled<MODE>(r1, p.rs1);
+                r2 = scaled<MODE>(r2, p.rs2);
             }
             r1 = fma_rn(-xlo.b, xlo.m1, fma_rn(xhi.b, xhi.m1, r1));
             r2 = fma_rn(-xlo.b, xlo.m2, fma_rn(xhi.b, xhi.m2, r2));
@@ -523,7 +534,7 @@ __device__ __forceinline__ bool tile_item(TileCtx& c, FluxParams<double> const& 
                 double const v2 = mul_alu(u[4], r);
                 double const mv = fma_rn(u[4], v2, fma_rn(u[3], v1, mul_alu(u[2], v0))); // |m|^2 / rho
                 double const pr = fma_rn(-p.half_gm1, mv, mul_alu(p.gm1, u[1])); // (gamma-1)(e - |m|^2/(2 rho))
-                double const cs = fast_sound_speed(mul_alu(mul_alu(p.gamma, r), pr));
+                double const cs = sqrt_alu(mul_alu(mul_alu(p.gamma, r), pr));
                 p.h_out[o] = u[1] + pr; // staged as e + p at the next step
                 p.prim_out.f[0][o] = u[0];
                 p.prim_out.f[1][o] = pr;
