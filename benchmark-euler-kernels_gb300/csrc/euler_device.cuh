@@ -76,20 +76,6 @@ __device__ __forceinline__ double half_exact(double x)
 __device__ __forceinline__ float half_exact(float x) { return __fmul_rn(x, 0.5f); }
 __device__ __forceinline__ float abs_(float a) { return fabsf(a); }
 
-// Correctly rounded x / y given r = RN(1/y): q0 = RN(x r) is within one ulp
-// of x/y, the remainder x - q0 y is exact through one FMA, and
-// RN(q0 + rem r) is the correctly rounded quotient (Markstein's correction
-// step; P. Markstein, "Computation of elementary functions on the IBM RISC
-// System/6000 processor", IBM J. Res. Dev. 34(1), 1990).  Valid away from
-// overflow and underflow, which the Euler states here never approach.
-template <class T>
-__device__ __forceinline__ T div_by_rcp(T x, T y, T r)
-{
-    T const q0 = mul_rn(x, r);
-    T const rem = fma_rn(-q0, y, x);
-    return fma_rn(rem, r, q0);
-}
-
 // Faithful FP64 reciprocal and square root (within one ulp of the correctly
 // rounded result, not always equal to it) for the fused step, whose parity
 // bar is a relative tolerance.  Each refines the PTX hardware approximation
@@ -183,6 +169,252 @@ __device__ __forceinline__ T warp_max(T v)
     return v;
 }
 
+// ------------------------------------------------- integer-pipe predicates
+// On GB300 an FP64 compare, min or max takes a full slot of the FP64 pipe
+// (1/64 of the FP32 rate); the same decisions taken on the bit patterns run
+// on the integer pipe, which the flux kernels leave almost idle.
+// The bit pattern through an opaque move: tests written on the bits must stay
+// on the integer pipe.  With a plain reinterpretation the compiler rewrote
+// (bits << 1) != 0 into the equivalent FP64 compare x != 0, which takes an
+// FP64 slot (four per HLLC face: 12.6 FP64 instructions per cell of the step).
+__device__ __forceinline__ long long dbits(double x)
+{
+    long long b;
+    asm("mov.b64 %0, %1;" : "=l"(b) : "d"(x));
+    return b;
+}
+
+// Signed key with the order of the doubles (-0 sorts just below +0).
+__device__ __forceinline__ long long order_key(double x)
+{
+    long long const b = dbits(x);
+    return b ^ ((b >> 63) & 0x7fffffffffffffffLL);
+}
+
+// x is neither +0 nor -0.
+__device__ __forceinline__ bool nonzero_(double x) { return (dbits(x) << 1) != 0; }
+
+// a*b > 0 for non-NaN a, b, decided from signs: both non-zero and of one sign.
+__device__ __forceinline__ bool product_positive(double a, double b)
+{
+    return nonzero_(a) && nonzero_(b) && ((dbits(a) ^ dbits(b)) >= 0);
+}
+
+// a < b with IEEE semantics (false when either is NaN; -0 and +0 equal),
+// decided on the integer pipe: the bit patterns mapped to ordered keys with
+// both zeros at 0.  The same answer as the FP64 compare, which would take an
+// FP64 slot.
+__device__ __forceinline__ bool is_nan_bits(long long b) { return (b & 0x7fffffffffffffffLL) > 0x7ff0000000000000LL; }
+__device__ __forceinline__ bool less_ieee(double a, double b)
+{
+    long long const x = dbits(a), y = dbits(b);
+    long long const kx = (x << 1) == 0 ? 0 : (x ^ ((x >> 63) & 0x7fffffffffffffffLL));
+    long long const ky = (y << 1) == 0 ? 0 : (y ^ ((y >> 63) & 0x7fffffffffffffffLL));
+    return !is_nan_bits(x) && !is_nan_bits(y) && kx < ky;
+}
+__device__ __forceinline__ bool less_ieee(float a, float b) { return a < b; }
+
+// ------------------------------------------- FP64 work on the integer pipes
+// The FP64 unit's product, for the operands mul_alu does not take, zeros aside.
+// Out of line: inlined, it was predicated instead of branched around, and a
+// predicated-off FP64 instruction takes its slot of the pipe all the same.
+static __device__ __noinline__ double mul_rare(double a, double b)
+{
+    long long const ab = dbits(a), bb = dbits(b);
+    long long const inf = 0x7ff0000000000000LL;
+    if ((ab & inf) != inf && (bb & inf) != inf && ((ab << 1) == 0 || (bb << 1) == 0)) {
+        return __longlong_as_double((ab ^ bb) & static_cast<long long>(0x8000000000000000ull));
+    }
+    return mul_rn(a, b);
+}
+
+// a*b on the integer pipes: the 53 x 53-bit product of the significands in
+// four 32-bit multiplies, rounded to nearest.  A tie goes to the even
+// neighbour (EVEN: the bits of the FP64 multiply, for the kernels that owe
+// the reference's bits) or away from zero (the same error bound for three
+// instructions less: 3.5 % of a 512^3 step).  FP64 kernels leave 85 % of the
+// issue slots idle while the FP64 pipe is full, and one FP64 instruction
+// holds that pipe as long as about 60 issue slots last; this takes about 30.
+// A step of 512^3 went from 31.2 ms to 27.4 with 22 of 127 FP64 instructions a
+// cell replaced by it, to 24.2 with rcp_alu and ten more products, to 23.9
+// with sqrt_alu and add_alu, and to 20.6 with the FP64 unit's forms out of
+// line.
+// Operands with a magnitude outside [2^-255, 2^257) take the FP64 multiply,
+// except zeros.
+template <bool EVEN>
+__device__ __forceinline__ double mul_int(double a, double b)
+{
+    long long const ab = dbits(a), bb = dbits(b);
+    unsigned const a0 = static_cast<unsigned>(ab), a1 = static_cast<unsigned>(ab >> 32);
+    unsigned const b0 = static_cast<unsigned>(bb), b1 = static_cast<unsigned>(bb >> 32);
+    if (((2u * a1 - 0x60000000u) | (2u * b1 - 0x60000000u)) >= 0x40000000u) {
+        return mul_rare(a, b);
+    }
+    unsigned const am = (a1 & 0xfffffu) | 0x100000u, bm = (b1 & 0xfffffu) | 0x100000u;
+    unsigned long long const t = static_cast<unsigned long long>(a0) * b0;
+    unsigned long long const u = static_cast<unsigned long long>(a0) * bm + (t >> 32);
+    unsigned long long const v = static_cast<unsigned long long>(am) * b0 + static_cast<unsigned>(u);
+    unsigned long long w = static_cast<unsigned long long>(am) * bm + (u >> 32) + (v >> 32);
+    // the product w : low word of v : low word of t has 106 bits (c = 1) or 105
+    unsigned const c = static_cast<unsigned>(w >> 41);
+    unsigned const x = static_cast<unsigned>(v);
+    unsigned const y = x + (0x80000u << c);
+    w += y < x ? 1u : 0u;
+    unsigned lo = __funnelshift_r(y, static_cast<unsigned>(w), 20u + c);
+    if (EVEN) {
+        bool const tie = (x << (12u - c)) == 0x80000000u && static_cast<unsigned>(t) == 0u;
+        lo &= tie ? ~1u : ~0u;
+    }
+    unsigned const hi = __funnelshift_r(static_cast<unsigned>(w), static_cast<unsigned>(w >> 32), 20u + c) +
+                        (a1 & 0xfff00000u) + (b1 & 0xfff00000u) - 0x40000000u + (c << 20);
+    return __hiloint2double(static_cast<int>(hi), static_cast<int>(lo));
+}
+
+static __device__ __noinline__ double rcp_rare(double x) { return rcp_faithful(x); }
+static __device__ __noinline__ double rcp_rn_rare(double x) { return rcp_rn(x); }
+static __device__ __noinline__ double sqrt_rare(double x) { return sqrt_faithful(x); }
+static __device__ __noinline__ double add_rare(double a, double b) { return add_rn(a, b); }
+
+// 2^53 / f, f the significand of x in [1, 2), rounded to nearest but for an
+// error of up to 0.5001 units: an FP32 seed q of 1/f, its error E = 1 - f q
+// exactly in 64-bit fixed point, and q (1 + E + E^2), for a seed within two
+// FP32 ulps.
+__device__ __forceinline__ unsigned long long rcp_significand(unsigned x0, unsigned x1)
+{
+    // f to 24 bits; q / 2^24 in [1/2, 1)
+    unsigned const f24 = (((__funnelshift_l(x0, x1, 4) & 0xffffffu) + 1u) >> 1) + 0x3f800000u;
+    unsigned const seed = min(max(__float_as_uint(rcp_approx(__uint_as_float(f24))), 0x3f000000u), 0x3f7fffffu);
+    unsigned const q = (seed & 0x7fffffu) | 0x800000u;
+    // E in units of 2^-76, from f q modulo 2^64
+    unsigned long long const t = static_cast<unsigned long long>(x0) * q;
+    unsigned const u = ((x1 & 0xfffffu) | 0x100000u) * q + static_cast<unsigned>(t >> 32);
+    long long const e = -static_cast<long long>((static_cast<unsigned long long>(u) << 32) | static_cast<unsigned>(t));
+    int const eh = static_cast<int>(e >> 24);
+    long long const e2 = e + ((static_cast<long long>(eh) * eh) >> 28);
+    // q (1 + E + E^2) in units of 2^-53
+    unsigned long long const p = static_cast<unsigned long long>(q) * static_cast<unsigned>(e2);
+    long long const c = static_cast<long long>(static_cast<int>(q)) * static_cast<int>(e2 >> 32) + static_cast<long long>(p >> 32);
+    return (static_cast<unsigned long long>(q) << 29) + static_cast<unsigned long long>((c + 0x4000) >> 15);
+}
+
+// g 2^-53 / 2^n for x = f 2^n, with the sign of x.
+__device__ __forceinline__ double rcp_pack(unsigned long long g, unsigned x1)
+{
+    unsigned const hi = static_cast<unsigned>(g >> 32) + 0x7fc00000u - (x1 & 0xfff00000u);
+    return __hiloint2double(static_cast<int>(hi), static_cast<int>(static_cast<unsigned>(g)));
+}
+
+// 1/x on the integer pipes, within 0.5001 ulp.  Magnitudes outside
+// [2^-255, 2^257) take rcp_faithful.
+__device__ __forceinline__ double rcp_alu(double x)
+{
+    long long const xb = dbits(x);
+    unsigned const x0 = static_cast<unsigned>(xb), x1 = static_cast<unsigned>(xb >> 32);
+    if (2u * x1 - 0x60000000u >= 0x40000000u) {
+        return rcp_rare(x);
+    }
+    return rcp_pack(rcp_significand(x0, x1), x1);
+}
+
+// 1/x correctly rounded, on the integer pipes: the remainder 2^105 - f 2^52 g
+// is exact modulo 2^64, and g moves by one where it exceeds half of f 2^52
+// (equality cannot occur).
+__device__ __forceinline__ double rcp_rn_alu(double x)
+{
+    long long const xb = dbits(x);
+    unsigned const x0 = static_cast<unsigned>(xb), x1 = static_cast<unsigned>(xb >> 32);
+    if (2u * x1 - 0x60000000u >= 0x40000000u) {
+        return rcp_rn_rare(x);
+    }
+    unsigned long long const m = (static_cast<unsigned long long>((x1 & 0xfffffu) | 0x100000u) << 32) | x0;
+    unsigned long long g = rcp_significand(x0, x1);
+    long long const rem2 = -static_cast<long long>((m * g) << 1);
+    if (rem2 > static_cast<long long>(m)) {
+        ++g;
+    } else if (rem2 < -static_cast<long long>(m)) {
+        --g;
+    }
+    return rcp_pack(g, x1);
+}
+
+// sqrt(x) on the integer pipes: s = f y from an FP32 seed y of 1/sqrt(f), cut
+// to 32 bits, the exact residual R = f - s^2 in 64-bit fixed point and
+// s + R y/2 (1 + (3/2 d - cut) y), d = R y/2: within 0.52 ulp for a seed
+// within two FP32 ulps.  Magnitudes outside [2^-255, 2^257), zeros and
+// negative values take sqrt_faithful.
+__device__ __forceinline__ double sqrt_alu(double x)
+{
+    long long const xb = dbits(x);
+    unsigned const x0 = static_cast<unsigned>(xb), x1 = static_cast<unsigned>(xb >> 32);
+    if (x1 - 0x30000000u >= 0x20000000u) {
+        return sqrt_rare(x);
+    }
+    // x = f 4^n with f in [1, 4), m = f 2^52; q / 2^24 in [1/2, 1)
+    unsigned const odd = (~x1 >> 20) & 1u;
+    unsigned long long const m = ((static_cast<unsigned long long>((x1 & 0xfffffu) | 0x100000u) << 32) | x0) << odd;
+    unsigned const f24 = (((__funnelshift_l(x0, x1, 4) & 0xffffffu) + 1u) >> 1) + 0x3f800000u + (odd << 23);
+    unsigned const seed = min(max(__float_as_uint(rsqrt_approx(__uint_as_float(f24))), 0x3f000000u), 0x3f7fffffu);
+    unsigned const q = (seed & 0x7fffffu) | 0x800000u;
+    unsigned long long const t = static_cast<unsigned long long>(static_cast<unsigned>(m)) * q;
+    unsigned long long const s = static_cast<unsigned long long>(static_cast<unsigned>(m >> 32)) * q + (t >> 32); // 2^-44
+    unsigned const sh = (s >> 45) != 0 ? 0xffffffffu : static_cast<unsigned>(s >> 13);                            // 2^-31
+    long long const res = static_cast<long long>((m << 10) - static_cast<unsigned long long>(sh) * sh);           // 2^-62
+    long long const d = (res >> 5) * static_cast<long long>(q);                                                   // 2^-82
+    int const dh = static_cast<int>(d >> 32);                                                                     // 2^-50
+    int const cut = static_cast<int>((static_cast<unsigned>(s) - (sh << 13)) << 6);                               // 2^-50
+    int const z = static_cast<int>((static_cast<long long>(dh) * (dh + (dh >> 1) - cut)) >> 40);                  // 2^-60
+    long long const z2 = static_cast<long long>(z) * static_cast<int>(q);                                         // 2^-84
+    unsigned long long const g = ((static_cast<unsigned long long>(sh) << 31) + static_cast<unsigned long long>(d >> 20) +
+                                  static_cast<unsigned long long>(z2 >> 22) + 512u) >> 10;                        // 2^-52
+    unsigned const hi = static_cast<unsigned>(g >> 32) + (((x1 >> 1) + 0x1ff80000u - (odd << 19)) & 0xfff00000u) - 0x100000u;
+    return __hiloint2double(static_cast<int>(hi), static_cast<int>(static_cast<unsigned>(g)));
+}
+
+// a + b on the integer pipes for a, b >= 0, rounded to nearest even as the
+// FP64 add.  Exponents 32 or more apart, and operands or sums out of the
+// normal range, take the FP64 add.
+__device__ __forceinline__ double add_alu(double a, double b)
+{
+    unsigned long long const x = static_cast<unsigned long long>(dbits(a)), y = static_cast<unsigned long long>(dbits(b));
+    unsigned long long const g = x > y ? x : y, l = x > y ? y : x;
+    unsigned const g1 = static_cast<unsigned>(g >> 32), l1 = static_cast<unsigned>(l >> 32), l0 = static_cast<unsigned>(l);
+    unsigned const d = (g1 >> 20) - (l1 >> 20);
+    if (d >= 32u || g1 >= 0x7fe00000u || l1 < 0x00100000u) {
+        return add_rare(a, b);
+    }
+    unsigned const lm = (l1 & 0xfffffu) | 0x100000u;
+    unsigned const rest = __funnelshift_r(0u, l0, d); // what the alignment shifts out
+    unsigned long long t = (g & 0xfffffffffffffull) + 0x10000000000000ull +
+                           ((static_cast<unsigned long long>(lm >> d) << 32) | __funnelshift_r(l0, lm, d));
+    unsigned const c = static_cast<unsigned>(t >> 53);
+    bool const tie = c != 0 ? (rest == 0u && (t & 1u) != 0) : rest == 0x80000000u;
+    t += c != 0 ? 1u : rest >> 31;
+    t >>= c;
+    t -= tie ? (t & 1u) : 0u;
+    return __longlong_as_double(static_cast<long long>(t + (static_cast<unsigned long long>((g1 >> 20) - 1u + c) << 52)));
+}
+
+__device__ __forceinline__ double mul_alu(double a, double b) { return mul_int<false>(a, b); }
+__device__ __forceinline__ double mul_rn_alu(double a, double b) { return mul_int<true>(a, b); }
+
+// The same names for the kernels that are templates of the type.
+__device__ __forceinline__ float mul_rn_alu(float a, float b) { return mul_rn(a, b); }
+__device__ __forceinline__ float rcp_rn_alu(float x) { return rcp_rn(x); }
+
+// Correctly rounded x / y given r = RN(1/y): q0 = RN(x r) is within one ulp
+// of x/y, the remainder x - q0 y is exact through one FMA, and
+// RN(q0 + rem r) is the correctly rounded quotient (Markstein's correction
+// step; P. Markstein, "Computation of elementary functions on the IBM RISC
+// System/6000 processor", IBM J. Res. Dev. 34(1), 1990).  Valid away from
+// overflow and underflow, which the Euler states here never approach.
+template <class T>
+__device__ __forceinline__ T div_by_rcp(T x, T y, T r)
+{
+    T const q0 = mul_rn_alu(x, r);
+    T const rem = fma_rn(-q0, y, x);
+    return fma_rn(rem, r, q0);
+}
+
 // cons_to_prim of one cell, bit-identical to cons_to_prim.hpp:20-32 with
 // kinetic_energy(cons) (euler_arrays.hpp:44-48), PerfectGas::pressure
 // (perfect_gas.hpp:25-28) and to_prim (euler_arrays.hpp:66-75):
@@ -191,13 +423,13 @@ __device__ __forceinline__ T warp_max(T v)
 template <class T>
 __device__ __forceinline__ void cons_to_prim_exact(T d, T e, T m0, T m1, T m2, T gm1, T& p, T& u0, T& u1, T& u2)
 {
-    T const r = rcp_rn(d);
-    T const mm = add_rn(add_rn(mul_rn(m0, m0), mul_rn(m1, m1)), mul_rn(m2, m2));
+    T const r = rcp_rn_alu(d);
+    T const mm = add_rn(add_rn(mul_rn_alu(m0, m0), mul_rn_alu(m1, m1)), mul_rn_alu(m2, m2));
     T const ke = half_exact(div_by_rcp(mm, d, r));
-    p = mul_rn(gm1, sub_rn(e, ke));
-    u0 = mul_rn(m0, r);
-    u1 = mul_rn(m1, r);
-    u2 = mul_rn(m2, r);
+    p = mul_rn_alu(gm1, sub_rn(e, ke));
+    u0 = mul_rn_alu(m0, r);
+    u1 = mul_rn_alu(m1, r);
+    u2 = mul_rn_alu(m2, r);
 }
 
 // (c + |u0|)/dx0 + (c + |u1|)/dx1 + (c + |u2|)/dx2 of one cell with
@@ -284,195 +516,11 @@ struct StagedSide {
     double d, p, un, mn, c, h;
 };
 
-// ------------------------------------------------- integer-pipe predicates
-// On GB300 an FP64 compare, min or max takes a full slot of the FP64 pipe
-// (1/64 of the FP32 rate); the same decisions taken on the bit patterns run
-// on the integer pipe, which the flux kernels leave almost idle.
-// The bit pattern through an opaque move: tests written on the bits must stay
-// on the integer pipe.  With a plain reinterpretation the compiler rewrote
-// (bits << 1) != 0 into the equivalent FP64 compare x != 0, which takes an
-// FP64 slot (four per HLLC face: 12.6 FP64 instructions per cell of the step).
-__device__ __forceinline__ long long dbits(double x)
-{
-    long long b;
-    asm("mov.b64 %0, %1;" : "=l"(b) : "d"(x));
-    return b;
-}
-
-// Signed key with the order of the doubles (-0 sorts just below +0).
-__device__ __forceinline__ long long order_key(double x)
-{
-    long long const b = dbits(x);
-    return b ^ ((b >> 63) & 0x7fffffffffffffffLL);
-}
-
-// x is neither +0 nor -0.
-__device__ __forceinline__ bool nonzero_(double x) { return (dbits(x) << 1) != 0; }
-
-// a*b > 0 for non-NaN a, b, decided from signs: both non-zero and of one sign.
-__device__ __forceinline__ bool product_positive(double a, double b)
-{
-    return nonzero_(a) && nonzero_(b) && ((dbits(a) ^ dbits(b)) >= 0);
-}
-
-// a < b with IEEE semantics (false when either is NaN; -0 and +0 equal),
-// decided on the integer pipe: the bit patterns mapped to ordered keys with
-// both zeros at 0.  The same answer as the FP64 compare, which would take an
-// FP64 slot.
-__device__ __forceinline__ bool is_nan_bits(long long b) { return (b & 0x7fffffffffffffffLL) > 0x7ff0000000000000LL; }
-__device__ __forceinline__ bool less_ieee(double a, double b)
-{
-    long long const x = dbits(a), y = dbits(b);
-    long long const kx = (x << 1) == 0 ? 0 : (x ^ ((x >> 63) & 0x7fffffffffffffffLL));
-    long long const ky = (y << 1) == 0 ? 0 : (y ^ ((y >> 63) & 0x7fffffffffffffffLL));
-    return !is_nan_bits(x) && !is_nan_bits(y) && kx < ky;
-}
-__device__ __forceinline__ bool less_ieee(float a, float b) { return a < b; }
-
 // Finite and > 0.
 __device__ __forceinline__ bool finite_positive(double x)
 {
     long long const b = dbits(x);
     return b > 0 && b < 0x7ff0000000000000LL;
-}
-
-// ------------------------------------------- FP64 work on the integer pipes
-// The FP64 unit's product, for the operands mul_alu does not take, zeros aside.
-// Out of line: inlined, it was predicated instead of branched around, and a
-// predicated-off FP64 instruction takes its slot of the pipe all the same.
-static __device__ __noinline__ double mul_rare(double a, double b)
-{
-    long long const ab = dbits(a), bb = dbits(b);
-    long long const inf = 0x7ff0000000000000LL;
-    if ((ab & inf) != inf && (bb & inf) != inf && ((ab << 1) == 0 || (bb << 1) == 0)) {
-        return __longlong_as_double((ab ^ bb) & static_cast<long long>(0x8000000000000000ull));
-    }
-    return mul_rn(a, b);
-}
-
-// a*b on the integer pipes: the 53 x 53-bit product of the significands in
-// four 32-bit multiplies, rounded to nearest (a tie away from zero, where the
-// FP64 multiply takes the even neighbour).  FP64 kernels leave 85 % of the
-// issue slots idle while the FP64 pipe is full, and one FP64 instruction
-// holds that pipe as long as about 60 issue slots last; this takes about 30.
-// A step of 512^3 went from 31.2 ms to 27.4 with 22 of 127 FP64 instructions a
-// cell replaced by it, to 24.2 with rcp_alu and ten more products, to 23.9
-// with sqrt_alu and add_alu, and to 20.6 with the FP64 unit's forms out of
-// line.
-// Operands with a magnitude outside [2^-255, 2^257) take the FP64 multiply,
-// except zeros.
-__device__ __forceinline__ double mul_alu(double a, double b)
-{
-    long long const ab = dbits(a), bb = dbits(b);
-    unsigned const a0 = static_cast<unsigned>(ab), a1 = static_cast<unsigned>(ab >> 32);
-    unsigned const b0 = static_cast<unsigned>(bb), b1 = static_cast<unsigned>(bb >> 32);
-    if (((2u * a1 - 0x60000000u) | (2u * b1 - 0x60000000u)) >= 0x40000000u) {
-        return mul_rare(a, b);
-    }
-    unsigned const am = (a1 & 0xfffffu) | 0x100000u, bm = (b1 & 0xfffffu) | 0x100000u;
-    unsigned long long const t = static_cast<unsigned long long>(a0) * b0;
-    unsigned long long const u = static_cast<unsigned long long>(a0) * bm + (t >> 32);
-    unsigned long long const v = static_cast<unsigned long long>(am) * b0 + static_cast<unsigned>(u);
-    unsigned long long w = static_cast<unsigned long long>(am) * bm + (u >> 32) + (v >> 32);
-    // the product w : low word of v : low word of t has 106 bits (c = 1) or 105
-    unsigned const c = static_cast<unsigned>(w >> 41);
-    unsigned const x = static_cast<unsigned>(v);
-    unsigned const y = x + (0x80000u << c);
-    w += y < x ? 1u : 0u;
-    unsigned const lo = __funnelshift_r(y, static_cast<unsigned>(w), 20u + c);
-    unsigned const hi = __funnelshift_r(static_cast<unsigned>(w), static_cast<unsigned>(w >> 32), 20u + c) +
-                        (a1 & 0xfff00000u) + (b1 & 0xfff00000u) - 0x40000000u + (c << 20);
-    return __hiloint2double(static_cast<int>(hi), static_cast<int>(lo));
-}
-
-static __device__ __noinline__ double rcp_rare(double x) { return rcp_faithful(x); }
-static __device__ __noinline__ double sqrt_rare(double x) { return sqrt_faithful(x); }
-static __device__ __noinline__ double add_rare(double a, double b) { return add_rn(a, b); }
-
-// 1/x on the integer pipes: an FP32 seed q of the significand's reciprocal,
-// its error E = 1 - f q exactly in 64-bit fixed point, and q (1 + E + E^2)
-// rounded to nearest: within 0.5001 ulp for a seed within two FP32 ulps.
-// Magnitudes outside [2^-255, 2^257) take rcp_faithful.
-__device__ __forceinline__ double rcp_alu(double x)
-{
-    long long const xb = dbits(x);
-    unsigned const x0 = static_cast<unsigned>(xb), x1 = static_cast<unsigned>(xb >> 32);
-    if (2u * x1 - 0x60000000u >= 0x40000000u) {
-        return rcp_rare(x);
-    }
-    // f, the significand, to 24 bits; q / 2^24 in [1/2, 1)
-    unsigned const f24 = (((__funnelshift_l(x0, x1, 4) & 0xffffffu) + 1u) >> 1) + 0x3f800000u;
-    unsigned const seed = min(max(__float_as_uint(rcp_approx(__uint_as_float(f24))), 0x3f000000u), 0x3f7fffffu);
-    unsigned const q = (seed & 0x7fffffu) | 0x800000u;
-    // E in units of 2^-76, from f q modulo 2^64
-    unsigned long long const t = static_cast<unsigned long long>(x0) * q;
-    unsigned const u = ((x1 & 0xfffffu) | 0x100000u) * q + static_cast<unsigned>(t >> 32);
-    long long const e = -static_cast<long long>((static_cast<unsigned long long>(u) << 32) | static_cast<unsigned>(t));
-    int const eh = static_cast<int>(e >> 24);
-    long long const e2 = e + ((static_cast<long long>(eh) * eh) >> 28);
-    // q (1 + E + E^2) in units of 2^-53
-    unsigned long long const p = static_cast<unsigned long long>(q) * static_cast<unsigned>(e2);
-    long long const c = static_cast<long long>(static_cast<int>(q)) * static_cast<int>(e2 >> 32) + static_cast<long long>(p >> 32);
-    unsigned long long const g = (static_cast<unsigned long long>(q) << 29) + static_cast<unsigned long long>((c + 0x4000) >> 15);
-    unsigned const hi = static_cast<unsigned>(g >> 32) + 0x7fc00000u - (x1 & 0xfff00000u);
-    return __hiloint2double(static_cast<int>(hi), static_cast<int>(static_cast<unsigned>(g)));
-}
-
-// sqrt(x) on the integer pipes: s = f y from an FP32 seed y of 1/sqrt(f), cut
-// to 32 bits, the exact residual R = f - s^2 in 64-bit fixed point and
-// s + R y/2 (1 + (3/2 d - cut) y), d = R y/2: within 0.52 ulp for a seed
-// within two FP32 ulps.  Magnitudes outside [2^-255, 2^257), zeros and
-// negative values take sqrt_faithful.
-__device__ __forceinline__ double sqrt_alu(double x)
-{
-    long long const xb = dbits(x);
-    unsigned const x0 = static_cast<unsigned>(xb), x1 = static_cast<unsigned>(xb >> 32);
-    if (x1 - 0x30000000u >= 0x20000000u) {
-        return sqrt_rare(x);
-    }
-    // x = f 4^n with f in [1, 4), m = f 2^52; q / 2^24 in [1/2, 1)
-    unsigned const odd = (~x1 >> 20) & 1u;
-    unsigned long long const m = ((static_cast<unsigned long long>((x1 & 0xfffffu) | 0x100000u) << 32) | x0) << odd;
-    unsigned const f24 = (((__funnelshift_l(x0, x1, 4) & 0xffffffu) + 1u) >> 1) + 0x3f800000u + (odd << 23);
-    unsigned const seed = min(max(__float_as_uint(rsqrt_approx(__uint_as_float(f24))), 0x3f000000u), 0x3f7fffffu);
-    unsigned const q = (seed & 0x7fffffu) | 0x800000u;
-    unsigned long long const t = static_cast<unsigned long long>(static_cast<unsigned>(m)) * q;
-    unsigned long long const s = static_cast<unsigned long long>(static_cast<unsigned>(m >> 32)) * q + (t >> 32); // 2^-44
-    unsigned const sh = (s >> 45) != 0 ? 0xffffffffu : static_cast<unsigned>(s >> 13);                            // 2^-31
-    long long const res = static_cast<long long>((m << 10) - static_cast<unsigned long long>(sh) * sh);           // 2^-62
-    long long const d = (res >> 5) * static_cast<long long>(q);                                                   // 2^-82
-    int const dh = static_cast<int>(d >> 32);                                                                     // 2^-50
-    int const cut = static_cast<int>((static_cast<unsigned>(s) - (sh << 13)) << 6);                               // 2^-50
-    int const z = static_cast<int>((static_cast<long long>(dh) * (dh + (dh >> 1) - cut)) >> 40);                  // 2^-60
-    long long const z2 = static_cast<long long>(z) * static_cast<int>(q);                                         // 2^-84
-    unsigned long long const g = ((static_cast<unsigned long long>(sh) << 31) + static_cast<unsigned long long>(d >> 20) +
-                                  static_cast<unsigned long long>(z2 >> 22) + 512u) >> 10;                        // 2^-52
-    unsigned const hi = static_cast<unsigned>(g >> 32) + (((x1 >> 1) + 0x1ff80000u - (odd << 19)) & 0xfff00000u) - 0x100000u;
-    return __hiloint2double(static_cast<int>(hi), static_cast<int>(static_cast<unsigned>(g)));
-}
-
-// a + b on the integer pipes for a, b >= 0, rounded to nearest even as the
-// FP64 add.  Exponents 32 or more apart, and operands or sums out of the
-// normal range, take the FP64 add.
-__device__ __forceinline__ double add_alu(double a, double b)
-{
-    unsigned long long const x = static_cast<unsigned long long>(dbits(a)), y = static_cast<unsigned long long>(dbits(b));
-    unsigned long long const g = x > y ? x : y, l = x > y ? y : x;
-    unsigned const g1 = static_cast<unsigned>(g >> 32), l1 = static_cast<unsigned>(l >> 32), l0 = static_cast<unsigned>(l);
-    unsigned const d = (g1 >> 20) - (l1 >> 20);
-    if (d >= 32u || g1 >= 0x7fe00000u || l1 < 0x00100000u) {
-        return add_rare(a, b);
-    }
-    unsigned const lm = (l1 & 0xfffffu) | 0x100000u;
-    unsigned const rest = __funnelshift_r(0u, l0, d); // what the alignment shifts out
-    unsigned long long t = (g & 0xfffffffffffffull) + 0x10000000000000ull +
-                           ((static_cast<unsigned long long>(lm >> d) << 32) | __funnelshift_r(l0, lm, d));
-    unsigned const c = static_cast<unsigned>(t >> 53);
-    bool const tie = c != 0 ? (rest == 0u && (t & 1u) != 0) : rest == 0x80000000u;
-    t += c != 0 ? 1u : rest >> 31;
-    t >>= c;
-    t -= tie ? (t & 1u) : 0u;
-    return __longlong_as_double(static_cast<long long>(t + (static_cast<unsigned long long>((g1 >> 20) - 1u + c) << 52)));
 }
 
 // HLLC flux of hllc::operator() (euler_operators/hllc.hpp:50-105) in the face

