@@ -12,6 +12,7 @@
 #include "halve.cuh"
 
 #if defined(__CUDACC__)
+#include "euler_device.cuh"
 #define EULR_ADJ_FN __host__ __device__ __forceinline__
 #else
 #define EULR_ADJ_FN inline
@@ -19,19 +20,23 @@
 
 namespace eulr {
 
-// Reciprocal: correctly rounded on the host; on the GPU the faithful one of
-// the forward step (PTX rcp.approx.ftz.f64 and one third-order Newton step,
-// within one ulp), which costs three FP64 instructions.
+// Reciprocal and product: on the GPU on the integer pipes (rcp_alu within
+// 0.5001 ulp, mul_alu rounded to nearest), correctly rounded on the host.
 EULR_ADJ_FN double adj_rcp(double x)
 {
 #if defined(__CUDA_ARCH__)
-    double r;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
-    double e = __fma_rn(-x, r, 1.0);
-    e = __fma_rn(e, e, e);
-    return __fma_rn(r, e, r);
+    return rcp_alu(x);
 #else
     return 1.0 / x;
+#endif
+}
+
+EULR_ADJ_FN double adj_mul(double a, double b)
+{
+#if defined(__CUDA_ARCH__)
+    return mul_alu(a, b);
+#else
+    return a * b;
 #endif
 }
 
@@ -128,7 +133,9 @@ EULR_ADJ_FN double tie_side_bar(FaceSide const& q, double a, double S, double iS
 //   b = a ustar/(S - ustar):  mass d b, energy b (e + p + S d w), normal
 //   momentum d b ustar + p + a d w, tangential d b t.
 // One acoustic speed in place of two wave speeds and two impedances: about 83
-// FP64 instructions a face where the form with both took 103.  The pressure
+// FP64 operations a face where the form with both took 103, and 18 of its
+// products and the reciprocal run on the integer pipes (a reverse godunov of
+// 128^3 1239 -> 1047 us, of 64^3 193 -> 165).  The pressure
 // term is the upwind side's, p_q + rc_q (ustar - un_q): the reference's mean
 // of the two sides' values is the same function wherever ustar = num/den.
 //
@@ -150,7 +157,7 @@ EULR_ADJ_FN void hllc_bar(FaceSide const& L, FaceSide const& R, double dd, doubl
     double const du = L.un - R.un;
     double const A = cmax + (u_gt ? du : 0.0);
     double const D = L.r + R.r;
-    double const G = A * D;
+    double const G = adj_mul(A, D);
     double const mom = L.r * L.un + R.r * R.un;
     double const n = A * mom - (R.p - L.p); // G > 0, so ustar has the sign of n
     bool const left = adj_pos(n);
@@ -221,27 +228,27 @@ EULR_ADJ_FN void hllc_bar(FaceSide const& L, FaceSide const& R, double dd, doubl
         bq.t2 = 0.0;
     } else {
         double const M = S * G - n; // G (S - ustar)
-        double const Rr = adj_rcp(G * M);
-        double const nR = n * Rr;
-        iG = M * Rr;
-        ustar = nR * M;
-        double const iu = nR * G;       // ustar/(S - ustar)
-        double const y = G * (G * Rr);  // 1/(S - ustar)
-        double const b = a * iu;
+        double const Rr = adj_rcp(adj_mul(G, M));
+        double const nR = adj_mul(n, Rr);
+        iG = adj_mul(M, Rr);
+        ustar = adj_mul(nR, M);
+        double const iu = adj_mul(nR, G);              // ustar/(S - ustar)
+        double const y = adj_mul(G, adj_mul(G, Rr));   // 1/(S - ustar)
+        double const b = adj_mul(a, iu);
         double const w = ustar - q.un;
-        double const dw = q.r * w;
-        double const m = q.r * b;
+        double const dw = adj_mul(q.r, w);
+        double const m = adj_mul(q.r, b);
         double const E = S * dw + (q.e + q.p);
         double const gm = gd + gn * ustar + gt1 * q.t1 + gt2 * q.t2; // d/d (d b)
         double const gb = gm * q.r + ge * E;                         // d/d b
-        double const gE = ge * b;                                    // d/d E
+        double const gE = adj_mul(ge, b);                            // d/d E
         double const K = gE * S + gn * a;                            // d/d (d w)
-        double const gw = q.r * K;
-        double const gby = gb * y;
+        double const gw = adj_mul(q.r, K);
+        double const gby = adj_mul(gb, y);
         double const gS = gE * dw - gby * b; // db/dS = -b y
         ga = gn * dw + gb * iu + gS;         // S = un + a
         gus = gn * m + gw + gby * (a + b);   // db/dustar = (a + b) y
-        double const gEd = gE * q.r;
+        double const gEd = adj_mul(gE, q.r);
         bq.r = gm * b + K * w + gE * q.ke;
         bq.p = gn + gE + gE * inv_gm1;
         bq.un = gS - gw + gEd * q.un;
@@ -261,13 +268,13 @@ EULR_ADJ_FN void hllc_bar(FaceSide const& L, FaceSide const& R, double dd, doubl
     bR.t1 = left ? 0.0 : bq.t1;
     bR.t2 = left ? 0.0 : bq.t2;
     // ustar = n / G
-    double const gN = gus * iG;
-    double const gG = -gN * ustar;
+    double const gN = adj_mul(gus, iG);
+    double const gG = adj_mul(-gN, ustar);
     bL.p += gN;
     bR.p -= gN;
     // n's momentum sum and G's density sum
-    double const gmom = gN * A;
-    double const gD = gG * A;
+    double const gmom = adj_mul(gN, A);
+    double const gD = adj_mul(gG, A);
     bL.r += gmom * L.un + gD;
     bR.r += gmom * R.un + gD;
     bL.un += gmom * L.r;
