@@ -14,8 +14,10 @@ Reported:
   e2e        the same step through the C ABI from host buffers: host->device
              prim, step, device->host prim, every step
   roofline   the fused kernel against the FP64 pipe: algorithmic FLOPs per
-             interior cell x cells / CUDA-event kernel time, over the FP64 FMA
-             rate measured on this GPU in the same run
+             interior cell x cells / CUDA-event kernel time, over the FP64
+             unit's nominal rate and the FMA rate measured in the same run
+             (part of the kernel's products run on the integer pipes, so the
+             fractions exceed one)
   operators  each reference operator alone at 514^3 (prim_to_cons,
              cons_to_prim, time_step, godunov), CUDA-event timed
   cpu_baseline  the CPU oracle (C restatement of the reference operators,
@@ -57,9 +59,10 @@ CFL = 0.4
 FLOPS_PER_CELL_DEFAULT = None
 
 # DRAM bytes (read + write) per interior cell of the fused FP64 kernel, from
-# one ncu capture at 192^3 (736 MB read + 640 MB written over 7.08 M interior
-# cells); the kernel streams each plane once, so traffic scales with cells.
-FLUX_F64_DRAM_BYTES_PER_CELL = 194.4
+# one ncu capture at 256^3 (4.93 GB read + 1.99 GB written over 16.8 M interior
+# cells: ten staged fields with their halos, tiles at different planes when they
+# read their neighbours'); traffic scales with cells.
+FLUX_F64_DRAM_BYTES_PER_CELL = 413.0
 
 
 def parse():
@@ -668,8 +671,8 @@ def time_ops(torch, E, prim, n_int, fpc=None, fp64_peak=None, hbm_peak=None):
                             "note": "eulr_godunov_exact_f64: bit-identical to the reference (its operation order, "
                                     "every operation rounded separately). Each face is solved once and each cell's "
                                     "sound speed and total energy computed once, as the default godunov does, so "
-                                    "the algorithmic FLOPs are the same; its 3 correctly rounded divides per face "
-                                    "and divide + sqrt per cell take several FP64 instructions each"}
+                                    "the algorithmic FLOPs are the same; its products and reciprocals run on the "
+                                    "integer pipes with the FP64 unit's bits"}
     del cons, prim2
     if fpc:
         flops = {"prim_to_cons": (fpc["prim_to_cons_per_cell"]["total"], cells),
@@ -771,8 +774,10 @@ def run_ours(args):
             "kernel": "flux_tile_kernel<double, step>", "kernel_ms": flux_ms,
             "step_ms_sum_of_launches": step_ms_launches,
             "traffic": FLUX_F64_DRAM_BYTES_PER_CELL * interior,
-            "traffic_note": "dram bytes read+write per launch: 194.4 B per interior cell from an ncu capture at "
-                            "192^3, scaled by cells"}
+            "traffic_note": "dram bytes read+write per launch: 413 B per interior cell from an ncu capture at "
+                            "256^3, scaled by cells",
+            "note": "products, reciprocals and square roots run on the integer pipes, so the algorithm's "
+                    "operations exceed what the FP64 unit alone could do"}
     if fpc:
         fl = fpc["fused_step_fp64"] * interior
         roof["achieved"] = fl / (flux_ms * 1e-3) / 1e12

@@ -69,8 +69,8 @@ constexpr int kWaitTries = 1 << 20; // mbarrier.try_wait attempts before giving 
 
 // How a plane slot is filled.
 enum Staging {
-    kStageTma,   // fused FP64 step, row pitch a multiple of 16 bytes: TMA boxes, ring of three slots
-    kStageAsync, // fused FP64 step, any pitch, and the batch: 8-byte cp.async, the same ring
+    kStageTma,   // fused FP64 step, row pitch a multiple of 16 bytes: TMA boxes
+    kStageAsync, // fused FP64 step, any pitch, and the batch: 8-byte cp.async
     kStageDerive, // only prim is stored (per-operator godunov, FluxParams::own_momenta): cp.async, the rest computed
 };
 constexpr int kSlots = 2; // plane slots of the ring
@@ -911,8 +911,8 @@ constexpr int kStepTX = 16, kStepTY = 16;
 // 1.1 us a plane with two CTAs on the SM and 1.6 us with one.  Whole
 // 16 x 16 tiles are the best for large grids, smaller ones where their number
 // leaves SMs idle.  Against whole 16 x 16 tiles in chunks of at least 8
-// planes: 16^3 97 -> 12.5 us a step, 48^3 97 -> 46, 64^3 97 -> 86,
-// 99 x 128 x 75 311 -> 270.
+// planes, all work on the FP64 pipe: 16^3 97 -> 12.5 us a step, 48^3 97 -> 46,
+// 64^3 97 -> 86, 99 x 128 x 75 311 -> 270 (now 14.4, 36, 63 and 215).
 TilePlan choose_tiles(int ix, int iy, int iz, int sms, int per_sm, int face, int cell, int stage, int q)
 {
     constexpr double kInstr = 9.0e-3, kWait2 = 1.1, kWait1 = 1.6; // us
