@@ -24,6 +24,7 @@
 #include <cstring>
 #include <new>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 using namespace eulr;
@@ -104,6 +105,7 @@ struct eulr_batch {
     unsigned* d_exited = nullptr; // CTAs of the running launch that found the queue empty
     int* d_idle = nullptr;        // grids without interior cells, finalized by the launch's last CTA
     int nidle = 0;
+    int cubic = 0;                // FP64: grids of cubic cells
     int shape = 0;                // tile-shape variant of the batch kernel
     int kchunk = 32;
     int per_sm = 1;
@@ -165,6 +167,7 @@ int upload_params(eulr_batch* b)
     for (int dir = 0; dir < 2; ++dir) {
         int const in = dir, out = 1 - dir;
         std::vector<FluxParams<T>> fp(n);
+        int cubic = 0;
         for (int g = 0; g < n; ++g) {
             GridState const& G = b->grids[g];
             T const gamma = static_cast<T>(G.gamma);
@@ -210,7 +213,11 @@ int upload_params(eulr_batch* b)
             p.fin = &b->sc[g];
             p.grid_items = G.items;
             fp[g] = p;
+            if constexpr (std::is_same<T, double>::value) {
+                cubic += cubic_mesh(p) ? 1 : 0;
+            }
         }
+        b->cubic = cubic;
         B_CUDA(cudaMemcpy(b->d_params[dir], fp.data(), sizeof(FluxParams<T>) * n, cudaMemcpyHostToDevice),
                "upload batch parameters");
     }
@@ -330,6 +337,8 @@ int enqueue_step_t(eulr_batch* b, int dir)
     bp.exited = b->d_exited;
     bp.idle = b->d_idle;
     bp.nidle = b->nidle;
+    bp.ngrids = static_cast<int>(b->grids.size());
+    bp.cubic = b->cubic;
     for (auto const& gs : b->grids) {
         bp.max_cells = std::max(bp.max_cells, gs.g.ncell());
     }

@@ -75,6 +75,15 @@ enum Staging {
 };
 constexpr int kSlots = 2; // plane slots of the ring
 
+// What a kernel knows of its mesh.  Code for the other kind of mesh is short
+// and FP64: kept beside a run-time test it is predicated, and takes its slots
+// of the FP64 pipe unused (11 of 77 instructions a cell of a cubic grid's step).
+enum Mesh {
+    kMeshAny,   // tested at run time: a batch with grids of both kinds, and the first step of FluxParams::own_momenta
+    kMeshCubic, // equal spacings and face areas
+    kMeshOther,
+};
+
 template <int TX, int TY, int NSLOT>
 struct TileLayout {
     static constexpr int HX = TX + 2;
@@ -318,29 +327,18 @@ __device__ __forceinline__ bool wait_slot(TileCtx& c, int s)
     return ok;
 }
 
-// a*b by a ratio of face areas.  The FP64 product is predicated on meshes of
-// equal areas, where it still takes its slots of the pipe; the integer one is
-// branched around, but its registers spill in the step (512^3: 20.6 ms a step
-// with the first, 20.8 with the second; godunov 22.2 and 21.1).
-template <int MODE>
-__device__ __forceinline__ double scaled(double a, double b)
-{
-    return MODE == kModeStep ? mul_rn(a, b) : mul_alu(a, b);
-}
-
 // One work item: interior planes [kb, ke) of tile (tx, ty), with the update
 // coefficient k0 (dt/dv times an x face's area).  Tiles are at most
 // TX x TY cells, cut evenly out of the grid (p.sx, p.sy), so a warp solves no
 // face and updates no cell that is not the grid's.  Returns false when a staged plane never arrived.
-template <int TX, int TY, int MODE, int STAGE>
+template <int TX, int TY, int MODE, int STAGE, int MESH>
 __device__ __forceinline__ bool tile_item(TileCtx& c, FluxParams<double> const& p, TmaMaps const& maps, double k0, int tx,
                                           int ty, int kb, int ke)
 {
     constexpr int NSLOT = kSlots;
     using L = TileLayout<TX, TY, NSLOT>;
     int const tid = threadIdx.x;
-    bool const cubic = p.invdx0 == p.invdx1 && p.invdx1 == p.invdx2;
-    bool const equal_areas = p.rs1 == 1.0 && p.rs2 == 1.0;
+    bool const cubic = MESH == kMeshAny ? cubic_mesh(p) : MESH == kMeshCubic;
     double* const smem = c.smem;
     double* const fx = c.fx;
     double* const fy = c.fy;
@@ -391,7 +389,7 @@ __device__ __forceinline__ bool tile_item(TileCtx& c, FluxParams<double> const& 
         double const* const q1 = slot_field<TX, TY, NSLOT>(smem, 1, 0);
         UpwindFlux const f0 = hllc_upwind(load_side<L::PLANE_PAD>(q0, center, 2), load_side<L::PLANE_PAD>(q1, center, 2));
         double const* const u = (dbits(f0.b) > 0 ? q0 : q1) + center;
-        zlo = FaceTerms{equal_areas ? f0.b : scaled<MODE>(f0.b, p.rs2), f0.h, f0.fn, u[0], u[7 * L::PLANE_PAD], u[8 * L::PLANE_PAD],
+        zlo = FaceTerms{cubic ? f0.b : mul_rn(f0.b, p.rs2), f0.h, f0.fn, u[0], u[7 * L::PLANE_PAD], u[8 * L::PLANE_PAD],
                         u[9 * L::PLANE_PAD]};
     }
     if (__syncthreads_or(c.timed_out)) { // slot 0 is refilled next
@@ -466,8 +464,8 @@ __device__ __forceinline__ bool tile_item(TileCtx& c, FluxParams<double> const& 
             double const* const qr = is_x || is_y ? qc : qn;
             int const ar = a + (is_x ? 1 : (is_y ? L::HX : 0));
             UpwindFlux u = hllc_upwind(load_side<L::PLANE_PAD>(qc, a, dir), load_side<L::PLANE_PAD>(qr, ar, dir));
-            if (!equal_areas) {
-                u.b = scaled<MODE>(u.b, is_x ? 1.0 : (is_y ? p.rs1 : p.rs2));
+            if (!cubic) {
+                u.b = mul_rn(u.b, is_x ? 1.0 : (is_y ? p.rs1 : p.rs2));
             }
             double* const out = (is_x ? fx : (is_y ? fy : fz)) + g;
             int const stride = is_x ? L::NFX : (is_y ? L::NFY : L::NFZ);
@@ -497,9 +495,9 @@ __device__ __forceinline__ bool tile_item(TileCtx& c, FluxParams<double> const& 
             FaceTerms const yhi = face_terms<L::PLANE_PAD>(fy, L::NFY, yb + t.w, qc + center, 0, L::HX);
             double r1 = sub_rn(yhi.fn, ylo.fn);
             double r2 = sub_rn(zhi.fn, zlo.fn);
-            if (!equal_areas) {
-                r1 = scaled<MODE>(r1, p.rs1);
-                r2 = scaled<MODE>(r2, p.rs2);
+            if (!cubic) {
+                r1 = mul_rn(r1, p.rs1);
+                r2 = mul_rn(r2, p.rs2);
             }
             r1 = fma_rn(-xlo.b, xlo.m1, fma_rn(xhi.b, xhi.m1, r1));
             r2 = fma_rn(-xlo.b, xlo.m2, fma_rn(xhi.b, xhi.m2, r2));
@@ -651,7 +649,7 @@ __device__ __forceinline__ TileCtx make_ctx(unsigned char* smem_dyn)
     return c;
 }
 
-template <int TX, int TY, int MODE, int STAGE>
+template <int TX, int TY, int MODE, int STAGE, int MESH>
 __global__ void __launch_bounds__(TX* TY, 3) flux_tile_kernel(const __grid_constant__ FluxParams<double> p,
                                                            const __grid_constant__ TmaMaps maps)
 {
@@ -680,7 +678,7 @@ __global__ void __launch_bounds__(TX* TY, 3) flux_tile_kernel(const __grid_const
         int const tile = w / iz;
         int const k = w - tile * iz;
         int const run = min(end - w, iz - k);
-        if (!tile_item<TX, TY, MODE, STAGE>(c, p, maps, k0, tile % p.tiles_x, tile / p.tiles_x, 1 + k, 1 + k + run)) {
+        if (!tile_item<TX, TY, MODE, STAGE, MESH>(c, p, maps, k0, tile % p.tiles_x, tile / p.tiles_x, 1 + k, 1 + k + run)) {
             break;
         }
         w += run;
@@ -711,7 +709,7 @@ __global__ void __launch_bounds__(TX* TY, 3) flux_tile_kernel(const __grid_const
 // copies the item's grid parameters to shared memory and runs the same tile
 // engine; each item's wavespeed goes to its own grid's accumulator, so every
 // grid keeps its own dt.  Staging by cp.async (grids of any shape).
-template <int TX, int TY>
+template <int TX, int TY, int MESH>
 __global__ void __launch_bounds__(TX* TY, TX* TY == 256 ? 3 : 6) flux_batch_kernel(const __grid_constant__ BatchParams<double> b)
 {
     constexpr int NSLOT = kSlots;
@@ -739,7 +737,7 @@ __global__ void __launch_bounds__(TX* TY, TX* TY == 256 ? 3 : 6) flux_batch_kern
         __syncthreads();
         double const dtodv = dt_over_dv(gp);
         int const kb = 1 + it.w * gp.kchunk;
-        tile_item<TX, TY, kModeStep, kStageAsync>(c, gp, TmaMaps{}, dtodv * gp.ds0, it.y, it.z, kb,
+        tile_item<TX, TY, kModeStep, kStageAsync, MESH>(c, gp, TmaMaps{}, dtodv * gp.ds0, it.y, it.z, kb,
                                                      min(kb + gp.kchunk, gp.g.n2 - 1));
         flush_wavespeed<NT>(c, gp.wmax, gp.status);
         item_done(gp);
@@ -967,16 +965,16 @@ TilePlan choose_tiles(int ix, int iy, int iz, int sms, int per_sm, int face, int
 
 namespace {
 
-template <int MODE, int STAGE>
+template <int MODE, int STAGE, int MESH>
 struct FluxKernel {
     using L = TileLayout<kStepTX, kStepTY, kSlots>;
-    static auto fn() { return flux_tile_kernel<kStepTX, kStepTY, MODE, STAGE>; }
+    static auto fn() { return flux_tile_kernel<kStepTX, kStepTY, MODE, STAGE, MESH>; }
 
     // Resident CTAs per SM.  Called outside any stream capture (by the entry
     // points before they enqueue work).
     static cudaError_t configure(int* per_sm)
     {
-        return resident_ctas<flux_tile_kernel<kStepTX, kStepTY, MODE, STAGE>>(L::NT, static_cast<int>(L::BYTES), per_sm);
+        return resident_ctas<flux_tile_kernel<kStepTX, kStepTY, MODE, STAGE, MESH>>(L::NT, static_cast<int>(L::BYTES), per_sm);
     }
 
     static cudaError_t launch(FluxParams<double> p, TmaMaps const& maps, int sms, cudaStream_t s)
@@ -994,8 +992,6 @@ struct FluxKernel {
         // staged one
         TilePlan const plan = MODE == kModeStep ? choose_tiles(ix, iy, iz, sms, per_sm, 16, 48, 0, q)
                                                 : choose_tiles(ix, iy, iz, sms, per_sm, 16, 30, 17, q);
-        p.rs1 = p.ds1 / p.ds0;
-        p.rs2 = p.ds2 / p.ds0;
         p.h_over_p = p.inv_gm1 + 1.0;
         p.sx = split_tiles(ix, plan.nx, q);
         p.sy = split_tiles(iy, plan.ny, 1);
@@ -1014,29 +1010,36 @@ struct FluxKernel {
 constexpr int kBatchShapes[][2] = {{32, 8}, {16, 8}, {16, 16}};
 constexpr int kNumBatchShapes = 3;
 
-template <int TX, int TY>
+template <int TX, int TY, int MESH>
 struct BatchKernel {
     using L = TileLayout<TX, TY, kSlots>;
-    static auto fn() { return flux_batch_kernel<TX, TY>; }
     static cudaError_t configure(int* per_sm)
     {
-        auto kern = fn();
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             static_cast<int>(L::BYTES));
-        if (e != cudaSuccess) {
-            return e;
-        }
-        int n = 0;
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, L::NT, L::BYTES);
-        *per_sm = n < 1 ? 1 : n;
-        return e;
+        return resident_ctas<flux_batch_kernel<TX, TY, MESH>>(L::NT, static_cast<int>(L::BYTES), per_sm);
     }
     static cudaError_t launch(BatchParams<double> const& b, int grid, cudaStream_t s)
     {
-        fn()<<<grid, L::NT, L::BYTES, s>>>(b);
+        flux_batch_kernel<TX, TY, MESH><<<grid, L::NT, L::BYTES, s>>>(b);
         return cudaGetLastError();
     }
 };
+
+// b == nullptr: configure for every kind of mesh (the fewest resident CTAs).
+template <int TX, int TY>
+cudaError_t run_batch(BatchParams<double> const* b, int grid, int* per_sm, cudaStream_t s)
+{
+    if (b != nullptr) {
+        return b->cubic == b->ngrids ? BatchKernel<TX, TY, kMeshCubic>::launch(*b, grid, s)
+               : b->cubic == 0       ? BatchKernel<TX, TY, kMeshOther>::launch(*b, grid, s)
+                                     : BatchKernel<TX, TY, kMeshAny>::launch(*b, grid, s);
+    }
+    int n[3] = {};
+    cudaError_t e = BatchKernel<TX, TY, kMeshAny>::configure(&n[0]);
+    e = e != cudaSuccess ? e : BatchKernel<TX, TY, kMeshCubic>::configure(&n[1]);
+    e = e != cudaSuccess ? e : BatchKernel<TX, TY, kMeshOther>::configure(&n[2]);
+    *per_sm = std::min(n[0], std::min(n[1], n[2]));
+    return e;
+}
 
 } // namespace
 
@@ -1055,9 +1058,9 @@ cudaError_t launch_flux_batch(int shape, int comp, BatchParams<T> const* b, int 
 {
     if constexpr (sizeof(T) == sizeof(double)) {
         switch (shape) {
-        case 0: return b ? BatchKernel<32, 8>::launch(*b, grid, s) : BatchKernel<32, 8>::configure(per_sm);
-        case 1: return b ? BatchKernel<16, 8>::launch(*b, grid, s) : BatchKernel<16, 8>::configure(per_sm);
-        default: return b ? BatchKernel<16, 16>::launch(*b, grid, s) : BatchKernel<16, 16>::configure(per_sm);
+        case 0: return run_batch<32, 8>(b, grid, per_sm, s);
+        case 1: return run_batch<16, 8>(b, grid, per_sm, s);
+        default: return run_batch<16, 16>(b, grid, per_sm, s);
         }
     } else {
         return launch_batch_f32col(comp, kBatchShapes[shape][0], b, grid, per_sm, s);
@@ -1072,31 +1075,44 @@ struct FluxDispatch;
 
 template <>
 struct FluxDispatch<double> {
+    // Both kinds of mesh, as the mesh is not known here; their kernels take
+    // the same shared memory and no more than the registers of three CTAs.
+    template <int MODE, int STAGE>
+    static cudaError_t configure_meshes(int* per_sm)
+    {
+        cudaError_t const e = FluxKernel<MODE, STAGE, kMeshOther>::configure(per_sm);
+        return e != cudaSuccess ? e : FluxKernel<MODE, STAGE, kMeshCubic>::configure(per_sm);
+    }
+    template <int MODE, int STAGE>
+    static cudaError_t launch_mesh(FluxParams<double> const& p, TmaMaps const& maps, int sms, cudaStream_t s)
+    {
+        return cubic_mesh(p) ? FluxKernel<MODE, STAGE, kMeshCubic>::launch(p, maps, sms, s)
+                             : FluxKernel<MODE, STAGE, kMeshOther>::launch(p, maps, sms, s);
+    }
+
     static cudaError_t configure(int mode, bool tma, int /*comp*/, int* per_sm)
     {
         if (mode == kModeStep) {
-            cudaError_t const e = FluxKernel<kModeStep, kStageDerive>::configure(per_sm);
+            cudaError_t const e = FluxKernel<kModeStep, kStageDerive, kMeshAny>::configure(per_sm);
             if (e != cudaSuccess) {
                 return e;
             }
-            return tma ? FluxKernel<kModeStep, kStageTma>::configure(per_sm)
-                       : FluxKernel<kModeStep, kStageAsync>::configure(per_sm);
+            return tma ? configure_meshes<kModeStep, kStageTma>(per_sm) : configure_meshes<kModeStep, kStageAsync>(per_sm);
         }
-        return FluxKernel<kModeGodunov, kStageDerive>::configure(per_sm);
+        return configure_meshes<kModeGodunov, kStageDerive>(per_sm);
     }
-    static cudaError_t launch(FluxParams<double> const& p, TmaMaps const* maps, int mode, int /*comp*/, int sms,
-                              cudaStream_t s)
+    static cudaError_t launch(FluxParams<double> p, TmaMaps const* maps, int mode, int /*comp*/, int sms, cudaStream_t s)
     {
+        p.rs1 = p.ds1 / p.ds0;
+        p.rs2 = p.ds2 / p.ds0;
         if (mode == kModeStep) {
             if (p.own_momenta) {
-                return FluxKernel<kModeStep, kStageDerive>::launch(p, TmaMaps{}, sms, s);
+                return FluxKernel<kModeStep, kStageDerive, kMeshAny>::launch(p, TmaMaps{}, sms, s);
             }
-            if (maps != nullptr) {
-                return FluxKernel<kModeStep, kStageTma>::launch(p, *maps, sms, s);
-            }
-            return FluxKernel<kModeStep, kStageAsync>::launch(p, TmaMaps{}, sms, s);
+            return maps != nullptr ? launch_mesh<kModeStep, kStageTma>(p, *maps, sms, s)
+                                   : launch_mesh<kModeStep, kStageAsync>(p, TmaMaps{}, sms, s);
         }
-        return FluxKernel<kModeGodunov, kStageDerive>::launch(p, TmaMaps{}, sms, s);
+        return launch_mesh<kModeGodunov, kStageDerive>(p, TmaMaps{}, sms, s);
     }
 };
 

@@ -137,6 +137,12 @@ struct FluxParams {
     int grid_items;   // batch: work items of this grid in the current item list
 };
 
+// Equal spacings and face areas.
+__host__ __device__ inline bool cubic_mesh(FluxParams<double> const& p)
+{
+    return p.invdx0 == p.invdx1 && p.invdx1 == p.invdx2 && p.rs1 == 1.0 && p.rs2 == 1.0;
+}
+
 // Launch parameters of the multi-grid batch kernel.
 template <class T>
 struct BatchParams {
@@ -147,6 +153,7 @@ struct BatchParams {
     unsigned* exited;           // CTAs that found the queue empty; the last resets head and itself
     const int* idle;            // grids without interior cells (no work item): finalized by the last CTA
     int nidle;
+    int ngrids, cubic;          // FP64: the grids, and how many of them have cubic cells
     long long max_cells;        // cells of the largest grid (selects 32-bit offsets where they suffice)
 };
 
