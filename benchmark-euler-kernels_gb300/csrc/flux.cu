@@ -34,8 +34,8 @@
 // and the sum of the densities run on the integer pipes (mul_alu, rcp_alu,
 // sqrt_alu, add_alu): 11 FP64 instructions stay of a face's 22 and seed, 34 of
 // a cell's 51 and two seeds.  With three CTAs on an SM (two plane slots, 80
-// registers) a step of 512^3 takes 20.6 ms where it took 31.0, the operator
-// godunov 21.1 where it took 31.6.
+// registers) and kernels that know their mesh, a step of 512^3 takes 19.2 ms
+// where it took 31.0, the operator godunov 21.1 where it took 31.6.
 // The fused step then finishes the cell on chip: cons_to_prim, sound speed
 // and the next step's CFL max-wavespeed, reduced warp -> block -> one
 // atomicMax per CTA, so dt never leaves the device.
@@ -77,7 +77,8 @@ constexpr int kSlots = 2; // plane slots of the ring
 
 // What a kernel knows of its mesh.  Code for the other kind of mesh is short
 // and FP64: kept beside a run-time test it is predicated, and takes its slots
-// of the FP64 pipe unused (11 of 77 instructions a cell of a cubic grid's step).
+// of the FP64 pipe unused: a step of 512^3 20.6 -> 19.2 ms, of 64^3 63.0 -> 58.1
+// us, of 24 batched grids 7.40 -> 7.22 ms with kernels of their own.
 enum Mesh {
     kMeshAny,   // tested at run time: a batch with grids of both kinds, and the first step of FluxParams::own_momenta
     kMeshCubic, // equal spacings and face areas
@@ -910,7 +911,7 @@ constexpr int kStepTX = 16, kStepTY = 16;
 // 16 x 16 tiles are the best for large grids, smaller ones where their number
 // leaves SMs idle.  Against whole 16 x 16 tiles in chunks of at least 8
 // planes, all work on the FP64 pipe: 16^3 97 -> 12.5 us a step, 48^3 97 -> 46,
-// 64^3 97 -> 86, 99 x 128 x 75 311 -> 270 (now 14.4, 36, 63 and 215).
+// 64^3 97 -> 86, 99 x 128 x 75 311 -> 270 (now 13.5, 34, 58 and 211).
 TilePlan choose_tiles(int ix, int iy, int iz, int sms, int per_sm, int face, int cell, int stage, int q)
 {
     constexpr double kInstr = 9.0e-3, kWait2 = 1.1, kWait1 = 1.6; // us
