@@ -97,6 +97,25 @@ def test_step_and_godunov_scale_with_density_and_pressure(cuda, euler, oracle_li
         assert max(rel_linf(np.ldexp(a, -k), b)) <= 1e-13
 
 
+@pytest.mark.parametrize("kinds", ["cubic", "both"])
+def test_batch_of_cubic_and_other_meshes_equals_single_grids(cuda, euler, oracle_lib, kinds):
+    """A batch whose grids are all of cubic cells, and one with both kinds: the bits of each grid stepped alone."""
+    shapes = [(19, 19, 5), (20, 35, 3), (35, 21, 26), (18, 18, 18)]
+    meshes = [(0.1, 0.1, 0.1) if kinds == "cubic" or i % 2 else (0.11, 0.07, 0.13) for i in range(len(shapes))]
+    prims = [oracle_lib.random_prim(*s, seed=50 + i) for i, s in enumerate(shapes)]
+    with euler.Batch([(*s, 1.4, *dx) for s, dx in zip(shapes, meshes)], cfl=0.4) as b:
+        for g, p in enumerate(prims):
+            b.set_prim(g, p)
+        b.advance(4)
+        got = [b.state_numpy(g) for g in range(len(shapes))]
+    for shape, dx, p0, (pb, cb) in zip(shapes, meshes, prims, got):
+        with euler.Simulation(*shape, 1.4, dx, 0.4) as s:
+            s.set_prim(p0)
+            s.advance(4)
+            ps, cs = s.state_numpy()
+        assert np.array_equal(pb, ps) and np.array_equal(cb, cs), shape
+
+
 @pytest.mark.parametrize("precision", ["f32", "f32c", "f32c_hilo"])
 def test_fp32_columns_match_oracle_and_batch(cuda, euler, oracle_lib, precision):
     """The FP32 column engine at its tile widths and chunk edges.  Against the FP64 oracle after four steps: 4 steps
