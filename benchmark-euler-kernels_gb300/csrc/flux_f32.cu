@@ -136,6 +136,22 @@ __device__ __forceinline__ float col_pressure(Raw5 const& r, float u0, float u1,
     return pressure_f64_rescue(r.d, r.e, r.m[0], r.m[1], r.m[2], ir, gm1, COMP == kCompHiLo ? lo : nullptr);
 }
 
+// sqrt(x / d) of the per-operator godunov's cells, x = gamma p: x / sqrt(x d)
+// from the hardware reciprocal square root and one Newton step, within 1.5
+// ulps of the correctly rounded value, where x d is a normal number.  Elsewhere
+// that is NaN, and a root and a division answer, out of line so that they cost
+// the others only the test (256^3: the operator 2 %):
+// x d leaves FP32's range though x / d does not in a dilute gas in CGS units
+// (rho 1e-27, p 1e-12), and p = 0 has c = 0.
+static __device__ __noinline__ float sound_speed_rare(float x, float d) { return sqrtf(x * (1.0f / d)); }
+__device__ __forceinline__ float operator_sound_speed(float x, float d)
+{
+    float const z = x * d;
+    float const y = rsqrt_approx(z);
+    float const c = x * fmaf(0.5f * y, fmaf(-z * y, y, 1.0f), y);
+    return c == c ? c : sound_speed_rare(x, d);
+}
+
 // Primitive state, sound speed and e + p of an FP32 conservative cell.  1/rho
 // is the hardware reciprocal (one MUFU.RCP), not the correctly rounded
 // sequence: the FP32 step's error budget is set by the state's own rounding,
@@ -145,18 +161,13 @@ __device__ __forceinline__ Prim7 prim_of(Raw5 const& r, FluxParams<float> const&
 {
     Prim7 q;
     if constexpr (COMP == kCompOperator) {
-        // r holds prim (d, p, u).  The sound speed gamma p / sqrt(gamma p d):
-        // the hardware reciprocal square root and one Newton step, within
-        // 1.5 ulps of the correctly rounded sqrt(gamma p / d).
+        // r holds prim (d, p, u)
         q.d = r.d;
         q.p = r.e;
         q.u[0] = r.m[0];
         q.u[1] = r.m[1];
         q.u[2] = r.m[2];
-        float const gp = p.gamma * r.e;
-        float const z = gp * r.d;
-        float const y = rsqrt_approx(z);
-        q.c = gp * fmaf(0.5f * y, fmaf(-z * y, y, 1.0f), y);
+        q.c = operator_sound_speed(p.gamma * r.e, r.d);
         float const uu = fmaf(r.m[2], r.m[2], fmaf(r.m[1], r.m[1], __fmul_rn(r.m[0], r.m[0])));
         q.e = __fadd_rn(fmaf(r.e, p.inv_gm1, __fmul_rn(0.5f * r.d, uu)), r.e);
         return q;
