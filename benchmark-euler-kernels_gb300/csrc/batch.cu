@@ -10,9 +10,12 @@
 // picked by eulr_batch_autotune, which times every combination on the loaded
 // state; without it they are 16x16 and 32.
 //
-// State layout: each grid owns, inside one allocation, the same fields as a
-// single simulation of its precision (FP64: prim, cons, sound speed, two
-// copies; FP32 states: cons and optional low words, two copies).  The
+// State layout: each grid owns, inside one allocation, two copies of the
+// fields a step of its precision reads and writes.  FP64: prim, cons, sound
+// speed and e + p, 11 fields; prim and cons share the density, which is always
+// the same in both, as cons comes from prim (a single simulation may be loaded
+// with a cons of its own, and keeps both).  FP32 states: cons and optional low
+// words.  The
 // per-grid launch parameters of both copy directions live in device arrays
 // built once at creation.
 #include "euler_gb300.h"
@@ -601,7 +604,7 @@ int eulr_batch_create(int precision, int ngrids, const eulr_grid_desc* grids, do
         b->own_stream = true;
     }
     b->grids.resize(ngrids);
-    int const per_copy = is_f64(b) ? 12 : (b->comp == kCompHiLo ? 10 : 5);
+    int const per_copy = is_f64(b) ? 11 : (b->comp == kCompHiLo ? 10 : 5);
     size_t bytes = 0;
     size_t max_items = 0;
     for (int g = 0; g < ngrids; ++g) {
@@ -633,10 +636,11 @@ int eulr_batch_create(int precision, int ngrids, const eulr_grid_desc* grids, do
         size_t const field = pad256(static_cast<size_t>(G.g.ncell()) * b->esize);
         for (int c = 0; c < 2; ++c) {
             if (is_f64(b)) {
-                for (int f = 0; f < 5; ++f) {
+                for (int f = 1; f < 5; ++f) {
                     G.prim[c][f] = p;
                     p += field;
                 }
+                G.prim[c][0] = p + 2 * field; // cons' density, which follows
                 G.cs[c] = p;
                 p += field;
                 G.h[c] = p;
