@@ -206,38 +206,46 @@ def _stream(stream=None) -> int:
 _operators: dict = {}  # (entry point, suffix) -> its C function
 
 
-def _operator(name: str, sfx: str):
+def _operator(name: str, sfx: str, *args) -> None:
     fn = _operators.get((name, sfx))
     if fn is None:
         fn = _operators[name, sfx] = getattr(load(), f"eulr_{name}_{sfx}")
-    return fn
+    try:
+        status = fn(*args)
+    except ctypes.ArgumentError:
+        for value, kind in zip(args, fn.argtypes):
+            if kind in (_D, _F):
+                kind(value)  # raises what the value itself does: TypeError, OverflowError
+        raise
+    if status != EULR_SUCCESS:
+        check(status)
 
 
 def init_implode(n0, n1, n2, dx, dtype=None, device="cuda", stream=None):
     torch = _torch()
     dtype = dtype or torch.float64
     prim = torch.empty((5, n2, n1, n0), dtype=dtype, device=device)
-    check(_operator("init_implode", _sfx(prim))(bundle(prim), n0, n1, n2, dx[0], dx[1], dx[2], _stream(stream)))
+    _operator("init_implode", _sfx(prim), bundle(prim), n0, n1, n2, dx[0], dx[1], dx[2], _stream(stream))
     return prim
 
 
 def prim_to_cons(prim, gamma, out=None, stream=None):
     cons = out if out is not None else _torch().empty_like(prim)
-    check(_operator("prim_to_cons", _sfx(prim))(bundle(prim), bundle(cons), *dims(prim), gamma, _stream(stream)))
+    _operator("prim_to_cons", _sfx(prim), bundle(prim), bundle(cons), *dims(prim), gamma, _stream(stream))
     return cons
 
 
 def cons_to_prim(cons, gamma, out=None, stream=None):
     prim = out if out is not None else _torch().empty_like(cons)
-    check(_operator("cons_to_prim", _sfx(cons))(bundle(cons), bundle(prim), *dims(cons), gamma, _stream(stream)))
+    _operator("cons_to_prim", _sfx(cons), bundle(cons), bundle(prim), *dims(cons), gamma, _stream(stream))
     return prim
 
 
 def time_step(prim, gamma, dx, out=None, stream=None):
     """Device scalar tensor holding time_step(prim) (not multiplied by CFL)."""
     dt = out if out is not None else _torch().empty((), dtype=prim.dtype, device=prim.device)
-    check(_operator("time_step", _sfx(prim))(bundle(prim), *dims(prim), gamma, dx[0], dx[1], dx[2], dt.data_ptr(),
-                                             _stream(stream)))
+    _operator("time_step", _sfx(prim), bundle(prim), *dims(prim), gamma, dx[0], dx[1], dx[2], dt.data_ptr(),
+              _stream(stream))
     return dt
 
 
@@ -250,17 +258,17 @@ def godunov(prim, cons, gamma, dx, dt, stream=None, exact=False):
     if exact:
         if isinstance(dt, tuple):
             raise ValueError("the exact godunov takes dt as a number")
-        check(_operator("godunov_exact", sfx)(bundle(prim), bundle(cons), *dims(prim), gamma, dx[0], dx[1], dx[2], dt,
-                                              _stream(stream)))
+        _operator("godunov_exact", sfx, bundle(prim), bundle(cons), *dims(prim), gamma, dx[0], dx[1], dx[2], dt,
+                  _stream(stream))
     elif isinstance(dt, tuple):
         if sfx != "f64":
             raise ctypes.ArgumentError("a device dt needs FP64 bundles")
         dt_t, cfl = dt
-        check(_operator("godunov_devdt", "f64")(bundle(prim), bundle(cons), *dims(prim), gamma, dx[0], dx[1], dx[2],
-                                                dt_t.data_ptr(), cfl, _stream(stream)))
+        _operator("godunov_devdt", "f64", bundle(prim), bundle(cons), *dims(prim), gamma, dx[0], dx[1], dx[2],
+                  dt_t.data_ptr(), cfl, _stream(stream))
     else:
-        check(_operator("godunov", sfx)(bundle(prim), bundle(cons), *dims(prim), gamma, dx[0], dx[1], dx[2], dt,
-                                        _stream(stream)))
+        _operator("godunov", sfx, bundle(prim), bundle(cons), *dims(prim), gamma, dx[0], dx[1], dx[2], dt,
+                  _stream(stream))
     return cons
 
 
@@ -443,7 +451,7 @@ def godunov_adjoint(prim, cons_bar, gamma, dx, dt, out=None, workspace=None, str
     check(load().eulr_godunov_adjoint_f64(bundle(prim), bundle(cons_bar), bundle(prim_bar), n0, n1, n2,
                                           float(gamma), float(dx[0]), float(dx[1]), float(dx[2]), float(dt),
                                           ctypes.c_void_p(workspace.data_ptr()), workspace.numel(),
-                                          _stream(stream)))
+              _stream(stream)))
     return prim_bar
 
 
