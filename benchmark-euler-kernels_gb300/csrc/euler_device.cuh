@@ -77,8 +77,9 @@ __device__ __forceinline__ float half_exact(float x) { return __fmul_rn(x, 0.5f)
 __device__ __forceinline__ float abs_(float a) { return fabsf(a); }
 
 // Faithful FP64 reciprocal and square root (within one ulp of the correctly
-// rounded result, not always equal to it) for the fused step, whose parity
-// bar is a relative tolerance.  Each refines the PTX hardware approximation
+// rounded result, not always equal to it) for kernels whose parity bar is a
+// relative tolerance: for the operands that rcp_alu and sqrt_alu below leave to
+// the FP64 unit, and the adjoint's cell conversion.  Each refines the PTX hardware approximation
 // (rcp.approx.ftz.f64, rsqrt.approx.ftz.f64; both measured at most 2^-19.9
 // relative error on sm_103a) by one Newton-Raphson step carried to third
 // order, from the series 1/(1-e) = 1 + e + e^2 + ... and
@@ -100,7 +101,6 @@ __device__ __forceinline__ double rcp_faithful(double x)
     e = __fma_rn(e, e, e);
     return __fma_rn(r, e, r);
 }
-__device__ __forceinline__ float rcp_faithful(float x) { return __frcp_rn(x); }
 
 __device__ __forceinline__ double sqrt_faithful(double x)
 {
@@ -135,8 +135,8 @@ __device__ __forceinline__ float rsqrt_approx(float x)
 // (y (1 + e/2 + 3e^2/8), e = 1 - z y^2).  Seven FP64 instructions and one
 // seed where rcp_faithful + sqrt_faithful take ten and two; within two ulps
 // of the correctly rounded sqrt(x/d) (checked against it on 4M argument
-// pairs).  For the sound speed sqrt(gamma p / rho) of a state whose 1/rho
-// is not needed otherwise.
+// pairs).  (Sound speeds are formed by sqrt_alu and rcp_alu now; only its test
+// uses this one.)
 __device__ __forceinline__ double sqrt_quotient_faithful(double x, double d)
 {
     double const z = x * d;
@@ -184,17 +184,11 @@ __device__ __forceinline__ long long dbits(double x)
     return b;
 }
 
-// Signed key with the order of the doubles (-0 sorts just below +0).
-__device__ __forceinline__ long long order_key(double x)
-{
-    long long const b = dbits(x);
-    return b ^ ((b >> 63) & 0x7fffffffffffffffLL);
-}
-
 // x is neither +0 nor -0.
 __device__ __forceinline__ bool nonzero_(double x) { return (dbits(x) << 1) != 0; }
 
 // a*b > 0 for non-NaN a, b, decided from signs: both non-zero and of one sign.
+// (Only its test uses it: hllc_upwind needs the sign of one number.)
 __device__ __forceinline__ bool product_positive(double a, double b)
 {
     return nonzero_(a) && nonzero_(b) && ((dbits(a) ^ dbits(b)) >= 0);
@@ -555,7 +549,7 @@ __device__ __forceinline__ bool finite_positive(double x)
 //  * in the supersonic case the reference's ratio (S-u)/(S-u) is exactly 1
 //    and its energy correction exactly 0: ustar := u and b := u (so w = 0)
 //    give the upwind state's own flux with two selects.
-//  * min/max and the sign tests run on the integer pipe (order_key etc.).
+//  * max and the sign tests run on the integer pipe, on the bit patterns.
 // So four of the five fluxes are b times a value of the upwind side, and the
 // FP64 kernels never form them: the face keeps b, h = (e + p) + S d w and the
 // normal momentum's flux, the side is the sign of b, and each cell adds b d,

@@ -15,7 +15,8 @@ constexpr long long kInfBits = 0x7ff0000000000000LL;
 
 // g / D for 0 <= g < 2^12 and a compile-time 0 < D < 256, as one product and
 // a shift: floor(g (floor(2^20/D) + 1) / 2^20) exceeds g/D by less than
-// g/2^20 < 2^-8, which stays below the gap 1/D to the next integer.
+// g/2^20 < 2^-8, which stays below the gap 1/D to the next integer.  (The
+// kernels use the run-time form below; this one only its test does.)
 template <int D>
 __device__ __forceinline__ int div_small(int g)
 {
@@ -66,10 +67,6 @@ __device__ __forceinline__ long long wave_key(double v)
 }
 __device__ __forceinline__ long long wave_key(float v) { return wave_key(static_cast<double>(v)); }
 
-__device__ __forceinline__ bool cell_ok(double d, double pr, double invdt)
-{
-    return finite_positive(d) && finite_positive(pr) && dbits(invdt) < kInfBits;
-}
 __device__ __forceinline__ bool cell_ok(float d, float pr, float invdt)
 {
     return d > 0.0f && pr > 0.0f && invdt <= 3.0e38f;
