@@ -8,7 +8,7 @@
 // first step).  Pairs of steps are captured into a CUDA graph.  The tile shape
 // (32x8, 16x8 or 16x16) and the longest chunk (planes per work item) are
 // picked by eulr_batch_autotune, which times every combination on the loaded
-// state; without it they are 16x16 and 32.
+// state; without it default_shape and 32.
 //
 // State layout: each grid owns, inside one allocation, two copies of the
 // fields a step of its precision reads and writes.  FP64: prim, cons, sound
@@ -81,10 +81,7 @@ struct GridState {
 };
 
 constexpr int kKchunks[] = {8, 16, 32, 64};
-// Tiles of a batch that is not autotuned: 16 x 16, the autotuner's choice on
-// most mixes of grids and within 3 % of it on the others tried (24 grids
-// FP64: 5.70 Gcell/s, 5.77 tuned).
-constexpr int kDefaultShape = 2;
+constexpr int kDefaultShape = 2; // 16 x 16, of an FP64 batch (24 grids: 5.70 Gcell/s, 5.77 tuned)
 
 } // namespace
 
@@ -230,6 +227,41 @@ int upload_params(eulr_batch* b)
 int upload_params_any(eulr_batch* b)
 {
     return is_f64(b) ? upload_params<double>(b) : upload_params<float>(b);
+}
+
+// Tiles of a batch that is not autotuned.  FP64 tiles are cut to the grid:
+// 16 x 16, the autotuner's choice on most mixes of grids and within 3 % of it
+// on the others tried.  FP32 tiles are whole, so the shape that covers the
+// grids with the fewest columns, counted at what a column costs in it: a
+// double-float state has more CTAs on an SM with 16 x 8 tiles (16 grids of
+// 128^3: 1180 -> 1078 us a step), the others fewer halos with larger ones (plain
+// state 548 us, 600 with 16 x 8).  Within 5 % of the best shape on 22 mixes of
+// grids, but 14 % on one grid of 16^3.  200 grids of 24^3 (compensated): 115 us
+// with 16 x 16 tiles, 92 with the three 32 x 8 ones that cover a grid.
+int default_shape(eulr_batch const* b)
+{
+    if (is_f64(b)) {
+        return kDefaultShape;
+    }
+    int best = kDefaultShape;
+    double least = 0.0;
+    for (int s = batch_shape_count() - 1; s >= 0; --s) { // 16 x 16 first
+        int tx = 0, ty = 0;
+        batch_shape(s, &tx, &ty);
+        double const column = tx == 32 ? 1.03 : (ty == 16 ? 1.0 : (b->comp == kCompHiLo ? 0.92 : (b->comp == kCompSum ? 1.02 : 1.1)));
+        double cost = 0.0;
+        for (GridState const& G : b->grids) {
+            int const ix = G.g.n0 - 2, iy = G.g.n1 - 2, iz = G.g.n2 - 2;
+            if (ix > 0 && iy > 0 && iz > 0) {
+                cost += column * (tx * ty) * ((ix + tx - 1) / tx) * ((iy + ty - 1) / ty) * iz;
+            }
+        }
+        if (s == kDefaultShape || cost < least) {
+            least = cost;
+            best = s;
+        }
+    }
+    return best;
 }
 
 // Work items for tile shape `shape`, the largest grids first
@@ -677,7 +709,7 @@ int eulr_batch_create(int precision, int ngrids, const eulr_grid_desc* grids, do
     if (e != cudaSuccess) {
         return bail(cfail(e, "cudaMemset"));
     }
-    int const st = build_items(b, kDefaultShape, 32);
+    int const st = build_items(b, default_shape(b), 32);
     if (st != EULR_SUCCESS) {
         return bail(st);
     }
@@ -777,9 +809,6 @@ int eulr_batch_autotune(eulr_batch* b, int trial_steps, int* shape_out, int* kch
     int best_shape = 0, best_kc = 32;
     int st = EULR_SUCCESS;
     for (int shape = 0; shape < batch_shape_count() && st == EULR_SUCCESS; ++shape) {
-        if (!batch_shape_built(shape, is_f64(b))) {
-            continue;
-        }
         for (int kc : kKchunks) {
             st = build_items(b, shape, kc);
             if (st != EULR_SUCCESS) {

@@ -1006,8 +1006,7 @@ struct FluxKernel {
     }
 };
 
-// Tile shapes of the batch (the autotuner picks one); the FP32 states' column
-// engine has those of 256 columns.
+// Tile shapes of the batch (the autotuner picks one).
 constexpr int kBatchShapes[][2] = {{32, 8}, {16, 8}, {16, 16}};
 constexpr int kNumBatchShapes = 3;
 
@@ -1050,7 +1049,6 @@ void batch_shape(int shape, int* tx, int* ty)
     *tx = kBatchShapes[shape][0];
     *ty = kBatchShapes[shape][1];
 }
-bool batch_shape_built(int shape, bool f64) { return f64 || kBatchShapes[shape][0] * kBatchShapes[shape][1] == 256; }
 
 // b == nullptr: configure (dynamic shared memory opt-in) and report the
 // resident CTAs per SM; otherwise launch `grid` persistent CTAs.
@@ -1064,7 +1062,7 @@ cudaError_t launch_flux_batch(int shape, int comp, BatchParams<T> const* b, int 
         default: return run_batch<16, 16>(b, grid, per_sm, s);
         }
     } else {
-        return launch_batch_f32col(comp, kBatchShapes[shape][0], b, grid, per_sm, s);
+        return launch_batch_f32col(comp, kBatchShapes[shape][0], kBatchShapes[shape][1], b, grid, per_sm, s);
     }
 }
 

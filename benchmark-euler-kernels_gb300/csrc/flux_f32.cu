@@ -61,12 +61,13 @@ namespace {
 // 256^3): the state's own rounding and the FP32 fluxes dominate it.
 namespace f32col {
 
-constexpr int NT = 256;          // threads of a CTA, one column each
 constexpr int kCompOperator = 3; // the per-operator godunov
 
-// A tile of TX columns along x; a warp holds 32 / TX rows of it.
-template <int TX_>
+// A tile of TX columns along x, one per thread of its CTA; a warp holds
+// 32 / TX rows of it.
+template <int TX_, int NT_ = 256>
 struct Tile {
+    static constexpr int NT = NT_;
     static constexpr int TX = TX_;
     static constexpr int TY = NT / TX;
     static constexpr int HX = TX + 2;
@@ -77,7 +78,7 @@ struct Tile {
     // one without halo staging (threads 0..NHALO-1) and other than the top
     // row's warp (which solves the top boundary y faces), so that no warp
     // solves more than one extra face per plane.
-    static constexpr int kRightWarp = 3;
+    static constexpr int kRightWarp = NT == 256 ? 3 : 2;
     static_assert(kRightWarp * 32 >= NHALO && kRightWarp < NT / 32 - 1 && TY <= 32 && 32 % TX == 0, "right boundary warp");
 };
 
@@ -251,10 +252,10 @@ __device__ __forceinline__ Raw5 read_raw(float const* src, int stride)
     return Raw5{src[0], src[stride], {src[2 * stride], src[3 * stride], src[4 * stride]}};
 }
 
-template <int W>
+template <class W>
 __device__ __forceinline__ void halo_cell(int h, int& hx, int& hy)
 {
-    constexpr int TX = Tile<W>::TX, TY = Tile<W>::TY, HX = Tile<W>::HX, HY = Tile<W>::HY;
+    constexpr int TX = W::TX, TY = W::TY, HX = W::HX, HY = W::HY;
     if (h < TY) {
         hx = 0;
         hy = 1 + h;
@@ -274,20 +275,20 @@ __device__ __forceinline__ void halo_cell(int h, int& hx, int& hy)
 // (u2, c, e + p, -), written and read with two vector accesses (STS.128 and
 // LDS.128) instead of seven scalar ones.  Consecutive lanes touch
 // consecutive words, so the accesses are free of bank conflicts.
-template <int W>
+template <class W>
 struct SlotPlane {
-    float4 a[Tile<W>::PLANE];
-    float4 b[Tile<W>::PLANE];
+    float4 a[W::PLANE];
+    float4 b[W::PLANE];
 };
 
-template <int W>
+template <class W>
 __device__ __forceinline__ void put(SlotPlane<W>& q, int idx, Prim7 const& v)
 {
     q.a[idx] = make_float4(v.d, v.p, v.u[0], v.u[1]);
     q.b[idx] = make_float4(v.u[2], v.c, v.e, v.e);
 }
 
-template <int W>
+template <class W>
 __device__ __forceinline__ Prim7 get(SlotPlane<W> const& q, int idx)
 {
     float4 const a = q.a[idx];
@@ -378,9 +379,9 @@ __device__ __forceinline__ void hilo_update2(float2& u, float2& lo, float2 xl, f
     lo = sub2(err, sub2(u, sum));
 }
 
-template <int COMP, int W>
+template <int COMP, class W>
 struct ColShared {
-    static constexpr int TY = Tile<W>::TY, NHALO = Tile<W>::NHALO;
+    static constexpr int NT = W::NT, TY = W::TY, NHALO = W::NHALO;
     SlotPlane<W> slot[2];
     float4 yflux_a[NT]; // the y face below each cell
     float yflux_b[NT];
@@ -398,12 +399,12 @@ struct ColShared {
 // 1/dx_d too).  BRANCHED: the cell update sits inside the
 // interior test (the batch) rather than beside it (the single grid).
 // Accumulates this thread's max wavespeed and non-physical flag.
-template <int COMP, int W, bool UNIFORM, class Off, bool BRANCHED>
+template <int COMP, class W, bool UNIFORM, class Off, bool BRANCHED>
 __device__ __forceinline__ void col_item(FluxParams<float> const& p, float k0, float k1, float k2, int tx, int ty,
                                          int kb, int ke, ColShared<COMP, W>& sh, float& wmaxf, bool& bad)
 {
-    constexpr int TX = Tile<W>::TX, TY = Tile<W>::TY, HX = Tile<W>::HX, NHALO = Tile<W>::NHALO;
-    constexpr int kRightWarp = Tile<W>::kRightWarp;
+    constexpr int NT = W::NT, TX = W::TX, TY = W::TY, HX = W::HX, NHALO = W::NHALO;
+    constexpr int kRightWarp = W::kRightWarp;
     CBundle<float> const& src = staged<COMP>(p);
     int const tid = threadIdx.x;
     int const ti = tid % TX;
@@ -651,10 +652,11 @@ __device__ __forceinline__ void col_item(FluxParams<float> const& p, float k0, f
 
 // Block max of the threads' wavespeeds into *wmax (ordered bits, one
 // atomicMax per CTA) and the non-physical flag into *status; clears both.
-template <int COMP, int W>
+template <int COMP, class W>
 __device__ __forceinline__ void col_flush(ColShared<COMP, W>& sh, float& wmaxf, bool& bad, unsigned long long* wmax,
                                           int* status)
 {
+    constexpr int NT = W::NT;
     int const tid = threadIdx.x;
     long long wk = wave_key(wmaxf);
 #pragma unroll
@@ -690,12 +692,12 @@ __device__ __forceinline__ void col_flush(ColShared<COMP, W>& sh, float& wmaxf, 
 }
 
 // CTAs per SM the registers are cut for.
-template <int COMP>
-constexpr int kColPerSM = COMP == kCompHiLo ? 2 : 3;
+template <int COMP, class W>
+constexpr int kColPerSM = (COMP == kCompHiLo ? 512 : 768) / W::NT;
 
 // One launch over a single grid: the fused step, or the operator.
-template <int COMP, int W, bool UNIFORM, class Off>
-__global__ void __launch_bounds__(NT, kColPerSM<COMP>) f32_step_kernel(const __grid_constant__ FluxParams<float> p)
+template <int COMP, class W, bool UNIFORM, class Off>
+__global__ void __launch_bounds__(W::NT, kColPerSM<COMP, W>) f32_step_kernel(const __grid_constant__ FluxParams<float> p)
 {
     __shared__ __align__(16) ColShared<COMP, W> sh;
     float const dtodv = dt_over_dv(p);
@@ -723,8 +725,8 @@ __global__ void __launch_bounds__(NT, kColPerSM<COMP>) f32_step_kernel(const __g
 // The column engine over a batch: CTAs pop (grid, tile x, tile y, chunk)
 // items from the queue, as flux_batch_kernel does; each item's wavespeed goes
 // to its own grid.  Grids of cubic cells take the cubic update and wavespeed.
-template <int COMP, int W, class Off>
-__global__ void __launch_bounds__(NT, kColPerSM<COMP>) f32_batch_kernel(const __grid_constant__ BatchParams<float> b)
+template <int COMP, class W, class Off>
+__global__ void __launch_bounds__(W::NT, kColPerSM<COMP, W>) f32_batch_kernel(const __grid_constant__ BatchParams<float> b)
 {
     static_assert(sizeof(FluxParams<float>) % 4 == 0, "parameter copy in 4-byte words");
     __shared__ __align__(16) ColShared<COMP, W> sh;
@@ -744,7 +746,7 @@ __global__ void __launch_bounds__(NT, kColPerSM<COMP>) f32_batch_kernel(const __
             break;
         }
         int4 const it = b.items[item];
-        for (int w = tid; w < static_cast<int>(sizeof(FluxParams<float>) / 4); w += NT) {
+        for (int w = tid; w < static_cast<int>(sizeof(FluxParams<float>) / 4); w += W::NT) {
             reinterpret_cast<int*>(&gp)[w] = reinterpret_cast<const int*>(&b.grids[it.x])[w];
         }
         __syncthreads();
@@ -771,7 +773,7 @@ constexpr long long kNarrowCells = 0xffffffffLL;
 template <int COMP>
 cudaError_t configure_f32col(int* per_sm)
 {
-    return resident_ctas<f32col::f32_step_kernel<COMP, 32, false, long long>>(f32col::NT, 0, per_sm);
+    return resident_ctas<f32col::f32_step_kernel<COMP, f32col::Tile<32>, false, long long>>(256, 0, per_sm);
 }
 
 // Tile width and chunks of planes of a single-grid launch.
@@ -798,7 +800,7 @@ ColPlan choose_columns(int ix, int iy, int iz, int sms, int per_sm)
     double least = 1e300;
     long long tiles = 1;
     for (int tx : {32, 16, 8}) {
-        int const ty = f32col::NT / tx;
+        int const ty = 256 / tx;
         long long const n = static_cast<long long>((ix + tx - 1) / tx) * ((iy + ty - 1) / ty);
         double const cost = n * (tx == 32 ? (ix % 32 == 0 ? 1.0 : 1.06) : (tx == 16 ? 1.02 : 1.12));
         if (cost < least) {
@@ -825,14 +827,14 @@ ColPlan choose_columns(int ix, int iy, int iz, int sms, int per_sm)
     return best;
 }
 
-template <int COMP, int W, class Off>
+template <int COMP, class W, class Off>
 cudaError_t launch_f32col_as(FluxParams<float> p, int chunks, int sms, cudaStream_t s)
 {
     int const per_sm = p.per_sm > 0 ? p.per_sm : 1;
     int const ix = p.g.n0 - 2;
     int const iy = p.g.n1 - 2;
-    p.tiles_x = (ix + f32col::Tile<W>::TX - 1) / f32col::Tile<W>::TX;
-    p.tiles_y = (iy + f32col::Tile<W>::TY - 1) / f32col::Tile<W>::TY;
+    p.tiles_x = (ix + W::TX - 1) / W::TX;
+    p.tiles_y = (iy + W::TY - 1) / W::TY;
     long long const slots = static_cast<long long>(sms) * per_sm;
     p.kchunk = chunks;
     p.nwork = p.tiles_x * p.tiles_y * chunks;
@@ -840,9 +842,9 @@ cudaError_t launch_f32col_as(FluxParams<float> p, int chunks, int sms, cudaStrea
     // cubic cells: equal face areas give equal update coefficients dt/dv * ds_d,
     // and equal 1/dx_d the one-product wavespeed
     if (p.ds0 == p.ds1 && p.ds1 == p.ds2 && p.invdx0 == p.invdx1 && p.invdx1 == p.invdx2) {
-        f32col::f32_step_kernel<COMP, W, true, Off><<<grid, f32col::NT, 0, s>>>(p);
+        f32col::f32_step_kernel<COMP, W, true, Off><<<grid, W::NT, 0, s>>>(p);
     } else {
-        f32col::f32_step_kernel<COMP, W, false, Off><<<grid, f32col::NT, 0, s>>>(p);
+        f32col::f32_step_kernel<COMP, W, false, Off><<<grid, W::NT, 0, s>>>(p);
     }
     return cudaGetLastError();
 }
@@ -855,31 +857,31 @@ cudaError_t launch_f32col(FluxParams<float> const& p, int sms, cudaStream_t s)
     }
     ColPlan const plan = choose_columns(p.g.n0 - 2, p.g.n1 - 2, p.g.n2 - 2, sms, p.per_sm > 0 ? p.per_sm : 1);
     if (p.g.ncell() > kNarrowCells) { // 64-bit offsets are built for one width
-        return launch_f32col_as<COMP, 32, long long>(p, plan.chunks, sms, s);
+        return launch_f32col_as<COMP, f32col::Tile<32>, long long>(p, plan.chunks, sms, s);
     }
     switch (plan.width) {
-    case 8: return launch_f32col_as<COMP, 8, unsigned>(p, plan.chunks, sms, s);
-    case 16: return launch_f32col_as<COMP, 16, unsigned>(p, plan.chunks, sms, s);
-    default: return launch_f32col_as<COMP, 32, unsigned>(p, plan.chunks, sms, s);
+    case 8: return launch_f32col_as<COMP, f32col::Tile<8>, unsigned>(p, plan.chunks, sms, s);
+    case 16: return launch_f32col_as<COMP, f32col::Tile<16>, unsigned>(p, plan.chunks, sms, s);
+    default: return launch_f32col_as<COMP, f32col::Tile<32>, unsigned>(p, plan.chunks, sms, s);
     }
 }
 
-// The column engine as the 32 x 8 and 16 x 16 shapes of the FP32 batch.
-template <int COMP, int W>
+// The column engine as the shapes of the FP32 batch.
+template <int COMP, class W>
 struct ColBatchKernel {
     static cudaError_t run(BatchParams<float> const* b, int grid, int* per_sm, cudaStream_t s)
     {
         if (b == nullptr) {
             int n = 0;
             cudaError_t const e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-                    &n, f32col::f32_batch_kernel<COMP, W, long long>, f32col::NT, 0);
+                    &n, f32col::f32_batch_kernel<COMP, W, long long>, W::NT, 0);
             *per_sm = n < 1 ? 1 : n;
             return e;
         }
         if (b->max_cells <= kNarrowCells) {
-            f32col::f32_batch_kernel<COMP, W, unsigned><<<grid, f32col::NT, 0, s>>>(*b);
+            f32col::f32_batch_kernel<COMP, W, unsigned><<<grid, W::NT, 0, s>>>(*b);
         } else {
-            f32col::f32_batch_kernel<COMP, W, long long><<<grid, f32col::NT, 0, s>>>(*b);
+            f32col::f32_batch_kernel<COMP, W, long long><<<grid, W::NT, 0, s>>>(*b);
         }
         return cudaGetLastError();
     }
@@ -912,16 +914,22 @@ cudaError_t launch_godunov_f32(FluxParams<float> const& p, int sms, cudaStream_t
     return e != cudaSuccess ? e : launch_f32col<f32col::kCompOperator>(q, sms, s);
 }
 
-cudaError_t launch_batch_f32col(int comp, int tx, BatchParams<float> const* b, int grid, int* per_sm, cudaStream_t s)
+template <int COMP>
+static cudaError_t run_batch_f32col(int tx, int ty, BatchParams<float> const* b, int grid, int* per_sm, cudaStream_t s)
 {
-    bool const w = tx == 32;
+    if (tx * ty == 128) {
+        return ColBatchKernel<COMP, f32col::Tile<16, 128>>::run(b, grid, per_sm, s);
+    }
+    return tx == 32 ? ColBatchKernel<COMP, f32col::Tile<32>>::run(b, grid, per_sm, s)
+                    : ColBatchKernel<COMP, f32col::Tile<16>>::run(b, grid, per_sm, s);
+}
+
+cudaError_t launch_batch_f32col(int comp, int tx, int ty, BatchParams<float> const* b, int grid, int* per_sm, cudaStream_t s)
+{
     switch (comp) {
-    case kCompSum:
-        return w ? ColBatchKernel<kCompSum, 32>::run(b, grid, per_sm, s) : ColBatchKernel<kCompSum, 16>::run(b, grid, per_sm, s);
-    case kCompHiLo:
-        return w ? ColBatchKernel<kCompHiLo, 32>::run(b, grid, per_sm, s) : ColBatchKernel<kCompHiLo, 16>::run(b, grid, per_sm, s);
-    default:
-        return w ? ColBatchKernel<kCompNone, 32>::run(b, grid, per_sm, s) : ColBatchKernel<kCompNone, 16>::run(b, grid, per_sm, s);
+    case kCompSum: return run_batch_f32col<kCompSum>(tx, ty, b, grid, per_sm, s);
+    case kCompHiLo: return run_batch_f32col<kCompHiLo>(tx, ty, b, grid, per_sm, s);
+    default: return run_batch_f32col<kCompNone>(tx, ty, b, grid, per_sm, s);
     }
 }
 

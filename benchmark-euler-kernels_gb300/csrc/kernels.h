@@ -225,11 +225,9 @@ cudaError_t launch_godunov_exact(CBundle<T> prim, Bundle<T> cons, Geom g, T gamm
 int flux_tile_x();
 int flux_tile_y();
 
-// Multi-grid batch (batch.cu): tile-shape variants of the batch kernel; the
-// FP32 states have the 32 x 8 and 16 x 16 ones.
+// Multi-grid batch (batch.cu): tile-shape variants of the batch kernel.
 int batch_shape_count();
 void batch_shape(int shape, int* tx, int* ty);
-bool batch_shape_built(int shape, bool f64);
 template <class T>
 cudaError_t launch_flux_batch(int shape, int comp, BatchParams<T> const* b, int grid, int* per_sm, cudaStream_t s);
 template <class T>
@@ -243,7 +241,7 @@ cudaError_t configure_step_f32col(int comp, int* per_sm);
 cudaError_t launch_step_f32col(FluxParams<float> const& p, int comp, int sms, cudaStream_t s);
 cudaError_t launch_godunov_f32(FluxParams<float> const& p, int sms, cudaStream_t s);
 // b == nullptr: configure and report resident CTAs per SM; otherwise launch.
-cudaError_t launch_batch_f32col(int comp, int tx, BatchParams<float> const* b, int grid, int* per_sm, cudaStream_t s);
+cudaError_t launch_batch_f32col(int comp, int tx, int ty, BatchParams<float> const* b, int grid, int* per_sm, cudaStream_t s);
 
 cudaError_t launch_fma_probe(int kind, int blocks, int iters, float* sink, cudaStream_t s);
 template <class T>

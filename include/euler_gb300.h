@@ -329,8 +329,8 @@ int eulr_batch_set_prim_f64(eulr_batch* batch, int grid, eulr_prim_cf64 prim);
 int eulr_batch_init_step(eulr_batch* batch, int grid, double c, double rho_in, double p_in, double rho_out,
                          double p_out);
 
-/* Times every tile shape (32x8, 16x8, 16x16; FP32 states: those of 256 columns)
- * and longest chunk (8, 16, 32, 64 planes) on the loaded state over `trial_steps` steps each, keeps the
+/* Times every tile shape (32x8, 16x8, 16x16) and longest chunk (8, 16, 32,
+ * 64 planes) on the loaded state over `trial_steps` steps each, keeps the
  * fastest and restores the state's clocks.  Reports the choice as
  * TX*1000+TY, the chunk length and its step time in ms (any may be NULL). */
 int eulr_batch_autotune(eulr_batch* batch, int trial_steps, int* tile_shape, int* kchunk, double* step_ms);
