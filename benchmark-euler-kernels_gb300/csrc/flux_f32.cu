@@ -781,15 +781,19 @@ cudaError_t configure_f32col(int* per_sm)
 // 12 % dearer than a 32-column one (measured at 512^3: -2 to 8 % and 10 to
 // 15 %), and 32-column tiles 6 % dearer where they leave a remainder (200^3,
 // compensated state: 166 us a step in 32-wide tiles, 142 in 16-wide).
-// Chunks: about three items per CTA slot, in chunks of 8 to 64 planes -- with
-// fewer items the SMs are not full, longer chunks let neighbouring CTAs drift
-// apart and lose the halos they share in L2, shorter ones pay the plane and a
-// half that an item costs besides its own too often -- and, within half of
-// that count, the one with the least work on the busiest SM.  A grid with
-// fewer tiles than SMs is cut finer, to one item per SM.  Within 5 % of the
-// best count tried on grids of 64^3 to 512^3.  Against 32-wide tiles in chunks of
-// at least 8 planes (compensated state, a step): 99 x 128 x 75 43 -> 30 us,
-// 200 x 147 x 131 93 -> 83, 200^3 172 -> 142, 16^3 15 -> 8.
+// Chunks: the least time of the busiest SM.  n items over its CTA slots are
+// q full rounds and a rest of k items an SM.  A full round costs as many items'
+// time as the SM has slots.  The rest costs what kRest says: less than a full
+// round, but more than in proportion, as fewer CTAs hide less of each other's
+// waits; after two full rounds the CTAs are out of step and most of a single
+// item is hidden.  An item costs a plane besides its own (the z face and the
+// two planes below it), and 2 % more per 64 planes beyond 64: neighbouring CTAs
+// drift apart and lose the halos they share in L2.  Fitted to 10 to 30 counts
+// of chunks on each of 43 grids of 38^3 to 512^3 and three states, where it is
+// on average 1.6 % (plain and compensated) and 3.4 % (double-float) above the
+// best count; the items of the busiest SM alone, each as dear, gave 4.9 and
+// 6.9 %.  Plain state: 224^3 186 -> 169 us a step, 320^3 508 -> 470,
+// 1024 x 32^2 25.7 -> 24.5.
 struct ColPlan {
     int width, chunks;
 };
@@ -809,19 +813,23 @@ ColPlan choose_columns(int ix, int iy, int iz, int sms, int per_sm)
             tiles = n;
         }
     }
+    // time of a rest of k items an SM after 0, 1 and more full rounds, in 0.01 items
+    constexpr int kRest2[3][3] = {{0, 110, 200}, {0, 120, 200}, {0, 90, 200}};
+    constexpr int kRest3[3][4] = {{0, 130, 215, 300}, {0, 150, 250, 300}, {0, 90, 220, 300}};
     long long const slots = static_cast<long long>(sms) * per_sm;
-    long long planes = tiles * iz / (3 * slots);
-    planes = planes < 8 ? 8 : (planes > 64 ? 64 : planes);
-    int const aim = static_cast<int>((iz + planes - 1) / planes);
-    long long lo = aim * 2 / 3 > 0 ? aim * 2 / 3 : 1;
-    long long hi = aim * 3 / 2 > sms / tiles ? aim * 3 / 2 : sms / tiles;
-    hi = hi < iz ? (hi > lo ? hi : lo) : iz;
-    long long fewest = 0x7fffffffffffffffLL;
-    for (long long c = lo; c <= hi; ++c) {
-        long long const cost = (tiles * c + sms - 1) / sms * (2 * ((iz + c - 1) / c) + 3);
-        if (cost < fewest) {
-            fewest = cost;
-            best.chunks = static_cast<int>(c);
+    long long least_time = 0x7fffffffffffffffLL;
+    for (int planes = iz < 128 ? iz : 128; planes >= 1; --planes) {
+        int const c = (iz + planes - 1) / planes;
+        long long const q = tiles * c / slots;
+        int const k = static_cast<int>((tiles * c - q * slots + sms - 1) / sms);
+        int const after = q < 2 ? static_cast<int>(q) : 2;
+        int const rest = per_sm == 2 ? kRest2[after][k] : (per_sm == 3 ? kRest3[after][k] : 100 * k);
+        int const longest = (iz + c - 1) / c;
+        long long const time =
+                (100 * per_sm * q + rest) * (longest + 1) * (3200 + (longest > 64 ? longest - 64 : 0));
+        if (time < least_time) {
+            least_time = time;
+            best.chunks = c;
         }
     }
     return best;
