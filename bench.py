@@ -16,8 +16,9 @@ Reported:
   roofline   the fused kernel against the FP64 pipe: algorithmic FLOPs per
              interior cell x cells / CUDA-event kernel time, over the FP64
              unit's nominal rate and the FMA rate measured in the same run
-             (part of the kernel's products run on the integer pipes, so the
-             fractions exceed one)
+             (part of the kernel's products run on the integer pipes, so these
+             fractions exceed one), and the FP64 pipe's own instructions over
+             its issue rate
   operators  each reference operator alone at 514^3 (prim_to_cons,
              cons_to_prim, time_step, godunov), CUDA-event timed
   cpu_baseline  the CPU oracle (C restatement of the reference operators,
@@ -63,6 +64,9 @@ FLOPS_PER_CELL_DEFAULT = None
 # cells: ten staged fields with their halos, tiles at different planes when they
 # read their neighbours'); traffic scales with cells.
 FLUX_F64_DRAM_BYTES_PER_CELL = 413.0
+# FP64-pipe thread instructions per interior cell of the same kernel, from the
+# same capture; the algorithm's other operations run on the integer pipes.
+FLUX_F64_PIPE_INSTRUCTIONS_PER_CELL = 69.8
 
 
 def parse():
@@ -347,8 +351,8 @@ def run_fp32c_leg(torch, E, args, stream, n0, dx, interior, steps_total, prim_re
                         "achieved": bytes_step / (flux_ms * 1e-3) / 1e9, "peak": hbm_peak,
                         "peak_source": "MEASURED_PEAKS.json (measured)" if hbm_peak else None,
                         "kernel_ms": flux_ms,
-                        "limiter": "instruction issue, not HBM: ncu shows the SM issuing on 67% of cycles at "
-                                   "409 thread-instructions per cell, DRAM at the algorithmic 40 B/cell "
+                        "limiter": "instruction issue, not HBM: ncu shows the SM issuing on 68% of cycles at "
+                                   "391 thread-instructions per cell, DRAM at the algorithmic 40 B/cell "
                                    "(ncu at 256^3)"}}
     if hbm_peak:
         out["roofline"]["frac"] = out["roofline"]["achieved"] / hbm_peak
@@ -777,7 +781,14 @@ def run_ours(args):
             "traffic_note": "dram bytes read+write per launch: 413 B per interior cell from an ncu capture at "
                             "256^3, scaled by cells",
             "note": "products, reciprocals and square roots run on the integer pipes, so the algorithm's "
-                    "operations exceed what the FP64 unit alone could do"}
+                    "operations exceed what the FP64 unit alone could do: frac is no fraction of a ceiling, "
+                    "fp64_pipe is"}
+    # what the FP64 pipe itself does: its instructions against its issue rate
+    issued = FLUX_F64_PIPE_INSTRUCTIONS_PER_CELL * interior / (flux_ms * 1e-3)
+    roof["fp64_pipe"] = {"instructions_per_cell": FLUX_F64_PIPE_INSTRUCTIONS_PER_CELL,
+                         "instructions_note": "thread instructions per interior cell, from an ncu capture at 256^3",
+                         "achieved_ginstr_s": issued / 1e9, "peak_ginstr_s": nominal / 2 / 1e9,
+                         "frac": issued / (nominal / 2), "frac_of_probe": issued / (peak / 2)}
     if fpc:
         fl = fpc["fused_step_fp64"] * interior
         roof["achieved"] = fl / (flux_ms * 1e-3) / 1e12

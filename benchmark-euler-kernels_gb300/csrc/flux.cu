@@ -907,7 +907,11 @@ constexpr int kStepTX = 16, kStepTY = 16;
 // adds a wait that its neighbours do not cover (its barriers and its last,
 // partly filled pass of faces).  c and z count FP64 warp instructions, each
 // holding its SM for 9.0 ns; the wait measured
-// 1.1 us a plane with two CTAs on the SM and 1.6 us with one.  Whole
+// 1.1 us a plane with two CTAs on the SM and 1.6 us with one.  Both were
+// measured on the kernel with two CTAs and all its work on the FP64 pipe; for
+// today's, with three and half of its arithmetic on the integer pipes, they
+// rank the tiles but do not give the time (512^3: 25.6 ms for 19.2, 64^3: 60
+// us for 58), and count whole tiles too dear against small ones.  Whole
 // 16 x 16 tiles are the best for large grids, smaller ones where their number
 // leaves SMs idle.  Against whole 16 x 16 tiles in chunks of at least 8
 // planes, all work on the FP64 pipe: 16^3 97 -> 12.5 us a step, 48^3 97 -> 46,

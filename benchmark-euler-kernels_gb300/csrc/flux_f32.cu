@@ -11,7 +11,9 @@ namespace {
 // ------------------------------------------------- FP32 step, column engine
 // The fused step of the FP32 states (cons only in HBM) with a regular
 // face-per-thread mapping.  Thread (ti, tj) of a 256-column CTA (32 x 8,
-// 16 x 16 or 8 x 32) owns the column (i0 + ti, j0 + tj) and marches it up z,
+// 16 x 16 or 8 x 32; in a batch 128 columns of 16 x 8 too: tiny and narrow
+// grids leave fewer of its threads idle, and a double-float state has four CTAs
+// on an SM instead of two) owns the column (i0 + ti, j0 + tj) and marches it up z,
 // keeping its cell's primitive state of planes k and k+1 in registers.  Per
 // plane it solves
 //   x: the face on its cell's left  (the right one is lane+1's, by shuffle;
@@ -33,7 +35,7 @@ namespace {
 // of three planes for the update, which in registers cost spills.
 //
 // It is bound by instruction issue.  Measured (one step): compensated state
-// 70 Gcell/s at 512^3 and 67 at 256^3, plain 74 and 72, double-float 37 (27
+// 70 Gcell/s at 512^3 and 67 at 256^3, plain 73 and 72, double-float 37 (27
 // on the shared-memory tile engine it had before), operator 72 (40 before).
 //
 // The state is plain FP32 (kCompNone), compensated (kCompSum), or

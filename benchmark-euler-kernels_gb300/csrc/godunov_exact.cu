@@ -369,7 +369,8 @@ cudaError_t launch_godunov_exact(CBundle<T> prim, Bundle<T> cons, Geom g, T gamm
     if (e != cudaSuccess) {
         return e;
     }
-    // FP64 instructions: about 62 a face, 50 a cell's update, 27 a staged cell
+    // FP64 instructions: about 62 a face, 50 a cell's update, 27 a staged cell,
+    // as before its products moved to the integer pipes (134 a cell are left)
     TilePlan plan = choose_tiles(g.n0 - 2, g.n1 - 2, g.n2 - 2, sms, per_sm, 62, 50, 27, 1);
     int const fewest = (g.n1 - 2 + kExTY<T> - 1) / kExTY<T>;
     plan.ny = plan.ny < fewest ? fewest : plan.ny;

@@ -62,7 +62,9 @@ TilePlan choose_tiles(int ix, int iy, int iz, int sms, int per_sm, int face, int
 
 // Opts Kernel into `bytes` of dynamic shared memory and returns its resident
 // CTAs per SM for blocks of `threads`, once per device: asked on every call
-// it cost a small operator 3 us.  Not during stream capture's first call.
+// it cost a small operator 3 us.  (The runtime keeps the opt-in per kernel and
+// device, not per context: launches in a second driver-API context, and after
+// the primary one was reset, have it too.)
 template <auto Kernel>
 cudaError_t resident_ctas(int threads, int bytes, int* per_sm)
 {

@@ -212,9 +212,9 @@ __global__ void __launch_bounds__(256) invdt_max_cons_kernel(CBundle<float> cons
 //    place, not copied first (10.9 GB of traffic less at 514^3);
 //  * cons = prim_to_cons(prim) when cons is set, bit-identical to
 //    prim_to_cons_kernel;
-//  * the stored sound speed in the form the fused step stores it
-//    (fast_sound_speed of (gamma/rho) p, faithful), so a loaded state and a
-//    stepped one carry the same kind of value, and e + p;
+//  * the stored sound speed as the fused step computes it, within two ulps (a
+//    reciprocal of rho and a square root; the step multiplies gamma and 1/rho
+//    first, this gamma and p, so the two may differ by an ulp), and e + p;
 //  * the EXACT max wavespeed of time_step.hpp:28-33 for the first dt, with
 //    the exact per-cell value evaluated only where WaveScreen says it can be
 //    the max.
